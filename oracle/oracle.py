@@ -35,11 +35,11 @@ def _ptr(a):
 def reference_dir():
     """The reference checkout that oracle/Makefile compiles from (its REF,
     which $CS3D_REFERENCE overrides), or None where that directory does not
-    exist (the GPU machines carry no reference checkout)."""
+    exist or holds no sources (the GPU machines carry no reference checkout)."""
     import subprocess
     out = subprocess.run(["make", "-s", "-C", HERE, "print-ref"], capture_output=True, text=True)
     d = out.stdout.strip()
-    return d if out.returncode == 0 and d and os.path.isdir(d) else None
+    return d if out.returncode == 0 and d and os.path.isfile(os.path.join(d, "CSolver_AWS.cpp")) else None
 
 
 def build(ref=False, quiet=True):
