@@ -283,6 +283,78 @@ int upload_op(const HostOp &h, DevOp<T> &d, cudaStream_t s) {
     return CS3D_OK;
 }
 
+// How a periodic line of N points is cut for the segmented FP32 solves
+// (cs3d_seg.cuh): the fewest register rows SEG * G that hold it with segments
+// at most kSegSlack rows shorter than SEG; SEG = 0 where none does (N below 17 or
+// above 512) or the line is not periodic.  pair: elements are float2 (the
+// sweeps' tiles), else floats.
+SegPlan seg_plan(int N, int periodic, bool pair) {
+    SegPlan best{};
+    if (!periodic) return best;
+    for (int G = 2; G <= 16; G *= 2)
+        for (int SEG = 16; SEG <= 32; SEG += 8) {
+            const int S = (N + G - 1) / G;
+            if (S > SEG || S <= SEG - 8 || (best.SEG && SEG * G >= best.SEG * best.G)) continue;
+            SegPlan p{};
+            p.SEG = SEG;
+            p.G = G;
+            p.S = S;
+            p.nS = N - G * (S - 1);
+            p.full = SEG == 32 && N == SEG * G;
+            p.lgLW = 5;
+            while ((1 << p.lgLW) * G > 32) --p.lgLW;
+            // segments of one line on distinct banks: 32-bank rows of 16 pairs
+            // or 32 floats; a full segment's rows are a multiple of that
+            const int lw = 1 << p.lgLW, row = pair ? 16 : 32;
+            p.pad = p.full && lw < row ? lw : 0;
+            p.kS = SEG - S;
+            p.pair = pair;
+            best = p;
+        }
+    return best;
+}
+
+// The line split over a cluster of C blocks, two segments of at most 32 rows
+// each a block.  22 rows at least: a segment's carry then reaches no further
+// than the next one (0.382^22 = 6e-10; the second derivative's 0.188 falls
+// faster).  C = 0 where no C <= 8 gives that.
+SegPlan cluster_plan(int N, int periodic) {
+    SegPlan p{};
+    const int C = (N + 63) / 64;
+    if (!periodic || C > 8 || N < 44 * C) return p;
+    p.SEG = 32;
+    p.C = C;
+    p.G = 2 * C;
+    p.S = (N + p.G - 1) / p.G;
+    p.nS = N - p.G * (p.S - 1);
+    p.full = N == 64 * C;
+    p.lgLW = 4;
+    p.kS = 32 - p.S;
+    p.pair = 1;
+    return p;
+}
+
+// The periodic operator in that form: left-hand side (a, 1, a) with
+// a = l / (1 + l^2).
+SegOp seg_op(const HostOp &h, const SegPlan &p) {
+    SegOp o{};
+    if (!p.SEG) return o;
+    const double a = h.alo[h.N / 2];
+    const double l = a == 0.0 ? 0.0 : (1.0 - std::sqrt(1.0 - 4.0 * a * a)) / (2.0 * a);
+    o.nl = (float)-l;
+    for (int k = 0; k <= kMaxH; k++) o.s[k] = (float)(h.taps[kMaxH + k] * h.scale * (1.0 + l * l));
+    for (int k = 0; k < 32; k++) o.pw[k] = (float)std::pow(-l, k + 1);
+    o.qS = (float)std::pow(-l, p.S);
+    o.qS1 = (float)std::pow(-l, p.S - 1);
+    o.iS = (float)std::pow(-l, -p.kS);
+    o.iS1 = (float)std::pow(-l, -(p.kS + 1));
+    const int smin = p.nS < p.G ? p.S - 1 : p.S;
+    o.T = 1;
+    while (o.T < p.G && std::pow(std::fabs(l), (double)smin * o.T) > 9e-10) o.T++;
+    o.wrap = o.T == p.G ? (float)(1.0 / (1.0 - std::pow(-l, h.N))) : 1.0f;
+    return o;
+}
+
 struct DeviceGuard {
     int prev = -1;
     explicit DeviceGuard(int dev) {
@@ -338,8 +410,13 @@ struct cs3d_handle {
     DevOp<double> op64[3][3];
     DevOp<float> op32[3][3];
     DevOp<float> op32fc[3];  // FP32 filter correction F - I (mixed form)
+    SegPlan seg[3] = {};     // mixed form: the periodic directions' segmented solves
+    SegOp segop[3][2] = {};  // 1st and 2nd derivative
+    SegPlan segf[3] = {};    // the filter's, and its correction operator
+    SegOp segfop[3] = {};
     // tiles
     int L[3] = {1, 1, 1}, Lf[3] = {1, 1, 1}, threads[3] = {128, 128, 128};
+    int Lt[3] = {1, 1, 1}, threads_t[3] = {128, 128, 128};  // the transposed sweeps of the mixed adjoint
     // step state
     int timeStep = 0, filterTimeStep = 0;
     int ic_done = 0;
@@ -505,11 +582,12 @@ static int check_config(const cs3d_config *c) {
 // global access is then a full 32-byte sector, which measured faster than
 // narrower tiles with more blocks per SM.
 // sweep: the sweeps' tile layout (pair-interleaved in FP32), else planar.
-static int pick_L(size_t tb, int nbuf, int N, int pitch_plus, int budget_kb = 72, bool sweep = false) {
+static int pick_L(size_t tb, int nbuf, int N, int pitch_plus, int budget_kb = 72, bool sweep = false,
+                  const SegPlan *seg = nullptr) {
     const size_t budget = (size_t)budget_kb * 1024;
     int L = 32;
     auto bytes = [&](int l) {
-        return sweep ? sweep_smem_bytes((int)tb, nbuf, l, l + pitch_plus, N)
+        return sweep ? sweep_smem_bytes((int)tb, nbuf, l, l + pitch_plus, N, seg)
                      : planar_smem_bytes((int)tb, nbuf, l, l + pitch_plus, N);
     };
     while (L > 1 && bytes(L) > budget) L /= 2;
@@ -639,6 +717,15 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
             if (!r) r = upload_op<float>(ho, h->op32[d][k - 1], h->stream);
             if (!r && k == 3) r = upload_op<float>(make_filter_correction(ho), h->op32fc[d], h->stream);
             if (r) return fail_free(r);
+            if (h->mixed && k < 3) {
+                h->seg[d] = d > 0 ? cluster_plan(Nd[d], ho.periodic) : SegPlan{};
+                if (!h->seg[d].C) h->seg[d] = seg_plan(Nd[d], ho.periodic, d > 0);
+                h->segop[d][k - 1] = seg_op(ho, h->seg[d]);
+            } else if (h->mixed && std::fabs(cfg->alphaF) < 0.4999) {
+                // (|alphaF| = 1/2 has no factorisation with l < 1)
+                h->segf[d] = seg_plan(Nd[d], ho.periodic, false);
+                h->segfop[d] = seg_op(make_filter_correction(ho), h->segf[d]);
+            }
         }
     for (int d = 0; d < 3; d++) {
         // Tile shape.  Default: the widest tile within 75 kB for the mixed
@@ -650,16 +737,24 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
         // the 72 kB tile is already 16 lines wide (N = 42) one block per SM was
         // slower, its phases no longer overlapping another block's.
         const int nb = sweep_nbuf(d, (int)h->tb);
-        h->L[d] = pick_L(h->tb, nb, Nd[d], x_pitch_plus(h, d), d == 0 ? (h->mixed ? 75 : 115) : 72, true);
-        // FP64 x: at most 4 lines within 115 kB (2 blocks per SM at N = 256,
-        // 3 at 128, registers).  Against the former 75 kB tiles with a pad
-        // column (1 line at N = 256): HIT 256^3 x 51.7 -> 26.3 ms per step,
-        // shear layer 3.25 -> 1.84; 8 lines at 128^3 measured 4% slower.
-        if (!h->mixed && d == 0 && h->L[d] > 4) h->L[d] = 4;
-        h->threads[d] = h->mixed ? (d == 0 ? sweep_threads<float>(0) : 256) : sweep_threads<double>(d);
-        if (h->mixed && d > 0 && h->L[d] < 16) {
-            h->L[d] = pick_L(h->tb, nb, Nd[d], 0, 200, true);
-            h->threads[d] = sweep_threads<float>(d);
+        auto shape = [&](const SegPlan *seg, int &L, int &threads) {
+            L = pick_L(h->tb, nb, Nd[d], x_pitch_plus(h, d), d == 0 ? (h->mixed ? 75 : 115) : 72, true, seg);
+            // FP64 x: at most 4 lines within 115 kB (2 blocks per SM at N = 256,
+            // 3 at 128, registers).  Against the former 75 kB tiles with a pad
+            // column (1 line at N = 256): HIT 256^3 x 51.7 -> 26.3 ms per step,
+            // shear layer 3.25 -> 1.84; 8 lines at 128^3 measured 4% slower.
+            if (!h->mixed && d == 0 && L > 4) L = 4;
+            threads = h->mixed ? (d == 0 ? sweep_threads<float>(0) : 256) : sweep_threads<double>(d);
+            if (h->mixed && d > 0 && L < 16) {
+                L = pick_L(h->tb, nb, Nd[d], 0, 200, true, seg);
+                threads = sweep_threads<float>(d);
+            }
+        };
+        shape(nullptr, h->Lt[d], h->threads_t[d]);
+        shape(&h->seg[d], h->L[d], h->threads[d]);
+        if (h->seg[d].C) {
+            h->L[d] = kClusterLines;
+            h->threads[d] = kTpbYZ;
         }
         h->Lf[d] = pick_L(h->tb, h->mixed ? 10 : 5, Nd[d], d == 0 ? 1 : 0);
         // a mixed filter tile narrower than 8 lines within 72 kB (N = 256: 4
@@ -667,6 +762,13 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
         // blocks per SM): HIT 256^3 filter 2.27 -> 1.81 ms per step; at
         // N = 128 the 8-line tile stays (16 lines measured slower)
         if (h->mixed && h->Lf[d] < 8) h->Lf[d] = pick_L(h->tb, 10, Nd[d], d == 0 ? 1 : 0, 110);
+        if (h->segf[d].SEG) {
+            // 32 lines a tile, 128-byte rows, where a block of them fits; half
+            // of that along x, whose lines are contiguous
+            int L = d == 0 ? 16 : 32;
+            while (L > 1 && filter_seg_smem(L, L + (d == 0), Nd[d], h->segf[d]) > 200 * 1024) L /= 2;
+            h->Lf[d] = L;
+        }
         if (sweep_smem_bytes((int)h->tb, nb, 1, 2, Nd[d]) > 200 * 1024)
             return fail_free(fail(CS3D_ERR_SHAPE, "N[%d]=%d: a line does not fit in shared memory", d, Nd[d]));
     }
@@ -914,6 +1016,9 @@ static int run_stage(cs3d_handle *h, int st, int last) {
         a.lgL = ilog2(a.L);
         a.divN = make_fastdiv((unsigned)(d == 0 ? h->g.Nx : d == 1 ? h->g.Ny : h->g.Nz));
         a.P = a.L + x_pitch_plus(h, d);
+        a.seg = h->seg[d];
+        a.g1 = h->segop[d][0];
+        a.g2 = h->segop[d][1];
         if (sizeof(T) == 8) {
             a.d1 = *reinterpret_cast<const LineOp<T> *>(&h->op64[d][0].op);
             a.d2 = *reinterpret_cast<const LineOp<T> *>(&h->op64[d][1].op);
@@ -942,7 +1047,9 @@ static int run_stage(cs3d_handle *h, int st, int last) {
                 fa.lgL = ilog2(h->Lf[d]);
                 fa.divN = make_fastdiv((unsigned)(d == 0 ? h->g.Nx : d == 1 ? h->g.Ny : h->g.Nz));
                 fa.P = h->Lf[d] + (d == 0 ? 1 : 0);
-                fa.threads = sizeof(T) == 4 ? filter_threads<float>() : filter_threads<double>();
+                fa.seg = h->segf[d];
+                fa.sg = h->segfop[d];
+                fa.threads = fa.seg.SEG ? kFilterSegTpb : sizeof(T) == 4 ? filter_threads<float>() : filter_threads<double>();
                 if (sizeof(T) == 8) fa.op = *reinterpret_cast<const LineOp<T> *>(&h->op64[d][2].op);
                 else fa.op = *reinterpret_cast<const LineOp<T> *>(&h->op32fc[d].op);
                 void **src = pass == 1 ? h->ft1 : h->ft2;
@@ -1768,10 +1875,10 @@ static int adj_vjp_tape(cs3d_handle *h, const T *const qin[5], void *const Gv[48
         for (int d = 2; d >= 0; d--) {
             TSweepArgs ta{};
             ta.g = h->g;
-            ta.L = h->L[d];
-            ta.lgL = ilog2(h->L[d]);
-            ta.P = h->L[d] + (d == 0 ? 1 : 0);
-            ta.threads = h->threads[d];
+            ta.L = h->Lt[d];
+            ta.lgL = ilog2(h->Lt[d]);
+            ta.P = h->Lt[d] + (d == 0 ? 1 : 0);
+            ta.threads = h->threads_t[d];
             ta.divN = make_fastdiv((unsigned)(d == 0 ? h->g.Nx : d == 1 ? h->g.Ny : h->g.Nz));
             ta.d1 = h->op32[d][0].op;
             ta.d2 = h->op32[d][1].op;

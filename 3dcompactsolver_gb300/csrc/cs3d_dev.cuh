@@ -47,6 +47,31 @@ struct LineOp {
     int periodic;
 };
 
+// How a periodic line is cut into register segments (cs3d_seg.cuh): G
+// segments (a power of two, one lane each), the first nS of S rows and the
+// others of S - 1, walked by a kernel compiled for SEG rows a segment.
+struct SegPlan {
+    int SEG;   // 0: not cut (the Thomas solves run instead)
+    int full;  // every segment has SEG rows
+    int S, nS, G;
+    int lgLW;  // log2 of the lines a warp holds: 32 / G
+    int pad;   // full only: shared-memory elements between a line's segments
+    int kS;    // SEG - S
+    int pair;  // array elements are float2 (y and z sweeps), else float
+    int C;     // > 0: a cluster of C blocks holds the line, two segments each
+               // (G = 2 C, not restricted to a power of two)
+};
+
+// A periodic operator in that form: -l, the scaled taps (centre outwards),
+// the powers (-l)^(k+1), and what weights the carries between segments.
+struct SegOp {
+    float nl, s[kMaxH + 1], pw[32];
+    float qS, qS1;  // (-l)^S, (-l)^(S-1)
+    float iS, iS1;  // (-l)^-kS, (-l)^-(kS+1)
+    float wrap;     // 1, or 1 / (1 - (-l)^N) where T = G
+    int T;
+};
+
 // Loads of operator coefficients (a few kB per operator, read by every line
 // solve) through the read-only data path.
 __device__ __forceinline__ float ldc(const float *p) { return __ldg(p); }
@@ -142,26 +167,28 @@ __device__ __forceinline__ int faces_of(const Geom &g, int i, int j, int k) {
     return f;
 }
 
-// T^0.76, the exponent of the viscosity law mu = mu_ref T^0.76 (IdealGas.hpp).
-// FP32: exp2(0.76 log2 T) with the hardware log2 (absolute error about 2^-22,
-// so about 1.5e-7 relative in the result: an FP32 rounding).  FP64, whose pipe issues two operations per SM and
-// clock: y^25 = T^19 solved by one step of Halley's method (cubic
-// convergence) from an FP32 estimate exp2(0.76 log2 T) (relative error below
-// 2e-6), written as the correction y + y (c - a) / (13 a + 12 c) with
-// a = y^25, c = T^19 by repeated squaring: about 20 FP64 operations and one
-// division, within 2 ulp of the library pow on [1e-6, 1e6] (sampled against
-// it: the cubic step leaves the estimate's error at ~1e-17).  Outside that
-// range, and for NaN, the library pow.
-__device__ __forceinline__ float visc_pow(float T) { return exp2f(0.76f * __log2f(T)); }
-__device__ __forceinline__ double visc_pow(double T) {
-    if (!(T > 1e-6 && T < 1e6)) return pow(T, 0.76);
-    const double y = (double)exp2f(0.76f * log2f((float)T));
-    const double t2 = T * T, t4 = t2 * t2, t8 = t4 * t4, t16 = t8 * t8;
-    const double c = t16 * t2 * T;
+// T^-0.24, from which both the viscosity law mu = mu_ref T^0.76 (IdealGas.hpp)
+// and its slope 0.76 mu / T follow by multiplications.
+// FP32: exp2(-0.24 log2 T) with the hardware log2 (absolute error about 2^-22,
+// so about 4e-8 relative in the result).  FP64, whose pipe issues two
+// operations per SM and clock: y = T^-0.24 solves T^6 y^25 = 1; from an FP32
+// estimate (relative error below 6e-7) the residual e = 1 - T^6 y^25 gives
+// y (1 - e)^(-1/25) = y (1 + e/25 + 13 e^2/625 + ...), the next term below
+// 5e-17: 14 FP64 operations and no division, within 1 ulp of the library pow
+// on [1e-6, 1e6].  Outside that range, and for NaN, the library pow.
+__device__ __forceinline__ float visc_rpow(float T) { return exp2f(-0.24f * __log2f(T)); }
+__device__ __forceinline__ double visc_rpow(double T) {
+    if (!(T > 1e-6 && T < 1e6)) return pow(T, -0.24);
+    const double y = (double)exp2f(-0.24f * log2f((float)T));
+    const double t2 = T * T, t6 = t2 * t2 * t2;
     const double y2 = y * y, y4 = y2 * y2, y8 = y4 * y4, y16 = y8 * y8;
-    const double a = y16 * y8 * y;
-    return y + y * ((c - a) / (13.0 * a + 12.0 * c));
+    const double e = fma(-t6, y16 * y8 * y, 1.0);
+    return fma(y, e * fma(e, 13.0 / 625.0, 1.0 / 25.0), y);
 }
+
+// T^0.76
+template <typename T>
+__device__ __forceinline__ T visc_pow(T t) { return t * visc_rpow(t); }
 
 // Direction whose continuity derivative survives at a wall point: the
 // reference applies the wall faces in the order X0,X1,Y0,Y1,Z0,Z1 and the

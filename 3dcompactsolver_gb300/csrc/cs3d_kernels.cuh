@@ -6,6 +6,8 @@ namespace cs3d {
 
 constexpr int kTpbX = 256;   // threads per block of the mixed-form x sweep
 constexpr int kTpbYZ = 512;  // most threads per block of the mixed-form y and z sweeps
+constexpr int kFilterSegTpb = 320;  // threads per block of the segmented mixed filter
+constexpr int kClusterLines = 32;  // lines of a tile whose lines are split over a cluster
 constexpr int kFilterTpb = 256;  // threads per block of the mixed-form filter
 
 // Most threads per block the stage sweeps in work type T, direction dir, are
@@ -42,6 +44,8 @@ struct SweepArgs {
     int P;          // shared-memory pitch between positions of a line
     int threads;    // threads per block
     LineOp<T> d1, d2;
+    SegPlan seg;    // mixed form, periodic lines (seg.SEG > 0): the segmented
+    SegOp g1, g2;   // solves' plan and operators
     GasParams gas;
     const T *qs[5]; // stage input q* in the work precision (FP64 q* itself, or
                     // its FP32 shadow in the mixed form)
@@ -83,6 +87,8 @@ struct FilterArgs {
     int L, lgL, P, threads;
     FastDiv divN;
     LineOp<T> op;
+    SegPlan seg;       // mixed form, periodic lines: the segmented solves' plan
+    SegOp sg;          // and operator (SEG = 0: op's Thomas factors)
     Q5 src64;          // FP64 source (or null pointers)
     T *src32[5];       // work-precision source
     Q5 dst64;          // FP64 destination (or null pointers)
@@ -357,8 +363,9 @@ cudaError_t launch_ke_seed(const KeSeedArgs &a, cudaStream_t s);
 
 // shared memory of a sweep tile (pair-interleaved for prec_bytes 4) and of
 // a planar tile (filter, single operators, adjoint operators)
-size_t sweep_smem_bytes(int prec_bytes, int nbuf, int L, int P, int N);
+size_t sweep_smem_bytes(int prec_bytes, int nbuf, int L, int P, int N, const SegPlan *seg = nullptr);
 size_t planar_smem_bytes(int prec_bytes, int nbuf, int L, int P, int N);
+size_t filter_seg_smem(int L, int P, int N, const SegPlan &p);
 int sweep_nbuf(int dir, int prec_bytes);
 int sweep_ntask(int dir);
 int filter_ntask();

@@ -1,0 +1,354 @@
+// cs3d_seg.cuh -- compact line solves of periodic lines in register segments
+// (FP32), shared by the stage sweeps, the filter and the adjoint kernels.
+//
+// On a periodic line the compact operators' left-hand side is the circulant
+// tridiagonal (a, 1, a), which factors exactly into two first-order
+// recurrences with constant coefficients,
+//   (a, 1, a) = (1 + l E^-1)(1 + l E) / (1 + l^2),   a = l / (1 + l^2), |l| < 1
+// (E the shift by one row), so that with the right-hand side scaled by
+// (1 + l^2) -- folded into the taps --
+//   forward   y_n = r_n - l y_{n-1},     backward   x_n = y_n - l x_{n+1}
+// around the circle.  No row needs factors from memory, a division or a
+// Sherman-Morrison correction, and the recurrences are cut anywhere: a line is
+// split into G segments, one lane each, held in registers.  Each lane runs its
+// segment from a zero start; the value entering it is the ends of the segments
+// before it, weighted by powers of -l,
+//   Y_j = e_{j-1} + q_{j-1} (e_{j-2} + q_{j-2} (...)),   q = (-l)^length,
+// taken from the T nearest segments by shuffles (T: until the weight is below
+// 2^-30; the whole circle, with the geometric factor 1 / (1 - (-l)^N), where
+// that takes all of them), and is added to the first rows with the same
+// powers.  The backward pass mirrors it.
+//
+// What bounds it: the one-thread-per-line Thomas solve it replaces
+// (solve_lanes) was a chain of N rows, each with two shared-memory reads and
+// two writes and about 22 instructions, run by half of the block's warps; here
+// a row is read once and written once in about 11 instructions, the chain is a
+// segment, and a warp holds all segments of its lines (no block barrier inside
+// a solve).  The consume phases read solutions without a correction.  Against
+// solve_lanes, per step: 128^3 y 0.359 -> 0.283 ms, z 0.602 -> 0.527; 256^3 y
+// 2.92 -> 2.19 ms; the error against 64 bits falls by a tenth (differences
+// before products).
+#pragma once
+#include "cs3d_dev.cuh"
+
+namespace cs3d {
+
+// Rows at the start of a segment whose carry is added: (-l)^(k+1) falls below
+// 5e-9 after these many rows.  The first derivative has l = 0.382, the second
+// 0.188; the filter's l depends on its coefficient (all rows).
+constexpr int kSegRows1 = 20, kSegRows2 = 12, kSegRowsAll = 64;
+// Segments are at most kSegSlack rows shorter than the compiled length (seg_plan keeps
+// 8, cluster_plan 10).
+constexpr int kSegSlack = 10;
+
+// One lane's place in its line's segments, in elements of the array walked:
+// register row k is at row[k * P] (k >= k0), rows before the segment at
+// lo[k * P] (k < k0), rows after it at hi[h * P].
+template <typename E>
+struct SegLane {
+    int seg, k0;  // k0: unused leading rows of the register segment
+    E *row, *lo, *hi;
+};
+
+// First row of segment s.
+__device__ __forceinline__ int seg_row0(const SegPlan &pl, int s) { return s * pl.S - max(0, s - pl.nS); }
+
+// The lane of a line that lies whole in this block's tile (line at base, rows
+// P elements apart, pl.pad more after every full segment).
+template <int SEG, bool FULL, typename E>
+__device__ __forceinline__ SegLane<E> seg_lane(const SegPlan &pl, E *base, int seg, int N, int P) {
+    SegLane<E> s;
+    s.seg = seg;
+    if constexpr (FULL) {
+        s.k0 = 0;
+        s.row = base + seg * (SEG * P + pl.pad);
+        s.lo = seg > 0 ? s.row - pl.pad : base + N * P + (pl.G - 1) * pl.pad;
+        s.hi = seg < pl.G - 1 ? s.row + SEG * P + pl.pad : base;
+    } else {
+        const int n0 = seg_row0(pl, seg), len = pl.S - (seg >= pl.nS);
+        s.k0 = SEG - len;
+        s.row = base + (n0 - s.k0) * P;
+        s.lo = n0 > 0 ? s.row : s.row + N * P;
+        s.hi = seg < pl.G - 1 ? base + (n0 + len) * P : base;
+    }
+    return s;
+}
+
+// The window of a segment: register row k at w[k + H], H rows either side.
+// Rows before the segment's own (ragged segments) come from the halo or stay
+// zero; the callers zero their right-hand sides.
+template <int SEG, bool FULL, int H, typename W, typename E, typename LD>
+__device__ __forceinline__ void seg_load(W (&w)[SEG + 2 * H], const SegLane<E> &s, int P, LD &&ld) {
+#pragma unroll
+    for (int k = -H; k < SEG; ++k) {
+        if (FULL) {
+            w[k + H] = k < 0 ? ld(s.lo + k * P) : ld(s.row + k * P);
+        } else if (k < kSegSlack) {
+            w[k + H] = W{};
+            if (k >= s.k0 - H) w[k + H] = k < s.k0 ? ld(s.lo + k * P) : ld(s.row + k * P);
+        } else {
+            w[k + H] = ld(s.row + k * P);
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < H; ++h) w[SEG + H + h] = ld(s.hi + h * P);
+}
+
+// Right-hand sides from a window (taps scaled by 1/h, 1/h^2 and 1 + l^2): the
+// differences first, so that their products round relative to the differences.
+template <int SEG>
+__device__ __forceinline__ float seg_r1(const float (&w)[SEG + 4], const SegOp &o, int k) {
+    return fmaf(o.s[1], w[k + 3] - w[k + 1], o.s[2] * (w[k + 4] - w[k]));
+}
+template <int SEG>
+__device__ __forceinline__ float seg_r2(const float (&w)[SEG + 4], const SegOp &o, int k) {
+    return fmaf(o.s[1], (w[k + 3] - w[k + 2]) - (w[k + 2] - w[k + 1]),
+                o.s[2] * ((w[k + 4] - w[k + 2]) - (w[k + 2] - w[k])));
+}
+
+// y: right-hand sides (zero in rows before k0).  Forward from zero: the
+// segment's end value.
+template <int SEG>
+__device__ __forceinline__ float seg_fwd(float (&y)[SEG], const SegOp &o) {
+    float c = y[0];
+#pragma unroll
+    for (int k = 1; k < SEG; ++k) y[k] = c = fmaf(o.nl, c, y[k]);
+    return c;
+}
+// Add the value entering the segment (KU: rows that take it), then backward
+// from zero: the value at the segment's first row.
+template <int SEG, bool FULL, int KU>
+__device__ __forceinline__ float seg_bwd(float (&y)[SEG], const SegOp &o, const SegPlan &pl, int k0, float in) {
+    constexpr int KF = KU + (FULL ? 0 : kSegSlack) < SEG ? KU + (FULL ? 0 : kSegSlack) : SEG;
+    if constexpr (!FULL) in *= k0 == pl.kS ? o.iS : o.iS1;  // the powers count from row k0
+#pragma unroll
+    for (int k = 0; k < KF; ++k) y[k] = fmaf(o.pw[k], in, y[k]);
+    float c = y[SEG - 1], b = c;
+#pragma unroll
+    for (int k = SEG - 2; k >= 0; --k) {
+        y[k] = c = fmaf(o.nl, c, y[k]);
+        if (!FULL && k <= kSegSlack) b = k == k0 ? c : b;
+    }
+    return FULL ? c : b;
+}
+// Add the value at the next segment's first row.
+template <int SEG, int KU>
+__device__ __forceinline__ void seg_end(float (&y)[SEG], const SegOp &o, float in) {
+#pragma unroll
+    for (int k = 0; k < (KU < SEG ? KU : SEG); ++k) y[SEG - 1 - k] = fmaf(o.pw[k], in, y[SEG - 1 - k]);
+}
+
+// What enters this lane's segment: e of the DIR-side neighbours (DIR = -1:
+// segments before, +1: after), weighted.  lane0: the line's first lane.
+template <int DIR>
+__device__ __forceinline__ float seg_carry(float e, const SegOp &o, const SegPlan &pl, int seg, int lane0) {
+    float c = 0.f;
+    for (int t = o.T; t >= 1; --t) {
+        const int src = (seg + DIR * t) & (pl.G - 1);
+        const float es = __shfl_sync(0xffffffffu, e, lane0 + (src << pl.lgLW));
+        c = fmaf(src < pl.nS ? o.qS : o.qS1, c, es);
+    }
+    return c * o.wrap;
+}
+
+// The whole solve, all segments of the line in this warp.
+template <int SEG, bool FULL, int KU>
+__device__ __forceinline__ void seg_solve(float (&y)[SEG], const SegOp &o, const SegPlan &pl, int seg, int k0,
+                                          int lane0) {
+    const float e = seg_fwd<SEG>(y, o);
+    const float b = seg_bwd<SEG, FULL, KU>(y, o, pl, k0, seg_carry<-1>(e, o, pl, seg, lane0));
+    seg_end<SEG, KU>(y, o, seg_carry<1>(b, o, pl, seg, lane0));
+}
+
+// Store the segment's own rows.
+template <int SEG, bool FULL, typename E, typename ST>
+__device__ __forceinline__ void seg_store(const SegLane<E> &s, int P, ST &&st) {
+#pragma unroll
+    for (int k = 0; k < SEG; ++k)
+        if (FULL || k >= kSegSlack || k >= s.k0) st(s.row + k * P, k);
+}
+
+// The right-hand sides of two solves of the pair-interleaved tile (element n
+// of a pair: a float2).  MODE 0: lane x's field by the 1st (y1) and 2nd (y2)
+// derivative, 1: both lanes' fields by the 1st derivative, 2: lane x's field
+// alone by the 1st, 3: lane x's field by the 1st, lane y's by the 2nd.
+template <int SEG, bool FULL, int MODE>
+__device__ __forceinline__ void seg_pair_rhs(float (&y1)[SEG], float (&y2)[SEG], const SegLane<float2> &s, int P,
+                                             const SegOp &o1, const SegOp &o2) {
+    float w1[SEG + 4], w2[SEG + 4];
+    if constexpr (MODE == 0 || MODE == 2) {
+        seg_load<SEG, FULL, 2>(w1, s, P, [](const float2 *p) { return p->x; });
+    } else {
+        float2 w[SEG + 4];
+        seg_load<SEG, FULL, 2>(w, s, P, [](const float2 *p) { return *p; });
+#pragma unroll
+        for (int k = 0; k < SEG + 4; ++k) { w1[k] = w[k].x; w2[k] = w[k].y; }
+    }
+#pragma unroll
+    for (int k = 0; k < SEG; ++k) {
+        y1[k] = seg_r1<SEG>(w1, o1, k);
+        if constexpr (MODE == 0) y2[k] = seg_r2<SEG>(w1, o2, k);
+        if constexpr (MODE == 1) y2[k] = seg_r1<SEG>(w2, o1, k);
+        if constexpr (MODE == 3) y2[k] = seg_r2<SEG>(w2, o2, k);
+        if constexpr (MODE == 2) y2[k] = 0.f;
+        if (!FULL && k < kSegSlack && k < s.k0) y1[k] = y2[k] = 0.f;
+    }
+}
+
+// Two solves of the tile in place, all segments of their lines in this warp.
+template <int SEG, bool FULL, int MODE>
+__device__ __forceinline__ void seg_pair(const SegLane<float2> &s, int P, const SegOp &o1, const SegOp &o2,
+                                         const SegPlan &pl, int lane0, bool active) {
+    float y1[SEG], y2[SEG];
+    seg_pair_rhs<SEG, FULL, MODE>(y1, y2, s, P, o1, o2);
+    seg_solve<SEG, FULL, kSegRows1>(y1, o1, pl, s.seg, s.k0, lane0);
+    if constexpr (MODE == 0 || MODE == 3) seg_solve<SEG, FULL, kSegRows2>(y2, o2, pl, s.seg, s.k0, lane0);
+    if constexpr (MODE == 1) seg_solve<SEG, FULL, kSegRows1>(y2, o1, pl, s.seg, s.k0, lane0);
+    __syncwarp();  // every lane of the line has read its window
+    if (!active) return;
+    seg_store<SEG, FULL>(s, P, [&](float2 *p, int k) {
+        if constexpr (MODE == 2) p->x = y1[k];
+        else *p = make_float2(y1[k], y2[k]);
+    });
+}
+
+// One solve of a planar tile: the KIND-th derivative of the segment at `s`,
+// its rows stored to the same places `shift` elements on (0: in place).
+template <int SEG, bool FULL, int KIND>
+__device__ __forceinline__ void seg_one(const SegLane<float> &s, int P, const SegOp &o, const SegPlan &pl, int lane0,
+                                        bool active, int shift) {
+    float y[SEG];
+    {
+        float w[SEG + 4];
+        seg_load<SEG, FULL, 2>(w, s, P, [](const float *p) { return *p; });
+#pragma unroll
+        for (int k = 0; k < SEG; ++k) {
+            y[k] = KIND == 1 ? seg_r1<SEG>(w, o, k) : seg_r2<SEG>(w, o, k);
+            if (!FULL && k < kSegSlack && k < s.k0) y[k] = 0.f;
+        }
+    }
+    seg_solve<SEG, FULL, KIND == 1 ? kSegRows1 : kSegRows2>(y, o, pl, s.seg, s.k0, lane0);
+    __syncwarp();  // every lane of the line has read its window
+    if (active) seg_store<SEG, FULL>(s, P, [&](float *p, int k) { p[shift] = y[k]; });
+    __syncwarp();
+}
+
+// The filter's correction (F - I) v of the segment at `s` (nine symmetric
+// taps), added to v in place.
+template <int SEG, bool FULL>
+__device__ __forceinline__ void seg_filter(const SegLane<float> &s, int P, const SegOp &o, const SegPlan &pl,
+                                           int lane0, bool active) {
+    float y[SEG];
+    {
+        float w[SEG + 8];
+        seg_load<SEG, FULL, 4>(w, s, P, [](const float *p) { return *p; });
+#pragma unroll
+        for (int k = 0; k < SEG; ++k) {
+            float r = o.s[0] * w[k + 4];
+#pragma unroll
+            for (int h = 1; h <= 4; ++h) r = fmaf(o.s[h], w[k + 4 - h] + w[k + 4 + h], r);
+            if (!FULL && k < kSegSlack && k < s.k0) r = 0.f;
+            y[k] = r;
+        }
+    }
+    seg_solve<SEG, FULL, kSegRowsAll>(y, o, pl, s.seg, s.k0, lane0);
+    __syncwarp();  // every lane of the line has read its window
+    if (active) seg_store<SEG, FULL>(s, P, [&](float *p, int k) { *p += y[k]; });
+}
+
+// ---------------------------------------------------------------------
+// lines split over a thread-block cluster
+// ---------------------------------------------------------------------
+// A tile of 32 neighbouring lines is 128 bytes a row, whole memory lines; 16
+// solves of 32 lines fit one SM's shared memory for 64 rows only, so a cluster
+// of C blocks holds the line, two segments (kClRows rows at most) a block.  Halo
+// rows are read from the neighbours' shared memory; the carries (T = 1: the
+// plan keeps segments long enough for the nearest neighbour alone) go through
+// a mailbox forward, and backward through the row that the receiving lane
+// itself overwrites next.  A warp holds 16 lines' two segments.
+// Why: beyond the L2 the memory system delivers in proportion to the bytes a
+// tile's row takes of its 128-byte line -- a copy kernel of z tiles on 256^3
+// measured 2.0 / 3.9 / 6.5 TB/s at 8 / 16 / 32 FP32 lines a row (5.2 / 5.6 /
+// 5.3 TB/s at 128^3, which the L2 holds).  The 8-line tiles that whole lines
+// leave room for at N = 256: z 6.66 ms a step; clusters of 4: 4.03.
+constexpr int kClRows = 64, kClLines = 32, kClWarps = 16;  // (kClLines: kClusterLines)
+
+__device__ __forceinline__ void cluster_sync() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The address of p (this block's shared memory) in block `rank` of the cluster.
+template <typename E>
+__device__ __forceinline__ E *cluster_map(E *p, int rank) {
+    E *r;
+    asm("mapa.u64 %0, %1, %2;" : "=l"(r) : "l"(p), "r"(rank));
+    return r;
+}
+
+// The solves of a sweep tile (tasks as run_seg_tasks), one unit a warp: task
+// warp / 2, lines 16 (warp & 1) + lane.  mail: 2 * 8 * kClLines floats.  Every
+// thread of every block of the cluster calls it.
+template <bool FULL, int NT, bool SINGLE>
+__device__ __forceinline__ void run_cluster_tasks(float2 *tile, int pstride2, float2 *mail, const SegPlan &pl,
+                                                  const SegOp &o1, const SegOp &o2, int rank, int tid) {
+    constexpr int SEG = 32, P = kClLines;
+    const int warp = tid >> 5, t = warp >> 1, half = (tid >> 4) & 1;
+    const int l = ((warp & 1) << 4) | (tid & 15);
+    const int C = pl.C, prev = rank > 0 ? rank - 1 : C - 1, next = rank < C - 1 ? rank + 1 : 0;
+    const int seg = 2 * rank + half;
+    float2 *line = tile + t * pstride2 + l;
+    SegLane<float2> s;
+    s.seg = seg;
+    const int n0 = seg_row0(pl, seg) - seg_row0(pl, 2 * rank), len = pl.S - (seg >= pl.nS);
+    s.k0 = FULL ? 0 : SEG - len;
+    s.row = line + (n0 - s.k0) * P;
+    // (rows of the previous block: its last row precedes this block's first)
+    const int nprev = FULL ? kClRows : seg_row0(pl, 2 * prev + 2) - seg_row0(pl, 2 * prev);
+    s.lo = half ? cluster_map(s.row, rank) : cluster_map(line + (nprev - s.k0) * P, prev);
+    s.hi = half ? cluster_map(line, next) : cluster_map(line + (n0 + len) * P, rank);
+    const bool dd = t < 4, single = SINGLE && t == NT - 1;
+    float y1[SEG], y2[SEG];
+    float2 e;
+    if (dd) {
+        seg_pair_rhs<SEG, FULL, 0>(y1, y2, s, P, o1, o2);
+        e = make_float2(seg_fwd<SEG>(y1, o1), seg_fwd<SEG>(y2, o2));
+    } else if (single) {
+        seg_pair_rhs<SEG, FULL, 2>(y1, y2, s, P, o1, o2);
+        e = make_float2(seg_fwd<SEG>(y1, o1), 0.f);
+    } else {
+        seg_pair_rhs<SEG, FULL, 1>(y1, y2, s, P, o1, o2);
+        e = make_float2(seg_fwd<SEG>(y1, o1), seg_fwd<SEG>(y2, o1));
+    }
+    float2 in;
+    in.x = __shfl_sync(0xffffffffu, e.x, tid & 15);
+    in.y = __shfl_sync(0xffffffffu, e.y, tid & 15);
+    float2 *box = mail + t * kClLines + l;
+    if (half) *cluster_map(box, next) = e;
+    cluster_sync();  // the forward carries are there, and every window has been read
+    if (!half) in = *box;
+    if (dd) {
+        e = make_float2(seg_bwd<SEG, FULL, kSegRows1>(y1, o1, pl, s.k0, in.x),
+                        seg_bwd<SEG, FULL, kSegRows2>(y2, o2, pl, s.k0, in.y));
+    } else if (single) {
+        e.x = seg_bwd<SEG, FULL, kSegRows1>(y1, o1, pl, s.k0, in.x);
+    } else {
+        e = make_float2(seg_bwd<SEG, FULL, kSegRows1>(y1, o1, pl, s.k0, in.x),
+                        seg_bwd<SEG, FULL, kSegRows1>(y2, o1, pl, s.k0, in.y));
+    }
+    in.x = __shfl_sync(0xffffffffu, e.x, (tid & 15) | 16);
+    in.y = __shfl_sync(0xffffffffu, e.y, (tid & 15) | 16);
+    // the previous block's last row of this line, stored next by its own lane
+    if (!half) *cluster_map(line + (nprev - 1) * P, prev) = e;
+    cluster_sync();  // (the last access to another block's shared memory)
+    if (half) in = s.row[(SEG - 1) * P];
+    if (dd) {
+        seg_end<SEG, kSegRows1>(y1, o1, in.x);
+        seg_end<SEG, kSegRows2>(y2, o2, in.y);
+    } else {
+        seg_end<SEG, kSegRows1>(y1, o1, in.x);
+        if (!single) seg_end<SEG, kSegRows1>(y2, o1, in.y);
+    }
+    seg_store<SEG, FULL>(s, P, [&](float2 *p, int k) { *p = make_float2(y1[k], y2[k]); });
+}
+
+}  // namespace cs3d

@@ -55,6 +55,91 @@ constexpr int kMinBlocksX = 3, kMinBlocksY = 1, kMinBlocksZ = 1;
 // form's usual pitches (x: 9 and 5; y, z: 16 and 8), where every
 // shared-memory access of a solve chunk becomes an immediate off one base
 // register: x 0.358 -> 0.336 ms, y and z 2-4% faster per step at 128^3.
+//
+// SEG > 0 (mixed form, periodic lines): the segmented solves of cs3d_seg.cuh,
+// SEG rows a segment, FULL when the line length is a multiple; the tile then
+// has no line factors and its solutions need no correction on read.  SEG = 0:
+// the Thomas solves with precomputed factors (the plain form, wall lines, and
+// lengths that seg_plan does not cut).
+template <typename T, int SEG>
+struct TileOf {
+    using SM = typename SweepSmem<T>::type;
+    static __device__ __forceinline__ SM at(int nbuf, int L, int P, int N, const SegPlan &) {
+        return SweepSmem<T>::at(smem_raw, nbuf, L, P, N);
+    }
+    static __device__ __forceinline__ void put1f(const SM &sm, int t, int o, T v) { put1(sm, t, o, v); }
+    static __device__ __forceinline__ Zn<T> z(const LineOp<T> &d1, const LineOp<T> &d2, int n) { return zn(d1, d2, n); }
+    static __device__ __forceinline__ void two(const SM &sm, int t, const Pt &p, int L, T za, T zb, T &a, T &b) {
+        get2(sm, t, p, L, za, zb, a, b);
+    }
+    static __device__ __forceinline__ T one(const SM &sm, int k, const Pt &p, int L, T z) { return get1(sm, k, p, L, z); }
+};
+// Segmented x tiles are planar: 80 registers a thread (3 blocks of 256 per SM)
+// hold one solve's segment, not a pair's.  Buffers as XU..XF4; a task's
+// buffers are 2t and 2t + 1.
+struct SmemSegX {
+    float *buf;
+    int stride;
+    __device__ float &at(int k, int o) const { return buf[k * stride + o]; }
+};
+template <int SEG>
+struct TileSegX {
+    using SM = SmemSegX;
+    static __device__ __forceinline__ SM at(int, int, int P, int N, const SegPlan &pl) {
+        return {reinterpret_cast<float *>(smem_raw), seg_stride(N, P, pl.G, pl.pad)};
+    }
+    static __device__ __forceinline__ void put1f(const SM &sm, int t, int o, float v) { sm.at(2 * t, o) = v; }
+    static __device__ __forceinline__ Zn<float> z(const LineOp<float> &, const LineOp<float> &, int) { return {0.f, 0.f}; }
+    static __device__ __forceinline__ void two(const SM &sm, int t, const Pt &p, int, float, float, float &a, float &b) {
+        a = sm.at(2 * t, p.o);
+        b = sm.at(2 * t + 1, p.o);
+    }
+    static __device__ __forceinline__ float one(const SM &sm, int k, const Pt &p, int, float) { return sm.at(k, p.o); }
+};
+__device__ __forceinline__ void put2(const SmemSegX &sm, int t, int o, float v0, float v1) {
+    sm.at(2 * t, o) = v0;
+    sm.at(2 * t + 1, o) = v1;
+}
+// The 13 solves of a segmented x tile, seven units of two (the last of one) on
+// the lines a warp holds.
+template <int SEG, bool FULL>
+__device__ __forceinline__ void run_seg_x(const SmemSegX &sm, int P, int L, int N, const SegPlan &pl, const SegOp &o1,
+                                          const SegOp &o2, int tid, int nthr) {
+    const int lane0 = tid & ((1 << pl.lgLW) - 1), seg = (tid & 31) >> pl.lgLW;
+    const int groups = max(1, L >> pl.lgLW);
+    for (int u = tid >> 5; u < 7 * groups; u += nthr >> 5) {
+        const int t = u / groups, l = ((u - t * groups) << pl.lgLW) + lane0;
+        const bool active = l < L;
+        SegLane<float> s = seg_lane<SEG, FULL>(pl, &sm.at(2 * t, active ? l : 0), seg, N, P);
+        // t < 4: the 2nd derivative to the next buffer, then the 1st in place
+        if (t < 4) seg_one<SEG, FULL, 2>(s, P, o2, pl, lane0, active, sm.stride);
+        seg_one<SEG, FULL, 1>(s, P, o1, pl, lane0, active, 0);
+        if (t < 4 || t == 6) continue;
+        s.row += sm.stride;
+        s.lo += sm.stride;
+        s.hi += sm.stride;
+        seg_one<SEG, FULL, 1>(s, P, o1, pl, lane0, active, 0);
+    }
+}
+template <int SEG>
+struct TileSeg {
+    using SM = SmemPair;
+    static __device__ __forceinline__ SM at(int, int, int P, int N, const SegPlan &pl) { return smem_pair_seg(P, N, pl); }
+    static __device__ __forceinline__ void put1f(const SM &sm, int t, int o, float v) { sm.at(2 * t, o) = v; }
+    static __device__ __forceinline__ Zn<float> z(const LineOp<float> &, const LineOp<float> &, int) { return {0.f, 0.f}; }
+    static __device__ __forceinline__ void two(const SM &sm, int t, const Pt &p, int, float, float, float &a, float &b) {
+        const float2 v = sm.pair(t)[p.o];
+        a = v.x;
+        b = v.y;
+    }
+    static __device__ __forceinline__ float one(const SM &sm, int k, const Pt &p, int, float) { return sm.at(k, p.o); }
+};
+// (cluster tiles: 8 pair arrays, then the mailbox)
+__device__ __forceinline__ float2 *cluster_mail(const SmemPair &sm) { return sm.pair(8); }
+template <> struct TileOf<float, 16> : TileSeg<16> {};
+template <> struct TileOf<float, 24> : TileSeg<24> {};
+template <> struct TileOf<float, 32> : TileSeg<32> {};
+
 // ---------------------------------------------------------------------
 // sweep x
 // ---------------------------------------------------------------------
@@ -71,12 +156,13 @@ __constant__ Task kTasksX2[7] = {{XU, XU, 0, XU, XU2, 1}, {XV, XV, 0, XV, XV2, 1
                                  {XT, XT, 0, XT, XT2, 1}, {XRU, XRU, 0, XF1, XF1, 0},
                                  {XF2, XF2, 0, XF3, XF3, 0}, {XF4, XF4, 0, XF4, XDUM, 0}};
 
-template <typename T, int PC>
-__global__ void __launch_bounds__(sweep_threads<T>(0), sizeof(T) == 4 ? kMinBlocksX : 2) k_sweep_x(SweepArgs<T> a) {
+template <typename T, int PC, int SEG = 0, bool FULL = false>
+__global__ void __launch_bounds__(sweep_threads<T>(0), sizeof(T) == 4 && (SEG == 0 || FULL) ? kMinBlocksX : 2) k_sweep_x(SweepArgs<T> a) {
+    using TS = std::conditional_t<(SEG > 0), TileSegX<SEG>, TileOf<T, 0>>;
     const int L = a.L, P = PC > 0 ? PC : a.P;
     const Tile t = make_tile<0>(a.g, L);
-    const int N = t.N, NL = N * L;
-    const auto sm = SweepSmem<T>::at(smem_raw, sizeof(T) == 4 ? XNB2 : XNB, L, P, N);
+    const int N = t.N, NL = N * L, pad = FULL ? a.seg.pad : 0;
+    const auto sm = TS::at(sizeof(T) == 4 ? XNB2 : XNB, L, P, N, a.seg);
     const GasParams gp = a.gas;
     // FP64 tiles: points across the lines first, pitch P = L (no pad column)
     constexpr bool kXLineFirst = sizeof(T) == 8;
@@ -84,7 +170,7 @@ __global__ void __launch_bounds__(sweep_threads<T>(0), sizeof(T) == 4 ? kMinBloc
     struct InA { Pt pt; T q[5]; };
     batched<InA, sizeof(T) == 4 ? 4 : 2>(NL,
         [&](InA &in, int p) {
-            in.pt = point<0, kXLineFirst>(t, p, L, P, a.lgL, a.divN);
+            in.pt = point<0, kXLineFirst>(t, p, L, P, a.lgL, a.divN, pad);
 #pragma unroll
             for (int f = 0; f < 5; ++f) in.q[f] = a.qs[f][in.pt.gi];
         },
@@ -108,24 +194,27 @@ __global__ void __launch_bounds__(sweep_threads<T>(0), sizeof(T) == 4 ? kMinBloc
                                    to_work<T>(a.backup.f[4][gi]));
             }
             const int o = in.pt.o;
-            put1(sm, 0, o, ss.U);
-            put1(sm, 1, o, ss.V);
-            put1(sm, 2, o, ss.W);
-            put1(sm, 3, o, ss.Tt);
+            TS::put1f(sm, 0, o, ss.U);
+            TS::put1f(sm, 1, o, ss.V);
+            TS::put1f(sm, 2, o, ss.W);
+            TS::put1f(sm, 3, o, ss.Tt);
             put2(sm, 4, o, s.ru, s.ru * ss.U + ss.p);
             put2(sm, 5, o, s.rv * ss.U, s.rw * ss.U);
-            put1(sm, 6, o, s.re * ss.U + ss.U * ss.p);
+            TS::put1f(sm, 6, o, s.re * ss.U + ss.U * ss.p);
         });
     __syncthreads();
-    run_sweep_solves<2, PC>(sm, sizeof(T) == 4 ? kTasksX2 : kTasksX, 7, L, t.nlines, a.d1, a.d2, threadIdx.x,
-                            blockDim.x, XDUM);
+    if constexpr (SEG > 0)
+        run_seg_x<SEG, FULL>(sm, P, L, N, a.seg, a.g1, a.g2, threadIdx.x, blockDim.x);
+    else
+        run_sweep_solves<2, PC>(sm, sizeof(T) == 4 ? kTasksX2 : kTasksX, 7, L, t.nlines, a.d1, a.d2, threadIdx.x,
+                                blockDim.x, XDUM);
     __syncthreads();
     // phase C
     const T c43 = T(4.0 / 3.0), cpPr = (T)gp.cpPr, muref = (T)gp.mu_ref;
     struct InC { Pt pt; T v[4]; };
     batched<InC, sizeof(T) == 4 ? 4 : 2>(NL,
         [&](InC &in, int p) {
-            in.pt = point<0, kXLineFirst>(t, p, L, P, a.lgL, a.divN);
+            in.pt = point<0, kXLineFirst>(t, p, L, P, a.lgL, a.divN, pad);
             const unsigned gi = in.pt.gi;
             in.v[0] = a.prim[0][gi]; in.v[1] = a.prim[1][gi]; in.v[2] = a.prim[2][gi]; in.v[3] = a.prim[4][gi];
         },
@@ -133,20 +222,20 @@ __global__ void __launch_bounds__(sweep_threads<T>(0), sizeof(T) == 4 ? kMinBloc
             if (!in.pt.ok) return;
             const Pt &p = in.pt;
             const unsigned gi = p.gi;
-            const Zn<T> zz = zn(a.d1, a.d2, p.n);
+            const Zn<T> zz = TS::z(a.d1, a.d2, p.n);
             const T U = in.v[0], V = in.v[1], W = in.v[2], Tt = in.v[3];
-            const T mu = muref * visc_pow(Tt);
-            const T amu = (T)0.76 * mu / Tt;
+            const T vz = muref * visc_rpow(Tt);
+            const T mu = vz * Tt, amu = (T)0.76 * vz;
             a.mu[gi] = mu;
             a.amu[gi] = amu;
             T Ux, Uxx, Vx, Vxx, Wx, Wxx, Tx, Txx, cex, f1, f2, f3;
-            get2(sm, 0, p, L, zz.z1, zz.z2, Ux, Uxx);
-            get2(sm, 1, p, L, zz.z1, zz.z2, Vx, Vxx);
-            get2(sm, 2, p, L, zz.z1, zz.z2, Wx, Wxx);
-            get2(sm, 3, p, L, zz.z1, zz.z2, Tx, Txx);
-            get2(sm, 4, p, L, zz.z1, zz.z1, cex, f1);
-            get2(sm, 5, p, L, zz.z1, zz.z1, f2, f3);
-            const T f4 = get1(sm, XF4, p, L, zz.z1);
+            TS::two(sm, 0, p, L, zz.z1, zz.z2, Ux, Uxx);
+            TS::two(sm, 1, p, L, zz.z1, zz.z2, Vx, Vxx);
+            TS::two(sm, 2, p, L, zz.z1, zz.z2, Wx, Wxx);
+            TS::two(sm, 3, p, L, zz.z1, zz.z2, Tx, Txx);
+            TS::two(sm, 4, p, L, zz.z1, zz.z1, cex, f1);
+            TS::two(sm, 5, p, L, zz.z1, zz.z1, f2, f3);
+            const T f4 = TS::one(sm, XF4, p, L, zz.z1);
             a.dx[0][gi] = Ux; a.dx[1][gi] = Vx; a.dx[2][gi] = Wx; a.dx[3][gi] = Tx;
             if (a.tape[0]) {  // the tape's x entries (kIn* 0..16)
                 T *const *g = a.tape;
@@ -156,10 +245,12 @@ __global__ void __launch_bounds__(sweep_threads<T>(0), sizeof(T) == 4 ? kMinBloc
                 g[12][gi] = cex; g[13][gi] = f1; g[14][gi] = f2; g[15][gi] = f3; g[16][gi] = f4;
             }
             a.R[0][gi] = -cex;
-            a.R[1][gi] = mu * (c43 * Uxx) - f1;
-            a.R[2][gi] = mu * Vxx - f2;
-            a.R[3][gi] = mu * Wxx - f3;
-            a.R[4][gi] = cpPr * mu * Txx + mu * (U * (c43 * Uxx) + V * Vxx + W * Wxx) - f4;
+            // viscous terms of the momenta; their work is U, V, W times them
+            const T v1 = mu * c43 * Uxx, v2 = mu * Vxx, v3 = mu * Wxx;
+            a.R[1][gi] = v1 - f1;
+            a.R[2][gi] = v2 - f2;
+            a.R[3][gi] = v3 - f3;
+            a.R[4][gi] = cpPr * mu * Txx + U * v1 + V * v2 + W * v3 - f4;
         });
 }
 
@@ -179,16 +270,18 @@ __constant__ Task kTasksY2[8] = {{YU, YU, 0, YU, YU2, 1}, {YV, YV, 0, YV, YV2, 1
 
 // FP64: 3 blocks per SM (168 registers, no spills): 2.93 -> 2.67 ms per step at
 // TGV 128^3, 37.5 -> 27.1 at HIT 256^3, the same bits
-template <typename T, int PC>
+template <typename T, int PC, int SEG = 0, bool FULL = false, bool CL = false>
 __global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBlocksY : 3) k_sweep_y(SweepArgs<T> a) {
-    const int L = a.L, P = PC > 0 ? PC : a.P;
-    const Tile t = make_tile<1>(a.g, L);
-    const int N = t.N, NL = N * L;
-    const auto sm = SweepSmem<T>::at(smem_raw, sizeof(T) == 4 ? YNB2 : YNB, L, P, N);
+    using TS = TileOf<T, SEG>;
+    const int L = CL ? kClLines : a.L, P = PC > 0 ? PC : a.P;
+    const int rank = CL ? (int)blockIdx.x % a.seg.C : 0;
+    const Tile t = CL ? make_cluster_tile<1>(a.g, a.seg, rank) : make_tile<1>(a.g, L);
+    const int N = t.N, NL = N * L, pad = FULL && !CL ? a.seg.pad : 0;
+    const auto sm = TS::at(sizeof(T) == 4 ? YNB2 : YNB, L, P, CL ? kClRows : N, a.seg);
     struct InA { Pt pt; T v[11]; };
     batched<InA, sizeof(T) == 4 ? 4 : 2>(NL,
         [&](InA &in, int p) {
-            in.pt = point<1>(t, p, L, P, a.lgL, a.divN);
+            in.pt = point<1>(t, p, L, P, CL ? 5 : a.lgL, a.divN, pad);
             const unsigned gi = in.pt.gi;
 #pragma unroll
             for (int f = 0; f < 4; ++f) in.v[f] = a.qs[f + 1][gi];
@@ -202,24 +295,31 @@ __global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBloc
             const int o = in.pt.o;
             const T ru = in.v[0], rv = in.v[1], rw = in.v[2], re = in.v[3];
             const T V = in.v[5], pp = in.v[7];
-            put1(sm, 0, o, in.v[4]);
-            put1(sm, 1, o, V);
-            put1(sm, 2, o, in.v[6]);
-            put1(sm, 3, o, in.v[8]);
+            TS::put1f(sm, 0, o, in.v[4]);
+            TS::put1f(sm, 1, o, V);
+            TS::put1f(sm, 2, o, in.v[6]);
+            TS::put1f(sm, 3, o, in.v[8]);
             put2(sm, 4, o, in.v[9], in.v[10]);
             put2(sm, 5, o, rv, ru * V);
             put2(sm, 6, o, rv * V + pp, rw * V);
-            put1(sm, 7, o, re * V + V * pp);
+            TS::put1f(sm, 7, o, re * V + V * pp);
         });
-    __syncthreads();
-    run_sweep_solves<2, PC>(sm, sizeof(T) == 4 ? kTasksY2 : kTasksY, 8, L, t.nlines, a.d1, a.d2, threadIdx.x,
-                            blockDim.x, YDUM);
+    if constexpr (CL) cluster_sync();
+    else __syncthreads();
+    if constexpr (CL)
+        run_cluster_tasks<FULL, 8, true>(sm.pair(0), sm.pstride / 2, cluster_mail(sm), a.seg, a.g1, a.g2, rank,
+                                         threadIdx.x);
+    else if constexpr (SEG > 0)
+        run_seg_tasks<SEG, FULL, 8, true>(sm, P, L, N, a.seg, a.g1, a.g2, threadIdx.x, blockDim.x);
+    else
+        run_sweep_solves<2, PC>(sm, sizeof(T) == 4 ? kTasksY2 : kTasksY, 8, L, t.nlines, a.d1, a.d2, threadIdx.x,
+                                blockDim.x, YDUM);
     __syncthreads();
     const T c43 = T(4.0 / 3.0), c13 = T(1.0 / 3.0), cpPr = (T)a.gas.cpPr;
     struct InC { Pt pt; T v[9]; };
     batched<InC, sizeof(T) == 4 ? kYConsumeBatch : 2>(NL,
         [&](InC &in, int p) {
-            in.pt = point<1>(t, p, L, P, a.lgL, a.divN);
+            in.pt = point<1>(t, p, L, P, CL ? 5 : a.lgL, a.divN, pad);
             const unsigned gi = in.pt.gi;
             in.v[0] = a.prim[0][gi]; in.v[1] = a.prim[1][gi]; in.v[2] = a.prim[2][gi];
             in.v[3] = a.mu[gi];
@@ -230,17 +330,17 @@ __global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBloc
             if (!in.pt.ok) return;
             const Pt &p = in.pt;
             const unsigned gi = p.gi;
-            const Zn<T> zz = zn(a.d1, a.d2, p.n);
+            const Zn<T> zz = TS::z(a.d1, a.d2, p.n);
             const T U = in.v[0], V = in.v[1], W = in.v[2], mu = in.v[3];
             T Uy, Uyy, Vy, Vyy, Wy, Wyy, Ty, Tyy, Uxy, Vxy, cey, f1, f2, f3;
-            get2(sm, 0, p, L, zz.z1, zz.z2, Uy, Uyy);
-            get2(sm, 1, p, L, zz.z1, zz.z2, Vy, Vyy);
-            get2(sm, 2, p, L, zz.z1, zz.z2, Wy, Wyy);
-            get2(sm, 3, p, L, zz.z1, zz.z2, Ty, Tyy);
-            get2(sm, 4, p, L, zz.z1, zz.z1, Uxy, Vxy);
-            get2(sm, 5, p, L, zz.z1, zz.z1, cey, f1);
-            get2(sm, 6, p, L, zz.z1, zz.z1, f2, f3);
-            const T f4 = get1(sm, YF4, p, L, zz.z1);
+            TS::two(sm, 0, p, L, zz.z1, zz.z2, Uy, Uyy);
+            TS::two(sm, 1, p, L, zz.z1, zz.z2, Vy, Vyy);
+            TS::two(sm, 2, p, L, zz.z1, zz.z2, Wy, Wyy);
+            TS::two(sm, 3, p, L, zz.z1, zz.z2, Ty, Tyy);
+            TS::two(sm, 4, p, L, zz.z1, zz.z1, Uxy, Vxy);
+            TS::two(sm, 5, p, L, zz.z1, zz.z1, cey, f1);
+            TS::two(sm, 6, p, L, zz.z1, zz.z1, f2, f3);
+            const T f4 = TS::one(sm, YF4, p, L, zz.z1);
             a.dy[0][gi] = Uy; a.dy[1][gi] = Vy; a.dy[2][gi] = Wy; a.dy[3][gi] = Ty;
             if (a.tape[0]) {  // the tape's y entries (kIn* 17..31)
                 T *const *g = a.tape;
@@ -254,11 +354,11 @@ __global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBloc
             const int wd = a.wall_faces ? wall_dir(faces_of(a.g, i, j, k) & a.wall_faces) : -1;
             if (wd == 1) a.R[0][gi] = -cey;
             else if (wd < 0) a.R[0][gi] = in.v[4] - cey;
-            a.R[1][gi] = in.v[5] + (mu * (Uyy + c13 * Vxy) - f1);
-            a.R[2][gi] = in.v[6] + (mu * (c43 * Vyy + c13 * Uxy) - f2);
-            a.R[3][gi] = in.v[7] + (mu * Wyy - f3);
-            a.R[4][gi] = in.v[8] +
-                         (cpPr * mu * Tyy + mu * (U * Uyy + V * (c43 * Vyy) + W * Wyy + c13 * (U * Vxy + V * Uxy)) - f4);
+            const T v1 = mu * (Uyy + c13 * Vxy), v2 = mu * (c43 * Vyy + c13 * Uxy), v3 = mu * Wyy;
+            a.R[1][gi] = in.v[5] + (v1 - f1);
+            a.R[2][gi] = in.v[6] + (v2 - f2);
+            a.R[3][gi] = in.v[7] + (v3 - f3);
+            a.R[4][gi] = in.v[8] + (cpPr * mu * Tyy + U * v1 + V * v2 + W * v3 - f4);
         });
 }
 
@@ -273,18 +373,19 @@ __constant__ Task kTasksZ[8] = {{ZU, ZU, 0, ZU, ZU2, 1}, {ZV, ZV, 0, ZV, ZV2, 1}
 
 // The z sweep's three phases as functions of (tile, shared-memory layout,
 // thread range).
-template <typename T, int PC>
+template <typename T, int PC, int SEG, bool FULL, bool CL>
 struct ZSweep {
+    using TS = TileOf<T, SEG>;
+    using SM = typename TS::SM;
     // A: stage the inputs of the 16 z-solves of tile t in sm
-    using SM = typename SweepSmem<T>::type;
     static __device__ __forceinline__ void load(const SweepArgs<T> &a, const Tile &t, const SM &sm, int tid,
                                                 int nthr) {
-        const int L = a.L, P = PC > 0 ? PC : a.P;
-        const int NL = t.N * L;
+        const int L = CL ? kClLines : a.L, P = PC > 0 ? PC : a.P, lgL = CL ? 5 : a.lgL;
+        const int NL = t.N * L, pad = FULL && !CL ? a.seg.pad : 0;
         struct InA { Pt pt; T v[13]; };
         batched<InA, sizeof(T) == 4 ? 4 : 2>(NL, tid, nthr,
             [&](InA &in, int p) {
-                in.pt = point<2>(t, p, L, P, a.lgL, a.divN);
+                in.pt = point<2>(t, p, L, P, lgL, a.divN, pad);
                 const unsigned gi = in.pt.gi;
 #pragma unroll
                 for (int f = 0; f < 4; ++f) in.v[f] = a.qs[f + 1][gi];
@@ -300,10 +401,10 @@ struct ZSweep {
                 const int o = in.pt.o;
                 const T ru = in.v[0], rv = in.v[1], rw = in.v[2], re = in.v[3];
                 const T W = in.v[6], pp = in.v[7];
-                put1(sm, 0, o, in.v[4]);
-                put1(sm, 1, o, in.v[5]);
-                put1(sm, 2, o, W);
-                put1(sm, 3, o, in.v[8]);
+                TS::put1f(sm, 0, o, in.v[4]);
+                TS::put1f(sm, 1, o, in.v[5]);
+                TS::put1f(sm, 2, o, W);
+                TS::put1f(sm, 3, o, in.v[8]);
                 put2(sm, 4, o, in.v[9] + in.v[10], in.v[11]);
                 put2(sm, 5, o, in.v[12], rw);
                 put2(sm, 6, o, ru * W, rv * W);
@@ -313,14 +414,20 @@ struct ZSweep {
     // B: the 16 solves (8 pairs) of every line of the tile
     static __device__ __forceinline__ void solve(const SweepArgs<T> &a, const Tile &t, const SM &sm, int tid,
                                                  int nthr) {
-        run_sweep_solves<2, PC>(sm, kTasksZ, 8, a.L, t.nlines, a.d1, a.d2, tid, nthr, -1);
+        if constexpr (CL)
+            run_cluster_tasks<FULL, 8, false>(sm.pair(0), sm.pstride / 2, cluster_mail(sm), a.seg, a.g1, a.g2,
+                                              (int)blockIdx.x % a.seg.C, tid);
+        else if constexpr (SEG > 0)
+            run_seg_tasks<SEG, FULL, 8, false>(sm, PC > 0 ? PC : a.P, a.L, t.N, a.seg, a.g1, a.g2, tid, nthr);
+        else
+            run_sweep_solves<2, PC>(sm, kTasksZ, 8, a.L, t.nlines, a.d1, a.d2, tid, nthr, -1);
     }
     // C: right-hand side, dq and the RK update of every point of the tile
     static __device__ __forceinline__ void consume(const SweepArgs<T> &a, const Tile &t, const SM &sm, int tid,
                                                    int nthr) {
-        const int L = a.L, P = PC > 0 ? PC : a.P;
-        const int NL = t.N * L;
-        const T c43 = T(4.0 / 3.0), c13 = T(1.0 / 3.0), c23 = T(2.0 / 3.0), cpPr = (T)a.gas.cpPr;
+        const int L = CL ? kClLines : a.L, P = PC > 0 ? PC : a.P, lgL = CL ? 5 : a.lgL;
+        const int NL = t.N * L, pad = FULL && !CL ? a.seg.pad : 0;
+        const T c43 = T(4.0 / 3.0), c13 = T(1.0 / 3.0), cpPr = (T)a.gas.cpPr;
         const double dt = *a.dt;
         const T dtw = (T)dt;
         const int st = a.rk_step;
@@ -349,7 +456,7 @@ struct ZSweep {
         };
         pipelined<InC1>(NL, tid, nthr,
             [&](InC1 &in, int p) {
-                in.pt = point<2>(t, p, L, P, a.lgL, a.divN);
+                in.pt = point<2>(t, p, L, P, lgL, a.divN, pad);
                 const unsigned gi = in.pt.gi;
                 in.v[0] = a.prim[0][gi]; in.v[1] = a.prim[1][gi]; in.v[2] = a.prim[2][gi];
                 in.v[3] = a.mu[gi]; in.v[4] = a.amu[gi];
@@ -365,19 +472,19 @@ struct ZSweep {
                 if (!in.pt.ok) return;
                 const Pt &p = in.pt;
                 const unsigned gi = p.gi;
-                const Zn<T> zz = zn(a.d1, a.d2, p.n);
+                const Zn<T> zz = TS::z(a.d1, a.d2, p.n);
                 const T U = in.v[0], V = in.v[1], W = in.v[2], mu = in.v[3], amu = in.v[4];
                 const T Ux = in.v[5], Vx = in.v[6], Wx = in.v[7], Tx = in.v[8];
                 const T Uy = in.v[9], Vy = in.v[10], Wy = in.v[11], Ty = in.v[12];
                 T Uz, Uzz, Vz, Vzz, Wz, Wzz, Tz, Tzz, S, Wxz, Wyz, cez, f1, f2, f3, f4;
-                get2(sm, 0, p, L, zz.z1, zz.z2, Uz, Uzz);
-                get2(sm, 1, p, L, zz.z1, zz.z2, Vz, Vzz);
-                get2(sm, 2, p, L, zz.z1, zz.z2, Wz, Wzz);
-                get2(sm, 3, p, L, zz.z1, zz.z2, Tz, Tzz);
-                get2(sm, 4, p, L, zz.z1, zz.z1, S, Wxz);  // S = d/dz (Ux + Vy)
-                get2(sm, 5, p, L, zz.z1, zz.z1, Wyz, cez);
-                get2(sm, 6, p, L, zz.z1, zz.z1, f1, f2);
-                get2(sm, 7, p, L, zz.z1, zz.z1, f3, f4);
+                TS::two(sm, 0, p, L, zz.z1, zz.z2, Uz, Uzz);
+                TS::two(sm, 1, p, L, zz.z1, zz.z2, Vz, Vzz);
+                TS::two(sm, 2, p, L, zz.z1, zz.z2, Wz, Wzz);
+                TS::two(sm, 3, p, L, zz.z1, zz.z2, Tz, Tzz);
+                TS::two(sm, 4, p, L, zz.z1, zz.z1, S, Wxz);  // S = d/dz (Ux + Vy)
+                TS::two(sm, 5, p, L, zz.z1, zz.z1, Wyz, cez);
+                TS::two(sm, 6, p, L, zz.z1, zz.z1, f1, f2);
+                TS::two(sm, 7, p, L, zz.z1, zz.z1, f3, f4);
                 T src[5] = {T(0), T(0), T(0), T(0), T(0)};
                 if (a.sponge) {  // sigma (avg - q), SpongeBC / CSolver_AWS.hpp:228
                     const T sg = to_work<T>(a.sigma[gi]);
@@ -385,25 +492,24 @@ struct ZSweep {
                     for (int f = 0; f < 5; ++f) src[f] = sg * (to_work<T>(a.savg.f[f][gi]) - in.qsv[f]);
                 }
                 const T MuX = amu * Tx, MuY = amu * Ty, MuZ = amu * Tz;
+                // shear rates, and the normal stresses' 3/4: c43 h1 is
+                // (4/3) Ux - (2/3)(Vy + Wz)
+                const T s12 = Uy + Vx, s13 = Wx + Uz, s23 = Wy + Vz;
+                const T h1 = Ux - T(0.5) * (Vy + Wz), h2 = Vy - T(0.5) * (Ux + Wz), h3 = Wz - T(0.5) * (Ux + Vy);
+                // the viscous terms of the momenta: mu times second derivatives
+                // and the viscosity gradient times the stresses; their work is
+                // U, V, W times them, plus the dissipation
+                const T w1 = mu * (Uzz + c13 * Wxz) + (c43 * MuX * h1 + MuY * s12 + MuZ * s13);
+                const T w2 = mu * (Vzz + c13 * Wyz) + (c43 * MuY * h2 + MuX * s12 + MuZ * s23);
+                const T w3 = mu * (c43 * Wzz + c13 * S) + (c43 * MuZ * h3 + MuX * s13 + MuY * s23);
+                const T diss = c43 * (Ux * h1 + Vy * h2 + Wz * h3) + (s12 * s12 + s13 * s13 + s23 * s23);
                 T R[5];
                 R[0] = in.v[13];
-                R[1] = in.v[14] + mu * (Uzz + c13 * Wxz) - f1 + c43 * MuX * (Ux - T(0.5) * Vy - T(0.5) * Wz) +
-                       MuY * (Uy + Vx) + MuZ * (Wx + Uz) + src[1];
-                R[2] = in.v[15] + mu * (Vzz + c13 * Wyz) - f2 + c43 * MuY * (Vy - T(0.5) * Ux - T(0.5) * Wz) +
-                       MuX * (Uy + Vx) + MuZ * (Wy + Vz) + src[2];
-                R[3] = in.v[16] + mu * (c43 * Wzz + c13 * S) - f3 + c43 * MuZ * (Wz - T(0.5) * Ux - T(0.5) * Vy) +
-                       MuX * (Wx + Uz) + MuY * (Wy + Vz) + src[3];
-                const T q2s = Ux * Ux + Vy * Vy + Wz * Wz;
-                const T sq = Uy * Uy + Uz * Uz + Vx * Vx + Vz * Vz + Wx * Wx + Wy * Wy;
-                const T cr = Ux * Vy + Ux * Wz + Vy * Wz;
-                const T sh = Uy * Vx + Uz * Wx + Vz * Wy;
-                const T v1 = mu * (U * Uzz + V * Vzz + W * (c43 * Wzz) + c13 * (U * Wxz + V * Wyz + W * S) + c43 * q2s +
-                                   sq - c43 * cr + T(2.0) * sh);
-                const T v2 = c43 * (U * MuX * Ux + V * MuY * Vy + W * MuZ * Wz) - c23 * U * MuX * (Vy + Wz) -
-                             c23 * V * MuY * (Ux + Wz) - c23 * W * MuZ * (Ux + Vy) + U * MuY * (Uy + Vx) +
-                             U * MuZ * (Uz + Wx) + V * MuX * (Uy + Vx) + V * MuZ * (Vz + Wy) + W * MuX * (Uz + Wx) +
-                             W * MuY * (Vz + Wy);
-                R[4] = in.v[17] + cpPr * (MuX * Tx + MuY * Ty + MuZ * Tz + mu * Tzz) + v1 + v2 - f4 + T(2.0) * src[4];
+                R[1] = in.v[14] + (w1 - f1) + src[1];
+                R[2] = in.v[15] + (w2 - f2) + src[2];
+                R[3] = in.v[16] + (w3 - f3) + src[3];
+                R[4] = in.v[17] + cpPr * (MuX * Tx + MuY * Ty + MuZ * Tz + mu * Tzz) +
+                       (U * w1 + V * w2 + W * w3 + mu * diss) - f4 + T(2.0) * src[4];
                 // continuity and the post-step boundary fix-up (CSolver_AWS.cpp:1506-1679)
                 int i, j, k;
                 coords<2>(t, p.l, p.n, i, j, k);
@@ -439,7 +545,7 @@ struct ZSweep {
         };
         batched<InC2, kZUpdateBatch>(NL, tid, nthr,
             [&](InC2 &in, int p) {
-                in.pt = point<2>(t, p, L, P, a.lgL, a.divN);
+                in.pt = point<2>(t, p, L, P, lgL, a.divN, pad);
                 const unsigned gi = in.pt.gi;
 #pragma unroll
                 for (int f = 0; f < 5; ++f) {
@@ -503,15 +609,17 @@ struct ZSweep {
 
 // FP64: 3 blocks per SM (168 registers; 88 bytes of spill stores): 4.70 ->
 // 4.52 ms per step at TGV 128^3, 52.5 -> 44.9 at HIT 256^3, the same bits
-template <typename T, int PC>
+template <typename T, int PC, int SEG = 0, bool FULL = false, bool CL = false>
 __global__ void __launch_bounds__(sweep_threads<T>(2), sizeof(T) == 4 ? kMinBlocksZ : 3) k_sweep_z(SweepArgs<T> a) {
-    const Tile t = make_tile<2>(a.g, a.L);
-    const auto sm = SweepSmem<T>::at(smem_raw, ZNB, a.L, PC > 0 ? PC : a.P, t.N);
-    ZSweep<T, PC>::load(a, t, sm, threadIdx.x, blockDim.x);
+    using Z = ZSweep<T, PC, SEG, FULL, CL>;
+    const Tile t = CL ? make_cluster_tile<2>(a.g, a.seg, (int)blockIdx.x % a.seg.C) : make_tile<2>(a.g, a.L);
+    const auto sm = Z::TS::at(ZNB, a.L, PC > 0 ? PC : a.P, CL ? kClRows : t.N, a.seg);
+    Z::load(a, t, sm, threadIdx.x, blockDim.x);
+    if constexpr (CL) cluster_sync();
+    else __syncthreads();
+    Z::solve(a, t, sm, threadIdx.x, blockDim.x);
     __syncthreads();
-    ZSweep<T, PC>::solve(a, t, sm, threadIdx.x, blockDim.x);
-    __syncthreads();
-    ZSweep<T, PC>::consume(a, t, sm, threadIdx.x, blockDim.x);
+    Z::consume(a, t, sm, threadIdx.x, blockDim.x);
 }
 
 // ---------------------------------------------------------------------
@@ -610,6 +718,72 @@ __global__ void __launch_bounds__(filter_threads<T>(), sizeof(T) == 4 ? kFilterM
     }
 }
 
+// The mixed filter on periodic lines: the five fields' corrections by the
+// segmented solves (cs3d_seg.cuh), added in place, so a tile is five buffers
+// and the y and z tiles are 32 lines (128 bytes a row) wide.
+template <int DIR, int SEG, bool FULL>
+__global__ void __launch_bounds__(kFilterSegTpb, 2) k_filter_seg(FilterArgs<float> a) {
+    const int L = a.L, P = a.P;
+    const Tile t = make_tile<DIR>(a.g, L);
+    const int N = t.N, NL = N * L, pad = FULL ? a.seg.pad : 0;
+    const int stride = seg_stride(N, P, a.seg.G, a.seg.pad);
+    float *buf = reinterpret_cast<float *>(smem_raw);
+    struct In { Pt pt; float v[5]; };
+    batched<In, kFilterBatch>(NL,
+        [&](In &in, int p) {
+            in.pt = point<DIR>(t, p, L, P, a.lgL, a.divN, pad);
+            const unsigned gi = in.pt.gi;
+#pragma unroll
+            for (int f = 0; f < 5; ++f) in.v[f] = a.src64.f[0] ? narrow(a.src64.f[f][gi] - a.ref[f]) : a.src32[f][gi];
+        },
+        [&](In &in) {
+            if (!in.pt.ok) return;
+#pragma unroll
+            for (int f = 0; f < 5; ++f) buf[f * stride + in.pt.o] = in.v[f];
+        });
+    __syncthreads();
+    {
+        const int lane0 = threadIdx.x & ((1 << a.seg.lgLW) - 1), seg = (threadIdx.x & 31) >> a.seg.lgLW;
+        const int groups = max(1, L >> a.seg.lgLW);
+        for (int u = threadIdx.x >> 5; u < 5 * groups; u += blockDim.x >> 5) {
+            const int f = u / groups, l = ((u - f * groups) << a.seg.lgLW) + lane0;
+            const bool active = l < L;
+            seg_filter<SEG, FULL>(seg_lane<SEG, FULL>(a.seg, buf + f * stride + (active ? l : 0), seg, N, P), P, a.sg,
+                                  a.seg, lane0, active);
+        }
+    }
+    __syncthreads();
+    struct Out { Pt pt; double q[5]; float u[5]; };
+    batched<Out, kFilterConsumeBatch>(NL,
+        [&](Out &o, int p) {
+            o.pt = point<DIR>(t, p, L, P, a.lgL, a.divN, pad);
+#pragma unroll
+            for (int f = 0; f < 5; ++f) {
+                o.q[f] = a.delta_from.f[0] ? a.delta_from.f[f][o.pt.gi] : 0.0;
+                o.u[f] = a.unf[0] ? a.unf[f][o.pt.gi] : 0.f;
+            }
+        },
+        [&](Out &o) {
+            if (!o.pt.ok) return;
+            const unsigned gi = o.pt.gi;
+#pragma unroll
+            for (int f = 0; f < 5; ++f) {
+                const float v = buf[f * stride + o.pt.o];
+                if (a.dst64.f[0]) {
+                    // q1 = q2 + (filtered - unfiltered); the unfiltered value is
+                    // the first pass's FP32 input, or formed again from q2 (the
+                    // same number either way)
+                    const float v0 = a.unf[0] ? o.u[f] : narrow(o.q[f] - a.ref[f]);
+                    const double nv = o.q[f] + widen(v - v0);
+                    a.dst64.f[f][gi] = nv;
+                    a.shadow_out[f][gi] = narrow(nv);
+                } else {
+                    a.dst32[f][gi] = v;
+                }
+            }
+        });
+}
+
 // ---------------------------------------------------------------------
 // single operator on contiguous lines (Derivatives::calc1stDerivField etc.)
 // ---------------------------------------------------------------------
@@ -665,7 +839,11 @@ static size_t pair_tile_smem(int nbuf, int L, int P, int N) {
 size_t planar_smem_bytes(int prec_bytes, int nbuf, int L, int P, int N) {
     return prec_bytes == 8 ? tile_smem<double>(nbuf, L, P, N) : tile_smem<float>(nbuf, L, P, N);
 }
-size_t sweep_smem_bytes(int prec_bytes, int nbuf, int L, int P, int N) {
+size_t sweep_smem_bytes(int prec_bytes, int nbuf, int L, int P, int N, const SegPlan *seg) {
+    if (prec_bytes == 4 && seg && seg->C) return 8 * (8 * (size_t)kClRows * kClLines + 8 * kClLines);
+    if (prec_bytes == 4 && seg && seg->SEG && !seg->pair) return (size_t)XNB * 4 * seg_stride(N, P, seg->G, seg->pad);
+    // segmented solves: the pair arrays alone (no line factors, no read-ahead)
+    if (prec_bytes == 4 && seg && seg->SEG) return (size_t)((nbuf + 1) / 2) * 4 * seg_pair_stride(N, P, seg->G, seg->pad);
     return prec_bytes == 8 ? tile_smem<double>(nbuf, L, P, N) : pair_tile_smem(nbuf, L, P, N);
 }
 int sweep_nbuf(int dir, int prec_bytes) {
@@ -689,12 +867,68 @@ static dim3 tile_grid(int dir, const Geom &g, int L) {
     return dim3((g.Nx + L - 1) / L, g.Ny);
 }
 
+// the segmented instances: compile-time pitches for the full segments, the
+// three segment lengths at run-time pitch for the others
+static cudaError_t launch_cluster(void (*kernel)(SweepArgs<float>), const SweepArgs<float> &a, dim3 grid, size_t sm,
+                                  cudaStream_t s) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid.x * a.seg.C, grid.y);
+    c.blockDim = dim3(32 * kClWarps);
+    c.dynamicSmemBytes = sm;
+    c.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = a.seg.C;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    e = cudaLaunchKernelEx(&c, kernel, a);
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+static cudaError_t launch_seg_sweep(int dir, const SweepArgs<float> &a, dim3 grid, size_t sm, cudaStream_t s) {
+    if (a.seg.C) {
+        const bool f = a.seg.full;
+        if (dir == 1) return launch_cluster(f ? k_sweep_y<float, 32, 32, true, true> : k_sweep_y<float, 32, 32, false, true>, a, grid, sm, s);
+        return launch_cluster(f ? k_sweep_z<float, 32, 32, true, true> : k_sweep_z<float, 32, 32, false, true>, a, grid, sm, s);
+    }
+#define SEG_CASE(K, PC, SEG, FULL) return launch_tile_kernel(K<float, PC, SEG, FULL>, a, grid, sm, s)
+    if (a.seg.full) {
+        if (dir == 0 && a.P == 9) SEG_CASE(k_sweep_x, 9, 32, true);
+        if (dir == 0 && a.P == 5) SEG_CASE(k_sweep_x, 5, 32, true);
+        if (dir == 1 && a.P == 16) SEG_CASE(k_sweep_y, 16, 32, true);
+        if (dir == 1 && a.P == 8) SEG_CASE(k_sweep_y, 8, 32, true);
+        if (dir == 2 && a.P == 16) SEG_CASE(k_sweep_z, 16, 32, true);
+        if (dir == 2 && a.P == 8) SEG_CASE(k_sweep_z, 8, 32, true);
+        if (dir == 0) SEG_CASE(k_sweep_x, 0, 32, true);
+        if (dir == 1) SEG_CASE(k_sweep_y, 0, 32, true);
+        SEG_CASE(k_sweep_z, 0, 32, true);
+    }
+    if (a.seg.SEG == 32) {
+        if (dir == 0) SEG_CASE(k_sweep_x, 0, 32, false);
+        if (dir == 1) SEG_CASE(k_sweep_y, 0, 32, false);
+        SEG_CASE(k_sweep_z, 0, 32, false);
+    }
+    if (a.seg.SEG == 24) {
+        if (dir == 0) SEG_CASE(k_sweep_x, 0, 24, false);
+        if (dir == 1) SEG_CASE(k_sweep_y, 0, 24, false);
+        SEG_CASE(k_sweep_z, 0, 24, false);
+    }
+    if (dir == 0) SEG_CASE(k_sweep_x, 0, 16, false);
+    if (dir == 1) SEG_CASE(k_sweep_y, 0, 16, false);
+    SEG_CASE(k_sweep_z, 0, 16, false);
+#undef SEG_CASE
+}
+
 template <typename T>
 cudaError_t launch_sweep(int dir, const SweepArgs<T> &a, cudaStream_t s) {
     const int N = dir == 0 ? a.g.Nx : dir == 1 ? a.g.Ny : a.g.Nz;
-    const size_t sm = sweep_smem_bytes((int)sizeof(T), sweep_nbuf(dir, (int)sizeof(T)), a.L, a.P, N);
+    const size_t sm = sweep_smem_bytes((int)sizeof(T), sweep_nbuf(dir, (int)sizeof(T)), a.L, a.P, N, &a.seg);
     const dim3 grid = tile_grid(dir, a.g, a.L);
     if constexpr (sizeof(T) == 4) {
+        if (a.seg.SEG) return launch_seg_sweep(dir, a, grid, sm, s);
         if (dir == 0 && a.P == 9) return launch_tile_kernel(k_sweep_x<T, 9>, a, grid, sm, s);
         if (dir == 0 && a.P == 5) return launch_tile_kernel(k_sweep_x<T, 5>, a, grid, sm, s);
         if (dir == 1 && a.P == 16) return launch_tile_kernel(k_sweep_y<T, 16>, a, grid, sm, s);
@@ -707,9 +941,28 @@ cudaError_t launch_sweep(int dir, const SweepArgs<T> &a, cudaStream_t s) {
     return launch_tile_kernel(k_sweep_z<T, 0>, a, grid, sm, s);
 }
 
+size_t filter_seg_smem(int L, int P, int N, const SegPlan &p) { return (size_t)5 * 4 * seg_stride(N, P, p.G, p.pad); }
+
+template <int DIR>
+static cudaError_t launch_filter_seg(const FilterArgs<float> &a, dim3 grid, size_t sm, cudaStream_t s) {
+    if (a.seg.full) return launch_tile_kernel(k_filter_seg<DIR, 32, true>, a, grid, sm, s);
+    if (a.seg.SEG == 32) return launch_tile_kernel(k_filter_seg<DIR, 32, false>, a, grid, sm, s);
+    if (a.seg.SEG == 24) return launch_tile_kernel(k_filter_seg<DIR, 24, false>, a, grid, sm, s);
+    return launch_tile_kernel(k_filter_seg<DIR, 16, false>, a, grid, sm, s);
+}
+
 template <typename T>
 cudaError_t launch_filter(int dir, const FilterArgs<T> &a, cudaStream_t s) {
     const int N = dir == 0 ? a.g.Nx : dir == 1 ? a.g.Ny : a.g.Nz;
+    if constexpr (sizeof(T) == 4) {
+        if (a.seg.SEG) {
+            const size_t fs = filter_seg_smem(a.L, a.P, N, a.seg);
+            const dim3 fg = tile_grid(dir, a.g, a.L);
+            if (dir == 0) return launch_filter_seg<0>(a, fg, fs, s);
+            if (dir == 1) return launch_filter_seg<1>(a, fg, fs, s);
+            return launch_filter_seg<2>(a, fg, fs, s);
+        }
+    }
     const size_t sm = tile_smem<T>(sizeof(T) == 4 ? 10 : 5, a.L, a.P, N);
     const dim3 grid = tile_grid(dir, a.g, a.L);
     if constexpr (sizeof(T) == 4) {

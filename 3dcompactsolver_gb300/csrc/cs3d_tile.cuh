@@ -4,6 +4,7 @@
 #pragma once
 #include "cs3d_dev.cuh"
 #include "cs3d_kernels.cuh"
+#include "cs3d_seg.cuh"
 #include <type_traits>
 
 namespace cs3d {
@@ -368,7 +369,7 @@ struct Tile {
     unsigned sl, sn;  // strides between lines and along a line
     int nlines;       // valid lines in this tile (<= L)
     int N;            // line length
-    int ci, cj, ck;   // coordinates of (line 0, position 0)
+    int ci, cj, ck;   // coordinates of (line 0, position 0 of this tile)
 };
 
 // The tile of block coordinates (bx, by): bx counts tiles across the lines'
@@ -408,6 +409,18 @@ __device__ __forceinline__ Tile make_tile(const Geom &g, int L) {
     return make_tile_at<DIR>(g, L, blockIdx.x, blockIdx.y);
 }
 
+// The rows of a cluster's tile (32 lines) that block `rank` holds.
+template <int DIR>
+__device__ __forceinline__ Tile make_cluster_tile(const Geom &g, const SegPlan &pl, int rank) {
+    Tile t = make_tile_at<DIR>(g, kClLines, (int)blockIdx.x / pl.C, blockIdx.y);
+    const int n0 = seg_row0(pl, 2 * rank);
+    t.N = seg_row0(pl, 2 * rank + 2) - n0;
+    t.base += (unsigned)n0 * t.sn;
+    if (DIR == 1) t.cj = n0;
+    else t.ck = n0;
+    return t;
+}
+
 // Point p of a tile: consecutive threads touch consecutive global addresses
 // (position-major for x-lines, line-major otherwise).  L is a power of two
 // (lgL its logarithm); division by the x-line length uses a precomputed
@@ -425,8 +438,9 @@ struct Pt {
 // tile's lines first (y and z tiles, whose lines are adjacent in memory, and
 // the FP64 x tiles: 8-byte elements give each line a 32- or 64-byte run per
 // warp, whole sectors, and the stores are then conflict-free at P = L).
+// segpad: elements between a line's full segments (cs3d_seg.cuh), else 0.
 template <int DIR, bool LF = (DIR != 0)>
-__device__ __forceinline__ Pt point(const Tile &t, int p, int L, int P, int lgL, FastDiv dv) {
+__device__ __forceinline__ Pt point(const Tile &t, int p, int L, int P, int lgL, FastDiv dv, int segpad = 0) {
     Pt q;
     if (!LF) {
         q.l = (int)((__umulhi((unsigned)p, dv.mul) + (unsigned)p) >> dv.sh);
@@ -437,15 +451,15 @@ __device__ __forceinline__ Pt point(const Tile &t, int p, int L, int P, int lgL,
     }
     q.ok = q.l < t.nlines && q.n < t.N;
     q.gi = q.ok ? t.base + (unsigned)q.l * t.sl + (unsigned)q.n * t.sn : t.base;
-    q.o = q.n * P + q.l;
+    q.o = q.n * P + q.l + (q.n >> 5) * segpad;
     return q;
 }
 
 template <int DIR>
 __device__ __forceinline__ void coords(const Tile &t, int l, int n, int &i, int &j, int &k) {
     if (DIR == 0) { i = n; j = t.cj + l; k = t.ck; }
-    else if (DIR == 1) { i = t.ci + l; j = n; k = t.ck; }
-    else { i = t.ci + l; j = t.cj; k = n; }
+    else if (DIR == 1) { i = t.ci + l; j = t.cj + n; k = t.ck; }
+    else { i = t.ci + l; j = t.cj; k = t.ck + n; }
 }
 
 // ---------------------------------------------------------------------
@@ -508,6 +522,21 @@ __device__ __forceinline__ Smem<T> smem_layout_at(unsigned char *base, int nbuf,
 }
 
 extern __shared__ __align__(16) unsigned char smem_raw[];
+
+// Elements of one array of a segmented tile.
+__host__ __device__ inline int seg_stride(int N, int P, int G, int pad) { return N * P + (G - 1) * pad; }
+
+// The same tile for the segmented solves: no line factors, the segments'
+// pads between the rows.
+__host__ __device__ inline int seg_pair_stride(int N, int P, int G, int pad) { return 2 * seg_stride(N, P, G, pad); }
+__device__ __forceinline__ SmemPair smem_pair_seg(int P, int N, const SegPlan &pl) {
+    SmemPair s;
+    s.P = P;
+    s.pstride = seg_pair_stride(N, P, pl.G, pl.pad);
+    s.fact = nullptr;
+    s.buf = reinterpret_cast<float *>(smem_raw);
+    return s;
+}
 
 __device__ __forceinline__ SmemPair smem_pair_at(unsigned char *base, int nbuf, int L, int P, int N) {
     SmemPair s;
@@ -673,6 +702,24 @@ __device__ __forceinline__ void run_sweep_solves(const SmemPair &sm, const Task 
                                                  int nlines, const LineOp<float> &op0, const LineOp<float> &op1,
                                                  int tid, int nthr, int skip) {
     run_sweep_tasks<H, PC>(sm, tasks, ntask, L, nlines, op0, op1, tid, nthr, skip);
+}
+
+// The segmented solves of a sweep tile: tasks 0..3 the 1st and 2nd derivative
+// of one field, the others the 1st derivatives of two (SINGLE: the last task
+// has one field).  A unit is a task's solves on the lines one warp holds.
+template <int SEG, bool FULL, int NT, bool SINGLE>
+__device__ __forceinline__ void run_seg_tasks(const SmemPair &sm, int P, int L, int N, const SegPlan &pl,
+                                              const SegOp &o1, const SegOp &o2, int tid, int nthr) {
+    const int lane0 = tid & ((1 << pl.lgLW) - 1), seg = (tid & 31) >> pl.lgLW;
+    const int groups = max(1, L >> pl.lgLW);
+    for (int u = tid >> 5; u < NT * groups; u += nthr >> 5) {
+        const int t = u / groups, l = ((u - t * groups) << pl.lgLW) + lane0;
+        const bool active = l < L;
+        const SegLane<float2> s = seg_lane<SEG, FULL>(pl, sm.pair(t) + (active ? l : 0), seg, N, P);
+        if (t < 4) seg_pair<SEG, FULL, 0>(s, P, o1, o2, pl, lane0, active);
+        else if (SINGLE && t == NT - 1) seg_pair<SEG, FULL, 2>(s, P, o1, o2, pl, lane0, active);
+        else seg_pair<SEG, FULL, 1>(s, P, o1, o2, pl, lane0, active);
+    }
 }
 
 // Phase-A stores of task t's inputs at offset o: put1 for a task whose two

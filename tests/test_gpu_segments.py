@@ -1,0 +1,47 @@
+"""The mixed form's segmented line solves (csrc/cs3d_seg.cuh) at the line
+lengths where their plan changes: the shortest and longest of each segment
+count, full and ragged segments, lines split over a cluster of blocks and
+lines in one block, and the lengths left to the Thomas solves (16, 87, 513)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# one block: 17..43, 65..87, 129..131; clusters: 44..64, 88..128, 132..512
+LENGTHS = [16, 17, 18, 31, 32, 33, 43, 44, 63, 64, 65, 77, 87, 88, 101, 127, 128, 129, 131, 132, 176, 191, 192, 193,
+           256, 257, 320, 511, 512, 513]
+
+# One RK4 step plus filter of a state of order one at CFL 0.5: each of the four
+# stages and the filter adds at most about four FP32 roundings (2^-24) of terms
+# (dt/h) * flux of order one, weighted by the operators' row sums (below 4).
+TOL = 5 * 4 * 4 * 2.0 ** -24
+
+
+def _noise(shape, seed):
+    rng = np.random.default_rng(seed)
+    one = np.ones(shape)
+    u = [0.2 * np.cos(rng.uniform(0, 6.28) + sum(2 * np.pi * rng.integers(0, 3) * np.arange(n).reshape(
+        [-1 if a == b else 1 for b in range(3)]) / n for a, n in enumerate(shape)))
+        + 0.02 * rng.standard_normal(shape) for _ in range(4)]
+    return one + 0.1 * u[3], one / 1.4 + 0.05 * u[0] ** 2, u[0], u[1], u[2]
+
+
+@pytest.mark.parametrize("N", LENGTHS)
+@pytest.mark.parametrize("d", [0, 1, 2])
+def test_mixed_step_tracks_fp64_at_plan_edges(gpu_pkg, N, d):
+    abi = gpu_pkg._abi
+    n = [12, 12, 12]
+    n[d] = N
+    n[(d + 1) % 3] = 19  # a tile that is not full
+    ic = _noise((n[2], n[1], n[0]), 100 * d + N)
+    out = []
+    for prec in (abi.FP64, abi.FP32_MIXED):
+        L = [6.283185307179586 * (1.0 - 1.0 / k) for k in n]
+        s = gpu_pkg.Solver(gpu_pkg.make_config(tuple(n), tuple(L), mu_ref=1e-3, CFL=0.5, precision=prec))
+        s.set_initial_conditions(*ic)
+        s.step()
+        s.sync()
+        out.append(s.conserved())
+        s.close()
+    scale = np.maximum(np.abs(out[0]).reshape(5, -1).max(1), 1.0).reshape(5, 1, 1, 1)
+    assert float((np.abs(out[1] - out[0]) / scale).max()) <= TOL
