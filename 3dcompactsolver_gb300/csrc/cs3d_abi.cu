@@ -286,13 +286,12 @@ int upload_op(const HostOp &h, DevOp<T> &d, cudaStream_t s) {
 // How a periodic line of N points is cut for the segmented FP32 solves
 // (cs3d_seg.cuh): the fewest register rows SEG * G that hold it with segments
 // at most kSegSlack rows shorter than SEG; SEG = 0 where none does (N below 17 or
-// above 512) or the line is not periodic.  pair: elements are float2 (the
-// sweeps' tiles), else floats.
-SegPlan seg_plan(int N, int periodic, bool pair) {
+// above 32 maxG).  pair: elements are float2 (the sweeps' tiles), else scalars.
+// step: between the compiled segment lengths 16 .. 32.
+SegPlan seg_plan(int N, bool pair, int maxG = 16, int step = 8) {
     SegPlan best{};
-    if (!periodic) return best;
-    for (int G = 2; G <= 16; G *= 2)
-        for (int SEG = 16; SEG <= 32; SEG += 8) {
+    for (int G = 2; G <= maxG; G *= 2)
+        for (int SEG = 16; SEG <= 32; SEG += step) {
             const int S = (N + G - 1) / G;
             if (S > SEG || S <= SEG - 8 || (best.SEG && SEG * G >= best.SEG * best.G)) continue;
             SegPlan p{};
@@ -336,23 +335,117 @@ SegPlan cluster_plan(int N, int periodic) {
 
 // The periodic operator in that form: left-hand side (a, 1, a) with
 // a = l / (1 + l^2).
-SegOp seg_op(const HostOp &h, const SegPlan &p) {
-    SegOp o{};
+// bits: below 2^-bits a carry is left out.
+template <typename R>
+SegOp<R> seg_op(const HostOp &h, const SegPlan &p, int bits) {
+    SegOp<R> o{};
     if (!p.SEG) return o;
     const double a = h.alo[h.N / 2];
     const double l = a == 0.0 ? 0.0 : (1.0 - std::sqrt(1.0 - 4.0 * a * a)) / (2.0 * a);
-    o.nl = (float)-l;
-    for (int k = 0; k <= kMaxH; k++) o.s[k] = (float)(h.taps[kMaxH + k] * h.scale * (1.0 + l * l));
-    for (int k = 0; k < 32; k++) o.pw[k] = (float)std::pow(-l, k + 1);
-    o.qS = (float)std::pow(-l, p.S);
-    o.qS1 = (float)std::pow(-l, p.S - 1);
-    o.iS = (float)std::pow(-l, -p.kS);
-    o.iS1 = (float)std::pow(-l, -(p.kS + 1));
+    o.nl = (R)-l;
+    for (int k = 0; k <= kMaxH; k++) o.s[k] = (R)(h.taps[kMaxH + k] * h.scale * (1.0 + l * l));
+    for (int k = 0; k < 32; k++) o.pw[k] = (R)std::pow(-l, k + 1);
+    o.qS = (R)std::pow(-l, p.S);
+    o.qS1 = (R)std::pow(-l, p.S - 1);
+    o.iS = (R)std::pow(-l, -p.kS);
+    o.iS1 = (R)std::pow(-l, -(p.kS + 1));
     const int smin = p.nS < p.G ? p.S - 1 : p.S;
     o.T = 1;
-    while (o.T < p.G && std::pow(std::fabs(l), (double)smin * o.T) > 9e-10) o.T++;
-    o.wrap = o.T == p.G ? (float)(1.0 / (1.0 - std::pow(-l, h.N))) : 1.0f;
+    while (o.T < p.G && std::pow(std::fabs(l), (double)smin * o.T) > std::ldexp(1.0, -bits)) o.T++;
+    o.wrap = o.T == p.G ? (R)(1.0 / (1.0 - std::pow(-l, h.N))) : R(1);
     return o;
+}
+
+// Whether the left-hand side (a, 1, a) factors with l < 1 (|alphaF| = 1/2
+// does not; the derivatives' a are 1/3 and 2/11).
+bool factors(const HostOp &h) { return std::fabs(h.alo[h.N / 2]) < 0.4999; }
+
+// The plain form's lines (cs3d_seg.cuh, one thread a line): the rows of a
+// line in blocks of a cluster along y and z, 64 at most where 8 blocks allow
+// it, 40 at least (0.382^40 = 2e-17: a carry reaches the next block alone);
+// along x the whole line in one block, in two halves from 80 rows on (its 13
+// solves of 4 lines fill 2 of 3 warps otherwise).
+SegPlan seq_plan(int N, int d) {
+    SegPlan p{};
+    p.SEG = kSeqSeg;
+    p.C = d == 0 ? 1 : std::min(8, (N + 63) / 64);
+    while (p.C > 1 && N / p.C < 40) p.C--;
+    p.G = d == 0 && N >= 80 ? 2 : p.C;
+    p.S = (N + p.G - 1) / p.G;
+    p.nS = N - p.G * (p.S - 1);
+    return p;
+}
+
+// bits: below 2^-bits a carry is left out; pw: the powers' device copy.
+SeqOp seq_op(const HostOp &h, const SegPlan &p, double **pw, cudaStream_t s, int *rc) {
+    SeqOp o{};
+    const SegOp<double> g = seg_op<double>(h, p, 56);
+    o.nl = g.nl;
+    o.s0 = g.s[0];
+    o.s1 = g.s[1];
+    o.s2 = g.s[2];
+    o.wrap = p.G == 1 ? 1.0 / (1.0 - std::pow(g.nl, h.N)) : 1.0;
+    while (std::pow(std::fabs(g.nl), o.K) > std::ldexp(1.0, -56)) o.K++;
+    std::vector<double> t(o.K);
+    for (int k = 0; k < o.K; k++) t[k] = std::pow(g.nl, k + 1);
+    *rc = CS3D_OK;
+    if (cudaMalloc(pw, o.K * 8) != cudaSuccess ||
+        cudaMemcpyAsync(*pw, t.data(), o.K * 8, cudaMemcpyHostToDevice, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess)
+        *rc = fail(CS3D_ERR_CUDA, "operator upload failed");
+    o.pw = *pw;
+    return o;
+}
+
+// One operator of contiguous FP64 lines in register segments: the launch
+// arguments but for the arrays, and a wall line's table in device memory.
+struct LineSeg {
+    LineSegArgs a{};  // a.seg.SEG = 0: not cut, the Thomas solve runs
+    double *mem = nullptr;
+};
+
+int make_line_seg(const HostOp &h, LineSeg &ls, cudaStream_t s) {
+    const int N = h.N;
+    LineSegArgs &a = ls.a;
+    if (!factors(h)) return CS3D_OK;
+    a.seg = seg_plan(N, false, 32, 4);
+    if (!a.seg.SEG) return CS3D_OK;
+    const SegPlan &p = a.seg;
+    a.N = N;
+    while ((1 << a.lgG) < p.G) a.lgG++;
+    a.wall = !h.periodic;
+    a.divN = make_fastdiv((unsigned)N);
+    a.divS = make_fastdiv((unsigned)p.S);
+    a.divS1 = make_fastdiv((unsigned)(p.S - 1));
+    a.op = seg_op<double>(h, p, 60);
+    if (!a.wall) return CS3D_OK;
+    for (int k = 0; k <= kMaxH; k++) a.op.s[k] = h.taps[kMaxH + k] * h.scale;  // (the table scales the rows)
+    for (int b = 0; b < 2 * kMaxH; b++) {
+        for (int k = 0; k < kTaps; k++) a.btaps[b][k] = h.btaps[b][k] * h.scale;
+        a.boff[b] = h.boff[b];
+    }
+    const size_t n = (size_t)p.G * p.SEG;
+    std::vector<double> t(5 * n, 0.0);
+    for (int sg = 0, row = 0; sg < p.G; sg++) {
+        const int len = p.S - (sg >= p.nS), k0 = p.SEG - len;
+        double *sc = &t[sg * p.SEG], *f = sc + n, *b = f + n, *pf = b + n, *pb = pf + n;
+        for (int k = k0; k < p.SEG; k++, row++) {
+            sc[k] = h.iw[row];
+            f[k] = row > 0 ? -h.alo[row] * h.iw[row] : 0.0;
+            b[k] = row < N - 1 ? -h.c[row] * h.iw[row] : 0.0;
+            pf[k] = f[k] * (k > k0 ? pf[k - 1] : 1.0);
+        }
+        for (int k = p.SEG - 1; k >= k0; k--) pb[k] = b[k] * (k < p.SEG - 1 ? pb[k + 1] : 1.0);
+    }
+    CS3D_CUDA(cudaMalloc(&ls.mem, t.size() * 8));
+    CS3D_CUDA(cudaMemcpyAsync(ls.mem, t.data(), t.size() * 8, cudaMemcpyHostToDevice, s));
+    CS3D_CUDA(cudaStreamSynchronize(s));
+    a.tab.s = ls.mem;
+    a.tab.f = ls.mem + n;
+    a.tab.b = ls.mem + 2 * n;
+    a.tab.pf = ls.mem + 3 * n;
+    a.tab.pb = ls.mem + 4 * n;
+    return CS3D_OK;
 }
 
 struct DeviceGuard {
@@ -409,11 +502,15 @@ struct cs3d_handle {
     // operators: [dir][kind-1]
     DevOp<double> op64[3][3];
     DevOp<float> op32[3][3];
+    LineSeg lseg[3][3];
     DevOp<float> op32fc[3];  // FP32 filter correction F - I (mixed form)
     SegPlan seg[3] = {};     // mixed form: the periodic directions' segmented solves
-    SegOp segop[3][2] = {};  // 1st and 2nd derivative
+    SegOp<float> segop[3][2] = {};  // 1st and 2nd derivative
     SegPlan segf[3] = {};    // the filter's, and its correction operator
-    SegOp segfop[3] = {};
+    SegOp<float> segfop[3] = {};
+    SeqOp seqop[3][2] = {};  // plain form: the sequential solves (plan in seg)
+    double *seqpw[3][2] = {};
+    SegOp<double> segfop64[3] = {};
     // tiles
     int L[3] = {1, 1, 1}, Lf[3] = {1, 1, 1}, threads[3] = {128, 128, 128};
     int Lt[3] = {1, 1, 1}, threads_t[3] = {128, 128, 128};  // the transposed sweeps of the mixed adjoint
@@ -715,16 +812,23 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
             HostOp ho = make_op(k, Nd[d], cfg->bc_type[d], dd[d], cfg->alphaF);
             int r = upload_op<double>(ho, h->op64[d][k - 1], h->stream);
             if (!r) r = upload_op<float>(ho, h->op32[d][k - 1], h->stream);
+            if (!r) r = make_line_seg(ho, h->lseg[d][k - 1], h->stream);
             if (!r && k == 3) r = upload_op<float>(make_filter_correction(ho), h->op32fc[d], h->stream);
             if (r) return fail_free(r);
-            if (h->mixed && k < 3) {
+            if (!h->mixed && ho.periodic && k < 3) {
+                h->seg[d] = seq_plan(Nd[d], d);
+                h->seqop[d][k - 1] = seq_op(ho, h->seg[d], &h->seqpw[d][k - 1], h->stream, &r);
+                if (r) return fail_free(r);
+            } else if (!h->mixed && ho.periodic && factors(ho)) {
+                h->segf[d] = seg_plan(Nd[d], true);
+                h->segfop64[d] = seg_op<double>(ho, h->segf[d], 60);
+            } else if (h->mixed && k < 3) {
                 h->seg[d] = d > 0 ? cluster_plan(Nd[d], ho.periodic) : SegPlan{};
-                if (!h->seg[d].C) h->seg[d] = seg_plan(Nd[d], ho.periodic, d > 0);
-                h->segop[d][k - 1] = seg_op(ho, h->seg[d]);
-            } else if (h->mixed && std::fabs(cfg->alphaF) < 0.4999) {
-                // (|alphaF| = 1/2 has no factorisation with l < 1)
-                h->segf[d] = seg_plan(Nd[d], ho.periodic, false);
-                h->segfop[d] = seg_op(make_filter_correction(ho), h->segf[d]);
+                if (ho.periodic && !h->seg[d].C) h->seg[d] = seg_plan(Nd[d], d > 0);
+                h->segop[d][k - 1] = seg_op<float>(ho, h->seg[d], 30);
+            } else if (h->mixed && ho.periodic && factors(ho)) {
+                h->segf[d] = seg_plan(Nd[d], false);
+                h->segfop[d] = seg_op<float>(make_filter_correction(ho), h->segf[d], 30);
             }
         }
     for (int d = 0; d < 3; d++) {
@@ -752,7 +856,15 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
         };
         shape(nullptr, h->Lt[d], h->threads_t[d]);
         shape(&h->seg[d], h->L[d], h->threads[d]);
-        if (h->seg[d].C) {
+        const int other = d == 0 ? cfg->Ny : cfg->Nx, planes = d == 2 ? cfg->Ny : cfg->Nz;
+        if (!h->mixed && h->seg[d].SEG) {
+            // y and z: 8 lines (64-byte rows, a warp's solves of one kind), 3
+            // blocks an SM at 64 rows; fewer lines where the grid would leave
+            // SMs without a block (16^3: 2 lines, 128 blocks a launch)
+            int &L = h->L[d];
+            if (d > 0) L = std::min(8, pick_L(8, nb, Nd[d], 0, 84, true, &h->seg[d]));
+            while (L > 2 && (long long)h->seg[d].C * ((other + L - 1) / L) * planes < 152) L /= 2;
+        } else if (h->seg[d].C) {
             h->L[d] = kClusterLines;
             h->threads[d] = kTpbYZ;
         }
@@ -763,10 +875,10 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
         // N = 128 the 8-line tile stays (16 lines measured slower)
         if (h->mixed && h->Lf[d] < 8) h->Lf[d] = pick_L(h->tb, 10, Nd[d], d == 0 ? 1 : 0, 110);
         if (h->segf[d].SEG) {
-            // 32 lines a tile, 128-byte rows, where a block of them fits; half
-            // of that along x, whose lines are contiguous
-            int L = d == 0 ? 16 : 32;
-            while (L > 1 && filter_seg_smem(L, L + (d == 0), Nd[d], h->segf[d]) > 200 * 1024) L /= 2;
+            // 128-byte rows where a block of them fits; half of that along x,
+            // whose lines are contiguous
+            int L = h->mixed ? (d == 0 ? 16 : 32) : (d == 0 ? 8 : 16);
+            while (L > 1 && filter_seg_smem((int)h->tb, L, L + (d == 0), Nd[d], h->segf[d]) > 200 * 1024) L /= 2;
             h->Lf[d] = L;
         }
         if (sweep_smem_bytes((int)h->tb, nb, 1, 2, Nd[d]) > 200 * 1024)
@@ -788,6 +900,8 @@ extern "C" int cs3d_destroy(cs3d_handle *h) {
         for (int k = 0; k < 3; k++) {
             if (h->op64[d][k].mem) cudaFree(h->op64[d][k].mem);
             if (h->op32[d][k].mem) cudaFree(h->op32[d][k].mem);
+            if (h->lseg[d][k].mem) cudaFree(h->lseg[d][k].mem);
+            if (k < 2 && h->seqpw[d][k]) cudaFree(h->seqpw[d][k]);
         }
     for (int d = 0; d < 3; d++)
         if (h->op32fc[d].mem) cudaFree(h->op32fc[d].mem);
@@ -1019,6 +1133,8 @@ static int run_stage(cs3d_handle *h, int st, int last) {
         a.seg = h->seg[d];
         a.g1 = h->segop[d][0];
         a.g2 = h->segop[d][1];
+        a.h1 = h->seqop[d][0];
+        a.h2 = h->seqop[d][1];
         if (sizeof(T) == 8) {
             a.d1 = *reinterpret_cast<const LineOp<T> *>(&h->op64[d][0].op);
             a.d2 = *reinterpret_cast<const LineOp<T> *>(&h->op64[d][1].op);
@@ -1048,8 +1164,9 @@ static int run_stage(cs3d_handle *h, int st, int last) {
                 fa.divN = make_fastdiv((unsigned)(d == 0 ? h->g.Nx : d == 1 ? h->g.Ny : h->g.Nz));
                 fa.P = h->Lf[d] + (d == 0 ? 1 : 0);
                 fa.seg = h->segf[d];
-                fa.sg = h->segfop[d];
-                fa.threads = fa.seg.SEG ? kFilterSegTpb : sizeof(T) == 4 ? filter_threads<float>() : filter_threads<double>();
+                if constexpr (sizeof(T) == 4) fa.sg = h->segfop[d];
+                else fa.sg = h->segfop64[d];
+                fa.threads = fa.seg.SEG ? (sizeof(T) == 4 ? kFilterSegTpb : kFilterSegTpb64) : sizeof(T) == 4 ? filter_threads<float>() : filter_threads<double>();
                 if (sizeof(T) == 8) fa.op = *reinterpret_cast<const LineOp<T> *>(&h->op64[d][2].op);
                 else fa.op = *reinterpret_cast<const LineOp<T> *>(&h->op32fc[d].op);
                 void **src = pass == 1 ? h->ft1 : h->ft2;
@@ -1344,24 +1461,39 @@ extern "C" int cs3d_kernel_times(cs3d_handle *h, double *ms, long long *count, i
 // ---------------------------------------------------------------------
 // single operators
 // ---------------------------------------------------------------------
+// The operator on every line of npts points: in register segments where the
+// line is cut, else one Thomas solve a thread.
+static int line_op_on(const LineOp<double> &op, const LineSegArgs &seg, int kind, long long npts, const double *in,
+                      double *out, cudaStream_t s) {
+    if (seg.seg.SEG) {
+        LineSegArgs a = seg;
+        a.nlines = npts / op.N;
+        a.in = in;
+        a.out = out;
+        CS3D_CUDA(launch_line_seg(kind, a, s));
+        return CS3D_OK;
+    }
+    LineOpArgs a{};
+    a.op = op;
+    a.nlines = npts / op.N;
+    a.L = 32;
+    while (a.L > 1 && planar_smem_bytes(8, 1, a.L, a.L + 1, op.N) > 72 * 1024) a.L /= 2;
+    a.P = a.L + 1;
+    a.threads = 128;
+    a.in = in;
+    a.out = out;
+    CS3D_CUDA(launch_line_op(a, s));
+    return CS3D_OK;
+}
+
 static int line_op(cs3d_handle *h, int kind, int dir, const double *in, double *out) {
     if (!h || !in || !out) return fail(CS3D_ERR_ARG, "null argument");
     if (dir < 0 || dir > 2) return fail(CS3D_ERR_ARG, "dir=%d", dir);
     if (in == out) return fail(CS3D_ERR_ARG, "in and out must not overlap");
     DeviceGuard dg(h->dev);
-    LineOpArgs a{};
-    a.op = h->op64[dir][kind - 1].op;
-    const int N = a.op.N;
-    a.nlines = h->g.npts / N;
-    a.L = 32;
-    while (a.L > 1 && planar_smem_bytes(8, 1, a.L, a.L + 1, N) > 72 * 1024) a.L /= 2;
-    a.P = a.L + 1;
-    a.threads = 128;
-    a.in = in;
-    a.out = out;
-    CS3D_CUDA(launch_line_op(a, h->stream));
-    h->launches++;
-    return CS3D_OK;
+    const int rc = line_op_on(h->op64[dir][kind - 1].op, h->lseg[dir][kind - 1].a, kind, h->g.npts, in, out, h->stream);
+    if (!rc) h->launches++;
+    return rc;
 }
 
 extern "C" int cs3d_deriv1(cs3d_handle *h, int dir, const double *in_dev, double *out_dev) {
@@ -1382,6 +1514,7 @@ struct cs3d_op {
     cudaStream_t stream = nullptr;
     long long npts = 0;
     DevOp<double> ops[3];
+    LineSeg seg[3];
     double *stage = nullptr;  // 2 * npts doubles for the host-array calls (allocated on first use)
 };
 
@@ -1416,7 +1549,9 @@ extern "C" int cs3d_op_create(const cs3d_config *cfg, int dir, cs3d_op **out) {
     // Domain.hpp:31-45: dx = x[1] - x[0]
     const double dh = (1.0 / ((double)Nd[dir] - 1.0)) * Ld[dir] - 0.0;
     for (int k = 1; k <= 3; k++) {
-        int r = upload_op<double>(make_op(k, Nd[dir], bc, dh, cfg->alphaF), o->ops[k - 1], o->stream);
+        const HostOp ho = make_op(k, Nd[dir], bc, dh, cfg->alphaF);
+        int r = upload_op<double>(ho, o->ops[k - 1], o->stream);
+        if (!r) r = make_line_seg(ho, o->seg[k - 1], o->stream);
         if (r) return fail_free(r);
     }
     if (cudaStreamSynchronize(o->stream) != cudaSuccess)
@@ -1431,6 +1566,8 @@ extern "C" int cs3d_op_destroy(cs3d_op *o) {
     if (o->stream) cudaStreamSynchronize(o->stream);
     for (auto &d : o->ops)
         if (d.mem) cudaFree(d.mem);
+    for (auto &d : o->seg)
+        if (d.mem) cudaFree(d.mem);
     if (o->stage) cudaFree(o->stage);
     if (o->stream) cudaStreamDestroy(o->stream);
     delete o;
@@ -1438,18 +1575,7 @@ extern "C" int cs3d_op_destroy(cs3d_op *o) {
 }
 
 static int op_launch(cs3d_op *o, int kind, const double *in, double *out) {
-    LineOpArgs a{};
-    a.op = o->ops[kind - 1].op;
-    const int N = a.op.N;
-    a.nlines = o->npts / N;
-    a.L = 32;
-    while (a.L > 1 && planar_smem_bytes(8, 1, a.L, a.L + 1, N) > 72 * 1024) a.L /= 2;
-    a.P = a.L + 1;
-    a.threads = 128;
-    a.in = in;
-    a.out = out;
-    CS3D_CUDA(launch_line_op(a, o->stream));
-    return CS3D_OK;
+    return line_op_on(o->ops[kind - 1].op, o->seg[kind - 1].a, kind, o->npts, in, out, o->stream);
 }
 
 extern "C" int cs3d_op_apply(cs3d_op *o, int kind, const double *in_dev, double *out_dev) {

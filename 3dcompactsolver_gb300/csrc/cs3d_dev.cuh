@@ -47,6 +47,8 @@ struct LineOp {
     int periodic;
 };
 
+constexpr int kSeqSeg = 64;  // SegPlan::SEG of the plain form's sequential solves
+
 // How a periodic line is cut into register segments (cs3d_seg.cuh): G
 // segments (a power of two, one lane each), the first nS of S rows and the
 // others of S - 1, walked by a kernel compiled for SEG rows a segment.
@@ -64,11 +66,12 @@ struct SegPlan {
 
 // A periodic operator in that form: -l, the scaled taps (centre outwards),
 // the powers (-l)^(k+1), and what weights the carries between segments.
+template <typename R>
 struct SegOp {
-    float nl, s[kMaxH + 1], pw[32];
-    float qS, qS1;  // (-l)^S, (-l)^(S-1)
-    float iS, iS1;  // (-l)^-kS, (-l)^-(kS+1)
-    float wrap;     // 1, or 1 / (1 - (-l)^N) where T = G
+    R nl, s[kMaxH + 1], pw[32];
+    R qS, qS1;  // (-l)^S, (-l)^(S-1)
+    R iS, iS1;  // (-l)^-kS, (-l)^-(kS+1)
+    R wrap;     // 1, or 1 / (1 - (-l)^N) where T = G
     int T;
 };
 

@@ -1,12 +1,14 @@
 // cs3d_kernels.cuh -- kernel argument blocks and launch functions.
 #pragma once
 #include "cs3d_dev.cuh"
+#include "cs3d_seg.cuh"
 
 namespace cs3d {
 
 constexpr int kTpbX = 256;   // threads per block of the mixed-form x sweep
 constexpr int kTpbYZ = 512;  // most threads per block of the mixed-form y and z sweeps
-constexpr int kFilterSegTpb = 320;  // threads per block of the segmented mixed filter
+// threads per block of the segmented filter
+constexpr int kFilterSegTpb = 320, kFilterSegTpb64 = 160;
 constexpr int kClusterLines = 32;  // lines of a tile whose lines are split over a cluster
 constexpr int kFilterTpb = 256;  // threads per block of the mixed-form filter
 
@@ -45,7 +47,8 @@ struct SweepArgs {
     int threads;    // threads per block
     LineOp<T> d1, d2;
     SegPlan seg;    // mixed form, periodic lines (seg.SEG > 0): the segmented
-    SegOp g1, g2;   // solves' plan and operators
+    SegOp<float> g1, g2;  // solves' plan and operators; plain form: the
+    SeqOp h1, h2;   // sequential solves' (seg: G = C blocks' rows of a line)
     GasParams gas;
     const T *qs[5]; // stage input q* in the work precision (FP64 q* itself, or
                     // its FP32 shadow in the mixed form)
@@ -87,8 +90,8 @@ struct FilterArgs {
     int L, lgL, P, threads;
     FastDiv divN;
     LineOp<T> op;
-    SegPlan seg;       // mixed form, periodic lines: the segmented solves' plan
-    SegOp sg;          // and operator (SEG = 0: op's Thomas factors)
+    SegPlan seg;       // periodic lines: the segmented solves' plan and
+    SegOp<T> sg;       // operator (SEG = 0: op's Thomas factors)
     Q5 src64;          // FP64 source (or null pointers)
     T *src32[5];       // work-precision source
     Q5 dst64;          // FP64 destination (or null pointers)
@@ -103,6 +106,27 @@ struct LineOpArgs {
     int L, P, threads;
     long long nlines;
     LineOp<double> op;
+    const double *in;
+    double *out;
+};
+
+// Factors of a line with wall closures in the segments' register rows
+// (seg * SEG + k, zero in unused ones): y_n = s_n r_n + f_n y_{n-1},
+// x_n = y_n + b_n x_{n+1}; pf and pb their running products from the segment's
+// first and last row.
+struct SegTab {
+    const double *s, *f, *b, *pf, *pb;
+};
+// One operator on contiguous lines in register segments (cs3d_lineop.cu).
+struct LineSegArgs {
+    int N, lgG, wall;
+    long long nlines;
+    FastDiv divN, divS, divS1;  // by N, S, S - 1
+    SegPlan seg;
+    SegOp<double> op;
+    SegTab tab;
+    double btaps[2 * kMaxH][kTaps];
+    int boff[2 * kMaxH];
     const double *in;
     double *out;
 };
@@ -187,6 +211,7 @@ cudaError_t launch_sweep(int dir, const SweepArgs<T> &a, cudaStream_t s);
 template <typename T>
 cudaError_t launch_filter(int dir, const FilterArgs<T> &a, cudaStream_t s);
 cudaError_t launch_line_op(const LineOpArgs &a, cudaStream_t s);
+cudaError_t launch_line_seg(int kind, const LineSegArgs &a, cudaStream_t s);
 template <typename T>
 cudaError_t launch_tgv(const TgvArgs<T> &a, int blocks, cudaStream_t s);
 // calcTurbulenceQuantities / shearLayerInfoCalc sums over q1 and the
@@ -365,7 +390,7 @@ cudaError_t launch_ke_seed(const KeSeedArgs &a, cudaStream_t s);
 // a planar tile (filter, single operators, adjoint operators)
 size_t sweep_smem_bytes(int prec_bytes, int nbuf, int L, int P, int N, const SegPlan *seg = nullptr);
 size_t planar_smem_bytes(int prec_bytes, int nbuf, int L, int P, int N);
-size_t filter_seg_smem(int L, int P, int N, const SegPlan &p);
+size_t filter_seg_smem(int prec_bytes, int L, int P, int N, const SegPlan &p);
 int sweep_nbuf(int dir, int prec_bytes);
 int sweep_ntask(int dir);
 int filter_ntask();

@@ -1,0 +1,184 @@
+// cs3d_lineop.cu -- one compact operator on contiguous FP64 lines
+// (Derivatives::calc1stDerivField, calc2ndDerivField, Filter::filterField) in
+// register segments (sm_103a).
+//
+// A warp owns 32 / G whole lines, G segments each, one segment a lane: it
+// copies its lines (one contiguous range of memory) to its own shared memory,
+// every lane solves its segment in registers (cs3d_seg.cuh), and the warp copies
+// the result out.  Nothing is shared between warps, so loads, solves and
+// stores of different warps overlap without block barriers.  Segments are
+// SEG + 1 doubles apart: 32 lanes at the same row touch all banks.
+//
+// What bounds it: FP64 issue (two operations an SM and clock).  The kernel it
+// replaces on these lengths (k_line_op: one thread a line, a quarter of the
+// block's threads) left that pipe idle most of the time: 128^3, three operators,
+// 235 us; walls of 301 points (3850 lines), 161 us.
+#include "cs3d_seg.cuh"
+#include "cs3d_kernels.cuh"
+
+namespace cs3d {
+
+constexpr int kLineSegTpb = 128;
+
+extern __shared__ __align__(16) unsigned char smem_line[];
+
+// The solve of a line with wall closures: the factors vary along the line, so
+// each row's come from a table (SegTab), walked like the registers.
+template <int SEG>
+__device__ __forceinline__ void seg_solve_tab(double (&y)[SEG], const SegTab &tb, int T, int G, int seg, int k0,
+                                              int lane0) {
+    const double *f = tb.f + seg * SEG, *b = tb.b + seg * SEG, *pf = tb.pf + seg * SEG, *pb = tb.pb + seg * SEG;
+    double c = 0.0;
+#pragma unroll
+    for (int k = 0; k < SEG; ++k) y[k] = c = fma(ldc(f + k), c, y[k]);
+    double in = 0.0, q = ldc(pf + SEG - 1);
+    for (int t = T; t >= 1; --t) {
+        const int src = max(seg - t, 0);
+        const double es = __shfl_sync(0xffffffffu, c, lane0 + src), qs = __shfl_sync(0xffffffffu, q, lane0 + src);
+        in = seg - t >= 0 ? fma(qs, in, es) : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < SEG; ++k) y[k] = fma(ldc(pf + k), in, y[k]);
+    c = 0.0;
+    double first = 0.0;
+#pragma unroll
+    for (int k = SEG - 1; k >= 0; --k) {
+        y[k] = c = fma(ldc(b + k), c, y[k]);
+        if (k <= kSegSlack) first = k == k0 ? c : first;
+    }
+    in = 0.0;
+    q = ldc(pb + k0);
+    for (int t = T; t >= 1; --t) {
+        const int src = min(seg + t, G - 1);
+        const double es = __shfl_sync(0xffffffffu, first, lane0 + src), qs = __shfl_sync(0xffffffffu, q, lane0 + src);
+        in = seg + t < G ? fma(qs, in, es) : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < SEG; ++k) y[k] = fma(ldc(pb + k), in, y[k]);
+}
+
+// KIND 1, 2: derivatives, 3: filter.  WALL: closures from op's explicit rows
+// and factors from a.tab; else periodic.
+template <int KIND, int SEG, bool FULL, bool WALL>
+__global__ void __launch_bounds__(kLineSegTpb, WALL && SEG > 24 ? 3 : 4) k_line_seg(LineSegArgs a) {
+    constexpr int H = KIND == 3 ? 4 : 2, LS = SEG + 1;
+    const int N = a.N, G = a.seg.G, lane = threadIdx.x & 31, lw = 32 >> a.lgG;
+    const long long l0 = ((long long)blockIdx.x * (kLineSegTpb / 32) + (threadIdx.x >> 5)) * lw;
+    if (l0 >= a.nlines) return;  // (whole warps)
+    const int total = (int)min((long long)lw, a.nlines - l0) * N;
+    double *sm = reinterpret_cast<double *>(smem_line) + (threadIdx.x >> 5) * 32 * LS;
+    const int nb = a.seg.nS * a.seg.S;
+    // shared-memory offset of the warp's element idx
+    auto place = [&](int idx) {
+        const int l = (int)((__umulhi((unsigned)idx, a.divN.mul) + (unsigned)idx) >> a.divN.sh), n = idx - l * N;
+        int seg, k;
+        if (FULL) {
+            seg = n / SEG;
+            k = n % SEG;
+        } else {
+            const bool lng = n < nb;
+            const FastDiv d = lng ? a.divS : a.divS1;
+            const int m = lng ? n : n - nb, s = (int)((__umulhi((unsigned)m, d.mul) + (unsigned)m) >> d.sh);
+            seg = lng ? s : s + a.seg.nS;
+            k = m - s * (lng ? a.seg.S : a.seg.S - 1);
+        }
+        return ((l << a.lgG) + seg) * LS + k;
+    };
+    const double *in = a.in + l0 * N;
+    for (int i0 = lane; i0 < total; i0 += 8 * 32) {
+        double v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = i0 + 32 * u < total ? in[i0 + 32 * u] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (i0 + 32 * u < total) sm[place(i0 + 32 * u)] = v[u];
+    }
+    __syncwarp();
+    const int seg = lane & (G - 1), lane0 = lane & ~(G - 1);
+    const int len = a.seg.S - (seg >= a.seg.nS), k0 = SEG - len;
+    const int sp = (seg - 1) & (G - 1), sn = (seg + 1) & (G - 1);
+    SegLane<double> s;
+    s.seg = seg;
+    s.k0 = k0;
+    s.row = sm + lane * LS - k0;
+    s.lo = sm + (lane0 + sp) * LS + a.seg.S - (sp >= a.seg.nS) - k0;
+    s.hi = sm + (lane0 + sn) * LS;
+    double y[SEG];
+    {
+        double w[SEG + 2 * H];
+        seg_load<SEG, FULL, H>(w, s, 1, [](const double *p) { return *p; });
+#pragma unroll
+        for (int k = 0; k < SEG; ++k) {
+            if constexpr (KIND == 1) y[k] = seg_r1<SEG>(w, a.op, k);
+            if constexpr (KIND == 2) y[k] = seg_r2<SEG>(w, a.op, k);
+            if constexpr (KIND == 3) y[k] = seg_r3<SEG>(w, a.op, k);
+            if (!FULL && k < kSegSlack && k < k0) y[k] = 0.0;
+        }
+    }
+    if constexpr (WALL) {
+        // the first and last H rows, from their explicit coefficients
+        const bool top = seg == 0, end = seg == G - 1;
+        if (top || end) {
+            const double *line0 = sm + lane0 * LS;
+#pragma unroll
+            for (int b = 0; b < H; ++b) {
+                const int r = top ? b : H + b;
+                double v = 0.0;
+                for (int k = 0; k < kTaps; ++k) {
+                    const int n = a.boff[r] + k;
+                    if (n >= N) break;
+                    const int sg = n < nb ? n / a.seg.S : a.seg.nS + (n - nb) / (a.seg.S - 1);
+                    v = fma(a.btaps[r][k], line0[sg * LS + n - seg_row0(a.seg, sg)], v);
+                }
+                if (end) y[SEG - H + b] = v;
+                if (top) {
+#pragma unroll
+                    for (int k = 0; k < kSegSlack + H; ++k)
+                        if (k == k0 + b) y[k] = v;
+                }
+            }
+        }
+        const double *sc = a.tab.s + seg * SEG;
+#pragma unroll
+        for (int k = 0; k < SEG; ++k) y[k] *= ldc(sc + k);
+        seg_solve_tab<SEG>(y, a.tab, a.op.T, G, seg, k0, lane0);
+    } else {
+        // 64 bits: the second derivative's powers fall below 1e-17 in 24 rows
+        seg_solve<SEG, FULL, (KIND == 2 ? 24 : SEG)>(y, a.op, a.seg, seg, k0, lane0, 0);
+    }
+    __syncwarp();  // every lane has read its window
+    seg_store<SEG, FULL>(s, 1, [&](double *p, int k) { *p = y[k]; });
+    __syncwarp();
+    double *out = a.out + l0 * N;
+#pragma unroll 8
+    for (int i = lane; i < total; i += 32) out[i] = sm[place(i)];
+}
+
+template <int KIND, int SEG, bool FULL, bool WALL>
+static cudaError_t launch(const LineSegArgs &a, cudaStream_t s) {
+    const size_t sm = (size_t)kLineSegTpb * (SEG + 1) * 8;
+    const long long per = (kLineSegTpb / 32) * (32 >> a.lgG);
+    k_line_seg<KIND, SEG, FULL, WALL><<<(unsigned)((a.nlines + per - 1) / per), kLineSegTpb, sm, s>>>(a);
+    return cudaGetLastError();
+}
+template <int KIND>
+static cudaError_t launch_kind(const LineSegArgs &a, cudaStream_t s) {
+    if (a.wall) {
+        if (a.seg.SEG == 32) return launch<KIND, 32, false, true>(a, s);
+        if (a.seg.SEG == 28) return launch<KIND, 28, false, true>(a, s);
+        if (a.seg.SEG == 24) return launch<KIND, 24, false, true>(a, s);
+        if (a.seg.SEG == 20) return launch<KIND, 20, false, true>(a, s);
+        return launch<KIND, 16, false, true>(a, s);
+    }
+    if (a.seg.full) return launch<KIND, 32, true, false>(a, s);
+    if (a.seg.SEG == 32) return launch<KIND, 32, false, false>(a, s);
+    if (a.seg.SEG == 28) return launch<KIND, 28, false, false>(a, s);
+    if (a.seg.SEG == 24) return launch<KIND, 24, false, false>(a, s);
+    if (a.seg.SEG == 20) return launch<KIND, 20, false, false>(a, s);
+    return launch<KIND, 16, false, false>(a, s);
+}
+cudaError_t launch_line_seg(int kind, const LineSegArgs &a, cudaStream_t s) {
+    return kind == 1 ? launch_kind<1>(a, s) : kind == 2 ? launch_kind<2>(a, s) : launch_kind<3>(a, s);
+}
+
+}  // namespace cs3d

@@ -1,5 +1,5 @@
-// cs3d_seg.cuh -- compact line solves of periodic lines in register segments
-// (FP32), shared by the stage sweeps, the filter and the adjoint kernels.
+// cs3d_seg.cuh -- compact line solves of periodic lines in register segments,
+// shared by the stage sweeps, the filter and the adjoint kernels.
 //
 // On a periodic line the compact operators' left-hand side is the circulant
 // tridiagonal (a, 1, a), which factors exactly into two first-order
@@ -33,8 +33,8 @@
 
 namespace cs3d {
 
-// Rows at the start of a segment whose carry is added: (-l)^(k+1) falls below
-// 5e-9 after these many rows.  The first derivative has l = 0.382, the second
+// FP32: rows at the start of a segment whose carry is added: (-l)^(k+1) falls
+// below 5e-9 after these many rows.  The first derivative has l = 0.382, the second
 // 0.188; the filter's l depends on its coefficient (all rows).
 constexpr int kSegRows1 = 20, kSegRows2 = 12, kSegRowsAll = 64;
 // Segments are at most kSegSlack rows shorter than the compiled length (seg_plan keeps
@@ -50,8 +50,9 @@ struct SegLane {
     E *row, *lo, *hi;
 };
 
-// First row of segment s.
+// First row of segment s, and the rows of segment s (-1: the last).
 __device__ __forceinline__ int seg_row0(const SegPlan &pl, int s) { return s * pl.S - max(0, s - pl.nS); }
+__device__ __forceinline__ int seg_rows(const SegPlan &pl, int s) { return pl.S - ((s < 0 ? pl.G - 1 : s) >= pl.nS); }
 
 // The lane of a line that lies whole in this block's tile (line at base, rows
 // P elements apart, pl.pad more after every full segment).
@@ -96,68 +97,81 @@ __device__ __forceinline__ void seg_load(W (&w)[SEG + 2 * H], const SegLane<E> &
 
 // Right-hand sides from a window (taps scaled by 1/h, 1/h^2 and 1 + l^2): the
 // differences first, so that their products round relative to the differences.
-template <int SEG>
-__device__ __forceinline__ float seg_r1(const float (&w)[SEG + 4], const SegOp &o, int k) {
-    return fmaf(o.s[1], w[k + 3] - w[k + 1], o.s[2] * (w[k + 4] - w[k]));
+template <int SEG, typename R>
+__device__ __forceinline__ R seg_r1(const R (&w)[SEG + 4], const SegOp<R> &o, int k) {
+    return fma(o.s[1], w[k + 3] - w[k + 1], o.s[2] * (w[k + 4] - w[k]));
 }
+template <int SEG, typename R>
+__device__ __forceinline__ R seg_r2(const R (&w)[SEG + 4], const SegOp<R> &o, int k) {
+    return fma(o.s[1], (w[k + 3] - w[k + 2]) - (w[k + 2] - w[k + 1]),
+               o.s[2] * ((w[k + 4] - w[k + 2]) - (w[k + 2] - w[k])));
+}
+// 64 bits: the plain sum, one operation less on the FP64 pipe.
 template <int SEG>
-__device__ __forceinline__ float seg_r2(const float (&w)[SEG + 4], const SegOp &o, int k) {
-    return fmaf(o.s[1], (w[k + 3] - w[k + 2]) - (w[k + 2] - w[k + 1]),
-                o.s[2] * ((w[k + 4] - w[k + 2]) - (w[k + 2] - w[k])));
+__device__ __forceinline__ double seg_r2(const double (&w)[SEG + 4], const SegOp<double> &o, int k) {
+    return fma(o.s[2], w[k + 4] + w[k], fma(o.s[1], w[k + 3] + w[k + 1], o.s[0] * w[k + 2]));
+}
+template <int SEG, typename R>
+__device__ __forceinline__ R seg_r3(const R (&w)[SEG + 8], const SegOp<R> &o, int k) {
+    R r = o.s[0] * w[k + 4];
+#pragma unroll
+    for (int h = 1; h <= 4; ++h) r = fma(o.s[h], w[k + 4 - h] + w[k + 4 + h], r);
+    return r;
 }
 
 // y: right-hand sides (zero in rows before k0).  Forward from zero: the
 // segment's end value.
-template <int SEG>
-__device__ __forceinline__ float seg_fwd(float (&y)[SEG], const SegOp &o) {
-    float c = y[0];
+template <int SEG, typename R>
+__device__ __forceinline__ R seg_fwd(R (&y)[SEG], const SegOp<R> &o) {
+    R c = y[0];
 #pragma unroll
-    for (int k = 1; k < SEG; ++k) y[k] = c = fmaf(o.nl, c, y[k]);
+    for (int k = 1; k < SEG; ++k) y[k] = c = fma(o.nl, c, y[k]);
     return c;
 }
 // Add the value entering the segment (KU: rows that take it), then backward
 // from zero: the value at the segment's first row.
-template <int SEG, bool FULL, int KU>
-__device__ __forceinline__ float seg_bwd(float (&y)[SEG], const SegOp &o, const SegPlan &pl, int k0, float in) {
+template <int SEG, bool FULL, int KU, typename R>
+__device__ __forceinline__ R seg_bwd(R (&y)[SEG], const SegOp<R> &o, const SegPlan &pl, int k0, R in) {
     constexpr int KF = KU + (FULL ? 0 : kSegSlack) < SEG ? KU + (FULL ? 0 : kSegSlack) : SEG;
     if constexpr (!FULL) in *= k0 == pl.kS ? o.iS : o.iS1;  // the powers count from row k0
 #pragma unroll
-    for (int k = 0; k < KF; ++k) y[k] = fmaf(o.pw[k], in, y[k]);
-    float c = y[SEG - 1], b = c;
+    for (int k = 0; k < KF; ++k) y[k] = fma(o.pw[k], in, y[k]);
+    R c = y[SEG - 1], b = c;
 #pragma unroll
     for (int k = SEG - 2; k >= 0; --k) {
-        y[k] = c = fmaf(o.nl, c, y[k]);
+        y[k] = c = fma(o.nl, c, y[k]);
         if (!FULL && k <= kSegSlack) b = k == k0 ? c : b;
     }
     return FULL ? c : b;
 }
 // Add the value at the next segment's first row.
-template <int SEG, int KU>
-__device__ __forceinline__ void seg_end(float (&y)[SEG], const SegOp &o, float in) {
+template <int SEG, int KU, typename R>
+__device__ __forceinline__ void seg_end(R (&y)[SEG], const SegOp<R> &o, R in) {
 #pragma unroll
-    for (int k = 0; k < (KU < SEG ? KU : SEG); ++k) y[SEG - 1 - k] = fmaf(o.pw[k], in, y[SEG - 1 - k]);
+    for (int k = 0; k < (KU < SEG ? KU : SEG); ++k) y[SEG - 1 - k] = fma(o.pw[k], in, y[SEG - 1 - k]);
 }
 
 // What enters this lane's segment: e of the DIR-side neighbours (DIR = -1:
-// segments before, +1: after), weighted.  lane0: the line's first lane.
-template <int DIR>
-__device__ __forceinline__ float seg_carry(float e, const SegOp &o, const SegPlan &pl, int seg, int lane0) {
-    float c = 0.f;
+// segments before, +1: after), weighted.  lane0: the line's first lane, its
+// segments 2^lgst lanes apart.
+template <int DIR, typename R>
+__device__ __forceinline__ R seg_carry(R e, const SegOp<R> &o, const SegPlan &pl, int seg, int lane0, int lgst) {
+    R c = R(0);
     for (int t = o.T; t >= 1; --t) {
         const int src = (seg + DIR * t) & (pl.G - 1);
-        const float es = __shfl_sync(0xffffffffu, e, lane0 + (src << pl.lgLW));
-        c = fmaf(src < pl.nS ? o.qS : o.qS1, c, es);
+        const R es = __shfl_sync(0xffffffffu, e, lane0 + (src << lgst));
+        c = fma(src < pl.nS ? o.qS : o.qS1, c, es);
     }
     return c * o.wrap;
 }
 
 // The whole solve, all segments of the line in this warp.
-template <int SEG, bool FULL, int KU>
-__device__ __forceinline__ void seg_solve(float (&y)[SEG], const SegOp &o, const SegPlan &pl, int seg, int k0,
-                                          int lane0) {
-    const float e = seg_fwd<SEG>(y, o);
-    const float b = seg_bwd<SEG, FULL, KU>(y, o, pl, k0, seg_carry<-1>(e, o, pl, seg, lane0));
-    seg_end<SEG, KU>(y, o, seg_carry<1>(b, o, pl, seg, lane0));
+template <int SEG, bool FULL, int KU, typename R>
+__device__ __forceinline__ void seg_solve(R (&y)[SEG], const SegOp<R> &o, const SegPlan &pl, int seg, int k0,
+                                          int lane0, int lgst) {
+    const R e = seg_fwd<SEG>(y, o);
+    const R b = seg_bwd<SEG, FULL, KU>(y, o, pl, k0, seg_carry<-1>(e, o, pl, seg, lane0, lgst));
+    seg_end<SEG, KU>(y, o, seg_carry<1>(b, o, pl, seg, lane0, lgst));
 }
 
 // Store the segment's own rows.
@@ -174,7 +188,7 @@ __device__ __forceinline__ void seg_store(const SegLane<E> &s, int P, ST &&st) {
 // alone by the 1st, 3: lane x's field by the 1st, lane y's by the 2nd.
 template <int SEG, bool FULL, int MODE>
 __device__ __forceinline__ void seg_pair_rhs(float (&y1)[SEG], float (&y2)[SEG], const SegLane<float2> &s, int P,
-                                             const SegOp &o1, const SegOp &o2) {
+                                             const SegOp<float> &o1, const SegOp<float> &o2) {
     float w1[SEG + 4], w2[SEG + 4];
     if constexpr (MODE == 0 || MODE == 2) {
         seg_load<SEG, FULL, 2>(w1, s, P, [](const float2 *p) { return p->x; });
@@ -197,13 +211,13 @@ __device__ __forceinline__ void seg_pair_rhs(float (&y1)[SEG], float (&y2)[SEG],
 
 // Two solves of the tile in place, all segments of their lines in this warp.
 template <int SEG, bool FULL, int MODE>
-__device__ __forceinline__ void seg_pair(const SegLane<float2> &s, int P, const SegOp &o1, const SegOp &o2,
+__device__ __forceinline__ void seg_pair(const SegLane<float2> &s, int P, const SegOp<float> &o1, const SegOp<float> &o2,
                                          const SegPlan &pl, int lane0, bool active) {
     float y1[SEG], y2[SEG];
     seg_pair_rhs<SEG, FULL, MODE>(y1, y2, s, P, o1, o2);
-    seg_solve<SEG, FULL, kSegRows1>(y1, o1, pl, s.seg, s.k0, lane0);
-    if constexpr (MODE == 0 || MODE == 3) seg_solve<SEG, FULL, kSegRows2>(y2, o2, pl, s.seg, s.k0, lane0);
-    if constexpr (MODE == 1) seg_solve<SEG, FULL, kSegRows1>(y2, o1, pl, s.seg, s.k0, lane0);
+    seg_solve<SEG, FULL, kSegRows1>(y1, o1, pl, s.seg, s.k0, lane0, pl.lgLW);
+    if constexpr (MODE == 0 || MODE == 3) seg_solve<SEG, FULL, kSegRows2>(y2, o2, pl, s.seg, s.k0, lane0, pl.lgLW);
+    if constexpr (MODE == 1) seg_solve<SEG, FULL, kSegRows1>(y2, o1, pl, s.seg, s.k0, lane0, pl.lgLW);
     __syncwarp();  // every lane of the line has read its window
     if (!active) return;
     seg_store<SEG, FULL>(s, P, [&](float2 *p, int k) {
@@ -215,7 +229,7 @@ __device__ __forceinline__ void seg_pair(const SegLane<float2> &s, int P, const 
 // One solve of a planar tile: the KIND-th derivative of the segment at `s`,
 // its rows stored to the same places `shift` elements on (0: in place).
 template <int SEG, bool FULL, int KIND>
-__device__ __forceinline__ void seg_one(const SegLane<float> &s, int P, const SegOp &o, const SegPlan &pl, int lane0,
+__device__ __forceinline__ void seg_one(const SegLane<float> &s, int P, const SegOp<float> &o, const SegPlan &pl, int lane0,
                                         bool active, int shift) {
     float y[SEG];
     {
@@ -227,33 +241,30 @@ __device__ __forceinline__ void seg_one(const SegLane<float> &s, int P, const Se
             if (!FULL && k < kSegSlack && k < s.k0) y[k] = 0.f;
         }
     }
-    seg_solve<SEG, FULL, KIND == 1 ? kSegRows1 : kSegRows2>(y, o, pl, s.seg, s.k0, lane0);
+    seg_solve<SEG, FULL, KIND == 1 ? kSegRows1 : kSegRows2>(y, o, pl, s.seg, s.k0, lane0, pl.lgLW);
     __syncwarp();  // every lane of the line has read its window
     if (active) seg_store<SEG, FULL>(s, P, [&](float *p, int k) { p[shift] = y[k]; });
     __syncwarp();
 }
 
-// The filter's correction (F - I) v of the segment at `s` (nine symmetric
-// taps), added to v in place.
-template <int SEG, bool FULL>
-__device__ __forceinline__ void seg_filter(const SegLane<float> &s, int P, const SegOp &o, const SegPlan &pl,
+// The filter (nine symmetric taps) of the segment at `s` in place.  FP32: o is
+// the correction F - I, added to the value; FP64: o is F itself.
+template <int SEG, bool FULL, typename R>
+__device__ __forceinline__ void seg_filter(const SegLane<R> &s, int P, const SegOp<R> &o, const SegPlan &pl,
                                            int lane0, bool active) {
-    float y[SEG];
+    R y[SEG];
     {
-        float w[SEG + 8];
-        seg_load<SEG, FULL, 4>(w, s, P, [](const float *p) { return *p; });
+        R w[SEG + 8];
+        seg_load<SEG, FULL, 4>(w, s, P, [](const R *p) { return *p; });
 #pragma unroll
         for (int k = 0; k < SEG; ++k) {
-            float r = o.s[0] * w[k + 4];
-#pragma unroll
-            for (int h = 1; h <= 4; ++h) r = fmaf(o.s[h], w[k + 4 - h] + w[k + 4 + h], r);
-            if (!FULL && k < kSegSlack && k < s.k0) r = 0.f;
-            y[k] = r;
+            y[k] = seg_r3<SEG>(w, o, k);
+            if (!FULL && k < kSegSlack && k < s.k0) y[k] = R(0);
         }
     }
-    seg_solve<SEG, FULL, kSegRowsAll>(y, o, pl, s.seg, s.k0, lane0);
+    seg_solve<SEG, FULL, kSegRowsAll>(y, o, pl, s.seg, s.k0, lane0, pl.lgLW);
     __syncwarp();  // every lane of the line has read its window
-    if (active) seg_store<SEG, FULL>(s, P, [&](float *p, int k) { *p += y[k]; });
+    if (active) seg_store<SEG, FULL>(s, P, [&](R *p, int k) { *p = sizeof(R) == 4 ? *p + y[k] : y[k]; });
 }
 
 // ---------------------------------------------------------------------
@@ -290,7 +301,7 @@ __device__ __forceinline__ E *cluster_map(E *p, int rank) {
 // thread of every block of the cluster calls it.
 template <bool FULL, int NT, bool SINGLE>
 __device__ __forceinline__ void run_cluster_tasks(float2 *tile, int pstride2, float2 *mail, const SegPlan &pl,
-                                                  const SegOp &o1, const SegOp &o2, int rank, int tid) {
+                                                  const SegOp<float> &o1, const SegOp<float> &o2, int rank, int tid) {
     constexpr int SEG = 32, P = kClLines;
     const int warp = tid >> 5, t = warp >> 1, half = (tid >> 4) & 1;
     const int l = ((warp & 1) << 4) | (tid & 15);
@@ -349,6 +360,153 @@ __device__ __forceinline__ void run_cluster_tasks(float2 *tile, int pstride2, fl
         if (!single) seg_end<SEG, kSegRows1>(y2, o1, in.y);
     }
     seg_store<SEG, FULL>(s, P, [&](float2 *p, int k) { *p = make_float2(y1[k], y2[k]); });
+}
+
+// ---------------------------------------------------------------------
+// FP64 lines, one thread a line
+// ---------------------------------------------------------------------
+// The plain form is bound by FP64 issue (two operations an SM and clock), so
+// its solves take the fewest operations: one thread walks the R rows of its
+// line that this block holds, in place in shared memory (4 or 5 operations for
+// the stencil, one a row forward, one backward), and the carries touch only
+// the K rows that they reach: 6.6 (first derivative) and 7.4 operations a row
+// at R = 128 against 9 of the Thomas sweep with its Sherman-Morrison
+// correction.  The line's other rows are in the blocks of a cluster, as in
+// run_cluster_tasks; R >= 40 there, so that a carry crosses one block at most.
+// Whole lines of one block: the circle closes on itself (wrap).
+struct SeqOp {
+    double nl, s0, s1, s2, wrap;
+    const double *pw;  // (-l)^(k+1)
+    int K;
+};
+
+// KIND 1, 2.  lo: the two rows before the first, hi: after the last (read
+// before any row is written; sync() between).  Returns the end value.
+template <int KIND, typename SYNC>
+__device__ __forceinline__ double seq_fwd(double *d, int P, int R, const SeqOp &o, const double *lo, const double *hi,
+                                          SYNC &&sync) {
+    double w0 = lo[-2 * P], w1 = lo[-P], w2 = d[0], w3 = d[P];
+    const double h0 = hi[0], h1 = hi[P];
+    sync();
+    const double nl = o.nl, s0 = o.s0, s1 = o.s1, s2 = o.s2;
+    double y = 0.0;
+    auto row = [&](double w4) {
+        const double r = KIND == 1 ? fma(s1, w3 - w1, s2 * (w4 - w0)) : fma(s2, w4 + w0, fma(s1, w3 + w1, s0 * w2));
+        y = fma(nl, y, r);
+        w0 = w1; w1 = w2; w2 = w3; w3 = w4;
+    };
+    double *q = d;
+    int n = 0;
+    for (; n + 6 <= R; n += 4, q += 4 * P) {
+        double c[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[j] = q[(j + 2) * P];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            row(c[j]);
+            q[j * P] = y;
+        }
+    }
+    for (; n < R; ++n, q += P) {
+        row(n + 2 < R ? q[2 * P] : n + 2 == R ? h0 : h1);
+        q[0] = y;
+    }
+    return y;
+}
+// Backward, `in` entering at the first row; returns the first row's value.
+__device__ __forceinline__ double seq_bwd(double *d, int P, int R, const SeqOp &o, double in) {
+    const double nl = o.nl;
+    const int K = min(o.K, R);
+    double x = 0.0;
+    double *q = d + (R - 1) * P;
+    int n = R;
+    for (; n - 4 >= K; n -= 4, q -= 4 * P) {
+        double c[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[j] = q[-j * P];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) q[-j * P] = x = fma(nl, x, c[j]);
+    }
+    for (; n > K; --n, q -= P) q[0] = x = fma(nl, x, q[0]);
+    for (; n - 4 >= 0; n -= 4, q -= 4 * P) {
+        double c[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[j] = fma(ldc(o.pw + n - 1 - j), in, q[-j * P]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) q[-j * P] = x = fma(nl, x, c[j]);
+    }
+    for (; n > 0; --n, q -= P) q[0] = x = fma(nl, x, fma(ldc(o.pw + n - 1), in, q[0]));
+    return x;
+}
+__device__ __forceinline__ void seq_end(double *d, int P, int R, const SeqOp &o, double in) {
+    const int K = min(o.K, R);
+    double *q = d + (R - 1) * P;
+#pragma unroll 4
+    for (int k = 0; k < K; ++k) q[-k * P] = fma(ldc(o.pw + k), in, q[-k * P]);
+}
+
+// The solves of a tile of L lines (a power of two <= 32), planar buffers
+// `stride` apart: n1 first derivatives in buffers 0 .., then second derivatives
+// of the first four fields in n1 .. n1 + 3, each in place.  A line's segments:
+// one a block of a cluster of pl.C blocks (R rows here), or pl.G in this block
+// (R: all rows).  Warps are uniform: the second derivatives start at a warp's
+// first lane.  mail: 2 (n1 + 4) L doubles per segment of the block.  Every
+// thread of every block of the cluster calls it.
+__device__ __forceinline__ void run_seq_tasks(double *tile, int stride, double *mail, int n1, int L, int lgL, int R,
+                                              const SegPlan &pl, const SeqOp &o1, const SeqOp &o2, int rank, int tid) {
+    const int C = pl.C, B = C > 1 ? 1 : pl.G;      // segments of a line in this block: 1 or 2
+    const int per = 32 >> lgL;                     // solves a warp holds
+    const int n1p = (n1 * B + per - 1) & ~(per - 1);
+    int k = tid >> lgL;
+    const int l = tid & (L - 1);
+    const bool second = k >= n1p;
+    const bool on = second ? k < n1p + 4 * B : k < n1 * B;
+    if (second) k -= n1p;
+    if (!on) k = 0;
+    const int h = B > 1 ? k & 1 : 0;
+    k = (B > 1 ? k >> 1 : k) + (second && on ? n1 : 0);
+    const int R0 = seg_rows(pl, 0);
+    double *line = tile + k * stride + l, *d = line + h * R0 * L;
+    const int rows = B > 1 ? seg_rows(pl, h) : R;
+    double *box = mail + (2 * k + h) * L + l, *box2 = box + 2 * (n1 + 4) * L;
+    const SeqOp &o = second ? o2 : o1;
+    double v = 0.0;
+    if (C > 1) {
+        const int prev = rank > 0 ? rank - 1 : C - 1, next = rank < C - 1 ? rank + 1 : 0;
+        const double *lo = cluster_map(d + seg_rows(pl, rank - 1) * L, prev), *hi = cluster_map(d, next);
+        auto sync = [] { cluster_sync(); };
+        if (second) v = seq_fwd<2>(d, L, on ? R : 0, o, lo, hi, sync);
+        else v = seq_fwd<1>(d, L, on ? R : 0, o, lo, hi, sync);
+        if (on) *cluster_map(box, next) = v;
+        cluster_sync();
+        if (on) {
+            v = seq_bwd(d, L, R, o, *box);
+            *cluster_map(box2, prev) = v;
+        }
+        cluster_sync();  // (the last access to another block's shared memory)
+        if (on) seq_end(d, L, R, o, *box2);
+    } else if (B > 1) {
+        // the halves' ends are each other's neighbours
+        const double *lo = line + (h ? R0 : R) * L, *hi = line + (h ? 0 : R0) * L;
+        const int other = h ? -L : L;
+        auto sync = [] { __syncthreads(); };
+        if (second) v = seq_fwd<2>(d, L, on ? rows : 0, o, lo, hi, sync);
+        else v = seq_fwd<1>(d, L, on ? rows : 0, o, lo, hi, sync);
+        if (on) box[other] = v;
+        __syncthreads();
+        if (on) {
+            v = seq_bwd(d, L, rows, o, *box);
+            box2[other] = v;
+        }
+        __syncthreads();
+        if (on) seq_end(d, L, rows, o, *box2);
+    } else if (on) {
+        auto sync = [] {};
+        if (second) v = seq_fwd<2>(d, L, R, o, d + R * L, d, sync);
+        else v = seq_fwd<1>(d, L, R, o, d + R * L, d, sync);
+        v = seq_bwd(d, L, R, o, v * o.wrap);
+        seq_end(d, L, R, o, v * o.wrap);
+    }
 }
 
 }  // namespace cs3d

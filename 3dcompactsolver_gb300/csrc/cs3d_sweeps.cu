@@ -61,6 +61,7 @@ constexpr int kMinBlocksX = 3, kMinBlocksY = 1, kMinBlocksZ = 1;
 // has no line factors and its solutions need no correction on read.  SEG = 0:
 // the Thomas solves with precomputed factors (the plain form, wall lines, and
 // lengths that seg_plan does not cut).
+constexpr int ZS_ = 8;  // the first of the z tile's slots that park dq (ZS)
 template <typename T, int SEG>
 struct TileOf {
     using SM = typename SweepSmem<T>::type;
@@ -73,7 +74,47 @@ struct TileOf {
         get2(sm, t, p, L, za, zb, a, b);
     }
     static __device__ __forceinline__ T one(const SM &sm, int k, const Pt &p, int L, T z) { return get1(sm, k, p, L, z); }
+    // the z sweep parks dq in five of the point's spent solve slots
+    static __device__ __forceinline__ T &dq(const SM &sm, int f, int o) { return sm.at(ZS_ + f, o); }
 };
+// FP64, periodic lines: planar buffers of the sequential solves, the n1 first
+// derivatives, then the four second derivatives (each solved in place, so the
+// load phase stores those fields twice).
+constexpr int kSeq = kSeqSeg;
+struct SmemSeq {
+    double *buf;
+    int stride, n1;
+    __device__ double &at(int k, int o) const { return buf[k * stride + o]; }
+};
+template <>
+struct TileOf<double, kSeq> {
+    using SM = SmemSeq;
+    static __device__ __forceinline__ SM at(int n1, int L, int, int R, const SegPlan &) {
+        return {reinterpret_cast<double *>(smem_raw), seq_stride(R, L), n1};
+    }
+    static __device__ __forceinline__ void put1f(const SM &sm, int t, int o, double v) {
+        if (t < 4) {
+            sm.at(t, o) = v;
+            sm.at(sm.n1 + t, o) = v;
+        } else {
+            sm.at(2 * t - 4, o) = v;
+        }
+    }
+    static __device__ __forceinline__ Zn<double> z(const LineOp<double> &, const LineOp<double> &, int) { return {0.0, 0.0}; }
+    static __device__ __forceinline__ void two(const SM &sm, int t, const Pt &p, int, double, double, double &a, double &b) {
+        a = sm.at(t < 4 ? t : 2 * t - 4, p.o);
+        b = sm.at(t < 4 ? sm.n1 + t : 2 * t - 3, p.o);
+    }
+    static __device__ __forceinline__ double one(const SM &sm, int, const Pt &p, int, double) { return sm.at(sm.n1 - 1, p.o); }
+    static __device__ __forceinline__ double &dq(const SM &sm, int f, int o) { return sm.at(4 + f, o); }
+    static __device__ __forceinline__ double *mail(const SM &sm) { return sm.buf + (sm.n1 + 4) * sm.stride; }
+};
+__device__ __forceinline__ void put2(const SmemSeq &sm, int t, int o, double v0, double v1) {
+    sm.at(2 * t - 4, o) = v0;
+    sm.at(2 * t - 3, o) = v1;
+}
+// first derivatives of a sweep
+constexpr int kSeqN1X = 9, kSeqN1Y = 11, kSeqN1Z = 12;
 // Segmented x tiles are planar: 80 registers a thread (3 blocks of 256 per SM)
 // hold one solve's segment, not a pair's.  Buffers as XU..XF4; a task's
 // buffers are 2t and 2t + 1.
@@ -103,8 +144,8 @@ __device__ __forceinline__ void put2(const SmemSegX &sm, int t, int o, float v0,
 // The 13 solves of a segmented x tile, seven units of two (the last of one) on
 // the lines a warp holds.
 template <int SEG, bool FULL>
-__device__ __forceinline__ void run_seg_x(const SmemSegX &sm, int P, int L, int N, const SegPlan &pl, const SegOp &o1,
-                                          const SegOp &o2, int tid, int nthr) {
+__device__ __forceinline__ void run_seg_x(const SmemSegX &sm, int P, int L, int N, const SegPlan &pl, const SegOp<float> &o1,
+                                          const SegOp<float> &o2, int tid, int nthr) {
     const int lane0 = tid & ((1 << pl.lgLW) - 1), seg = (tid & 31) >> pl.lgLW;
     const int groups = max(1, L >> pl.lgLW);
     for (int u = tid >> 5; u < 7 * groups; u += nthr >> 5) {
@@ -133,6 +174,7 @@ struct TileSeg {
         b = v.y;
     }
     static __device__ __forceinline__ float one(const SM &sm, int k, const Pt &p, int, float) { return sm.at(k, p.o); }
+    static __device__ __forceinline__ float &dq(const SM &sm, int f, int o) { return sm.at(ZS_ + f, o); }
 };
 // (cluster tiles: 8 pair arrays, then the mailbox)
 __device__ __forceinline__ float2 *cluster_mail(const SmemPair &sm) { return sm.pair(8); }
@@ -158,11 +200,11 @@ __constant__ Task kTasksX2[7] = {{XU, XU, 0, XU, XU2, 1}, {XV, XV, 0, XV, XV2, 1
 
 template <typename T, int PC, int SEG = 0, bool FULL = false>
 __global__ void __launch_bounds__(sweep_threads<T>(0), sizeof(T) == 4 && (SEG == 0 || FULL) ? kMinBlocksX : 2) k_sweep_x(SweepArgs<T> a) {
-    using TS = std::conditional_t<(SEG > 0), TileSegX<SEG>, TileOf<T, 0>>;
+    using TS = std::conditional_t<(SEG > 0 && sizeof(T) == 4), TileSegX<SEG>, TileOf<T, SEG>>;
     const int L = a.L, P = PC > 0 ? PC : a.P;
     const Tile t = make_tile<0>(a.g, L);
     const int N = t.N, NL = N * L, pad = FULL ? a.seg.pad : 0;
-    const auto sm = TS::at(sizeof(T) == 4 ? XNB2 : XNB, L, P, N, a.seg);
+    const auto sm = TS::at(SEG == kSeq ? kSeqN1X : sizeof(T) == 4 ? XNB2 : XNB, L, P, N, a.seg);
     const GasParams gp = a.gas;
     // FP64 tiles: points across the lines first, pitch P = L (no pad column)
     constexpr bool kXLineFirst = sizeof(T) == 8;
@@ -203,7 +245,9 @@ __global__ void __launch_bounds__(sweep_threads<T>(0), sizeof(T) == 4 && (SEG ==
             TS::put1f(sm, 6, o, s.re * ss.U + ss.U * ss.p);
         });
     __syncthreads();
-    if constexpr (SEG > 0)
+    if constexpr (SEG == kSeq)
+        run_seq_tasks(sm.buf, sm.stride, TS::mail(sm), kSeqN1X, L, a.lgL, N, a.seg, a.h1, a.h2, 0, threadIdx.x);
+    else if constexpr (SEG > 0)
         run_seg_x<SEG, FULL>(sm, P, L, N, a.seg, a.g1, a.g2, threadIdx.x, blockDim.x);
     else
         run_sweep_solves<2, PC>(sm, sizeof(T) == 4 ? kTasksX2 : kTasksX, 7, L, t.nlines, a.d1, a.d2, threadIdx.x,
@@ -273,15 +317,17 @@ __constant__ Task kTasksY2[8] = {{YU, YU, 0, YU, YU2, 1}, {YV, YV, 0, YV, YV2, 1
 template <typename T, int PC, int SEG = 0, bool FULL = false, bool CL = false>
 __global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBlocksY : 3) k_sweep_y(SweepArgs<T> a) {
     using TS = TileOf<T, SEG>;
-    const int L = CL ? kClLines : a.L, P = PC > 0 ? PC : a.P;
+    constexpr bool SQ = SEG == kSeq;
+    const int L = CL && !SQ ? kClLines : a.L, P = PC > 0 ? PC : a.P, lgL = CL && !SQ ? 5 : a.lgL;
     const int rank = CL ? (int)blockIdx.x % a.seg.C : 0;
-    const Tile t = CL ? make_cluster_tile<1>(a.g, a.seg, rank) : make_tile<1>(a.g, L);
+    const Tile t = SQ ? make_seq_tile<1>(a.g, a.seg, L, rank)
+                      : CL ? make_cluster_tile<1>(a.g, a.seg, rank) : make_tile<1>(a.g, L);
     const int N = t.N, NL = N * L, pad = FULL && !CL ? a.seg.pad : 0;
-    const auto sm = TS::at(sizeof(T) == 4 ? YNB2 : YNB, L, P, CL ? kClRows : N, a.seg);
+    const auto sm = TS::at(SQ ? kSeqN1Y : sizeof(T) == 4 ? YNB2 : YNB, L, P, SQ ? (a.seg.C > 1 ? a.seg.S : N) : CL ? kClRows : N, a.seg);
     struct InA { Pt pt; T v[11]; };
     batched<InA, sizeof(T) == 4 ? 4 : 2>(NL,
         [&](InA &in, int p) {
-            in.pt = point<1>(t, p, L, P, CL ? 5 : a.lgL, a.divN, pad);
+            in.pt = point<1>(t, p, L, P, lgL, a.divN, pad);
             const unsigned gi = in.pt.gi;
 #pragma unroll
             for (int f = 0; f < 4; ++f) in.v[f] = a.qs[f + 1][gi];
@@ -306,7 +352,9 @@ __global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBloc
         });
     if constexpr (CL) cluster_sync();
     else __syncthreads();
-    if constexpr (CL)
+    if constexpr (SQ)
+        run_seq_tasks(sm.buf, sm.stride, TS::mail(sm), kSeqN1Y, L, lgL, N, a.seg, a.h1, a.h2, rank, threadIdx.x);
+    else if constexpr (CL)
         run_cluster_tasks<FULL, 8, true>(sm.pair(0), sm.pstride / 2, cluster_mail(sm), a.seg, a.g1, a.g2, rank,
                                          threadIdx.x);
     else if constexpr (SEG > 0)
@@ -319,7 +367,7 @@ __global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBloc
     struct InC { Pt pt; T v[9]; };
     batched<InC, sizeof(T) == 4 ? kYConsumeBatch : 2>(NL,
         [&](InC &in, int p) {
-            in.pt = point<1>(t, p, L, P, CL ? 5 : a.lgL, a.divN, pad);
+            in.pt = point<1>(t, p, L, P, lgL, a.divN, pad);
             const unsigned gi = in.pt.gi;
             in.v[0] = a.prim[0][gi]; in.v[1] = a.prim[1][gi]; in.v[2] = a.prim[2][gi];
             in.v[3] = a.mu[gi];
@@ -375,12 +423,13 @@ __constant__ Task kTasksZ[8] = {{ZU, ZU, 0, ZU, ZU2, 1}, {ZV, ZV, 0, ZV, ZV2, 1}
 // thread range).
 template <typename T, int PC, int SEG, bool FULL, bool CL>
 struct ZSweep {
+    static constexpr bool SQ = SEG == kSeq;
     using TS = TileOf<T, SEG>;
     using SM = typename TS::SM;
     // A: stage the inputs of the 16 z-solves of tile t in sm
     static __device__ __forceinline__ void load(const SweepArgs<T> &a, const Tile &t, const SM &sm, int tid,
                                                 int nthr) {
-        const int L = CL ? kClLines : a.L, P = PC > 0 ? PC : a.P, lgL = CL ? 5 : a.lgL;
+        const int L = CL && !SQ ? kClLines : a.L, P = PC > 0 ? PC : a.P, lgL = CL && !SQ ? 5 : a.lgL;
         const int NL = t.N * L, pad = FULL && !CL ? a.seg.pad : 0;
         struct InA { Pt pt; T v[13]; };
         batched<InA, sizeof(T) == 4 ? 4 : 2>(NL, tid, nthr,
@@ -414,9 +463,12 @@ struct ZSweep {
     // B: the 16 solves (8 pairs) of every line of the tile
     static __device__ __forceinline__ void solve(const SweepArgs<T> &a, const Tile &t, const SM &sm, int tid,
                                                  int nthr) {
-        if constexpr (CL)
+        const int rank = CL ? (int)blockIdx.x % a.seg.C : 0;
+        if constexpr (SQ)
+            run_seq_tasks(sm.buf, sm.stride, TS::mail(sm), kSeqN1Z, a.L, a.lgL, t.N, a.seg, a.h1, a.h2, rank, tid);
+        else if constexpr (CL)
             run_cluster_tasks<FULL, 8, false>(sm.pair(0), sm.pstride / 2, cluster_mail(sm), a.seg, a.g1, a.g2,
-                                              (int)blockIdx.x % a.seg.C, tid);
+                                              rank, tid);
         else if constexpr (SEG > 0)
             run_seg_tasks<SEG, FULL, 8, false>(sm, PC > 0 ? PC : a.P, a.L, t.N, a.seg, a.g1, a.g2, tid, nthr);
         else
@@ -425,9 +477,9 @@ struct ZSweep {
     // C: right-hand side, dq and the RK update of every point of the tile
     static __device__ __forceinline__ void consume(const SweepArgs<T> &a, const Tile &t, const SM &sm, int tid,
                                                    int nthr) {
-        const int L = CL ? kClLines : a.L, P = PC > 0 ? PC : a.P, lgL = CL ? 5 : a.lgL;
+        const int L = CL && !SQ ? kClLines : a.L, P = PC > 0 ? PC : a.P, lgL = CL && !SQ ? 5 : a.lgL;
         const int NL = t.N * L, pad = FULL && !CL ? a.seg.pad : 0;
-        const T c43 = T(4.0 / 3.0), c13 = T(1.0 / 3.0), cpPr = (T)a.gas.cpPr;
+        const T c43 = T(4.0 / 3.0), c13 = T(1.0 / 3.0), c23 = T(2.0 / 3.0), cpPr = (T)a.gas.cpPr;
         const double dt = *a.dt;
         const T dtw = (T)dt;
         const int st = a.rk_step;
@@ -448,7 +500,7 @@ struct ZSweep {
         // side and parks dq = dt*RHS in the point's own, now unused, solve slots;
         // C2 streams the FP64 state through the RK update.  Each pass keeps fewer
         // values live than one fused pass, so more points' loads are in flight.
-        constexpr int kDq[5] = {ZS, ZWX, ZWY, ZRW, ZF1};
+        static_assert(ZS == ZS_ && ZF1 == ZS_ + 4, "dq slots");
         struct InC1 {
             Pt pt;
             T v[18];
@@ -485,38 +537,39 @@ struct ZSweep {
                 TS::two(sm, 5, p, L, zz.z1, zz.z1, Wyz, cez);
                 TS::two(sm, 6, p, L, zz.z1, zz.z1, f1, f2);
                 TS::two(sm, 7, p, L, zz.z1, zz.z1, f3, f4);
-                T src[5] = {T(0), T(0), T(0), T(0), T(0)};
-                if (a.sponge) {  // sigma (avg - q), SpongeBC / CSolver_AWS.hpp:228
-                    const T sg = to_work<T>(a.sigma[gi]);
-#pragma unroll
-                    for (int f = 0; f < 5; ++f) src[f] = sg * (to_work<T>(a.savg.f[f][gi]) - in.qsv[f]);
-                }
                 const T MuX = amu * Tx, MuY = amu * Ty, MuZ = amu * Tz;
-                // shear rates, and the normal stresses' 3/4: c43 h1 is
-                // (4/3) Ux - (2/3)(Vy + Wz)
-                const T s12 = Uy + Vx, s13 = Wx + Uz, s23 = Wy + Vz;
-                const T h1 = Ux - T(0.5) * (Vy + Wz), h2 = Vy - T(0.5) * (Ux + Wz), h3 = Wz - T(0.5) * (Ux + Vy);
+                // shear rates, and the normal stresses 2 Ux - (2/3) div u
+                const T s12 = Uy + Vx, s13 = Wx + Uz, s23 = Wy + Vz, dv = c23 * (Ux + Vy + Wz);
+                const T g1 = T(2.0) * Ux - dv, g2 = T(2.0) * Vy - dv, g3 = T(2.0) * Wz - dv;
                 // the viscous terms of the momenta: mu times second derivatives
                 // and the viscosity gradient times the stresses; their work is
                 // U, V, W times them, plus the dissipation
-                const T w1 = mu * (Uzz + c13 * Wxz) + (c43 * MuX * h1 + MuY * s12 + MuZ * s13);
-                const T w2 = mu * (Vzz + c13 * Wyz) + (c43 * MuY * h2 + MuX * s12 + MuZ * s23);
-                const T w3 = mu * (c43 * Wzz + c13 * S) + (c43 * MuZ * h3 + MuX * s13 + MuY * s23);
-                const T diss = c43 * (Ux * h1 + Vy * h2 + Wz * h3) + (s12 * s12 + s13 * s13 + s23 * s23);
+                const T w1 = mu * (Uzz + c13 * Wxz) + (MuX * g1 + MuY * s12 + MuZ * s13);
+                const T w2 = mu * (Vzz + c13 * Wyz) + (MuY * g2 + MuX * s12 + MuZ * s23);
+                const T w3 = mu * (c43 * Wzz + c13 * S) + (MuZ * g3 + MuX * s13 + MuY * s23);
+                const T diss = Ux * g1 + Vy * g2 + Wz * g3 + (s12 * s12 + s13 * s13 + s23 * s23);
                 T R[5];
                 R[0] = in.v[13];
-                R[1] = in.v[14] + (w1 - f1) + src[1];
-                R[2] = in.v[15] + (w2 - f2) + src[2];
-                R[3] = in.v[16] + (w3 - f3) + src[3];
-                R[4] = in.v[17] + cpPr * (MuX * Tx + MuY * Ty + MuZ * Tz + mu * Tzz) +
-                       (U * w1 + V * w2 + W * w3 + mu * diss) - f4 + T(2.0) * src[4];
+                R[1] = in.v[14] + (w1 - f1);
+                R[2] = in.v[15] + (w2 - f2);
+                R[3] = in.v[16] + (w3 - f3);
+                R[4] = in.v[17] + (cpPr * (MuX * Tx + MuY * Ty + MuZ * Tz + mu * Tzz) +
+                                   (U * w1 + V * w2 + W * w3 + mu * diss) - f4);
+                T src0 = T(0);
+                if (a.sponge) {  // sigma (avg - q), SpongeBC / CSolver_AWS.hpp:228
+                    const T sg = to_work<T>(a.sigma[gi]);
+                    src0 = sg * (to_work<T>(a.savg.f[0][gi]) - in.qsv[0]);
+#pragma unroll
+                    for (int f = 1; f < 5; ++f)
+                        R[f] += (f == 4 ? T(2.0) * sg : sg) * (to_work<T>(a.savg.f[f][gi]) - in.qsv[f]);
+                }
                 // continuity and the post-step boundary fix-up (CSolver_AWS.cpp:1506-1679)
                 int i, j, k;
                 coords<2>(t, p.l, p.n, i, j, k);
                 const int fc = faces_of(a.g, i, j, k);
                 const int wd = a.wall_faces ? wall_dir(fc & a.wall_faces) : -1;
                 if (wd == 2) R[0] = -cez;
-                else if (wd < 0) R[0] = R[0] - cez + src[0];
+                else if (wd < 0) R[0] = a.sponge ? R[0] - cez + src0 : R[0] - cez;
                 const bool zero_all = (fc & a.sponge_kind_faces) != 0;
                 const bool zero_mom = wd >= 0;
                 if (a.diag[0]) {  // derivative fields of the last stage, for diagnostics
@@ -535,7 +588,7 @@ struct ZSweep {
                     T d = sizeof(T) == 8 ? (T)(dt * (double)R[f]) : dtw * R[f];
                     if (zero_all || (f > 0 && zero_mom)) d = T(0);
                     if (a.dq_out[0]) a.dq_out[f][gi] = to_f64(d);
-                    sm.at(kDq[f], p.o) = d;
+                    TS::dq(sm, f, p.o) = d;
                 }
             });
         struct InC2 {
@@ -561,7 +614,7 @@ struct ZSweep {
                     // plain form: the reference's RK update in FP64
 #pragma unroll
                     for (int f = 0; f < 5; ++f) {
-                        const double d = (double)sm.at(kDq[f], in.pt.o);
+                        const double d = (double)TS::dq(sm, f, in.pt.o);
                         if (tvd) {  // TVD-RK3 (TVDRK3.hpp:38-96); qa = q1, qb = qk
                             if (st == 1) a.qk.f[f][gi] = in.qa[f] + d;
                             else if (st == 2) a.qk.f[f][gi] = 0.75 * in.qa[f] + 0.25 * in.qb[f] + 0.25 * d;
@@ -578,7 +631,7 @@ struct ZSweep {
                     // mixed form: the FP32 increment accumulated into the FP64 state
 #pragma unroll
                     for (int f = 0; f < 5; ++f) {
-                        const T d = sm.at(kDq[f], in.pt.o);
+                        const T d = TS::dq(sm, f, in.pt.o);
                         if (tvd) {
                             const double dd = to_f64(d);
                             double nv;
@@ -612,8 +665,10 @@ struct ZSweep {
 template <typename T, int PC, int SEG = 0, bool FULL = false, bool CL = false>
 __global__ void __launch_bounds__(sweep_threads<T>(2), sizeof(T) == 4 ? kMinBlocksZ : 3) k_sweep_z(SweepArgs<T> a) {
     using Z = ZSweep<T, PC, SEG, FULL, CL>;
-    const Tile t = CL ? make_cluster_tile<2>(a.g, a.seg, (int)blockIdx.x % a.seg.C) : make_tile<2>(a.g, a.L);
-    const auto sm = Z::TS::at(ZNB, a.L, PC > 0 ? PC : a.P, CL ? kClRows : t.N, a.seg);
+    const int rank = CL ? (int)blockIdx.x % a.seg.C : 0;
+    const Tile t = Z::SQ ? make_seq_tile<2>(a.g, a.seg, a.L, rank)
+                         : CL ? make_cluster_tile<2>(a.g, a.seg, rank) : make_tile<2>(a.g, a.L);
+    const auto sm = Z::TS::at(Z::SQ ? kSeqN1Z : ZNB, a.L, PC > 0 ? PC : a.P, Z::SQ ? (a.seg.C > 1 ? a.seg.S : t.N) : CL ? kClRows : t.N, a.seg);
     Z::load(a, t, sm, threadIdx.x, blockDim.x);
     if constexpr (CL) cluster_sync();
     else __syncthreads();
@@ -721,20 +776,25 @@ __global__ void __launch_bounds__(filter_threads<T>(), sizeof(T) == 4 ? kFilterM
 // The mixed filter on periodic lines: the five fields' corrections by the
 // segmented solves (cs3d_seg.cuh), added in place, so a tile is five buffers
 // and the y and z tiles are 32 lines (128 bytes a row) wide.
-template <int DIR, int SEG, bool FULL>
-__global__ void __launch_bounds__(kFilterSegTpb, 2) k_filter_seg(FilterArgs<float> a) {
+// The plain form likewise, with F itself.
+template <typename T, int DIR, int SEG, bool FULL>
+__global__ void __launch_bounds__(sizeof(T) == 4 ? kFilterSegTpb : kFilterSegTpb64, sizeof(T) == 4 ? 2 : 3)
+k_filter_seg(FilterArgs<T> a) {
     const int L = a.L, P = a.P;
     const Tile t = make_tile<DIR>(a.g, L);
     const int N = t.N, NL = N * L, pad = FULL ? a.seg.pad : 0;
     const int stride = seg_stride(N, P, a.seg.G, a.seg.pad);
-    float *buf = reinterpret_cast<float *>(smem_raw);
-    struct In { Pt pt; float v[5]; };
+    T *buf = reinterpret_cast<T *>(smem_raw);
+    struct In { Pt pt; T v[5]; };
     batched<In, kFilterBatch>(NL,
         [&](In &in, int p) {
             in.pt = point<DIR>(t, p, L, P, a.lgL, a.divN, pad);
             const unsigned gi = in.pt.gi;
 #pragma unroll
-            for (int f = 0; f < 5; ++f) in.v[f] = a.src64.f[0] ? narrow(a.src64.f[f][gi] - a.ref[f]) : a.src32[f][gi];
+            for (int f = 0; f < 5; ++f) {
+                if constexpr (sizeof(T) == 8) in.v[f] = a.src64.f[0] ? a.src64.f[f][gi] : a.src32[f][gi];
+                else in.v[f] = a.src64.f[0] ? narrow(a.src64.f[f][gi] - a.ref[f]) : a.src32[f][gi];
+            }
         },
         [&](In &in) {
             if (!in.pt.ok) return;
@@ -753,6 +813,15 @@ __global__ void __launch_bounds__(kFilterSegTpb, 2) k_filter_seg(FilterArgs<floa
         }
     }
     __syncthreads();
+    if constexpr (sizeof(T) == 8) {
+        for (int p = threadIdx.x; p < NL; p += blockDim.x) {
+            const Pt pt = point<DIR>(t, p, L, P, a.lgL, a.divN, pad);
+            if (!pt.ok) continue;
+#pragma unroll
+            for (int f = 0; f < 5; ++f) (a.dst64.f[0] ? a.dst64.f[f] : a.dst32[f])[pt.gi] = buf[f * stride + pt.o];
+        }
+        return;
+    } else {
     struct Out { Pt pt; double q[5]; float u[5]; };
     batched<Out, kFilterConsumeBatch>(NL,
         [&](Out &o, int p) {
@@ -782,6 +851,7 @@ __global__ void __launch_bounds__(kFilterSegTpb, 2) k_filter_seg(FilterArgs<floa
                 }
             }
         });
+    }
 }
 
 // ---------------------------------------------------------------------
@@ -840,6 +910,9 @@ size_t planar_smem_bytes(int prec_bytes, int nbuf, int L, int P, int N) {
     return prec_bytes == 8 ? tile_smem<double>(nbuf, L, P, N) : tile_smem<float>(nbuf, L, P, N);
 }
 size_t sweep_smem_bytes(int prec_bytes, int nbuf, int L, int P, int N, const SegPlan *seg) {
+    // the buffers and the mailboxes (a line's rows here: one block's, or all)
+    if (prec_bytes == 8 && seg && seg->SEG)
+        return 8 * (size_t)nbuf * (seq_stride(seg->C > 1 ? seg->S : N, L) + (seg->G > 1 ? 4 * L : 0));
     if (prec_bytes == 4 && seg && seg->C) return 8 * (8 * (size_t)kClRows * kClLines + 8 * kClLines);
     if (prec_bytes == 4 && seg && seg->SEG && !seg->pair) return (size_t)XNB * 4 * seg_stride(N, P, seg->G, seg->pad);
     // segmented solves: the pair arrays alone (no line factors, no read-ahead)
@@ -869,13 +942,14 @@ static dim3 tile_grid(int dir, const Geom &g, int L) {
 
 // the segmented instances: compile-time pitches for the full segments, the
 // three segment lengths at run-time pitch for the others
-static cudaError_t launch_cluster(void (*kernel)(SweepArgs<float>), const SweepArgs<float> &a, dim3 grid, size_t sm,
+template <typename T>
+static cudaError_t launch_cluster(void (*kernel)(SweepArgs<T>), const SweepArgs<T> &a, dim3 grid, size_t sm,
                                   cudaStream_t s) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t c{};
     c.gridDim = dim3(grid.x * a.seg.C, grid.y);
-    c.blockDim = dim3(32 * kClWarps);
+    c.blockDim = dim3(a.threads);
     c.dynamicSmemBytes = sm;
     c.stream = s;
     cudaLaunchAttribute at{};
@@ -929,6 +1003,12 @@ cudaError_t launch_sweep(int dir, const SweepArgs<T> &a, cudaStream_t s) {
     const dim3 grid = tile_grid(dir, a.g, a.L);
     if constexpr (sizeof(T) == 4) {
         if (a.seg.SEG) return launch_seg_sweep(dir, a, grid, sm, s);
+    } else if (a.seg.SEG == kSeq) {
+        if (dir == 0) return launch_tile_kernel(k_sweep_x<T, 0, kSeq>, a, grid, sm, s);
+        return launch_cluster<T>(dir == 1 ? k_sweep_y<T, 0, kSeq, false, true> : k_sweep_z<T, 0, kSeq, false, true>, a, grid,
+                                 sm, s);
+    }
+    if constexpr (sizeof(T) == 4) {
         if (dir == 0 && a.P == 9) return launch_tile_kernel(k_sweep_x<T, 9>, a, grid, sm, s);
         if (dir == 0 && a.P == 5) return launch_tile_kernel(k_sweep_x<T, 5>, a, grid, sm, s);
         if (dir == 1 && a.P == 16) return launch_tile_kernel(k_sweep_y<T, 16>, a, grid, sm, s);
@@ -941,27 +1021,27 @@ cudaError_t launch_sweep(int dir, const SweepArgs<T> &a, cudaStream_t s) {
     return launch_tile_kernel(k_sweep_z<T, 0>, a, grid, sm, s);
 }
 
-size_t filter_seg_smem(int L, int P, int N, const SegPlan &p) { return (size_t)5 * 4 * seg_stride(N, P, p.G, p.pad); }
+size_t filter_seg_smem(int prec_bytes, int L, int P, int N, const SegPlan &p) {
+    return (size_t)5 * prec_bytes * seg_stride(N, P, p.G, p.pad);
+}
 
-template <int DIR>
-static cudaError_t launch_filter_seg(const FilterArgs<float> &a, dim3 grid, size_t sm, cudaStream_t s) {
-    if (a.seg.full) return launch_tile_kernel(k_filter_seg<DIR, 32, true>, a, grid, sm, s);
-    if (a.seg.SEG == 32) return launch_tile_kernel(k_filter_seg<DIR, 32, false>, a, grid, sm, s);
-    if (a.seg.SEG == 24) return launch_tile_kernel(k_filter_seg<DIR, 24, false>, a, grid, sm, s);
-    return launch_tile_kernel(k_filter_seg<DIR, 16, false>, a, grid, sm, s);
+template <int DIR, typename T>
+static cudaError_t launch_filter_seg(const FilterArgs<T> &a, dim3 grid, size_t sm, cudaStream_t s) {
+    if (a.seg.full) return launch_tile_kernel(k_filter_seg<T, DIR, 32, true>, a, grid, sm, s);
+    if (a.seg.SEG == 32) return launch_tile_kernel(k_filter_seg<T, DIR, 32, false>, a, grid, sm, s);
+    if (a.seg.SEG == 24) return launch_tile_kernel(k_filter_seg<T, DIR, 24, false>, a, grid, sm, s);
+    return launch_tile_kernel(k_filter_seg<T, DIR, 16, false>, a, grid, sm, s);
 }
 
 template <typename T>
 cudaError_t launch_filter(int dir, const FilterArgs<T> &a, cudaStream_t s) {
     const int N = dir == 0 ? a.g.Nx : dir == 1 ? a.g.Ny : a.g.Nz;
-    if constexpr (sizeof(T) == 4) {
-        if (a.seg.SEG) {
-            const size_t fs = filter_seg_smem(a.L, a.P, N, a.seg);
-            const dim3 fg = tile_grid(dir, a.g, a.L);
-            if (dir == 0) return launch_filter_seg<0>(a, fg, fs, s);
-            if (dir == 1) return launch_filter_seg<1>(a, fg, fs, s);
-            return launch_filter_seg<2>(a, fg, fs, s);
-        }
+    if (a.seg.SEG) {
+        const size_t fs = filter_seg_smem((int)sizeof(T), a.L, a.P, N, a.seg);
+        const dim3 fg = tile_grid(dir, a.g, a.L);
+        if (dir == 0) return launch_filter_seg<0>(a, fg, fs, s);
+        if (dir == 1) return launch_filter_seg<1>(a, fg, fs, s);
+        return launch_filter_seg<2>(a, fg, fs, s);
     }
     const size_t sm = tile_smem<T>(sizeof(T) == 4 ? 10 : 5, a.L, a.P, N);
     const dim3 grid = tile_grid(dir, a.g, a.L);

@@ -421,6 +421,18 @@ __device__ __forceinline__ Tile make_cluster_tile(const Geom &g, const SegPlan &
     return t;
 }
 
+// The rows of an FP64 tile (L lines, G = C segments) that block `rank` holds.
+template <int DIR>
+__device__ __forceinline__ Tile make_seq_tile(const Geom &g, const SegPlan &pl, int L, int rank) {
+    Tile t = make_tile_at<DIR>(g, L, (int)blockIdx.x / pl.C, blockIdx.y);
+    const int n0 = seg_row0(pl, rank);
+    t.N = seg_row0(pl, rank + 1) - n0;
+    t.base += (unsigned)n0 * t.sn;
+    if (DIR == 1) t.cj = n0;
+    if (DIR == 2) t.ck = n0;
+    return t;
+}
+
 // Point p of a tile: consecutive threads touch consecutive global addresses
 // (position-major for x-lines, line-major otherwise).  L is a power of two
 // (lgL its logarithm); division by the x-line length uses a precomputed
@@ -525,6 +537,10 @@ extern __shared__ __align__(16) unsigned char smem_raw[];
 
 // Elements of one array of a segmented tile.
 __host__ __device__ inline int seg_stride(int N, int P, int G, int pad) { return N * P + (G - 1) * pad; }
+
+// Elements of one buffer of an FP64 tile of the sequential solves (R rows of L
+// lines): a half-warp's solves on distinct banks.
+__host__ __device__ inline int seq_stride(int R, int L) { return R * L + (L < 16 ? ((L - R * L) & 15) : 0); }
 
 // The same tile for the segmented solves: no line factors, the segments'
 // pads between the rows.
@@ -709,7 +725,7 @@ __device__ __forceinline__ void run_sweep_solves(const SmemPair &sm, const Task 
 // has one field).  A unit is a task's solves on the lines one warp holds.
 template <int SEG, bool FULL, int NT, bool SINGLE>
 __device__ __forceinline__ void run_seg_tasks(const SmemPair &sm, int P, int L, int N, const SegPlan &pl,
-                                              const SegOp &o1, const SegOp &o2, int tid, int nthr) {
+                                              const SegOp<float> &o1, const SegOp<float> &o2, int tid, int nthr) {
     const int lane0 = tid & ((1 << pl.lgLW) - 1), seg = (tid & 31) >> pl.lgLW;
     const int groups = max(1, L >> pl.lgLW);
     for (int u = tid >> 5; u < NT * groups; u += nthr >> 5) {
