@@ -313,23 +313,27 @@ SegPlan seg_plan(int N, bool pair, int maxG = 16, int step = 8) {
     return best;
 }
 
-// The line split over a cluster of C blocks, two segments of at most 32 rows
-// each a block.  22 rows at least: a segment's carry then reaches no further
-// than the next one (0.382^22 = 6e-10; the second derivative's 0.188 falls
-// faster).  C = 0 where no C <= 8 gives that.
+// The line split over a cluster of C blocks, B segments of at most 32 rows
+// each a block: one to 256 points, else two.  22 rows at least: a segment's
+// carry then reaches no further than the next one (0.382^22 = 6e-10, a
+// hundredth of an FP32 rounding; the second derivative's 0.188 falls faster).  C = 0 where no C <= 8 gives that.
 SegPlan cluster_plan(int N, int periodic) {
     SegPlan p{};
-    const int C = (N + 63) / 64;
-    if (!periodic || C > 8 || N < 44 * C) return p;
-    p.SEG = 32;
-    p.C = C;
-    p.G = 2 * C;
-    p.S = (N + p.G - 1) / p.G;
-    p.nS = N - p.G * (p.S - 1);
-    p.full = N == 64 * C;
-    p.lgLW = 4;
-    p.kS = 32 - p.S;
-    p.pair = 1;
+    if (!periodic) return p;
+    for (int B = 1; B <= 2; B++) {
+        const int C = (N + 32 * B - 1) / (32 * B);
+        if (C > 8 || N < 22 * B * C) continue;
+        p.SEG = 32;
+        p.B = B;
+        p.C = C;
+        p.G = B * C;
+        p.S = (N + p.G - 1) / p.G;
+        p.nS = N - p.G * (p.S - 1);
+        p.full = N == 32 * p.G;
+        p.kS = 32 - p.S;
+        p.pair = 1;
+        break;
+    }
     return p;
 }
 
@@ -770,7 +774,7 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
         ALLOC(h->q1.f[f], n * 8);
         ALLOC(h->qk.f[f], n * 8);
         ALLOC(h->q2.f[f], n * 8);
-        ALLOC(h->prim[f], n * h->tb);
+        if (f != 3 || !h->mixed) ALLOC(h->prim[f], n * h->tb);  // (p, mu, amu: not stored by the mixed form)
         ALLOC(h->R[f], n * h->tb);
         ALLOC(h->ft1[f], n * h->tb);
         ALLOC(h->ft2[f], n * h->tb);
@@ -788,8 +792,10 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
             if (h->mixed_rk4) ALLOC(h->rfluct[f], n * 4);
         }
     }
-    ALLOC(h->mu, n * h->tb);
-    ALLOC(h->amu, n * h->tb);
+    if (!h->mixed) {
+        ALLOC(h->mu, n * h->tb);
+        ALLOC(h->amu, n * h->tb);
+    }
     ALLOC(h->scal, 8 * sizeof(double));
     ALLOC(h->flag, 4 * sizeof(int));
     ALLOC(h->red, 1024 * 8 * sizeof(double));
@@ -866,7 +872,7 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
             while (L > 2 && (long long)h->seg[d].C * ((other + L - 1) / L) * planes < 152) L /= 2;
         } else if (h->seg[d].C) {
             h->L[d] = kClusterLines;
-            h->threads[d] = kTpbYZ;
+            h->threads[d] = 256 * h->seg[d].B;
         }
         h->Lf[d] = pick_L(h->tb, h->mixed ? 10 : 5, Nd[d], d == 0 ? 1 : 0);
         // a mixed filter tile narrower than 8 lines within 72 kB (N = 256: 4
@@ -1109,7 +1115,8 @@ static int run_stage(cs3d_handle *h, int st, int last) {
     a.mixed_rk4 = h->mixed_rk4;
     for (int f = 0; f < 5; f++) {
         a.fluct[f] = h->rfluct[f];
-        a.fref[f] = h->fref[f];
+        a.fref_hi[f] = (float)h->fref[f];
+        a.fref_lo[f] = (float)(h->fref[f] - (double)a.fref_hi[f]);
     }
     a.fluct_out = h->mixed_rk4 && last && filtered;
     // FP32 shadow written by the z sweep: the next stage's input, or -- after
@@ -1173,6 +1180,8 @@ static int run_stage(cs3d_handle *h, int st, int last) {
                 void **dst = pass == 0 ? h->ft1 : h->ft2;
                 for (int f = 0; f < 5; f++) {
                     fa.ref[f] = h->mixed ? h->fref[f] : 0.0;
+                    fa.ref_hi[f] = (float)fa.ref[f];
+                    fa.ref_lo[f] = (float)(fa.ref[f] - (double)fa.ref_hi[f]);
                     // first pass: q2 - fref, in FP32 from the last stage (mixed
                     // RK4) or formed here from FP64 q2
                     const bool fl = pass == 0 && h->mixed_rk4;

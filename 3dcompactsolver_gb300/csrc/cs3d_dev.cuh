@@ -60,8 +60,8 @@ struct SegPlan {
     int pad;   // full only: shared-memory elements between a line's segments
     int kS;    // SEG - S
     int pair;  // array elements are float2 (y and z sweeps), else float
-    int C;     // > 0: a cluster of C blocks holds the line, two segments each
-               // (G = 2 C, not restricted to a power of two)
+    int C, B;  // C > 0: a cluster of C blocks holds the line, B segments each
+               // (G = B C, not restricted to a power of two)
 };
 
 // A periodic operator in that form: -l, the scaled taps (centre outwards),
@@ -152,6 +152,31 @@ __device__ __forceinline__ float narrow(double d) {
     bits = e32 <= 0 ? 0u : (e32 >= 255 ? 0x7f800000u : bits);
     bits = bits > 0x7f800000u ? 0x7f800000u : bits;
     return __uint_as_float(sign | bits);
+}
+
+// d as the unevaluated sum of two floats: hi its leading 24 bits, lo the next
+// 23, by integer instructions.  |d| below 2^-70 (or not finite): hi alone.
+__device__ __forceinline__ void split(double d, float &hi, float &lo) {
+    const unsigned h = (unsigned)__double2hiint(d), l = (unsigned)__double2loint(d);
+    const unsigned sign = h & 0x80000000u;
+    const int e32 = (int)((h >> 20) & 0x7ffu) - 896;
+    // truncated, so that the low 29 mantissa bits are the remainder
+    unsigned b = ((unsigned)e32 << 23) | ((h & 0xfffffu) << 3) | (l >> 29);
+    b = e32 <= 0 ? 0u : (e32 >= 255 ? 0x7f800000u : b);
+    hi = __uint_as_float(sign | b);
+    // the upper 23 of them as a float in [0, 1) ulp of hi
+    const float r = __uint_as_float(0x3f800000u | ((l >> 6) & 0x7fffffu)) - 1.0f;
+    const bool small = e32 <= 57 || e32 >= 255;
+    lo = small ? 0.0f : r * __uint_as_float(sign | ((unsigned)(e32 - 23) << 23));
+}
+
+// q - ref in FP32 (ref = ref_hi + ref_lo): both parts' differences, each exact
+// or rounded relative to the result.  An FP64 subtraction here would double
+// the last stage's work on the FP64 pipe.
+__device__ __forceinline__ float fluct_of(double q, float ref_hi, float ref_lo) {
+    float hi, lo;
+    split(q, hi, lo);
+    return (hi - ref_hi) + (lo - ref_lo);
 }
 
 // Work-precision <-> FP64 without the FP64 conversion pipe.

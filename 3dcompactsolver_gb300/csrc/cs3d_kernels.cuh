@@ -70,7 +70,7 @@ struct SweepArgs {
     const float *q1s[5];    // FP32 shadow of q1 (mixed RK4, stages 2-3)
     float *fluct[5];        // mixed RK4: q2 - fref in FP32, the filter's first input
     int fluct_out;          // mixed RK4, last stage of a filtered step: write fluct
-    double fref[5];         // the filter's per-field reference values
+    float fref_hi[5], fref_lo[5];  // the filter's per-field reference values, as sums of two floats
     float *shadow_out[5];   // FP32 shadow of the next stage input (mixed)
     int shadow_target;      // ShadowTarget
     int mixed_rk4;          // mixed form with RK4: qk kept only as FP32 shadow
@@ -99,7 +99,8 @@ struct FilterArgs {
     Q5 delta_from;     // mixed last pass: q1 = q2 + (filtered - unfiltered)
     const float *unf[5];   // mixed last pass: the unfiltered first-pass input, if kept
     float *shadow_out[5];  // mixed last pass: FP32 shadow of q1
-    double ref[5];     // per-field reference value subtracted on entry
+    double ref[5];     // per-field reference value subtracted on entry,
+    float ref_hi[5], ref_lo[5];  // and as a sum of two floats
 };
 
 struct LineOpArgs {

@@ -272,17 +272,18 @@ __device__ __forceinline__ void seg_filter(const SegLane<R> &s, int P, const Seg
 // ---------------------------------------------------------------------
 // A tile of 32 neighbouring lines is 128 bytes a row, whole memory lines; 16
 // solves of 32 lines fit one SM's shared memory for 64 rows only, so a cluster
-// of C blocks holds the line, two segments (kClRows rows at most) a block.  Halo
-// rows are read from the neighbours' shared memory; the carries (T = 1: the
-// plan keeps segments long enough for the nearest neighbour alone) go through
-// a mailbox forward, and backward through the row that the receiving lane
-// itself overwrites next.  A warp holds 16 lines' two segments.
+// of C blocks holds the line, B = one or two 32-row segments a block.  One (up to
+// 256 points) leaves room for two blocks an SM, one solving while the other's
+// loads and stores run.  Halo rows are read from the neighbours' shared memory;
+// the carries (T = 1: the plan keeps segments long enough for the nearest
+// neighbour alone) go through a mailbox forward, and backward through the row
+// that the receiving lane itself overwrites next.
 // Why: beyond the L2 the memory system delivers in proportion to the bytes a
 // tile's row takes of its 128-byte line -- a copy kernel of z tiles on 256^3
 // measured 2.0 / 3.9 / 6.5 TB/s at 8 / 16 / 32 FP32 lines a row (5.2 / 5.6 /
 // 5.3 TB/s at 128^3, which the L2 holds).  The 8-line tiles that whole lines
 // leave room for at N = 256: z 6.66 ms a step; clusters of 4: 4.03.
-constexpr int kClRows = 64, kClLines = 32, kClWarps = 16;  // (kClLines: kClusterLines)
+constexpr int kClLines = 32;  // (kClusterLines)
 
 __device__ __forceinline__ void cluster_sync() {
     __syncwarp();
@@ -296,27 +297,28 @@ __device__ __forceinline__ E *cluster_map(E *p, int rank) {
     return r;
 }
 
-// The solves of a sweep tile (tasks as run_seg_tasks), one unit a warp: task
-// warp / 2, lines 16 (warp & 1) + lane.  mail: 2 * 8 * kClLines floats.  Every
-// thread of every block of the cluster calls it.
+// The solves of a sweep tile (tasks as run_seg_tasks), one unit a warp: pl.B
+// segments of 32 / pl.B lines of one task.  mail: 2 * 8 * kClLines floats.
+// Every thread of every block of the cluster calls it.
 template <bool FULL, int NT, bool SINGLE>
 __device__ __forceinline__ void run_cluster_tasks(float2 *tile, int pstride2, float2 *mail, const SegPlan &pl,
                                                   const SegOp<float> &o1, const SegOp<float> &o2, int rank, int tid) {
     constexpr int SEG = 32, P = kClLines;
-    const int warp = tid >> 5, t = warp >> 1, half = (tid >> 4) & 1;
-    const int l = ((warp & 1) << 4) | (tid & 15);
+    const int B = pl.B, warp = tid >> 5, t = B == 2 ? warp >> 1 : warp, half = B == 2 ? (tid >> 4) & 1 : 0;
+    const int l = B == 2 ? ((warp & 1) << 4) | (tid & 15) : tid & 31;
     const int C = pl.C, prev = rank > 0 ? rank - 1 : C - 1, next = rank < C - 1 ? rank + 1 : 0;
-    const int seg = 2 * rank + half;
+    const int seg = B * rank + half;
+    const bool first = half == 0, last = half == B - 1;  // of this block
     float2 *line = tile + t * pstride2 + l;
     SegLane<float2> s;
     s.seg = seg;
-    const int n0 = seg_row0(pl, seg) - seg_row0(pl, 2 * rank), len = pl.S - (seg >= pl.nS);
+    const int n0 = seg_row0(pl, seg) - seg_row0(pl, B * rank), len = pl.S - (seg >= pl.nS);
     s.k0 = FULL ? 0 : SEG - len;
     s.row = line + (n0 - s.k0) * P;
     // (rows of the previous block: its last row precedes this block's first)
-    const int nprev = FULL ? kClRows : seg_row0(pl, 2 * prev + 2) - seg_row0(pl, 2 * prev);
-    s.lo = half ? cluster_map(s.row, rank) : cluster_map(line + (nprev - s.k0) * P, prev);
-    s.hi = half ? cluster_map(line, next) : cluster_map(line + (n0 + len) * P, rank);
+    const int nprev = FULL ? SEG * B : seg_row0(pl, B * (prev + 1)) - seg_row0(pl, B * prev);
+    s.lo = first ? cluster_map(line + (nprev - s.k0) * P, prev) : cluster_map(s.row, rank);
+    s.hi = last ? cluster_map(line, next) : cluster_map(line + (n0 + len) * P, rank);
     const bool dd = t < 4, single = SINGLE && t == NT - 1;
     float y1[SEG], y2[SEG];
     float2 e;
@@ -334,9 +336,9 @@ __device__ __forceinline__ void run_cluster_tasks(float2 *tile, int pstride2, fl
     in.x = __shfl_sync(0xffffffffu, e.x, tid & 15);
     in.y = __shfl_sync(0xffffffffu, e.y, tid & 15);
     float2 *box = mail + t * kClLines + l;
-    if (half) *cluster_map(box, next) = e;
+    if (last) *cluster_map(box, next) = e;
     cluster_sync();  // the forward carries are there, and every window has been read
-    if (!half) in = *box;
+    if (first) in = *box;
     if (dd) {
         e = make_float2(seg_bwd<SEG, FULL, kSegRows1>(y1, o1, pl, s.k0, in.x),
                         seg_bwd<SEG, FULL, kSegRows2>(y2, o2, pl, s.k0, in.y));
@@ -349,9 +351,9 @@ __device__ __forceinline__ void run_cluster_tasks(float2 *tile, int pstride2, fl
     in.x = __shfl_sync(0xffffffffu, e.x, (tid & 15) | 16);
     in.y = __shfl_sync(0xffffffffu, e.y, (tid & 15) | 16);
     // the previous block's last row of this line, stored next by its own lane
-    if (!half) *cluster_map(line + (nprev - 1) * P, prev) = e;
+    if (first) *cluster_map(line + (nprev - 1) * P, prev) = e;
     cluster_sync();  // (the last access to another block's shared memory)
-    if (half) in = s.row[(SEG - 1) * P];
+    if (last) in = s.row[(SEG - 1) * P];
     if (dd) {
         seg_end<SEG, kSegRows1>(y1, o1, in.x);
         seg_end<SEG, kSegRows2>(y2, o2, in.y);

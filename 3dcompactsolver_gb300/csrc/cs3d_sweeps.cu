@@ -42,13 +42,19 @@ namespace cs3d {
 constexpr int kFilterBatch = 4;         // the mixed filter's load and store loops
 constexpr int kFilterConsumeBatch = 2;  // the mixed filter's consume loop
 constexpr int kYConsumeBatch = 4;       // the y sweep's consume phase
-constexpr int kZUpdateBatch = 2;        // the z sweep's RK-update pass
 // Resident blocks per SM the mixed-form kernels are compiled for: the filter
 // at 4 (64 registers), the x sweep at 3 blocks of 256 threads (80 registers),
 // y and z at one block of 512 (128 registers); the plain form runs 128
 // threads, 2 blocks.
 constexpr int kFilterMinBlocks = 4;
 constexpr int kMinBlocksX = 3, kMinBlocksY = 1, kMinBlocksZ = 1;
+
+// Mixed form: the y and z sweeps form the pressure from what they read anyway
+// and the viscosity and its slope from T (a hardware log2 and exp2), so that x
+// stores neither: 32 of about 380 bytes a point and stage.  The plain form,
+// bound by FP64 issue, stores them.
+template <typename T>
+constexpr bool kRecompute = sizeof(T) == 4;
 
 // The sweep kernels take the shared-memory pitch of their tile as a template
 // parameter PC (0: read at run time).  The launcher instantiates the mixed
@@ -221,7 +227,8 @@ __global__ void __launch_bounds__(sweep_threads<T>(0), sizeof(T) == 4 && (SEG ==
             const unsigned gi = in.pt.gi;
             PrimW<T> s = prim_w<T>(gp, in.q[0], in.q[1], in.q[2], in.q[3], in.q[4]);
             a.prim[0][gi] = s.U; a.prim[1][gi] = s.V; a.prim[2][gi] = s.W;
-            a.prim[3][gi] = s.p; a.prim[4][gi] = s.Tt;
+            a.prim[4][gi] = s.Tt;
+            if constexpr (!kRecompute<T>) a.prim[3][gi] = s.p;
             // stage-start primitives: on stage 1, points of SPONGE faces (not
             // on a wall) use the state before the previous step's sponge
             // overwrite, which the reference's U,V,W,p,T arrays still hold.
@@ -269,9 +276,11 @@ __global__ void __launch_bounds__(sweep_threads<T>(0), sizeof(T) == 4 && (SEG ==
             const Zn<T> zz = TS::z(a.d1, a.d2, p.n);
             const T U = in.v[0], V = in.v[1], W = in.v[2], Tt = in.v[3];
             const T vz = muref * visc_rpow(Tt);
-            const T mu = vz * Tt, amu = (T)0.76 * vz;
-            a.mu[gi] = mu;
-            a.amu[gi] = amu;
+            const T mu = vz * Tt;
+            if constexpr (!kRecompute<T>) {
+                a.mu[gi] = mu;
+                a.amu[gi] = (T)0.76 * vz;
+            }
             T Ux, Uxx, Vx, Vxx, Wx, Wxx, Tx, Txx, cex, f1, f2, f3;
             TS::two(sm, 0, p, L, zz.z1, zz.z2, Ux, Uxx);
             TS::two(sm, 1, p, L, zz.z1, zz.z2, Vx, Vxx);
@@ -323,7 +332,7 @@ __global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBloc
     const Tile t = SQ ? make_seq_tile<1>(a.g, a.seg, L, rank)
                       : CL ? make_cluster_tile<1>(a.g, a.seg, rank) : make_tile<1>(a.g, L);
     const int N = t.N, NL = N * L, pad = FULL && !CL ? a.seg.pad : 0;
-    const auto sm = TS::at(SQ ? kSeqN1Y : sizeof(T) == 4 ? YNB2 : YNB, L, P, SQ ? (a.seg.C > 1 ? a.seg.S : N) : CL ? kClRows : N, a.seg);
+    const auto sm = TS::at(SQ ? kSeqN1Y : sizeof(T) == 4 ? YNB2 : YNB, L, P, SQ ? (a.seg.C > 1 ? a.seg.S : N) : CL ? 32 * a.seg.B : N, a.seg);
     struct InA { Pt pt; T v[11]; };
     batched<InA, sizeof(T) == 4 ? 4 : 2>(NL,
         [&](InA &in, int p) {
@@ -332,7 +341,8 @@ __global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBloc
 #pragma unroll
             for (int f = 0; f < 4; ++f) in.v[f] = a.qs[f + 1][gi];
 #pragma unroll
-            for (int f = 0; f < 5; ++f) in.v[4 + f] = a.prim[f][gi];
+            for (int f = 0; f < 5; ++f)
+                if (f != 3 || !kRecompute<T>) in.v[4 + f] = a.prim[f][gi];
             in.v[9] = a.dx[0][gi];
             in.v[10] = a.dx[1][gi];
         },
@@ -340,7 +350,8 @@ __global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBloc
             if (!in.pt.ok) return;
             const int o = in.pt.o;
             const T ru = in.v[0], rv = in.v[1], rw = in.v[2], re = in.v[3];
-            const T V = in.v[5], pp = in.v[7];
+            const T V = in.v[5];
+            const T pp = kRecompute<T> ? pressure<T>(a.gas, ru, rv, rw, re, in.v[4], V, in.v[6]) : in.v[7];
             TS::put1f(sm, 0, o, in.v[4]);
             TS::put1f(sm, 1, o, V);
             TS::put1f(sm, 2, o, in.v[6]);
@@ -363,14 +374,14 @@ __global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBloc
         run_sweep_solves<2, PC>(sm, sizeof(T) == 4 ? kTasksY2 : kTasksY, 8, L, t.nlines, a.d1, a.d2, threadIdx.x,
                                 blockDim.x, YDUM);
     __syncthreads();
-    const T c43 = T(4.0 / 3.0), c13 = T(1.0 / 3.0), cpPr = (T)a.gas.cpPr;
+    const T c43 = T(4.0 / 3.0), c13 = T(1.0 / 3.0), cpPr = (T)a.gas.cpPr, muref = (T)a.gas.mu_ref;
     struct InC { Pt pt; T v[9]; };
     batched<InC, sizeof(T) == 4 ? kYConsumeBatch : 2>(NL,
         [&](InC &in, int p) {
             in.pt = point<1>(t, p, L, P, lgL, a.divN, pad);
             const unsigned gi = in.pt.gi;
             in.v[0] = a.prim[0][gi]; in.v[1] = a.prim[1][gi]; in.v[2] = a.prim[2][gi];
-            in.v[3] = a.mu[gi];
+            in.v[3] = kRecompute<T> ? a.prim[4][gi] : a.mu[gi];
 #pragma unroll
             for (int f = 0; f < 5; ++f) in.v[4 + f] = a.R[f][gi];
         },
@@ -379,7 +390,8 @@ __global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBloc
             const Pt &p = in.pt;
             const unsigned gi = p.gi;
             const Zn<T> zz = TS::z(a.d1, a.d2, p.n);
-            const T U = in.v[0], V = in.v[1], W = in.v[2], mu = in.v[3];
+            const T U = in.v[0], V = in.v[1], W = in.v[2];
+            const T mu = kRecompute<T> ? muref * visc_rpow(in.v[3]) * in.v[3] : in.v[3];
             T Uy, Uyy, Vy, Vyy, Wy, Wyy, Ty, Tyy, Uxy, Vxy, cey, f1, f2, f3;
             TS::two(sm, 0, p, L, zz.z1, zz.z2, Uy, Uyy);
             TS::two(sm, 1, p, L, zz.z1, zz.z2, Vy, Vyy);
@@ -439,7 +451,8 @@ struct ZSweep {
 #pragma unroll
                 for (int f = 0; f < 4; ++f) in.v[f] = a.qs[f + 1][gi];
 #pragma unroll
-                for (int f = 0; f < 5; ++f) in.v[4 + f] = a.prim[f][gi];
+                for (int f = 0; f < 5; ++f)
+                    if (f != 3 || !kRecompute<T>) in.v[4 + f] = a.prim[f][gi];
                 in.v[9] = a.dx[0][gi];
                 in.v[10] = a.dy[1][gi];
                 in.v[11] = a.dx[2][gi];
@@ -449,7 +462,8 @@ struct ZSweep {
                 if (!in.pt.ok) return;
                 const int o = in.pt.o;
                 const T ru = in.v[0], rv = in.v[1], rw = in.v[2], re = in.v[3];
-                const T W = in.v[6], pp = in.v[7];
+                const T W = in.v[6];
+                const T pp = kRecompute<T> ? pressure<T>(a.gas, ru, rv, rw, re, in.v[4], in.v[5], W) : in.v[7];
                 TS::put1f(sm, 0, o, in.v[4]);
                 TS::put1f(sm, 1, o, in.v[5]);
                 TS::put1f(sm, 2, o, W);
@@ -480,6 +494,7 @@ struct ZSweep {
         const int L = CL && !SQ ? kClLines : a.L, P = PC > 0 ? PC : a.P, lgL = CL && !SQ ? 5 : a.lgL;
         const int NL = t.N * L, pad = FULL && !CL ? a.seg.pad : 0;
         const T c43 = T(4.0 / 3.0), c13 = T(1.0 / 3.0), c23 = T(2.0 / 3.0), cpPr = (T)a.gas.cpPr;
+        const T muref = (T)a.gas.mu_ref;
         const double dt = *a.dt;
         const T dtw = (T)dt;
         const int st = a.rk_step;
@@ -495,37 +510,51 @@ struct ZSweep {
         const bool need_qb = (!tvd && !a.mixed_rk4 && st > 1 && st < 4) || (tvd && st > 1);
         const bool need_q1s = a.mixed_rk4 && st > 1 && st < 4;
         const bool need_qs = a.mixed_rk4 && st == 1;
-        // Phase C runs in two passes over the same points, each point by the same
-        // thread in both (so no barrier between them): C1 forms the right-hand
-        // side and parks dq = dt*RHS in the point's own, now unused, solve slots;
-        // C2 streams the FP64 state through the RK update.  Each pass keeps fewer
-        // values live than one fused pass, so more points' loads are in flight.
+        // Right-hand side and update of a point in one pass: the FP64 additions
+        // of the update (two an SM and clock) run under the other warps' FP32
+        // work and loads.  As two passes over the tile, the update alone took 8.5 of a
+        // block's 20 us at 128^3.
         static_assert(ZS == ZS_ && ZF1 == ZS_ + 4, "dq slots");
-        struct InC1 {
+        struct InC {
             Pt pt;
             T v[18];
-            T qsv[5];
+            double qa[5];
+            double qb[5];  // FP64 state, or q1's FP32 shadow in the low word
         };
-        pipelined<InC1>(NL, tid, nthr,
-            [&](InC1 &in, int p) {
+        batched<InC, 1>(NL, tid, nthr,
+            [&](InC &in, int p) {
                 in.pt = point<2>(t, p, L, P, lgL, a.divN, pad);
                 const unsigned gi = in.pt.gi;
                 in.v[0] = a.prim[0][gi]; in.v[1] = a.prim[1][gi]; in.v[2] = a.prim[2][gi];
-                in.v[3] = a.mu[gi]; in.v[4] = a.amu[gi];
+                if constexpr (kRecompute<T>) {
+                    in.v[3] = a.prim[4][gi];
+                } else {
+                    in.v[3] = a.mu[gi];
+                    in.v[4] = a.amu[gi];
+                }
 #pragma unroll
                 for (int f = 0; f < 4; ++f) { in.v[5 + f] = a.dx[f][gi]; in.v[9 + f] = a.dy[f][gi]; }
 #pragma unroll
                 for (int f = 0; f < 5; ++f) {
                     in.v[13 + f] = a.R[f][gi];
-                    in.qsv[f] = a.sponge ? a.qs[f][gi] : T(0);
+                    in.qa[f] = use_q1a ? a.q1.f[f][gi] : a.q2.f[f][gi];
+                    if constexpr (sizeof(T) == 4) {
+                        if (need_qs || need_q1s)
+                            in.qb[f] = __hiloint2double(0, __float_as_int(need_qs ? a.qs[f][gi] : a.q1s[f][gi]));
+                        else in.qb[f] = need_qb ? a.qk.f[f][gi] : 0.0;
+                    } else {
+                        in.qb[f] = need_qb ? (tvd ? a.qk.f[f][gi] : a.q1.f[f][gi]) : 0.0;
+                    }
                 }
             },
-            [&](InC1 &in) {
+            [&](InC &in) {
                 if (!in.pt.ok) return;
                 const Pt &p = in.pt;
                 const unsigned gi = p.gi;
                 const Zn<T> zz = TS::z(a.d1, a.d2, p.n);
-                const T U = in.v[0], V = in.v[1], W = in.v[2], mu = in.v[3], amu = in.v[4];
+                const T U = in.v[0], V = in.v[1], W = in.v[2];
+                const T vz = kRecompute<T> ? muref * visc_rpow(in.v[3]) : T(0);
+                const T mu = kRecompute<T> ? vz * in.v[3] : in.v[3], amu = kRecompute<T> ? (T)0.76 * vz : in.v[4];
                 const T Ux = in.v[5], Vx = in.v[6], Wx = in.v[7], Tx = in.v[8];
                 const T Uy = in.v[9], Vy = in.v[10], Wy = in.v[11], Ty = in.v[12];
                 T Uz, Uzz, Vz, Vzz, Wz, Wzz, Tz, Tzz, S, Wxz, Wyz, cez, f1, f2, f3, f4;
@@ -558,10 +587,10 @@ struct ZSweep {
                 T src0 = T(0);
                 if (a.sponge) {  // sigma (avg - q), SpongeBC / CSolver_AWS.hpp:228
                     const T sg = to_work<T>(a.sigma[gi]);
-                    src0 = sg * (to_work<T>(a.savg.f[0][gi]) - in.qsv[0]);
+                    src0 = sg * (to_work<T>(a.savg.f[0][gi]) - a.qs[0][gi]);
 #pragma unroll
                     for (int f = 1; f < 5; ++f)
-                        R[f] += (f == 4 ? T(2.0) * sg : sg) * (to_work<T>(a.savg.f[f][gi]) - in.qsv[f]);
+                        R[f] += (f == 4 ? T(2.0) * sg : sg) * (to_work<T>(a.savg.f[f][gi]) - a.qs[f][gi]);
                 }
                 // continuity and the post-step boundary fix-up (CSolver_AWS.cpp:1506-1679)
                 int i, j, k;
@@ -588,33 +617,13 @@ struct ZSweep {
                     T d = sizeof(T) == 8 ? (T)(dt * (double)R[f]) : dtw * R[f];
                     if (zero_all || (f > 0 && zero_mom)) d = T(0);
                     if (a.dq_out[0]) a.dq_out[f][gi] = to_f64(d);
-                    TS::dq(sm, f, p.o) = d;
+                    R[f] = d;
                 }
-            });
-        struct InC2 {
-            Pt pt;
-            double qa[5], qb[5];
-            T qsv[5];    // q1's shadow: the stage input qs on stage 1, q1s on 2-3
-        };
-        batched<InC2, kZUpdateBatch>(NL, tid, nthr,
-            [&](InC2 &in, int p) {
-                in.pt = point<2>(t, p, L, P, lgL, a.divN, pad);
-                const unsigned gi = in.pt.gi;
-#pragma unroll
-                for (int f = 0; f < 5; ++f) {
-                    in.qa[f] = use_q1a ? a.q1.f[f][gi] : a.q2.f[f][gi];
-                    in.qb[f] = need_qb ? (tvd ? a.qk.f[f][gi] : a.q1.f[f][gi]) : 0.0;
-                    in.qsv[f] = need_qs ? a.qs[f][gi] : need_q1s ? (T)a.q1s[f][gi] : T(0);
-                }
-            },
-            [&](InC2 &in) {
-                if (!in.pt.ok) return;
-                const unsigned gi = in.pt.gi;
                 if (sizeof(T) == 8) {
                     // plain form: the reference's RK update in FP64
 #pragma unroll
                     for (int f = 0; f < 5; ++f) {
-                        const double d = (double)TS::dq(sm, f, in.pt.o);
+                        const double d = (double)R[f];
                         if (tvd) {  // TVD-RK3 (TVDRK3.hpp:38-96); qa = q1, qb = qk
                             if (st == 1) a.qk.f[f][gi] = in.qa[f] + d;
                             else if (st == 2) a.qk.f[f][gi] = 0.75 * in.qa[f] + 0.25 * in.qb[f] + 0.25 * d;
@@ -631,7 +640,7 @@ struct ZSweep {
                     // mixed form: the FP32 increment accumulated into the FP64 state
 #pragma unroll
                     for (int f = 0; f < 5; ++f) {
-                        const T d = TS::dq(sm, f, in.pt.o);
+                        const T d = R[f];
                         if (tvd) {
                             const double dd = to_f64(d);
                             double nv;
@@ -647,11 +656,11 @@ struct ZSweep {
                             a.q2.f[f][gi] = q2n;
                             if (st < 4) {
                                 // the next stage input qk = q1 + cb*dq, kept as an FP32 shadow
-                                a.shadow_out[f][gi] = fma(cb, d, in.qsv[f]);
+                                a.shadow_out[f][gi] = fma(cb, d, (T)__int_as_float(__double2loint(in.qb[f])));
                             } else {
                                 if (a.shadow_target == SHADOW_Q2) a.shadow_out[f][gi] = narrow(q2n);
                                 // the filter's first pass input, q2 - fref in FP32
-                                if (a.fluct_out) a.fluct[f][gi] = narrow(q2n - a.fref[f]);
+                                if (a.fluct_out) a.fluct[f][gi] = fluct_of(q2n, a.fref_hi[f], a.fref_lo[f]);
                             }
                         }
                     }
@@ -668,7 +677,7 @@ __global__ void __launch_bounds__(sweep_threads<T>(2), sizeof(T) == 4 ? kMinBloc
     const int rank = CL ? (int)blockIdx.x % a.seg.C : 0;
     const Tile t = Z::SQ ? make_seq_tile<2>(a.g, a.seg, a.L, rank)
                          : CL ? make_cluster_tile<2>(a.g, a.seg, rank) : make_tile<2>(a.g, a.L);
-    const auto sm = Z::TS::at(Z::SQ ? kSeqN1Z : ZNB, a.L, PC > 0 ? PC : a.P, Z::SQ ? (a.seg.C > 1 ? a.seg.S : t.N) : CL ? kClRows : t.N, a.seg);
+    const auto sm = Z::TS::at(Z::SQ ? kSeqN1Z : ZNB, a.L, PC > 0 ? PC : a.P, Z::SQ ? (a.seg.C > 1 ? a.seg.S : t.N) : CL ? 32 * a.seg.B : t.N, a.seg);
     Z::load(a, t, sm, threadIdx.x, blockDim.x);
     if constexpr (CL) cluster_sync();
     else __syncthreads();
@@ -793,7 +802,7 @@ k_filter_seg(FilterArgs<T> a) {
 #pragma unroll
             for (int f = 0; f < 5; ++f) {
                 if constexpr (sizeof(T) == 8) in.v[f] = a.src64.f[0] ? a.src64.f[f][gi] : a.src32[f][gi];
-                else in.v[f] = a.src64.f[0] ? narrow(a.src64.f[f][gi] - a.ref[f]) : a.src32[f][gi];
+                else in.v[f] = a.src64.f[0] ? fluct_of(a.src64.f[f][gi], a.ref_hi[f], a.ref_lo[f]) : a.src32[f][gi];
             }
         },
         [&](In &in) {
@@ -842,7 +851,7 @@ k_filter_seg(FilterArgs<T> a) {
                     // q1 = q2 + (filtered - unfiltered); the unfiltered value is
                     // the first pass's FP32 input, or formed again from q2 (the
                     // same number either way)
-                    const float v0 = a.unf[0] ? o.u[f] : narrow(o.q[f] - a.ref[f]);
+                    const float v0 = a.unf[0] ? o.u[f] : fluct_of(o.q[f], a.ref_hi[f], a.ref_lo[f]);
                     const double nv = o.q[f] + widen(v - v0);
                     a.dst64.f[f][gi] = nv;
                     a.shadow_out[f][gi] = narrow(nv);
@@ -913,7 +922,7 @@ size_t sweep_smem_bytes(int prec_bytes, int nbuf, int L, int P, int N, const Seg
     // the buffers and the mailboxes (a line's rows here: one block's, or all)
     if (prec_bytes == 8 && seg && seg->SEG)
         return 8 * (size_t)nbuf * (seq_stride(seg->C > 1 ? seg->S : N, L) + (seg->G > 1 ? 4 * L : 0));
-    if (prec_bytes == 4 && seg && seg->C) return 8 * (8 * (size_t)kClRows * kClLines + 8 * kClLines);
+    if (prec_bytes == 4 && seg && seg->C) return 8 * (8 * (size_t)(32 * seg->B) * kClLines + 8 * kClLines);
     if (prec_bytes == 4 && seg && seg->SEG && !seg->pair) return (size_t)XNB * 4 * seg_stride(N, P, seg->G, seg->pad);
     // segmented solves: the pair arrays alone (no line factors, no read-ahead)
     if (prec_bytes == 4 && seg && seg->SEG) return (size_t)((nbuf + 1) / 2) * 4 * seg_pair_stride(N, P, seg->G, seg->pad);

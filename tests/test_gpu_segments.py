@@ -7,9 +7,10 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-# one block: 17..43, 65..87, 129..131; clusters: 44..64, 88..128, 132..512
-LENGTHS = [16, 17, 18, 31, 32, 33, 43, 44, 63, 64, 65, 77, 87, 88, 101, 127, 128, 129, 131, 132, 176, 191, 192, 193,
-           256, 257, 320, 511, 512, 513]
+# clusters of one-segment blocks: 22..32, 44..64, 66..256; of two-segment
+# blocks: 264..512; one block: the others
+LENGTHS = [16, 17, 18, 21, 22, 31, 32, 33, 42, 43, 44, 63, 64, 65, 66, 77, 96, 97, 101, 127, 128, 129, 131, 176, 192, 193,
+           256, 257, 263, 264, 320, 511, 512, 513]
 
 # One RK4 step plus filter of a state of order one at CFL 0.5: each of the four
 # stages and the filter adds at most about four FP32 roundings (2^-24) of terms
