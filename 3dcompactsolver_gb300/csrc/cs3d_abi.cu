@@ -512,12 +512,14 @@ struct cs3d_handle {
     SegOp<float> segop[3][2] = {};  // 1st and 2nd derivative
     SegPlan segf[3] = {};    // the filter's, and its correction operator
     SegOp<float> segfop[3] = {};
+    // FP64 lines in register segments (post-processor, FP64 adjoint)
+    SegPlan segr[3] = {};
+    SegOp<double> segrop[3][3] = {};
     SeqOp seqop[3][2] = {};  // plain form: the sequential solves (plan in seg)
     double *seqpw[3][2] = {};
     SegOp<double> segfop64[3] = {};
     // tiles
     int L[3] = {1, 1, 1}, Lf[3] = {1, 1, 1}, threads[3] = {128, 128, 128};
-    int Lt[3] = {1, 1, 1}, threads_t[3] = {128, 128, 128};  // the transposed sweeps of the mixed adjoint
     // step state
     int timeStep = 0, filterTimeStep = 0;
     int ic_done = 0;
@@ -548,6 +550,7 @@ struct cs3d_handle {
     double *adj_f[kAdjFields][5] = {};
     double *adj_part = nullptr;
     int adj_nsteps = 0, adj_every = 0;
+    int adj_rec_every = 0;           // the interval that the record's storage was made for
     std::vector<double *> adj_ckpt;  // 5*npts each: the state before step k*adj_every
     std::vector<int> adj_ts, adj_fts;
     double *adj_seg = nullptr;       // adj_every states of the segment being reversed
@@ -821,6 +824,10 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
             if (!r) r = make_line_seg(ho, h->lseg[d][k - 1], h->stream);
             if (!r && k == 3) r = upload_op<float>(make_filter_correction(ho), h->op32fc[d], h->stream);
             if (r) return fail_free(r);
+            if (ho.periodic && factors(ho)) {
+                h->segr[d] = seg_plan(Nd[d], true);
+                h->segrop[d][k - 1] = seg_op<double>(ho, h->segr[d], 60);
+            }
             if (!h->mixed && ho.periodic && k < 3) {
                 h->seg[d] = seq_plan(Nd[d], d);
                 h->seqop[d][k - 1] = seq_op(ho, h->seg[d], &h->seqpw[d][k - 1], h->stream, &r);
@@ -860,7 +867,6 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
                 threads = sweep_threads<float>(d);
             }
         };
-        shape(nullptr, h->Lt[d], h->threads_t[d]);
         shape(&h->seg[d], h->L[d], h->threads[d]);
         const int other = d == 0 ? cfg->Ny : cfg->Nx, planes = d == 2 ? cfg->Ny : cfg->Nz;
         if (!h->mixed && h->seg[d].SEG) {
@@ -1886,10 +1892,27 @@ static int adj_apply(cs3d_handle *h, int d, int kind0, int kind1, std::initializ
     const int N = d == 0 ? h->g.Nx : d == 1 ? h->g.Ny : h->g.Nz;
     a.ntask = (int)tasks.size();
     const int nbuf = sizeof(T) == 4 ? 2 * ((a.ntask + 1) / 2) : a.ntask;
-    a.L = pick_L(sizeof(T), nbuf, N, d == 0 ? 1 : 0, 72, true);
+    // (the filter's operator does not factor where |alphaF| is near 1/2)
+    const bool filt = kind0 >= 2;
+    if constexpr (sizeof(T) == 8) {
+        if (h->segr[d].SEG && h->segrop[d][kind0].T && h->segrop[d][kind1].T) {
+            a.seg = h->segr[d];
+            a.g0 = h->segrop[d][kind0];
+            a.g1 = h->segrop[d][kind1];
+        }
+    } else if (f64io && filt && h->segf[d].SEG) {
+        a.seg = h->segf[d];
+        a.g0 = h->segfop[d];
+    }
+    if (a.seg.SEG) {
+        a.L = 16;
+        while (a.L > 1 && apply_seg_smem((int)sizeof(T), a.ntask, a.L, a.L + (d == 0), N, a.seg) > 72 * 1024) a.L /= 2;
+    } else {
+        a.L = pick_L(sizeof(T), nbuf, N, d == 0 ? 1 : 0, 72, true);
+    }
     a.lgL = ilog2(a.L);
     a.P = a.L + (d == 0 ? 1 : 0);
-    a.threads = apply_threads<T>();
+    a.threads = a.seg.SEG ? apply_seg_threads<T>() : apply_threads<T>();
     a.divN = make_fastdiv((unsigned)N);
     const DevOp<T> *ops = sizeof(T) == 8 ? reinterpret_cast<const DevOp<T> *>(h->op64[d])
                                          : reinterpret_cast<const DevOp<T> *>(h->op32[d]);
@@ -2010,10 +2033,13 @@ static int adj_vjp_tape(cs3d_handle *h, const T *const qin[5], void *const Gv[48
         for (int d = 2; d >= 0; d--) {
             TSweepArgs ta{};
             ta.g = h->g;
-            ta.L = h->Lt[d];
-            ta.lgL = ilog2(h->Lt[d]);
-            ta.P = h->Lt[d] + (d == 0 ? 1 : 0);
-            ta.threads = h->threads_t[d];
+            ta.L = h->L[d];
+            ta.lgL = ilog2(h->L[d]);
+            ta.P = h->L[d] + (d == 0 ? 1 : 0);
+            ta.threads = h->threads[d];
+            ta.seg = h->seg[d];
+            ta.g1 = h->segop[d][0];
+            ta.g2 = h->segop[d][1];
             ta.divN = make_fastdiv((unsigned)(d == 0 ? h->g.Nx : d == 1 ? h->g.Ny : h->g.Nz));
             ta.d1 = h->op32[d][0].op;
             ta.d2 = h->op32[d][1].op;
@@ -2292,33 +2318,43 @@ extern "C" int cs3d_adjoint_record(cs3d_handle *h, int nsteps, int checkpoint_ev
     if (every == 0) every = (int)std::ceil(std::sqrt((double)nsteps));
     if (every > nsteps) every = nsteps;
     CS3D_CUDA(cudaStreamSynchronize(h->stream));
-    for (void *p : h->adj_rec_allocs) cudaFree(p);
-    h->adj_rec_allocs.clear();
-    h->adj_ckpt.clear();
     h->adj_ts.clear();
     h->adj_fts.clear();
     h->adj_nsteps = 0;
     if ((rc = adj_workspace(h))) return rc;
     const size_t n5 = (size_t)h->g.npts * 5;
     const int nseg = (nsteps + every - 1) / every;
-    for (int k = 0; k < nseg; k++) {
-        void *p = nullptr;
-        if ((rc = adj_alloc(h, h->adj_rec_allocs, &p, n5 * 8))) return rc;
-        h->adj_ckpt.push_back((double *)p);
+    // the storage of the last record serves again where its shape is the same
+    // (allocating it cost as much as the four steps themselves at 64^3)
+    if ((int)h->adj_ckpt.size() != nseg || h->adj_rec_every != every || (h->adj_segmode && h->adj_recompute)) {
+        for (void *p : h->adj_rec_allocs) cudaFree(p);
+        h->adj_rec_allocs.clear();
+        h->adj_ckpt.clear();
+        h->adj_rec_every = 0;
+        h->adj_segmode = 0;
+        h->adj_segtape = h->adj_segyin = nullptr;
+        for (int k = 0; k < nseg; k++) {
+            void *p = nullptr;
+            if ((rc = adj_alloc(h, h->adj_rec_allocs, &p, n5 * 8))) return rc;
+            h->adj_ckpt.push_back((double *)p);
+        }
+        if ((rc = adj_alloc(h, h->adj_rec_allocs, (void **)&h->adj_seg, n5 * 8 * (size_t)every))) return rc;
+        h->adj_rec_every = every;
     }
-    if ((rc = adj_alloc(h, h->adj_rec_allocs, (void **)&h->adj_seg, n5 * 8 * (size_t)every))) return rc;
     // segment mode where the tapes and stage inputs of one segment (212 fields
     // in the work precision per step) fit in half of the free device memory
-    h->adj_segmode = 0;
-    h->adj_segtape = h->adj_segyin = nullptr;
-    {
+    if (!h->adj_segmode && !h->adj_recompute) {
         const size_t fb = (size_t)h->g.npts * h->tb;
         const size_t tape_b = (size_t)every * 4 * 48 * fb, yin_b = (size_t)every * 4 * 5 * fb;
         size_t free_b = 0, total_b = 0;
         CS3D_CUDA(cudaMemGetInfo(&free_b, &total_b));
-        if (!h->adj_recompute && tape_b + yin_b <= free_b / 2) {
-            if ((rc = adj_alloc(h, h->adj_rec_allocs, (void **)&h->adj_segtape, tape_b))) return rc;
-            if ((rc = adj_alloc(h, h->adj_rec_allocs, (void **)&h->adj_segyin, yin_b))) return rc;
+        if (tape_b + yin_b <= free_b / 2) {
+            rc = adj_alloc(h, h->adj_rec_allocs, (void **)&h->adj_segtape, tape_b);
+            if (!rc) rc = adj_alloc(h, h->adj_rec_allocs, (void **)&h->adj_segyin, yin_b);
+            if (rc) {
+                h->adj_rec_every = 0;  // (the next record starts afresh)
+                return rc;
+            }
             h->adj_segmode = 1;
         }
     }
@@ -2611,7 +2647,34 @@ extern "C" int cs3d_vorticity_q(cs3d_handle *h, double *vort, double *qcrit) {
     h->launches++;
     // the nine first derivatives with the solver's FP64 operators, one launch per direction
     for (int e = 0; e < 3; e++) {
-        int rc = adj_apply<double>(h, e, 0, 1,
+        const LineSegArgs &ls = h->lseg[e][0].a;
+        int rc = CS3D_OK;
+        if (e == 0 && ls.seg.SEG) {
+            for (int c = 0; c < 3 && !rc; c++)
+                rc = line_op_on(h->op64[e][0].op, ls, 1, h->g.npts, a.vel[c], d[c][e], h->stream);
+            h->launches += 3;
+            if (rc) return rc;
+            continue;
+        }
+        if (e > 0 && ls.seg.SEG && !ls.wall) {
+            ColumnArgs ca{};
+            ca.N = ls.N;
+            ca.lgG = ls.lgG;
+            ca.Nx = h->g.Nx;
+            const long long nxy = (long long)h->g.Nx * h->g.Ny;
+            ca.stride = e == 1 ? h->g.Nx : nxy;
+            ca.plane = e == 1 ? nxy : h->g.Nx;
+            ca.seg = ls.seg;
+            ca.op = ls.op;
+            for (int c = 0; c < 3; c++) {
+                ca.src[c] = a.vel[c];
+                ca.dst[c] = d[c][e];
+            }
+            CS3D_CUDA(launch_column_seg(ca, e == 1 ? h->g.Nz : h->g.Ny, h->stream));
+            h->launches++;
+            continue;
+        }
+        rc = adj_apply<double>(h, e, 0, 1,
                                    {{a.vel[0], nullptr, d[0][e], nullptr, 1.0, 0, 0},
                                     {a.vel[1], nullptr, d[1][e], nullptr, 1.0, 0, 0},
                                     {a.vel[2], nullptr, d[2][e], nullptr, 1.0, 0, 0}});

@@ -152,6 +152,112 @@ __global__ void __launch_bounds__(apply_threads<T>()) k_apply(ApplyArgs<T> a) {
         });
 }
 
+// The same on periodic lines by the register-segment solves (cs3d_seg.cuh): the
+// FP64 forms, and the FP32 filter correction of FP64 fields (F64IO).  Planar
+// buffers, one a task, solved in place; no correction on read.  k_apply's one
+// thread a line left the FP64 pipe idle (three first derivatives on 128^3: 249
+// us, three launches of 41 M FP64 warp operations in all).
+template <typename T, int DIR, int H, int SEG, bool FULL>
+__global__ void __launch_bounds__(apply_seg_threads<T>(), sizeof(T) == 4 ? 3 : 4) k_apply_seg(ApplyArgs<T> a) {
+    constexpr bool F64IO = sizeof(T) == 4;
+    const int L = a.L, P = a.P;
+    const Tile t = make_tile<DIR>(a.g, L);
+    const int N = t.N, NL = N * L, nt = a.ntask, pad = FULL ? a.seg.pad : 0;
+    T *buf = reinterpret_cast<T *>(smem_raw);
+    const int stride = seg_stride(N, P, a.seg.G, a.seg.pad);
+    struct In { Pt pt; T v[kApplyMax]; };
+    batched<In, 2>(NL,
+        [&](In &in, int p) {
+            in.pt = point<DIR>(t, p, L, P, a.lgL, a.divN, pad);
+            const unsigned gi = in.pt.gi;
+#pragma unroll
+            for (int k = 0; k < kApplyMax; ++k) {
+                if (k >= nt) break;
+                if constexpr (F64IO) {
+                    in.v[k] = to_work<T>(a.t[k].src64[gi]);
+                } else {
+                    in.v[k] = a.t[k].src[gi];
+                    if (a.t[k].src2) in.v[k] += a.t[k].src2[gi];
+                }
+            }
+        },
+        [&](In &in) {
+            if (!in.pt.ok) return;
+#pragma unroll
+            for (int k = 0; k < kApplyMax; ++k) {
+                if (k >= nt) break;
+                buf[k * stride + in.pt.o] = in.v[k];
+            }
+        });
+    __syncthreads();
+    {
+        const int lane0 = threadIdx.x & ((1 << a.seg.lgLW) - 1), seg = (threadIdx.x & 31) >> a.seg.lgLW;
+        const int groups = max(1, L >> a.seg.lgLW);
+        for (int u = threadIdx.x >> 5; u < nt * groups; u += blockDim.x >> 5) {
+            const int k = u / groups, l = ((u - k * groups) << a.seg.lgLW) + lane0;
+            const bool active = l < L;
+            const SegLane<T> s = seg_lane<SEG, FULL>(a.seg, buf + k * stride + (active ? l : 0), seg, N, P);
+            if constexpr (H == 4) seg_filter<SEG, FULL, false>(s, P, a.g0, a.seg, lane0, active);
+            else if (a.t[k].op == 1) seg_one<SEG, FULL, 2>(s, P, a.g1, a.seg, lane0, active, 0);
+            else seg_one<SEG, FULL, 1>(s, P, a.g0, a.seg, lane0, active, 0);
+        }
+    }
+    __syncthreads();
+    if constexpr (F64IO) {
+        struct Out64 { Pt pt; double e[kApplyMax]; };
+        batched<Out64, 2>(NL,
+            [&](Out64 &o, int p) {
+                o.pt = point<DIR>(t, p, L, P, a.lgL, a.divN, pad);
+#pragma unroll
+                for (int k = 0; k < kApplyMax; ++k) {
+                    if (k >= nt) break;
+                    o.e[k] = a.t[k].dst64[o.pt.gi];
+                }
+            },
+            [&](Out64 &o) {
+                if (!o.pt.ok) return;
+#pragma unroll
+                for (int k = 0; k < kApplyMax; ++k) {
+                    if (k >= nt) break;
+                    a.t[k].dst64[o.pt.gi] = o.e[k] + to_f64(a.t[k].scale * buf[k * stride + o.pt.o]);
+                }
+            });
+        return;
+    }
+    struct Out { Pt pt; T d[kApplyMax], d2[kApplyMax]; };
+    batched<Out, 1>(NL,
+        [&](Out &o, int p) {
+            o.pt = point<DIR>(t, p, L, P, a.lgL, a.divN, pad);
+            const unsigned gi = o.pt.gi;
+#pragma unroll
+            for (int k = 0; k < kApplyMax; ++k) {
+                if (k >= nt) break;
+                const ApplyTask<T> &tk = a.t[k];
+                const bool second = (k & 1) && a.merge[k / 2];
+                o.d[k] = (tk.dst && tk.acc && !second) ? tk.dst[gi] : T(0);
+                o.d2[k] = tk.dst2 ? tk.dst2[gi] : T(0);
+            }
+        },
+        [&](Out &o) {
+            if (!o.pt.ok) return;
+            const unsigned gi = o.pt.gi;
+#pragma unroll
+            for (int k = 0; k < kApplyMax; ++k) {
+                if (k >= nt) break;
+                const ApplyTask<T> &tk = a.t[k];
+                const T x = buf[k * stride + o.pt.o], v = tk.scale == T(1) ? x : tk.scale * x;
+                if ((k & 1) && a.merge[k / 2]) {
+                    tk.dst[gi] = tk.acc ? o.d[k - 1] + v : v;
+                } else if ((k & 1) == 0 && k + 1 < nt && a.merge[k / 2]) {
+                    o.d[k] = tk.acc ? o.d[k] + v : v;  // carried to task k + 1
+                } else if (tk.dst) {
+                    tk.dst[gi] = tk.acc ? o.d[k] + v : v;
+                }
+                if (tk.dst2) tk.dst2[gi] = o.d2[k] + v;
+            }
+        });
+}
+
 // ---------------------------------------------------------------------
 // transposed sweeps (FP32-mixed adjoint)
 // ---------------------------------------------------------------------
@@ -200,36 +306,59 @@ struct TSweepSrc<0> {
     }
 };
 
-template <int DIR, int PC>
-__global__ void __launch_bounds__(sweep_threads<float>(DIR), DIR == 0 ? kTMinBlocksX : 1) k_tsweep(TSweepArgs a) {
+// SEG > 0: the segmented solves of the forward sweeps (periodic lines always
+// here), x tiles planar, y and z lines in a cluster (CL) or one block.
+template <int DIR, int PC, int SEG = 0, bool FULL = false, bool CL = false>
+__global__ void __launch_bounds__(sweep_threads<float>(DIR), DIR == 0 && (SEG == 0 || FULL) ? kTMinBlocksX : 1)
+k_tsweep(TSweepArgs a) {
     using S = TSweepSrc<DIR>;
     constexpr int NP = (S::n + 1) / 2;
-    const int L = a.L, P = PC > 0 ? PC : a.P;
-    const Tile t = make_tile<DIR>(a.g, L);
-    const int N = t.N, NL = N * L;
-    const SmemPair sm = smem_pair_at(smem_raw, 2 * NP, L, P, N);
+    constexpr bool XP = DIR == 0 && SEG > 0;  // planar
+    const int L = CL ? kClLines : a.L, P = PC > 0 ? PC : a.P, lgL = CL ? 5 : a.lgL;
+    const int rank = CL ? (int)blockIdx.x % a.seg.C : 0;
+    const Tile t = CL ? make_cluster_tile<DIR>(a.g, a.seg, rank) : make_tile<DIR>(a.g, L);
+    const int N = t.N, NL = N * L, pad = FULL && !CL ? a.seg.pad : 0;
+    SmemPair sm;
+    SmemSegX sx;
+    if constexpr (XP) sx = {reinterpret_cast<float *>(smem_raw), seg_stride(N, P, a.seg.G, a.seg.pad)};
+    else if constexpr (SEG > 0) sm = smem_pair_seg(P, CL ? 32 * a.seg.B : N, a.seg);
+    else sm = smem_pair_at(smem_raw, 2 * NP, L, P, N);
     float *const *B = a.gbar;
     struct In { Pt pt; float v[S::n]; };
     batched<In, 4>(NL,
         [&](In &in, int p) {
-            in.pt = point<DIR>(t, p, L, P, a.lgL, a.divN);
+            in.pt = point<DIR>(t, p, L, P, lgL, a.divN, pad);
 #pragma unroll
             for (int k = 0; k < S::n; ++k) in.v[k] = B[S::e(k)][in.pt.gi];
         },
         [&](In &in) {
             if (!in.pt.ok) return;
+            if constexpr (XP) {
 #pragma unroll
-            for (int q = 0; q < NP; ++q) put2(sm, q, in.pt.o, in.v[2 * q], in.v[2 * q + 1 < S::n ? 2 * q + 1 : 2 * q]);
+                for (int k = 0; k < S::n; ++k) sx.at(k, in.pt.o) = in.v[k];
+            } else {
+#pragma unroll
+                for (int q = 0; q < NP; ++q) put2(sm, q, in.pt.o, in.v[2 * q], in.v[2 * q + 1 < S::n ? 2 * q + 1 : 2 * q]);
+            }
         });
-    __syncthreads();
-    run_sweep_tasks<2, PC>(sm, kTasksT, NP, L, t.nlines, a.d1, a.d2, threadIdx.x, blockDim.x);
+    if constexpr (CL) cluster_sync();
+    else __syncthreads();
+    if constexpr (CL)
+        run_cluster_tasks<FULL, 8, (S::n & 1), true>(sm.pair(0), sm.pstride / 2, cluster_mail(sm), a.seg, a.g1, a.g2,
+                                                     rank, threadIdx.x);
+    else if constexpr (XP)
+        run_seg_x<SEG, FULL, true>(sx, P, L, N, a.seg, a.g1, a.g2, threadIdx.x, blockDim.x);
+    else if constexpr (SEG > 0)
+        run_seg_tasks<SEG, FULL, NP, (S::n & 1), true>(sm, P, L, N, a.seg, a.g1, a.g2, threadIdx.x, blockDim.x);
+    else
+        run_sweep_tasks<2, PC>(sm, kTasksT, NP, L, t.nlines, a.d1, a.d2, threadIdx.x, blockDim.x);
     __syncthreads();
     // destinations added to: U V W T, then (z) Ux Vy Wx Wy / (y) Ux Vx
     constexpr int ND = DIR == 2 ? 8 : DIR == 1 ? 6 : 4;
     struct Out { Pt pt; float d[ND]; };
     batched<Out, 2>(NL,
         [&](Out &o, int p) {
-            o.pt = point<DIR>(t, p, L, P, a.lgL, a.divN);
+            o.pt = point<DIR>(t, p, L, P, lgL, a.divN, pad);
             const unsigned gi = o.pt.gi;
 #pragma unroll
             for (int f = 0; f < 4; ++f) o.d[f] = B[kInU + f][gi];
@@ -243,11 +372,23 @@ __global__ void __launch_bounds__(sweep_threads<float>(DIR), DIR == 0 ? kTMinBlo
             if (!o.pt.ok) return;
             const Pt &p = o.pt;
             const unsigned gi = p.gi;
-            const Zn<float> zz = zn(a.d1, a.d2, p.n);
             float g[2 * NP];
+            if constexpr (XP) {
 #pragma unroll
-            for (int q = 0; q < NP; ++q)
-                get2(sm, q, p, L, zz.z1, q < 4 ? zz.z2 : zz.z1, g[2 * q], g[2 * q + 1]);
+                for (int k = 0; k < S::n; ++k) g[k] = sx.at(k, p.o);
+            } else if constexpr (SEG > 0) {
+#pragma unroll
+                for (int q = 0; q < NP; ++q) {
+                    const float2 v = sm.pair(q)[p.o];
+                    g[2 * q] = v.x;
+                    g[2 * q + 1] = v.y;
+                }
+            } else {
+                const Zn<float> zz = zn(a.d1, a.d2, p.n);
+#pragma unroll
+                for (int q = 0; q < NP; ++q)
+                    get2(sm, q, p, L, zz.z1, q < 4 ? zz.z2 : zz.z1, g[2 * q], g[2 * q + 1]);
+            }
             // U V W T: (dst + (-D1 g_d)) + D2 g_dd
 #pragma unroll
             for (int f = 0; f < 4; ++f) B[kInU + f][gi] = (o.d[f] + (-g[2 * f])) + g[2 * f + 1];
@@ -313,9 +454,9 @@ __global__ void __launch_bounds__(128) k_vjp(VjpArgs<T> a) {
             if (a.qb2[0]) {
                 double v = a.ca * a.qb2[f][gi];
                 if (a.yt[0]) v += a.cb * a.yt[f][gi];
-                l[f] = (T)v;
+                l[f] = to_work<T>(v);
             } else {
-                l[f] = (T)a.lam[f][gi];
+                l[f] = to_work<T>(a.lam[f][gi]);
             }
         }
         rhs_vjp<T>(in, l, muref, cpPr, out);
@@ -393,7 +534,7 @@ __global__ void k_chain(ChainArgs<T> a) {
         grv += gV * ir - gm1 * V * gp;
         grw += gW * ir - gm1 * W * gp;
         gre += gm1 * gp;
-        const double o[5] = {(double)gr, (double)gru, (double)grv, (double)grw, (double)gre};
+        const double o[5] = {to_f64(gr), to_f64(gru), to_f64(grv), to_f64(grw), to_f64(gre)};
 #pragma unroll
         for (int f = 0; f < 5; ++f) {
             a.out[f][gi] = o[f];
@@ -450,6 +591,10 @@ static int pw_grid(long long n, int threads) {
     return (int)(b < 1 ? 1 : b);
 }
 
+size_t apply_seg_smem(int prec_bytes, int ntask, int L, int P, int N, const SegPlan &p) {
+    return (size_t)ntask * prec_bytes * seg_stride(N, P, p.G, p.pad);
+}
+
 template <typename K, typename A>
 static cudaError_t tile_launch(K kernel, const A &a, dim3 grid, size_t sm, cudaStream_t s) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
@@ -458,10 +603,33 @@ static cudaError_t tile_launch(K kernel, const A &a, dim3 grid, size_t sm, cudaS
     return cudaGetLastError();
 }
 
+template <typename T, int DIR, int H>
+static cudaError_t launch_apply_seg(const ApplyArgs<T> &a, dim3 grid, size_t sm, cudaStream_t s) {
+    if (a.seg.full) return tile_launch(k_apply_seg<T, DIR, H, 32, true>, a, grid, sm, s);
+    if (a.seg.SEG == 32) return tile_launch(k_apply_seg<T, DIR, H, 32, false>, a, grid, sm, s);
+    if (a.seg.SEG == 24) return tile_launch(k_apply_seg<T, DIR, H, 24, false>, a, grid, sm, s);
+    return tile_launch(k_apply_seg<T, DIR, H, 16, false>, a, grid, sm, s);
+}
+
 template <typename T>
 cudaError_t launch_apply(int dir, int H, const ApplyArgs<T> &a, cudaStream_t s) {
     if (a.ntask < 1 || a.ntask > kApplyMax) return cudaErrorInvalidValue;
     const int N = dir == 0 ? a.g.Nx : dir == 1 ? a.g.Ny : a.g.Nz;
+    if (a.seg.SEG) {
+        const size_t sb = apply_seg_smem((int)sizeof(T), a.ntask, a.L, a.P, N, a.seg);
+        const dim3 gr = dir == 0 ? dim3((a.g.Ny + a.L - 1) / a.L, a.g.Nz)
+                                 : dim3((a.g.Nx + a.L - 1) / a.L, dir == 1 ? a.g.Nz : a.g.Ny);
+        if constexpr (sizeof(T) == 8) {
+            if (H == 2) {
+                if (dir == 0) return launch_apply_seg<T, 0, 2>(a, gr, sb, s);
+                if (dir == 1) return launch_apply_seg<T, 1, 2>(a, gr, sb, s);
+                return launch_apply_seg<T, 2, 2>(a, gr, sb, s);
+            }
+        }
+        if (dir == 0) return launch_apply_seg<T, 0, 4>(a, gr, sb, s);
+        if (dir == 1) return launch_apply_seg<T, 1, 4>(a, gr, sb, s);
+        return launch_apply_seg<T, 2, 4>(a, gr, sb, s);
+    }
     const size_t sm = sweep_smem_bytes((int)sizeof(T), sizeof(T) == 4 ? 2 * ((a.ntask + 1) / 2) : a.ntask, a.L,
                                        a.P, N);
     const int L = a.L;
@@ -485,10 +653,30 @@ cudaError_t launch_apply(int dir, int H, const ApplyArgs<T> &a, cudaStream_t s) 
 cudaError_t launch_tsweep(int dir, const TSweepArgs &a, cudaStream_t s) {
     const int N = dir == 0 ? a.g.Nx : dir == 1 ? a.g.Ny : a.g.Nz;
     const int nbuf = dir == 0 ? 14 : 16;
-    const size_t sm = sweep_smem_bytes(4, nbuf, a.L, a.P, N);
+    const size_t sm = sweep_smem_bytes(4, nbuf, a.L, a.P, N, &a.seg);
     const int L = a.L;
     dim3 grid = dir == 0 ? dim3((a.g.Ny + L - 1) / L, a.g.Nz)
                          : dir == 1 ? dim3((a.g.Nx + L - 1) / L, a.g.Nz) : dim3((a.g.Nx + L - 1) / L, a.g.Ny);
+    const bool f = a.seg.full;
+    if (a.seg.C) {
+        if (dir == 1) return launch_cluster(f ? k_tsweep<1, 32, 32, true, true> : k_tsweep<1, 32, 32, false, true>, a, grid, sm, s);
+        return launch_cluster(f ? k_tsweep<2, 32, 32, true, true> : k_tsweep<2, 32, 32, false, true>, a, grid, sm, s);
+    }
+    if (a.seg.SEG) {
+#define T_CASE(SEG, FULL)                                                          \
+    do {                                                                           \
+        if (dir == 0) return tile_launch(k_tsweep<0, 0, SEG, FULL>, a, grid, sm, s); \
+        if (dir == 1) return tile_launch(k_tsweep<1, 0, SEG, FULL>, a, grid, sm, s); \
+        return tile_launch(k_tsweep<2, 0, SEG, FULL>, a, grid, sm, s);               \
+    } while (0)
+        if (dir == 0 && f && a.P == 17) return tile_launch(k_tsweep<0, 17, 32, true>, a, grid, sm, s);
+        if (dir == 0 && f && a.P == 9) return tile_launch(k_tsweep<0, 9, 32, true>, a, grid, sm, s);
+        if (f) T_CASE(32, true);
+        if (a.seg.SEG == 32) T_CASE(32, false);
+        if (a.seg.SEG == 24) T_CASE(24, false);
+        T_CASE(16, false);
+#undef T_CASE
+    }
     if (dir == 0 && a.P == 9) return tile_launch(k_tsweep<0, 9>, a, grid, sm, s);
     if (dir == 0 && a.P == 5) return tile_launch(k_tsweep<0, 5>, a, grid, sm, s);
     if (dir == 1 && a.P == 16) return tile_launch(k_tsweep<1, 16>, a, grid, sm, s);

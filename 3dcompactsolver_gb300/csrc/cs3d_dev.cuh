@@ -195,6 +195,24 @@ __device__ __forceinline__ int faces_of(const Geom &g, int i, int j, int k) {
     return f;
 }
 
+// Reciprocal and square root in FP64 from FP32 estimates by one step of a
+// cubically convergent Newton series (1/x = r (1 + e + e^2 + ...), e = 1 - x r;
+// sqrt x = g (1 - e)^(-1/2), g = x r, e = 1 - g r with r near 1/sqrt x): three and
+// five operations on the FP64 pipe, within an ulp.  Outside the FP32 range,
+// and for NaN, the library's.
+__device__ __forceinline__ double rcp_f64(double x) {
+    if (!(fabs(x) > 1e-30 && fabs(x) < 1e30)) return 1.0 / x;
+    const double r = widen(__frcp_rn(narrow(x)));
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+__device__ __forceinline__ double sqrt_f64(double x) {
+    if (!(x > 1e-30 && x < 1e30)) return sqrt(x);
+    const double r = widen(__frsqrt_rn(narrow(x))), g = x * r;
+    const double e = fma(-g, r, 1.0);
+    return fma(g * e, fma(0.375, e, 0.5), g);
+}
+
 // T^-0.24, from which both the viscosity law mu = mu_ref T^0.76 (IdealGas.hpp)
 // and its slope 0.76 mu / T follow by multiplications.
 // FP32: exp2(-0.24 log2 T) with the hardware log2 (absolute error about 2^-22,
@@ -207,7 +225,7 @@ __device__ __forceinline__ int faces_of(const Geom &g, int i, int j, int k) {
 __device__ __forceinline__ float visc_rpow(float T) { return exp2f(-0.24f * __log2f(T)); }
 __device__ __forceinline__ double visc_rpow(double T) {
     if (!(T > 1e-6 && T < 1e6)) return pow(T, -0.24);
-    const double y = (double)exp2f(-0.24f * log2f((float)T));
+    const double y = widen(exp2f(-0.24f * log2f(narrow(T))));
     const double t2 = T * T, t6 = t2 * t2 * t2;
     const double y2 = y * y, y4 = y2 * y2, y8 = y4 * y4, y16 = y8 * y8;
     const double e = fma(-t6, y16 * y8 * y, 1.0);

@@ -132,6 +132,16 @@ struct LineSegArgs {
     double *out;
 };
 
+// First derivative along y or z of three fields in XYZ layout.
+struct ColumnArgs {
+    int N, lgG, Nx;
+    long long stride, plane;  // elements between rows of a line, and between planes of lines
+    SegPlan seg;
+    SegOp<double> op;
+    const double *src[3];
+    double *dst[3];
+};
+
 struct BCArgs {
     Geom g;
     int face;
@@ -213,6 +223,7 @@ template <typename T>
 cudaError_t launch_filter(int dir, const FilterArgs<T> &a, cudaStream_t s);
 cudaError_t launch_line_op(const LineOpArgs &a, cudaStream_t s);
 cudaError_t launch_line_seg(int kind, const LineSegArgs &a, cudaStream_t s);
+cudaError_t launch_column_seg(const ColumnArgs &a, int planes, cudaStream_t s);
 template <typename T>
 cudaError_t launch_tgv(const TgvArgs<T> &a, int blocks, cudaStream_t s);
 // calcTurbulenceQuantities / shearLayerInfoCalc sums over q1 and the
@@ -296,6 +307,8 @@ struct ApplyArgs {
     int L, lgL, P, threads;
     FastDiv divN;
     LineOp<T> op0, op1;
+    SegPlan seg;      // periodic lines in register segments (FP64, and the FP32
+    SegOp<T> g0, g1;  // filter correction of FP64 fields); SEG = 0: op0, op1
     int ntask;
     ApplyTask<T> t[kApplyMax];
     // merge[i]: tasks 2i and 2i+1 write one destination (t[2i].dst), the
@@ -308,6 +321,9 @@ struct ApplyArgs {
 // sweeps), 128 in FP64 (the filter's solves use up to ~250 registers).
 template <typename T>
 __host__ __device__ constexpr int apply_threads() { return sizeof(T) == 4 ? 256 : 128; }
+template <typename T>
+__host__ __device__ constexpr int apply_seg_threads() { return sizeof(T) == 4 ? 256 : 128; }
+size_t apply_seg_smem(int prec_bytes, int ntask, int L, int P, int N, const SegPlan &p);
 // primitives U V W T and the 15 Euler fluxes of the state q, in the work type
 template <typename T>
 struct TapePrepArgs {
@@ -338,6 +354,8 @@ struct TSweepArgs {
     int L, lgL, P, threads;
     FastDiv divN;
     LineOp<float> d1, d2;
+    SegPlan seg;  // as SweepArgs
+    SegOp<float> g1, g2;
     float *gbar[48];  // cotangents, indexed as the tape (kIn* of cs3d_rhs_adjoint.cuh)
 };
 cudaError_t launch_tsweep(int dir, const TSweepArgs &a, cudaStream_t s);

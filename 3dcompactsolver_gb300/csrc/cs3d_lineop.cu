@@ -154,6 +154,56 @@ __global__ void __launch_bounds__(kLineSegTpb, WALL && SEG > 24 ? 3 : 4) k_line_
     for (int i = lane; i < total; i += 32) out[i] = sm[place(i)];
 }
 
+// First derivatives along y or z of fields in XYZ layout (periodic lines): a
+// lane's rows go from memory to registers and back, with no shared memory.  A
+// warp's 32 / G lines are adjacent in x, as are a block's warps.
+template <int SEG, bool FULL>
+__global__ void __launch_bounds__(kLineSegTpb, 4) k_column_seg(ColumnArgs a) {
+    const int G = a.seg.G, lane = threadIdx.x & 31, lw = 32 >> a.lgG;
+    const int l = lane & (lw - 1), seg = lane >> (5 - a.lgG);
+    const int i0 = ((int)blockIdx.x * (kLineSegTpb / 32) + (int)(threadIdx.x >> 5)) * lw;
+    if (i0 >= a.Nx) return;  // (whole warps)
+    const int i = min(i0 + l, a.Nx - 1);
+    const long long st = a.stride;
+    const long long base = (long long)blockIdx.y * a.plane + i;
+    const int n0 = seg_row0(a.seg, seg), len = a.seg.S - (seg >= a.seg.nS), k0 = SEG - len;
+    const double *src = a.src[blockIdx.z] + base;
+    SegLane<const double> s;
+    s.seg = seg;
+    s.k0 = k0;
+    s.row = src + (n0 - k0) * st;
+    s.lo = n0 > 0 ? s.row : s.row + a.N * st;
+    s.hi = seg < G - 1 ? src + (n0 + len) * st : src;
+    double y[SEG];
+    {
+        double w[SEG + 4];
+        seg_load<SEG, FULL, 2>(w, s, st, [](const double *p) { return __ldg(p); });
+#pragma unroll
+        for (int k = 0; k < SEG; ++k) {
+            y[k] = seg_r1<SEG>(w, a.op, k);
+            if (!FULL && k < kSegSlack && k < k0) y[k] = 0.0;
+        }
+    }
+    seg_solve<SEG, FULL, kSegRowsAll>(y, a.op, a.seg, seg, k0, l, 5 - a.lgG);
+    if (i0 + l >= a.Nx) return;
+    SegLane<double> d;
+    d.k0 = k0;
+    d.row = a.dst[blockIdx.z] + base + (n0 - k0) * st;
+    seg_store<SEG, FULL>(d, st, [&](double *p, int k) { *p = y[k]; });
+}
+
+cudaError_t launch_column_seg(const ColumnArgs &a, int planes, cudaStream_t s) {
+    const int per = (kLineSegTpb / 32) * (32 >> a.lgG);
+    const dim3 grid((a.Nx + per - 1) / per, planes, 3);
+    if (a.seg.full) k_column_seg<32, true><<<grid, kLineSegTpb, 0, s>>>(a);
+    else if (a.seg.SEG == 32) k_column_seg<32, false><<<grid, kLineSegTpb, 0, s>>>(a);
+    else if (a.seg.SEG == 28) k_column_seg<28, false><<<grid, kLineSegTpb, 0, s>>>(a);
+    else if (a.seg.SEG == 24) k_column_seg<24, false><<<grid, kLineSegTpb, 0, s>>>(a);
+    else if (a.seg.SEG == 20) k_column_seg<20, false><<<grid, kLineSegTpb, 0, s>>>(a);
+    else k_column_seg<16, false><<<grid, kLineSegTpb, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
 template <int KIND, int SEG, bool FULL, bool WALL>
 static cudaError_t launch(const LineSegArgs &a, cudaStream_t s) {
     const size_t sm = (size_t)kLineSegTpb * (SEG + 1) * 8;

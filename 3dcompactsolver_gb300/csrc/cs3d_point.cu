@@ -654,10 +654,10 @@ cudaError_t launch_aero(const AeroArgs &a, cudaStream_t s) {
 __global__ void k_velocity(PostArgs a) {
     for (long long gi = (long long)blockIdx.x * blockDim.x + threadIdx.x; gi < a.g.npts;
          gi += (long long)gridDim.x * blockDim.x) {
-        const double r = a.q.f[0][gi];
-        a.vel[0][gi] = a.q.f[1][gi] / r;
-        a.vel[1][gi] = a.q.f[2][gi] / r;
-        a.vel[2][gi] = a.q.f[3][gi] / r;
+        const double ir = rcp_f64(a.q.f[0][gi]);
+        a.vel[0][gi] = a.q.f[1][gi] * ir;
+        a.vel[1][gi] = a.q.f[2][gi] * ir;
+        a.vel[2][gi] = a.q.f[3][gi] * ir;
     }
 }
 
@@ -668,15 +668,10 @@ __global__ void k_vort_q(PostArgs a) {
         const double Vx = a.d[1][0][gi], Vy = a.d[1][1][gi], Vz = a.d[1][2][gi];
         const double Wx = a.d[2][0][gi], Wy = a.d[2][1][gi], Wz = a.d[2][2][gi];
         const double vx = Wy - Vz, vy = Uz - Wx, vz = Vx - Uy;
-        a.vort[gi] = sqrt(vx * vx + vy * vy + vz * vz);
-        const double s01 = 0.5 * (Uy + Vx), s12 = 0.5 * (Vz + Wy), s02 = 0.5 * (Uz + Wx);
-        const double w01 = 0.5 * (Uy - Vx), w12 = 0.5 * (Vz - Wy), w02 = 0.5 * (Uz - Wx);
-        // the nine products of each tensor in row order, as the reference sums them
-        const double om2 = 0.5 * (0.0 * 0.0 + w01 * w01 + w02 * w02 + (-w01) * (-w01) + 0.0 * 0.0 + w12 * w12 +
-                                  (-w02) * (-w02) + (-w12) * (-w12) + 0.0 * 0.0);
-        const double st2 = 0.5 * (Ux * Ux + s01 * s01 + s02 * s02 + s01 * s01 + Vy * Vy + s12 * s12 + s02 * s02 +
-                                  s12 * s12 + Wz * Wz);
-        a.qcrit[gi] = om2 - st2;
+        a.vort[gi] = sqrt_f64(vx * vx + vy * vy + vz * vz);
+        // |W|^2/2 - |S|^2/2 with the off-diagonal squares' differences taken:
+        // w_ij^2 - s_ij^2 = -u_i,j u_j,i
+        a.qcrit[gi] = -0.5 * (Ux * Ux + Vy * Vy + Wz * Wz) - (Uy * Vx + Uz * Wx + Vz * Wy);
     }
 }
 

@@ -78,8 +78,8 @@ __device__ __forceinline__ SegLane<E> seg_lane(const SegPlan &pl, E *base, int s
 // The window of a segment: register row k at w[k + H], H rows either side.
 // Rows before the segment's own (ragged segments) come from the halo or stay
 // zero; the callers zero their right-hand sides.
-template <int SEG, bool FULL, int H, typename W, typename E, typename LD>
-__device__ __forceinline__ void seg_load(W (&w)[SEG + 2 * H], const SegLane<E> &s, int P, LD &&ld) {
+template <int SEG, bool FULL, int H, typename W, typename E, typename I, typename LD>
+__device__ __forceinline__ void seg_load(W (&w)[SEG + 2 * H], const SegLane<E> &s, I P, LD &&ld) {
 #pragma unroll
     for (int k = -H; k < SEG; ++k) {
         if (FULL) {
@@ -175,8 +175,8 @@ __device__ __forceinline__ void seg_solve(R (&y)[SEG], const SegOp<R> &o, const 
 }
 
 // Store the segment's own rows.
-template <int SEG, bool FULL, typename E, typename ST>
-__device__ __forceinline__ void seg_store(const SegLane<E> &s, int P, ST &&st) {
+template <int SEG, bool FULL, typename E, typename I, typename ST>
+__device__ __forceinline__ void seg_store(const SegLane<E> &s, I P, ST &&st) {
 #pragma unroll
     for (int k = 0; k < SEG; ++k)
         if (FULL || k >= kSegSlack || k >= s.k0) st(s.row + k * P, k);
@@ -228,28 +228,29 @@ __device__ __forceinline__ void seg_pair(const SegLane<float2> &s, int P, const 
 
 // One solve of a planar tile: the KIND-th derivative of the segment at `s`,
 // its rows stored to the same places `shift` elements on (0: in place).
-template <int SEG, bool FULL, int KIND>
-__device__ __forceinline__ void seg_one(const SegLane<float> &s, int P, const SegOp<float> &o, const SegPlan &pl, int lane0,
+template <int SEG, bool FULL, int KIND, typename R>
+__device__ __forceinline__ void seg_one(const SegLane<R> &s, int P, const SegOp<R> &o, const SegPlan &pl, int lane0,
                                         bool active, int shift) {
-    float y[SEG];
+    R y[SEG];
     {
-        float w[SEG + 4];
-        seg_load<SEG, FULL, 2>(w, s, P, [](const float *p) { return *p; });
+        R w[SEG + 4];
+        seg_load<SEG, FULL, 2>(w, s, P, [](const R *p) { return *p; });
 #pragma unroll
         for (int k = 0; k < SEG; ++k) {
             y[k] = KIND == 1 ? seg_r1<SEG>(w, o, k) : seg_r2<SEG>(w, o, k);
-            if (!FULL && k < kSegSlack && k < s.k0) y[k] = 0.f;
+            if (!FULL && k < kSegSlack && k < s.k0) y[k] = R(0);
         }
     }
-    seg_solve<SEG, FULL, KIND == 1 ? kSegRows1 : kSegRows2>(y, o, pl, s.seg, s.k0, lane0, pl.lgLW);
+    constexpr int K1 = sizeof(R) == 4 ? kSegRows1 : kSegRowsAll, K2 = sizeof(R) == 4 ? kSegRows2 : 24;
+    seg_solve<SEG, FULL, KIND == 1 ? K1 : K2>(y, o, pl, s.seg, s.k0, lane0, pl.lgLW);
     __syncwarp();  // every lane of the line has read its window
-    if (active) seg_store<SEG, FULL>(s, P, [&](float *p, int k) { p[shift] = y[k]; });
+    if (active) seg_store<SEG, FULL>(s, P, [&](R *p, int k) { p[shift] = y[k]; });
     __syncwarp();
 }
 
 // The filter (nine symmetric taps) of the segment at `s` in place.  FP32: o is
-// the correction F - I, added to the value; FP64: o is F itself.
-template <int SEG, bool FULL, typename R>
+// the correction F - I, added to the value (ADD); FP64: o is F itself.
+template <int SEG, bool FULL, bool ADD, typename R>
 __device__ __forceinline__ void seg_filter(const SegLane<R> &s, int P, const SegOp<R> &o, const SegPlan &pl,
                                            int lane0, bool active) {
     R y[SEG];
@@ -264,7 +265,7 @@ __device__ __forceinline__ void seg_filter(const SegLane<R> &s, int P, const Seg
     }
     seg_solve<SEG, FULL, kSegRowsAll>(y, o, pl, s.seg, s.k0, lane0, pl.lgLW);
     __syncwarp();  // every lane of the line has read its window
-    if (active) seg_store<SEG, FULL>(s, P, [&](R *p, int k) { *p = sizeof(R) == 4 ? *p + y[k] : y[k]; });
+    if (active) seg_store<SEG, FULL>(s, P, [&](R *p, int k) { *p = ADD ? *p + y[k] : y[k]; });
 }
 
 // ---------------------------------------------------------------------
@@ -298,9 +299,10 @@ __device__ __forceinline__ E *cluster_map(E *p, int rank) {
 }
 
 // The solves of a sweep tile (tasks as run_seg_tasks), one unit a warp: pl.B
-// segments of 32 / pl.B lines of one task.  mail: 2 * 8 * kClLines floats.
-// Every thread of every block of the cluster calls it.
-template <bool FULL, int NT, bool SINGLE>
+// segments of 32 / pl.B lines of one task.  MIX: tasks 0..3 take the second
+// derivative of the lane y field.  mail: 2 * 8 * kClLines floats.  Every
+// thread of every block of the cluster calls it.
+template <bool FULL, int NT, bool SINGLE, bool MIX = false>
 __device__ __forceinline__ void run_cluster_tasks(float2 *tile, int pstride2, float2 *mail, const SegPlan &pl,
                                                   const SegOp<float> &o1, const SegOp<float> &o2, int rank, int tid) {
     constexpr int SEG = 32, P = kClLines;
@@ -323,7 +325,7 @@ __device__ __forceinline__ void run_cluster_tasks(float2 *tile, int pstride2, fl
     float y1[SEG], y2[SEG];
     float2 e;
     if (dd) {
-        seg_pair_rhs<SEG, FULL, 0>(y1, y2, s, P, o1, o2);
+        seg_pair_rhs<SEG, FULL, MIX ? 3 : 0>(y1, y2, s, P, o1, o2);
         e = make_float2(seg_fwd<SEG>(y1, o1), seg_fwd<SEG>(y2, o2));
     } else if (single) {
         seg_pair_rhs<SEG, FULL, 2>(y1, y2, s, P, o1, o2);

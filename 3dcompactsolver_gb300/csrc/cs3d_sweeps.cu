@@ -121,14 +121,6 @@ __device__ __forceinline__ void put2(const SmemSeq &sm, int t, int o, double v0,
 }
 // first derivatives of a sweep
 constexpr int kSeqN1X = 9, kSeqN1Y = 11, kSeqN1Z = 12;
-// Segmented x tiles are planar: 80 registers a thread (3 blocks of 256 per SM)
-// hold one solve's segment, not a pair's.  Buffers as XU..XF4; a task's
-// buffers are 2t and 2t + 1.
-struct SmemSegX {
-    float *buf;
-    int stride;
-    __device__ float &at(int k, int o) const { return buf[k * stride + o]; }
-};
 template <int SEG>
 struct TileSegX {
     using SM = SmemSegX;
@@ -143,31 +135,6 @@ struct TileSegX {
     }
     static __device__ __forceinline__ float one(const SM &sm, int k, const Pt &p, int, float) { return sm.at(k, p.o); }
 };
-__device__ __forceinline__ void put2(const SmemSegX &sm, int t, int o, float v0, float v1) {
-    sm.at(2 * t, o) = v0;
-    sm.at(2 * t + 1, o) = v1;
-}
-// The 13 solves of a segmented x tile, seven units of two (the last of one) on
-// the lines a warp holds.
-template <int SEG, bool FULL>
-__device__ __forceinline__ void run_seg_x(const SmemSegX &sm, int P, int L, int N, const SegPlan &pl, const SegOp<float> &o1,
-                                          const SegOp<float> &o2, int tid, int nthr) {
-    const int lane0 = tid & ((1 << pl.lgLW) - 1), seg = (tid & 31) >> pl.lgLW;
-    const int groups = max(1, L >> pl.lgLW);
-    for (int u = tid >> 5; u < 7 * groups; u += nthr >> 5) {
-        const int t = u / groups, l = ((u - t * groups) << pl.lgLW) + lane0;
-        const bool active = l < L;
-        SegLane<float> s = seg_lane<SEG, FULL>(pl, &sm.at(2 * t, active ? l : 0), seg, N, P);
-        // t < 4: the 2nd derivative to the next buffer, then the 1st in place
-        if (t < 4) seg_one<SEG, FULL, 2>(s, P, o2, pl, lane0, active, sm.stride);
-        seg_one<SEG, FULL, 1>(s, P, o1, pl, lane0, active, 0);
-        if (t < 4 || t == 6) continue;
-        s.row += sm.stride;
-        s.lo += sm.stride;
-        s.hi += sm.stride;
-        seg_one<SEG, FULL, 1>(s, P, o1, pl, lane0, active, 0);
-    }
-}
 template <int SEG>
 struct TileSeg {
     using SM = SmemPair;
@@ -182,8 +149,6 @@ struct TileSeg {
     static __device__ __forceinline__ float one(const SM &sm, int k, const Pt &p, int, float) { return sm.at(k, p.o); }
     static __device__ __forceinline__ float &dq(const SM &sm, int f, int o) { return sm.at(ZS_ + f, o); }
 };
-// (cluster tiles: 8 pair arrays, then the mailbox)
-__device__ __forceinline__ float2 *cluster_mail(const SmemPair &sm) { return sm.pair(8); }
 template <> struct TileOf<float, 16> : TileSeg<16> {};
 template <> struct TileOf<float, 24> : TileSeg<24> {};
 template <> struct TileOf<float, 32> : TileSeg<32> {};
@@ -249,7 +214,7 @@ __global__ void __launch_bounds__(sweep_threads<T>(0), sizeof(T) == 4 && (SEG ==
             TS::put1f(sm, 3, o, ss.Tt);
             put2(sm, 4, o, s.ru, s.ru * ss.U + ss.p);
             put2(sm, 5, o, s.rv * ss.U, s.rw * ss.U);
-            TS::put1f(sm, 6, o, s.re * ss.U + ss.U * ss.p);
+            TS::put1f(sm, 6, o, (s.re + ss.p) * ss.U);
         });
     __syncthreads();
     if constexpr (SEG == kSeq)
@@ -359,7 +324,7 @@ __global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBloc
             put2(sm, 4, o, in.v[9], in.v[10]);
             put2(sm, 5, o, rv, ru * V);
             put2(sm, 6, o, rv * V + pp, rw * V);
-            TS::put1f(sm, 7, o, re * V + V * pp);
+            TS::put1f(sm, 7, o, (re + pp) * V);
         });
     if constexpr (CL) cluster_sync();
     else __syncthreads();
@@ -471,7 +436,7 @@ struct ZSweep {
                 put2(sm, 4, o, in.v[9] + in.v[10], in.v[11]);
                 put2(sm, 5, o, in.v[12], rw);
                 put2(sm, 6, o, ru * W, rv * W);
-                put2(sm, 7, o, rw * W + pp, re * W + W * pp);
+                put2(sm, 7, o, rw * W + pp, (re + pp) * W);
             });
     }
     // B: the 16 solves (8 pairs) of every line of the tile
@@ -817,7 +782,7 @@ k_filter_seg(FilterArgs<T> a) {
         for (int u = threadIdx.x >> 5; u < 5 * groups; u += blockDim.x >> 5) {
             const int f = u / groups, l = ((u - f * groups) << a.seg.lgLW) + lane0;
             const bool active = l < L;
-            seg_filter<SEG, FULL>(seg_lane<SEG, FULL>(a.seg, buf + f * stride + (active ? l : 0), seg, N, P), P, a.sg,
+            seg_filter<SEG, FULL, sizeof(T) == 4>(seg_lane<SEG, FULL>(a.seg, buf + f * stride + (active ? l : 0), seg, N, P), P, a.sg,
                                   a.seg, lane0, active);
         }
     }
@@ -951,26 +916,6 @@ static dim3 tile_grid(int dir, const Geom &g, int L) {
 
 // the segmented instances: compile-time pitches for the full segments, the
 // three segment lengths at run-time pitch for the others
-template <typename T>
-static cudaError_t launch_cluster(void (*kernel)(SweepArgs<T>), const SweepArgs<T> &a, dim3 grid, size_t sm,
-                                  cudaStream_t s) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t c{};
-    c.gridDim = dim3(grid.x * a.seg.C, grid.y);
-    c.blockDim = dim3(a.threads);
-    c.dynamicSmemBytes = sm;
-    c.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = a.seg.C;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    c.attrs = &at;
-    c.numAttrs = 1;
-    e = cudaLaunchKernelEx(&c, kernel, a);
-    return e != cudaSuccess ? e : cudaGetLastError();
-}
-
 static cudaError_t launch_seg_sweep(int dir, const SweepArgs<float> &a, dim3 grid, size_t sm, cudaStream_t s) {
     if (a.seg.C) {
         const bool f = a.seg.full;
@@ -979,6 +924,7 @@ static cudaError_t launch_seg_sweep(int dir, const SweepArgs<float> &a, dim3 gri
     }
 #define SEG_CASE(K, PC, SEG, FULL) return launch_tile_kernel(K<float, PC, SEG, FULL>, a, grid, sm, s)
     if (a.seg.full) {
+        if (dir == 0 && a.P == 17) SEG_CASE(k_sweep_x, 17, 32, true);
         if (dir == 0 && a.P == 9) SEG_CASE(k_sweep_x, 9, 32, true);
         if (dir == 0 && a.P == 5) SEG_CASE(k_sweep_x, 5, 32, true);
         if (dir == 1 && a.P == 16) SEG_CASE(k_sweep_y, 16, 32, true);
@@ -1014,7 +960,7 @@ cudaError_t launch_sweep(int dir, const SweepArgs<T> &a, cudaStream_t s) {
         if (a.seg.SEG) return launch_seg_sweep(dir, a, grid, sm, s);
     } else if (a.seg.SEG == kSeq) {
         if (dir == 0) return launch_tile_kernel(k_sweep_x<T, 0, kSeq>, a, grid, sm, s);
-        return launch_cluster<T>(dir == 1 ? k_sweep_y<T, 0, kSeq, false, true> : k_sweep_z<T, 0, kSeq, false, true>, a, grid,
+        return launch_cluster(dir == 1 ? k_sweep_y<T, 0, kSeq, false, true> : k_sweep_z<T, 0, kSeq, false, true>, a, grid,
                                  sm, s);
     }
     if constexpr (sizeof(T) == 4) {

@@ -723,10 +723,14 @@ __device__ __forceinline__ void run_sweep_solves(const SmemPair &sm, const Task 
     run_sweep_tasks<H, PC>(sm, tasks, ntask, L, nlines, op0, op1, tid, nthr, skip);
 }
 
+// Cluster tiles: 8 pair arrays, then the mailbox.
+__device__ __forceinline__ float2 *cluster_mail(const SmemPair &sm) { return sm.pair(8); }
+
 // The segmented solves of a sweep tile: tasks 0..3 the 1st and 2nd derivative
 // of one field, the others the 1st derivatives of two (SINGLE: the last task
-// has one field).  A unit is a task's solves on the lines one warp holds.
-template <int SEG, bool FULL, int NT, bool SINGLE>
+// has one field; MIX: tasks 0..3 take the second derivative of the lane y
+// field).  A unit is a task's solves on the lines one warp holds.
+template <int SEG, bool FULL, int NT, bool SINGLE, bool MIX = false>
 __device__ __forceinline__ void run_seg_tasks(const SmemPair &sm, int P, int L, int N, const SegPlan &pl,
                                               const SegOp<float> &o1, const SegOp<float> &o2, int tid, int nthr) {
     const int lane0 = tid & ((1 << pl.lgLW) - 1), seg = (tid & 31) >> pl.lgLW;
@@ -735,12 +739,47 @@ __device__ __forceinline__ void run_seg_tasks(const SmemPair &sm, int P, int L, 
         const int t = u / groups, l = ((u - t * groups) << pl.lgLW) + lane0;
         const bool active = l < L;
         const SegLane<float2> s = seg_lane<SEG, FULL>(pl, sm.pair(t) + (active ? l : 0), seg, N, P);
-        if (t < 4) seg_pair<SEG, FULL, 0>(s, P, o1, o2, pl, lane0, active);
+        if (t < 4) seg_pair<SEG, FULL, MIX ? 3 : 0>(s, P, o1, o2, pl, lane0, active);
         else if (SINGLE && t == NT - 1) seg_pair<SEG, FULL, 2>(s, P, o1, o2, pl, lane0, active);
         else seg_pair<SEG, FULL, 1>(s, P, o1, o2, pl, lane0, active);
     }
 }
 
+// Segmented x tiles are planar: 80 registers a thread (3 blocks of 256 per SM)
+// hold one solve's segment, not a pair's.  Buffers as XU..XF4; a task's
+// buffers are 2t and 2t + 1.
+struct SmemSegX {
+    float *buf;
+    int stride;
+    __device__ float &at(int k, int o) const { return buf[k * stride + o]; }
+};
+__device__ __forceinline__ void put2(const SmemSegX &sm, int t, int o, float v0, float v1) {
+    sm.at(2 * t, o) = v0;
+    sm.at(2 * t + 1, o) = v1;
+}
+// The 13 solves of a segmented x tile, seven units of two (the last of one) on
+// the lines a warp holds.  MIX: units 0..3 take the second derivative of the
+// next buffer's own field.
+template <int SEG, bool FULL, bool MIX = false>
+__device__ __forceinline__ void run_seg_x(const SmemSegX &sm, int P, int L, int N, const SegPlan &pl, const SegOp<float> &o1,
+                                          const SegOp<float> &o2, int tid, int nthr) {
+    const int lane0 = tid & ((1 << pl.lgLW) - 1), seg = (tid & 31) >> pl.lgLW;
+    const int groups = max(1, L >> pl.lgLW);
+    for (int u = tid >> 5; u < 7 * groups; u += nthr >> 5) {
+        const int t = u / groups, l = ((u - t * groups) << pl.lgLW) + lane0;
+        const bool active = l < L;
+        SegLane<float> s = seg_lane<SEG, FULL>(pl, &sm.at(2 * t, active ? l : 0), seg, N, P);
+        // t < 4: the 2nd derivative to the next buffer, then the 1st in place
+        if (t < 4 && !MIX) seg_one<SEG, FULL, 2>(s, P, o2, pl, lane0, active, sm.stride);
+        seg_one<SEG, FULL, 1>(s, P, o1, pl, lane0, active, 0);
+        if ((t < 4 && !MIX) || t == 6) continue;
+        s.row += sm.stride;
+        s.lo += sm.stride;
+        s.hi += sm.stride;
+        if (MIX && t < 4) seg_one<SEG, FULL, 2>(s, P, o2, pl, lane0, active, 0);
+        else seg_one<SEG, FULL, 1>(s, P, o1, pl, lane0, active, 0);
+    }
+}
 // Phase-A stores of task t's inputs at offset o: put1 for a task whose two
 // solves read one field, put2 for two fields.  In the pair layout both are
 // one 64-bit store (put1 stores the field in both lanes); in the planar
@@ -812,13 +851,13 @@ __device__ __forceinline__ PrimW<T> prim_w(const GasParams &gp, T r0, T r1, T r2
     PrimW<T> s;
     s.ru = r1; s.rv = r2; s.rw = r3; s.re = r4;
     if constexpr (sizeof(T) == 8) {
-        // one correctly rounded reciprocal of rho instead of four FP64
-        // divisions (within an ulp of the quotients)
-        const double ir = __drcp_rn(r0);
+        // one reciprocal of rho instead of four FP64 divisions (within an
+        // ulp or two of the quotients)
+        const double ir = rcp_f64(r0);
         s.U = r1 * ir;
         s.V = r2 * ir;
         s.W = r3 * ir;
-        s.p = gp.gm1 * (r4 - 0.5 * r0 * (s.U * s.U + s.V * s.V + s.W * s.W));
+        s.p = gp.gm1 * (r4 - 0.5 * (r1 * s.U + r2 * s.V + r3 * s.W));
         s.Tt = s.p * ir * (1.0 / gp.R);  // 1/R: invariant, formed once per thread
     } else {
         // FP32 keeps the quotients: the reciprocal's rounding, shared by the
@@ -831,6 +870,27 @@ __device__ __forceinline__ PrimW<T> prim_w(const GasParams &gp, T r0, T r1, T r2
         s.Tt = s.p / (r0 * (T)gp.R);
     }
     return s;
+}
+
+// Launch of a kernel whose tiles are split over clusters of a.seg.C blocks
+// (grid: tiles).
+template <typename A>
+static cudaError_t launch_cluster(void (*kernel)(A), const A &a, dim3 grid, size_t sm, cudaStream_t s) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid.x * a.seg.C, grid.y);
+    c.blockDim = dim3(a.threads);
+    c.dynamicSmemBytes = sm;
+    c.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = a.seg.C;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    e = cudaLaunchKernelEx(&c, kernel, a);
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 // Pressure from the conserved variables and the velocity.
