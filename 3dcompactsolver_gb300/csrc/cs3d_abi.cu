@@ -285,7 +285,7 @@ int upload_op(const HostOp &h, DevOp<T> &d, cudaStream_t s) {
 
 // How a periodic line of N points is cut for the segmented FP32 solves
 // (cs3d_seg.cuh): the fewest register rows SEG * G that hold it with segments
-// at most kSegSlack rows shorter than SEG; SEG = 0 where none does (N below 17 or
+// at most kSegSlack rows shorter than SEG; SEG = 0 where none does (N = 8 or
 // above 32 maxG).  pair: elements are float2 (the sweeps' tiles), else scalars.
 // step: between the compiled segment lengths 16 .. 32.
 SegPlan seg_plan(int N, bool pair, int maxG = 16, int step = 8) {
@@ -310,6 +310,14 @@ SegPlan seg_plan(int N, bool pair, int maxG = 16, int step = 8) {
             p.pair = pair;
             best = p;
         }
+    if (!best.SEG && N > 8 && N <= 16) {  // one segment, closed on itself
+        best.SEG = 16;
+        best.G = 1;
+        best.S = best.nS = N;
+        best.lgLW = 5;
+        best.kS = 16 - N;
+        best.pair = pair;
+    }
     return best;
 }
 
@@ -525,6 +533,15 @@ struct cs3d_handle {
     int ic_done = 0;
     int store_dq = 0, store_diag = 0;
     long long launches = 0;
+    // small grids: the launches of a time step as CUDA graphs, one for each form
+    // that a step takes (see step_key)
+    struct StepGraph {
+        unsigned long long key = 0;
+        int seen = 0;
+        cudaGraphExec_t exec = nullptr;
+        long long launches = 0;
+    };
+    std::vector<StepGraph> graphs;
     // optional per-kernel timing with CUDA events on the handle's stream
     int timing = 0;
     std::vector<cudaEvent_t> ev_pool;
@@ -869,16 +886,22 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
         };
         shape(&h->seg[d], h->L[d], h->threads[d]);
         const int other = d == 0 ? cfg->Ny : cfg->Nx, planes = d == 2 ? cfg->Ny : cfg->Nz;
+        // fewer lines a tile where the grid would leave SMs without a block
+        // (16^3: 2 lines, 128 blocks a launch)
+        auto spread = [&](int &L) {
+            while (L > 2 && (long long)std::max(1, h->seg[d].C) * ((other + L - 1) / L) * planes < 152) L /= 2;
+        };
         if (!h->mixed && h->seg[d].SEG) {
             // y and z: 8 lines (64-byte rows, a warp's solves of one kind), 3
-            // blocks an SM at 64 rows; fewer lines where the grid would leave
-            // SMs without a block (16^3: 2 lines, 128 blocks a launch)
+            // blocks an SM at 64 rows
             int &L = h->L[d];
             if (d > 0) L = std::min(8, pick_L(8, nb, Nd[d], 0, 84, true, &h->seg[d]));
-            while (L > 2 && (long long)h->seg[d].C * ((other + L - 1) / L) * planes < 152) L /= 2;
+            spread(L);
         } else if (h->seg[d].C) {
             h->L[d] = kClusterLines;
             h->threads[d] = 256 * h->seg[d].B;
+        } else {
+            spread(h->L[d]);
         }
         h->Lf[d] = pick_L(h->tb, h->mixed ? 10 : 5, Nd[d], d == 0 ? 1 : 0);
         // a mixed filter tile narrower than 8 lines within 72 kB (N = 256: 4
@@ -893,6 +916,7 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
             while (L > 1 && filter_seg_smem((int)h->tb, L, L + (d == 0), Nd[d], h->segf[d]) > 200 * 1024) L /= 2;
             h->Lf[d] = L;
         }
+        while (h->Lf[d] > 2 && (long long)((other + h->Lf[d] - 1) / h->Lf[d]) * planes < 152) h->Lf[d] /= 2;
         if (sweep_smem_bytes((int)h->tb, nb, 1, 2, Nd[d]) > 200 * 1024)
             return fail_free(fail(CS3D_ERR_SHAPE, "N[%d]=%d: a line does not fit in shared memory", d, Nd[d]));
     }
@@ -903,10 +927,17 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
 #undef ALLOC
 }
 
+static void drop_graphs(cs3d_handle *h) {
+    for (auto &g : h->graphs)
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+    h->graphs.clear();
+}
+
 extern "C" int cs3d_destroy(cs3d_handle *h) {
     if (!h) return CS3D_OK;
     DeviceGuard dg(h->dev);
     if (h->stream) cudaStreamSynchronize(h->stream);
+    drop_graphs(h);
     for (void *p : h->allocs) cudaFree(p);
     for (int d = 0; d < 3; d++)
         for (int k = 0; k < 3; k++) {
@@ -1022,6 +1053,7 @@ static int init_after_state(cs3d_handle *h) {
             h->fref[f] = (double)(s / (long double)n);
         }
     }
+    drop_graphs(h);  // (fref is among the launches' arguments)
     if (h->mixed) {
         int r = launch_shadow_of(h, h->q1, h->q1s);
         if (r) return r;
@@ -1246,7 +1278,7 @@ extern "C" int cs3d_post_step(cs3d_handle *h) {
     return CS3D_OK;
 }
 
-extern "C" int cs3d_step(cs3d_handle *h) {
+static int plain_step(cs3d_handle *h) {
     int rc = cs3d_pre_step(h);
     if (rc) return rc;
     for (int s = 1; s <= h->nstages; s++) {
@@ -1254,6 +1286,87 @@ extern "C" int cs3d_step(cs3d_handle *h) {
         if (rc) return rc;
     }
     return cs3d_post_step(h);
+}
+
+// What the launches of a time step depend on besides the handle's constants:
+// the first step, whether it filters and in which order, the buffers that hold
+// q1 and q2 (exchanged by unfiltered steps), the sponge's backup, the options.
+static unsigned long long step_key(const cs3d_handle *h) {
+    const bool filtered = (h->timeStep + 1) % h->cfg.filter_step == 0;
+    unsigned long long k = (unsigned long long)(uintptr_t)h->q1.f[0];  // (a multiple of 256)
+    k |= (h->timeStep == 0) | (filtered << 1) | (h->backup_valid << 2) | (h->store_dq << 3) | (h->store_diag << 4);
+    if (filtered) k |= (unsigned long long)((h->filterTimeStep + 1) % 3) << 5;
+    return k;
+}
+
+// On the smallest grids a step's 18 launches and more take the host longer than
+// the GPU.  After kGraphAfter steps of one form its launches are recorded into
+// a graph, which later steps of that form launch as a whole: 16^3 FP64, three
+// handles in flight, 104 -> 90 us a step, one handle 246 -> 210.  To 2^16
+// points: on 64^3 a graph still helps one handle (203 -> 169 us a step), but
+// several handles' graphs overlap less than their launches (124 -> 143).
+constexpr long long kGraphPoints = 1 << 16;
+constexpr int kGraphAfter = 8;
+
+extern "C" int cs3d_step(cs3d_handle *h) {
+    if (!h) return fail(CS3D_ERR_ARG, "null handle");
+    if (!h->ic_done || h->g.npts > kGraphPoints || h->timing) return plain_step(h);
+    DeviceGuard dg(h->dev);
+    // (a caller's own capture of the stream takes the plain launches)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(h->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return plain_step(h);
+    const unsigned long long key = step_key(h);
+    size_t n = 0;
+    while (n < h->graphs.size() && h->graphs[n].key != key) n++;
+    if (n == h->graphs.size()) {
+        h->graphs.emplace_back();
+        h->graphs[n].key = key;
+    }
+    cs3d_handle::StepGraph &g = h->graphs[n];
+    if (!g.exec) {
+        if (++g.seen <= kGraphAfter) return plain_step(h);
+        // recorded with the host's side of the state set back afterwards, so that
+        // a failure leaves the step to the plain launches
+        const int ts = h->timeStep, fts = h->filterTimeStep, bv = h->backup_valid;
+        const Q5 q1 = h->q1, q2 = h->q2;
+        float *q1s[5], *q2s[5];
+        for (int f = 0; f < 5; f++) { q1s[f] = h->q1s[f]; q2s[f] = h->q2s[f]; }
+        const long long before = h->launches;
+        cudaGraph_t graph = nullptr;
+        bool ok = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+        if (ok) {
+            ok = plain_step(h) == CS3D_OK;
+            ok = cudaStreamEndCapture(h->stream, &graph) == cudaSuccess && ok;
+            ok = ok && cudaGraphInstantiate(&g.exec, graph, 0) == cudaSuccess;
+            if (graph) cudaGraphDestroy(graph);
+        }
+        g.launches = h->launches - before;
+        h->launches = before;
+        h->timeStep = ts;
+        h->filterTimeStep = fts;
+        h->backup_valid = bv;
+        h->q1 = q1;
+        h->q2 = q2;
+        for (int f = 0; f < 5; f++) { h->q1s[f] = q1s[f]; h->q2s[f] = q2s[f]; }
+        if (!ok) {
+            (void)cudaGetLastError();
+            g.exec = nullptr;
+            g.seen = -(1 << 30);
+            return plain_step(h);
+        }
+    }
+    CS3D_CUDA(cudaGraphLaunch(g.exec, h->stream));
+    // what plain_step does to the host's side of the state
+    h->launches += g.launches;
+    h->timeStep++;
+    if (h->timeStep % h->cfg.filter_step == 0) {
+        h->filterTimeStep++;
+    } else {
+        std::swap(h->q1, h->q2);
+        for (int f = 0; f < 5; f++) std::swap(h->q1s[f], h->q2s[f]);
+    }
+    if (h->sponge_kind_faces) h->backup_valid = 1;
+    return CS3D_OK;
 }
 
 extern "C" int cs3d_run(cs3d_handle *h, int n) {

@@ -117,25 +117,31 @@ __global__ void __launch_bounds__(kLineSegTpb, WALL && SEG > 24 ? 3 : 4) k_line_
     }
     if constexpr (WALL) {
         // the first and last H rows, from their explicit coefficients
-        const bool top = seg == 0, end = seg == G - 1;
-        if (top || end) {
-            const double *line0 = sm + lane0 * LS;
+        // (their columns lie in the line's first or last two segments)
+        const double *line0 = sm + lane0 * LS;
+        auto explicit_row = [&](int r, int sa) {
+            const int na = seg_row0(a.seg, sa), nb2 = seg_row0(a.seg, min(sa + 1, G - 1));
+            const double *pa = line0 + sa * LS - na, *pb = line0 + min(sa + 1, G - 1) * LS - nb2;
+            double v = 0.0;
+            for (int k = 0; k < kTaps; ++k) {
+                const int n = a.boff[r] + k;
+                if (n >= N) break;
+                v = fma(a.btaps[r][k], n >= nb2 ? pb[n] : pa[n], v);
+            }
+            return v;
+        };
+        if (seg == 0 || seg == G - 1) {
 #pragma unroll
             for (int b = 0; b < H; ++b) {
-                const int r = top ? b : H + b;
-                double v = 0.0;
-                for (int k = 0; k < kTaps; ++k) {
-                    const int n = a.boff[r] + k;
-                    if (n >= N) break;
-                    const int sg = n < nb ? n / a.seg.S : a.seg.nS + (n - nb) / (a.seg.S - 1);
-                    v = fma(a.btaps[r][k], line0[sg * LS + n - seg_row0(a.seg, sg)], v);
-                }
-                if (end) y[SEG - H + b] = v;
-                if (top) {
+                const double v = explicit_row(seg == 0 ? b : H + b, seg == 0 ? 0 : max(G - 2, 0));
+                if (seg == 0) {
 #pragma unroll
                     for (int k = 0; k < kSegSlack + H; ++k)
                         if (k == k0 + b) y[k] = v;
+                } else {
+                    y[SEG - H + b] = v;
                 }
+                if (G == 1) y[SEG - H + b] = explicit_row(H + b, 0);
             }
         }
         const double *sc = a.tab.s + seg * SEG;

@@ -1,7 +1,7 @@
 """Single operators in register segments (csrc/cs3d_lineop.cu) against the
 oracle at the line lengths where the cut changes: the shortest and longest of
 each segment count, full and ragged, a partly filled last warp, and the lengths
-left to the Thomas solve (16, 1025)."""
+left to the Thomas solve (8, 1025)."""
 import numpy as np
 import pytest
 
@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 TOL = 1e-13  # FP64, as the operators' other comparisons with the oracle
 
 
-@pytest.mark.parametrize("N", [16, 17, 18, 31, 32, 34, 41, 47, 48, 49, 65, 66, 96, 97, 127, 129, 193, 255, 257, 301,
+@pytest.mark.parametrize("N", [8, 9, 15, 16, 17, 18, 31, 32, 34, 41, 47, 48, 49, 65, 66, 96, 97, 127, 129, 193, 255, 257, 301,
                                512, 513, 767, 1023, 1024, 1025])
 @pytest.mark.parametrize("bc", [0, 1])
 @pytest.mark.parametrize("alphaF", [0.49, -0.3])

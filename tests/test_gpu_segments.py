@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 # clusters of one-segment blocks: 22..32, 44..64, 66..256; of two-segment
 # blocks: 264..512; one block: the others
-LENGTHS = [16, 17, 18, 21, 22, 31, 32, 33, 42, 43, 44, 63, 64, 65, 66, 77, 96, 97, 101, 127, 128, 129, 131, 176, 192, 193,
+LENGTHS = [9, 15, 16, 17, 18, 21, 22, 31, 32, 33, 42, 43, 44, 63, 64, 65, 66, 77, 96, 97, 101, 127, 128, 129, 131, 176, 192, 193,
            256, 257, 263, 264, 320, 511, 512, 513]
 
 # One RK4 step plus filter of a state of order one at CFL 0.5: each of the four
@@ -46,3 +46,38 @@ def test_mixed_step_tracks_fp64_at_plan_edges(gpu_pkg, N, d):
         s.close()
     scale = np.maximum(np.abs(out[0]).reshape(5, -1).max(1), 1.0).reshape(5, 1, 1, 1)
     assert float((np.abs(out[1] - out[0]) / scale).max()) <= TOL
+
+
+@pytest.mark.parametrize("kind", ["mixed", "fp64", "sponge"])
+def test_repeated_steps_equal_single_handles(gpu_pkg, kind):
+    """Steps launched as a recorded graph (small grids, after eight of a form)
+    leave the same bits as the sub-step calls, which are never recorded."""
+    cases = __import__("importlib").import_module("3dcompactsolver_gb300.cases")
+    abi = gpu_pkg._abi
+    if kind == "sponge":
+        cfg, ic = cases.wall_box(rk=abi.TVDRK3, moving=True, sponge=True)
+        cfg = cfg.copy(filter_step=2)
+    else:
+        cfg, ic = cases.tgv(16, precision=abi.FP32_MIXED if kind == "mixed" else abi.FP64, filter_step=2)
+    a, b = gpu_pkg.Solver(cfg), gpu_pkg.Solver(cfg)
+    for s in (a, b):
+        s.set_initial_conditions(*ic)
+    n = 70
+    a.run(n)
+    for _ in range(n):
+        b.pre_step()
+        ns = 3 if cfg.rk == abi.TVDRK3 else 4
+        for st in range(1, ns + 1):
+            b.sub_step(st, st == ns)
+        b.post_step()
+    assert a.scalars() == b.scalars()
+    assert a.launch_count() == b.launch_count()
+    assert np.array_equal(a.conserved(), b.conserved())
+    a.set_initial_conditions(*ic)  # (the graphs of the old state are dropped)
+    a.run(3)
+    c = gpu_pkg.Solver(cfg)
+    c.set_initial_conditions(*ic)
+    c.run(3)
+    assert np.array_equal(a.conserved(), c.conserved())
+    for s in (a, b, c):
+        s.close()
