@@ -355,6 +355,7 @@ SegOp<R> seg_op(const HostOp &h, const SegPlan &p, int bits) {
     const double a = h.alo[h.N / 2];
     const double l = a == 0.0 ? 0.0 : (1.0 - std::sqrt(1.0 - 4.0 * a * a)) / (2.0 * a);
     o.nl = (R)-l;
+    o.geo = (R)(1.0 / (1.0 - l * l));
     for (int k = 0; k <= kMaxH; k++) o.s[k] = (R)(h.taps[kMaxH + k] * h.scale * (1.0 + l * l));
     for (int k = 0; k < 32; k++) o.pw[k] = (R)std::pow(-l, k + 1);
     o.qS = (R)std::pow(-l, p.S);

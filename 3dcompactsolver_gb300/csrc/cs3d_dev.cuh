@@ -71,6 +71,7 @@ struct SegOp {
     R nl, s[kMaxH + 1], pw[32];
     R qS, qS1;  // (-l)^S, (-l)^(S-1)
     R iS, iS1;  // (-l)^-kS, (-l)^-(kS+1)
+    R geo;          // 1 / (1 - l^2)
     R wrap;     // 1, or 1 / (1 - (-l)^N) where T = G
     int T;
 };

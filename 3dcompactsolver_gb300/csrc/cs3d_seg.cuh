@@ -151,6 +151,31 @@ __device__ __forceinline__ void seg_end(R (&y)[SEG], const SegOp<R> &o, R in) {
     for (int k = 0; k < (KU < SEG ? KU : SEG); ++k) y[SEG - 1 - k] = fma(o.pw[k], in, y[SEG - 1 - k]);
 }
 
+// Backward from zero without the entering value: the value at the first row.
+template <int SEG, bool FULL, typename R>
+__device__ __forceinline__ R seg_bwd0(R (&y)[SEG], const SegOp<R> &o, int k0) {
+    R c = y[SEG - 1], b = c;
+#pragma unroll
+    for (int k = SEG - 2; k >= 0; --k) {
+        y[k] = c = fma(o.nl, c, y[k]);
+        if (!FULL && k <= kSegSlack) b = k == k0 ? c : b;
+    }
+    return FULL ? c : b;
+}
+// Both values added at once to a segment solved from zero on both sides, where
+// they reach no further than the segment: `in` entered the forward pass (the
+// backward pass answers (-l)^(k+1) with (-l)^(k+1) / (1 - l^2)), `next` is the
+// solution's value after the last row.
+template <int SEG, bool FULL, int KU, typename R>
+__device__ __forceinline__ void seg_close(R (&y)[SEG], const SegOp<R> &o, const SegPlan &pl, int k0, R in, R next) {
+    constexpr int KF = KU + (FULL ? 0 : kSegSlack) < SEG ? KU + (FULL ? 0 : kSegSlack) : SEG;
+    in *= o.geo;
+    if constexpr (!FULL) in *= k0 == pl.kS ? o.iS : o.iS1;  // the powers count from row k0
+#pragma unroll
+    for (int k = 0; k < KF; ++k) y[k] = fma(o.pw[k], in, y[k]);
+    seg_end<SEG, KU>(y, o, next);
+}
+
 // What enters this lane's segment: e of the DIR-side neighbours (DIR = -1:
 // segments before, +1: after), weighted.  lane0: the line's first lane, its
 // segments 2^lgst lanes apart.
@@ -277,8 +302,9 @@ __device__ __forceinline__ void seg_filter(const SegLane<R> &s, int P, const Seg
 // 256 points) leaves room for two blocks an SM, one solving while the other's
 // loads and stores run.  Halo rows are read from the neighbours' shared memory;
 // the carries (T = 1: the plan keeps segments long enough for the nearest
-// neighbour alone) go through a mailbox forward, and backward through the row
-// that the receiving lane itself overwrites next.
+// neighbour alone) cross in one exchange: every segment is solved from zero on
+// both sides, its last forward value goes to the next block's mailbox and its
+// first solution value to the previous one's (seg_close).
 // Why: beyond the L2 the memory system delivers in proportion to the bytes a
 // tile's row takes of its 128-byte line -- a copy kernel of z tiles on 256^3
 // measured 2.0 / 3.9 / 6.5 TB/s at 8 / 16 / 32 FP32 lines a row (5.2 / 5.6 /
@@ -300,7 +326,7 @@ __device__ __forceinline__ E *cluster_map(E *p, int rank) {
 
 // The solves of a sweep tile (tasks as run_seg_tasks), one unit a warp: pl.B
 // segments of 32 / pl.B lines of one task.  MIX: tasks 0..3 take the second
-// derivative of the lane y field.  mail: 2 * 8 * kClLines floats.  Every
+// derivative of the lane y field.  mail: 2 * 8 * kClLines float2s.  Every
 // thread of every block of the cluster calls it.
 template <bool FULL, int NT, bool SINGLE, bool MIX = false>
 __device__ __forceinline__ void run_cluster_tasks(float2 *tile, int pstride2, float2 *mail, const SegPlan &pl,
@@ -322,47 +348,37 @@ __device__ __forceinline__ void run_cluster_tasks(float2 *tile, int pstride2, fl
     s.lo = first ? cluster_map(line + (nprev - s.k0) * P, prev) : cluster_map(s.row, rank);
     s.hi = last ? cluster_map(line, next) : cluster_map(line + (n0 + len) * P, rank);
     const bool dd = t < 4, single = SINGLE && t == NT - 1;
+    const SegOp<float> &ob = dd ? o2 : o1;
     float y1[SEG], y2[SEG];
-    float2 e;
-    if (dd) {
-        seg_pair_rhs<SEG, FULL, MIX ? 3 : 0>(y1, y2, s, P, o1, o2);
-        e = make_float2(seg_fwd<SEG>(y1, o1), seg_fwd<SEG>(y2, o2));
-    } else if (single) {
-        seg_pair_rhs<SEG, FULL, 2>(y1, y2, s, P, o1, o2);
-        e = make_float2(seg_fwd<SEG>(y1, o1), 0.f);
+    if (dd) seg_pair_rhs<SEG, FULL, MIX ? 3 : 0>(y1, y2, s, P, o1, o2);
+    else if (single) seg_pair_rhs<SEG, FULL, 2>(y1, y2, s, P, o1, o2);
+    else seg_pair_rhs<SEG, FULL, 1>(y1, y2, s, P, o1, o2);
+    float2 e, b;  // the segment's last forward value, its first solution value
+    e.x = seg_fwd<SEG>(y1, o1);
+    b.x = seg_bwd0<SEG, FULL>(y1, o1, s.k0);
+    if (!single) {
+        e.y = seg_fwd<SEG>(y2, ob);
+        b.y = seg_bwd0<SEG, FULL>(y2, ob, s.k0);
     } else {
-        seg_pair_rhs<SEG, FULL, 1>(y1, y2, s, P, o1, o2);
-        e = make_float2(seg_fwd<SEG>(y1, o1), seg_fwd<SEG>(y2, o1));
+        e.y = b.y = 0.f;
     }
-    float2 in;
+    float2 *box = mail + t * kClLines + l, *box2 = box + 8 * kClLines;
+    if (last) *cluster_map(box, next) = e;
+    if (first) *cluster_map(box2, prev) = b;
+    float2 in, nb;  // the other half's, where this block holds two segments
     in.x = __shfl_sync(0xffffffffu, e.x, tid & 15);
     in.y = __shfl_sync(0xffffffffu, e.y, tid & 15);
-    float2 *box = mail + t * kClLines + l;
-    if (last) *cluster_map(box, next) = e;
-    cluster_sync();  // the forward carries are there, and every window has been read
+    nb.x = __shfl_sync(0xffffffffu, b.x, (tid & 15) | 16);
+    nb.y = __shfl_sync(0xffffffffu, b.y, (tid & 15) | 16);
+    // the neighbours' values are there, and every window has been read (the
+    // last access to another block's shared memory)
+    cluster_sync();
     if (first) in = *box;
-    if (dd) {
-        e = make_float2(seg_bwd<SEG, FULL, kSegRows1>(y1, o1, pl, s.k0, in.x),
-                        seg_bwd<SEG, FULL, kSegRows2>(y2, o2, pl, s.k0, in.y));
-    } else if (single) {
-        e.x = seg_bwd<SEG, FULL, kSegRows1>(y1, o1, pl, s.k0, in.x);
-    } else {
-        e = make_float2(seg_bwd<SEG, FULL, kSegRows1>(y1, o1, pl, s.k0, in.x),
-                        seg_bwd<SEG, FULL, kSegRows1>(y2, o1, pl, s.k0, in.y));
-    }
-    in.x = __shfl_sync(0xffffffffu, e.x, (tid & 15) | 16);
-    in.y = __shfl_sync(0xffffffffu, e.y, (tid & 15) | 16);
-    // the previous block's last row of this line, stored next by its own lane
-    if (first) *cluster_map(line + (nprev - 1) * P, prev) = e;
-    cluster_sync();  // (the last access to another block's shared memory)
-    if (last) in = s.row[(SEG - 1) * P];
-    if (dd) {
-        seg_end<SEG, kSegRows1>(y1, o1, in.x);
-        seg_end<SEG, kSegRows2>(y2, o2, in.y);
-    } else {
-        seg_end<SEG, kSegRows1>(y1, o1, in.x);
-        if (!single) seg_end<SEG, kSegRows1>(y2, o1, in.y);
-    }
+    if (last) nb = *box2;
+    // the next segment's first value answers this one's forward value too
+    seg_close<SEG, FULL, kSegRows1>(y1, o1, pl, s.k0, in.x, fmaf(e.x, o1.nl * o1.geo, nb.x));
+    if (dd) seg_close<SEG, FULL, kSegRows2>(y2, o2, pl, s.k0, in.y, fmaf(e.y, o2.nl * o2.geo, nb.y));
+    else if (!single) seg_close<SEG, FULL, kSegRows1>(y2, o1, pl, s.k0, in.y, fmaf(e.y, o1.nl * o1.geo, nb.y));
     seg_store<SEG, FULL>(s, P, [&](float2 *p, int k) { *p = make_float2(y1[k], y2[k]); });
 }
 

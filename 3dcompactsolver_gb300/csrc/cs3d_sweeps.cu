@@ -887,7 +887,7 @@ size_t sweep_smem_bytes(int prec_bytes, int nbuf, int L, int P, int N, const Seg
     // the buffers and the mailboxes (a line's rows here: one block's, or all)
     if (prec_bytes == 8 && seg && seg->SEG)
         return 8 * (size_t)nbuf * (seq_stride(seg->C > 1 ? seg->S : N, L) + (seg->G > 1 ? 4 * L : 0));
-    if (prec_bytes == 4 && seg && seg->C) return 8 * (8 * (size_t)(32 * seg->B) * kClLines + 8 * kClLines);
+    if (prec_bytes == 4 && seg && seg->C) return 8 * (8 * (size_t)(32 * seg->B) * kClLines + 16 * kClLines);
     if (prec_bytes == 4 && seg && seg->SEG && !seg->pair) return (size_t)XNB * 4 * seg_stride(N, P, seg->G, seg->pad);
     // segmented solves: the pair arrays alone (no line factors, no read-ahead)
     if (prec_bytes == 4 && seg && seg->SEG) return (size_t)((nbuf + 1) / 2) * 4 * seg_pair_stride(N, P, seg->G, seg->pad);

@@ -723,7 +723,7 @@ __device__ __forceinline__ void run_sweep_solves(const SmemPair &sm, const Task 
     run_sweep_tasks<H, PC>(sm, tasks, ntask, L, nlines, op0, op1, tid, nthr, skip);
 }
 
-// Cluster tiles: 8 pair arrays, then the mailbox.
+// Cluster tiles: 8 pair arrays, then the mailboxes.
 __device__ __forceinline__ float2 *cluster_mail(const SmemPair &sm) { return sm.pair(8); }
 
 // The segmented solves of a sweep tile: tasks 0..3 the 1st and 2nd derivative
