@@ -389,8 +389,7 @@ SegPlan seq_plan(int N, int d) {
     return p;
 }
 
-// bits: below 2^-bits a carry is left out; pw: the powers' device copy.
-SeqOp seq_op(const HostOp &h, const SegPlan &p, double **pw, cudaStream_t s, int *rc) {
+SeqOp seq_op(const HostOp &h, const SegPlan &p) {
     SeqOp o{};
     const SegOp<double> g = seg_op<double>(h, p, 56);
     o.nl = g.nl;
@@ -398,15 +397,8 @@ SeqOp seq_op(const HostOp &h, const SegPlan &p, double **pw, cudaStream_t s, int
     o.s1 = g.s[1];
     o.s2 = g.s[2];
     o.wrap = p.G == 1 ? 1.0 / (1.0 - std::pow(g.nl, h.N)) : 1.0;
-    while (std::pow(std::fabs(g.nl), o.K) > std::ldexp(1.0, -56)) o.K++;
-    std::vector<double> t(o.K);
-    for (int k = 0; k < o.K; k++) t[k] = std::pow(g.nl, k + 1);
-    *rc = CS3D_OK;
-    if (cudaMalloc(pw, o.K * 8) != cudaSuccess ||
-        cudaMemcpyAsync(*pw, t.data(), o.K * 8, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess)
-        *rc = fail(CS3D_ERR_CUDA, "operator upload failed");
-    o.pw = *pw;
+    while (o.K < kSeqRows && std::pow(std::fabs(g.nl), o.K) > std::ldexp(1.0, -56)) o.K++;
+    for (int k = 0; k < kSeqRows; k++) o.pw[k] = std::pow(g.nl, k + 1);
     return o;
 }
 
@@ -525,7 +517,6 @@ struct cs3d_handle {
     SegPlan segr[3] = {};
     SegOp<double> segrop[3][3] = {};
     SeqOp seqop[3][2] = {};  // plain form: the sequential solves (plan in seg)
-    double *seqpw[3][2] = {};
     SegOp<double> segfop64[3] = {};
     // tiles
     int L[3] = {1, 1, 1}, Lf[3] = {1, 1, 1}, threads[3] = {128, 128, 128};
@@ -848,8 +839,7 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
             }
             if (!h->mixed && ho.periodic && k < 3) {
                 h->seg[d] = seq_plan(Nd[d], d);
-                h->seqop[d][k - 1] = seq_op(ho, h->seg[d], &h->seqpw[d][k - 1], h->stream, &r);
-                if (r) return fail_free(r);
+                h->seqop[d][k - 1] = seq_op(ho, h->seg[d]);
             } else if (!h->mixed && ho.periodic && factors(ho)) {
                 h->segf[d] = seg_plan(Nd[d], true);
                 h->segfop64[d] = seg_op<double>(ho, h->segf[d], 60);
@@ -945,7 +935,6 @@ extern "C" int cs3d_destroy(cs3d_handle *h) {
             if (h->op64[d][k].mem) cudaFree(h->op64[d][k].mem);
             if (h->op32[d][k].mem) cudaFree(h->op32[d][k].mem);
             if (h->lseg[d][k].mem) cudaFree(h->lseg[d][k].mem);
-            if (k < 2 && h->seqpw[d][k]) cudaFree(h->seqpw[d][k]);
         }
     for (int d = 0; d < 3; d++)
         if (h->op32fc[d].mem) cudaFree(h->op32fc[d].mem);

@@ -394,10 +394,13 @@ __device__ __forceinline__ void run_cluster_tasks(float2 *tile, int pstride2, fl
 // correction.  The line's other rows are in the blocks of a cluster, as in
 // run_cluster_tasks; R >= 40 there, so that a carry crosses one block at most.
 // Whole lines of one block: the circle closes on itself (wrap).
+constexpr int kSeqRows = 44;  // powers kept: 0.382^41 < 2^-56
 struct SeqOp {
     double nl, s0, s1, s2, wrap;
-    const double *pw;  // (-l)^(k+1)
     int K;
+    double pw[kSeqRows];  // (-l)^(k+1), k < K (among the kernel's arguments: a
+                          // first read from memory costs a short line's solve
+                          // as much as its arithmetic)
 };
 
 // KIND 1, 2.  lo: the two rows before the first, hi: after the last (read
@@ -451,18 +454,18 @@ __device__ __forceinline__ double seq_bwd(double *d, int P, int R, const SeqOp &
     for (; n - 4 >= 0; n -= 4, q -= 4 * P) {
         double c[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) c[j] = fma(ldc(o.pw + n - 1 - j), in, q[-j * P]);
+        for (int j = 0; j < 4; ++j) c[j] = fma(o.pw[n - 1 - j], in, q[-j * P]);
 #pragma unroll
         for (int j = 0; j < 4; ++j) q[-j * P] = x = fma(nl, x, c[j]);
     }
-    for (; n > 0; --n, q -= P) q[0] = x = fma(nl, x, fma(ldc(o.pw + n - 1), in, q[0]));
+    for (; n > 0; --n, q -= P) q[0] = x = fma(nl, x, fma(o.pw[n - 1], in, q[0]));
     return x;
 }
 __device__ __forceinline__ void seq_end(double *d, int P, int R, const SeqOp &o, double in) {
     const int K = min(o.K, R);
     double *q = d + (R - 1) * P;
 #pragma unroll 4
-    for (int k = 0; k < K; ++k) q[-k * P] = fma(ldc(o.pw + k), in, q[-k * P]);
+    for (int k = 0; k < K; ++k) q[-k * P] = fma(o.pw[k], in, q[-k * P]);
 }
 
 // The solves of a tile of L lines (a power of two <= 32), planar buffers
