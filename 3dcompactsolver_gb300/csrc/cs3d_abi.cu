@@ -376,17 +376,24 @@ bool factors(const HostOp &h) { return std::fabs(h.alo[h.N / 2]) < 0.4999; }
 // The plain form's lines (cs3d_seg.cuh, one thread a line): the rows of a
 // line in blocks of a cluster along y and z, 64 at most where 8 blocks allow
 // it, 40 at least (0.382^40 = 2e-17: a carry reaches the next block alone);
-// along x the whole line in one block, in two halves from 80 rows on (its 13
-// solves of 4 lines fill 2 of 3 warps otherwise).
+// along x the whole line in one block, in two segments from 80 rows on and four
+// from 160 (more lanes for its 13 solves).
 SegPlan seq_plan(int N, int d) {
     SegPlan p{};
     p.SEG = kSeqSeg;
     p.C = d == 0 ? 1 : std::min(8, (N + 63) / 64);
     while (p.C > 1 && N / p.C < 40) p.C--;
-    p.G = d == 0 && N >= 80 ? 2 : p.C;
+    p.G = d > 0 ? p.C : N >= 160 ? 4 : N >= 80 ? 2 : 1;
     p.S = (N + p.G - 1) / p.G;
     p.nS = N - p.G * (p.S - 1);
     return p;
+}
+
+// Lanes per line that n1 first derivatives and four second ones take, B segments
+// each (run_seq_tasks: the second ones start at a warp's first lane).
+int seq_slots(int n1, int B, int L) {
+    const int per = 32 / std::min(L, 32);
+    return (n1 * B + per - 1) / per * per + 4 * B;
 }
 
 SeqOp seq_op(const HostOp &h, const SegPlan &p) {
@@ -864,12 +871,15 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
         const int nb = sweep_nbuf(d, (int)h->tb);
         auto shape = [&](const SegPlan *seg, int &L, int &threads) {
             L = pick_L(h->tb, nb, Nd[d], x_pitch_plus(h, d), d == 0 ? (h->mixed ? 75 : 115) : 72, true, seg);
-            // FP64 x: at most 4 lines within 115 kB (2 blocks per SM at N = 256,
-            // 3 at 128, registers).  Against the former 75 kB tiles with a pad
-            // column (1 line at N = 256): HIT 256^3 x 51.7 -> 26.3 ms per step,
-            // shear layer 3.25 -> 1.84; 8 lines at 128^3 measured 4% slower.
-            if (!h->mixed && d == 0 && L > 4) L = 4;
-            threads = h->mixed ? (d == 0 ? sweep_threads<float>(0) : 256) : sweep_threads<double>(d);
+            // FP64 x, Thomas solves: at most 4 lines within 115 kB (2 blocks per
+            // SM at N = 256, 3 at 128, registers).  Segmented: 8, as far as the
+            // 256 threads take them at once.
+            if (!h->mixed && d == 0) {
+                const int B = seg && seg->SEG ? seg->G : 0;
+                while (L > (B ? 8 : 4) || (B && seq_slots(9, B, L) * L > kSeqTpbX)) L /= 2;
+            }
+            threads = h->mixed ? (d == 0 ? sweep_threads<float>(0) : 256)
+                      : d == 0 && seg && seg->SEG ? kSeqTpbX : sweep_threads<double>(d);
             if (h->mixed && d > 0 && L < 16) {
                 L = pick_L(h->tb, nb, Nd[d], 0, 200, true, seg);
                 threads = sweep_threads<float>(d);

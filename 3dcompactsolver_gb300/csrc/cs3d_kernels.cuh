@@ -7,6 +7,7 @@ namespace cs3d {
 
 constexpr int kTpbX = 256;   // threads per block of the mixed-form x sweep
 constexpr int kTpbYZ = 512;  // most threads per block of the mixed-form y and z sweeps
+constexpr int kSeqTpbX = 256;  // threads per block of the FP64 segmented x sweep
 // threads per block of the segmented filter
 constexpr int kFilterSegTpb = 320, kFilterSegTpb64 = 160;
 constexpr int kClusterLines = 32;  // lines of a tile whose lines are split over a cluster

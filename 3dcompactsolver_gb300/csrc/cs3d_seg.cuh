@@ -477,7 +477,7 @@ __device__ __forceinline__ void seq_end(double *d, int P, int R, const SeqOp &o,
 // thread of every block of the cluster calls it.
 __device__ __forceinline__ void run_seq_tasks(double *tile, int stride, double *mail, int n1, int L, int lgL, int R,
                                               const SegPlan &pl, const SeqOp &o1, const SeqOp &o2, int rank, int tid) {
-    const int C = pl.C, B = C > 1 ? 1 : pl.G;      // segments of a line in this block: 1 or 2
+    const int C = pl.C, B = C > 1 ? 1 : pl.G;      // segments of a line in this block: 1, 2 or 4
     const int per = 32 >> lgL;                     // solves a warp holds
     const int n1p = (n1 * B + per - 1) & ~(per - 1);
     int k = tid >> lgL;
@@ -486,12 +486,11 @@ __device__ __forceinline__ void run_seq_tasks(double *tile, int stride, double *
     const bool on = second ? k < n1p + 4 * B : k < n1 * B;
     if (second) k -= n1p;
     if (!on) k = 0;
-    const int h = B > 1 ? k & 1 : 0;
-    k = (B > 1 ? k >> 1 : k) + (second && on ? n1 : 0);
-    const int R0 = seg_rows(pl, 0);
-    double *line = tile + k * stride + l, *d = line + h * R0 * L;
+    const int h = k & (B - 1);
+    k = (B == 4 ? k >> 2 : B == 2 ? k >> 1 : k) + (second && on ? n1 : 0);
+    double *line = tile + k * stride + l, *d = line + (B > 1 ? seg_row0(pl, h) : 0) * L;
     const int rows = B > 1 ? seg_rows(pl, h) : R;
-    double *box = mail + (2 * k + h) * L + l, *box2 = box + 2 * (n1 + 4) * L;
+    double *mbox = mail + B * k * L + l, *box = mbox + h * L, *box2 = box + B * (n1 + 4) * L;
     const SeqOp &o = second ? o2 : o1;
     double v = 0.0;
     if (C > 1) {
@@ -509,17 +508,16 @@ __device__ __forceinline__ void run_seq_tasks(double *tile, int stride, double *
         cluster_sync();  // (the last access to another block's shared memory)
         if (on) seq_end(d, L, R, o, *box2);
     } else if (B > 1) {
-        // the halves' ends are each other's neighbours
-        const double *lo = line + (h ? R0 : R) * L, *hi = line + (h ? 0 : R0) * L;
-        const int other = h ? -L : L;
+        const int hp = (h - 1) & (B - 1), hn = (h + 1) & (B - 1);
+        const double *lo = h ? d : line + R * L, *hi = hn ? d + rows * L : line;
         auto sync = [] { __syncthreads(); };
         if (second) v = seq_fwd<2>(d, L, on ? rows : 0, o, lo, hi, sync);
         else v = seq_fwd<1>(d, L, on ? rows : 0, o, lo, hi, sync);
-        if (on) box[other] = v;
+        if (on) mbox[hn * L] = v;
         __syncthreads();
         if (on) {
             v = seq_bwd(d, L, rows, o, *box);
-            box2[other] = v;
+            mbox[hp * L + B * (n1 + 4) * L] = v;
         }
         __syncthreads();
         if (on) seq_end(d, L, rows, o, *box2);

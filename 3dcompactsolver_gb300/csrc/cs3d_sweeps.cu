@@ -169,8 +169,12 @@ __constant__ Task kTasksX2[7] = {{XU, XU, 0, XU, XU2, 1}, {XV, XV, 0, XV, XV2, 1
                                  {XT, XT, 0, XT, XT2, 1}, {XRU, XRU, 0, XF1, XF1, 0},
                                  {XF2, XF2, 0, XF3, XF3, 0}, {XF4, XF4, 0, XF4, XDUM, 0}};
 
+// FP64 segmented: 256 threads (128 registers), the 13 solves' segments of a tile
+// fill 7 of 8 warps.  As 4-line tiles of 128 threads, 3 blocks an SM (3 of 4
+// warps, a quarter of the lanes idle): 128^3 2.62 -> 2.52 ms a step.
 template <typename T, int PC, int SEG = 0, bool FULL = false>
-__global__ void __launch_bounds__(sweep_threads<T>(0), sizeof(T) == 4 && (SEG == 0 || FULL) ? kMinBlocksX : 2) k_sweep_x(SweepArgs<T> a) {
+__global__ void __launch_bounds__(SEG == kSeq ? kSeqTpbX : sweep_threads<T>(0),
+                                  sizeof(T) == 4 && (SEG == 0 || FULL) ? kMinBlocksX : 2) k_sweep_x(SweepArgs<T> a) {
     using TS = std::conditional_t<(SEG > 0 && sizeof(T) == 4), TileSegX<SEG>, TileOf<T, SEG>>;
     const int L = a.L, P = PC > 0 ? PC : a.P;
     const Tile t = make_tile<0>(a.g, L);
@@ -886,7 +890,7 @@ size_t planar_smem_bytes(int prec_bytes, int nbuf, int L, int P, int N) {
 size_t sweep_smem_bytes(int prec_bytes, int nbuf, int L, int P, int N, const SegPlan *seg) {
     // the buffers and the mailboxes (a line's rows here: one block's, or all)
     if (prec_bytes == 8 && seg && seg->SEG)
-        return 8 * (size_t)nbuf * (seq_stride(seg->C > 1 ? seg->S : N, L) + (seg->G > 1 ? 4 * L : 0));
+        return 8 * (size_t)nbuf * (seq_stride(seg->C > 1 ? seg->S : N, L) + (seg->G == 1 ? 0 : 2 * (seg->C > 1 ? 1 : seg->G) * L));
     if (prec_bytes == 4 && seg && seg->C) return 8 * (8 * (size_t)(32 * seg->B) * kClLines + 16 * kClLines);
     if (prec_bytes == 4 && seg && seg->SEG && !seg->pair) return (size_t)XNB * 4 * seg_stride(N, P, seg->G, seg->pad);
     // segmented solves: the pair arrays alone (no line factors, no read-ahead)
