@@ -325,12 +325,13 @@ SegPlan seg_plan(int N, bool pair, int maxG = 16, int step = 8) {
 // each a block: one to 256 points, else two.  22 rows at least: a segment's
 // carry then reaches no further than the next one (0.382^22 = 6e-10, a
 // hundredth of an FP32 rounding; the second derivative's 0.188 falls faster).  C = 0 where no C <= 8 gives that.
+// Lines between walls: two blocks at least (their first and last segments differ), one segment each.
 SegPlan cluster_plan(int N, int periodic) {
     SegPlan p{};
-    if (!periodic) return p;
-    for (int B = 1; B <= 2; B++) {
+    for (int B = 1; B <= (periodic ? 2 : 1); B++) {
         const int C = (N + 32 * B - 1) / (32 * B);
-        if (C > 8 || N < 22 * B * C) continue;
+        if (C > 8 || N < 22 * B * C || (!periodic && C < 2)) continue;
+        p.wall = !periodic;
         p.SEG = 32;
         p.B = B;
         p.C = C;
@@ -407,6 +408,35 @@ SeqOp seq_op(const HostOp &h, const SegPlan &p) {
     while (o.K < kSeqRows && std::pow(std::fabs(g.nl), o.K) > std::ldexp(1.0, -56)) o.K++;
     for (int k = 0; k < kSeqRows; k++) o.pw[k] = std::pow(g.nl, k + 1);
     return o;
+}
+
+// The walls' rows of such a line: explicit rows, and the tables of the first
+// and last segment (device memory).
+int wall_op(const HostOp &h, const SegPlan &p, WallOp &w, float **mem, cudaStream_t s) {
+    const double a = h.alo[h.N / 2], l = (1.0 - std::sqrt(1.0 - 4.0 * a * a)) / (2.0 * a), q = 1.0 + l * l;
+    for (int b = 0; b < 4; b++)
+        for (int j = 0; j < 6; j++) {
+            // (rows N-2 and N-1 from column N - 6 on)
+            const int k = b < 2 ? j : h.N - 6 + j - h.boff[b];
+            w.bt[b][j] = k >= 0 ? (float)(h.btaps[b][k] * h.scale * q) : 0.f;
+        }
+    std::vector<float> t(3 * 64, 0.f);
+    for (int e = 0; e < 2; e++) {
+        const int len = e ? p.S - (p.G - 1 >= p.nS) : p.S, row0 = e ? h.N - len : 0;
+        for (int k = 32 - len; k < 32; k++) {
+            const int row = row0 + k - (32 - len);
+            t[32 * e + k] = (float)(h.iw[row] / q);
+            t[64 + 32 * e + k] = row > 0 ? (float)(-h.alo[row] * h.iw[row]) : 0.f;
+            t[128 + 32 * e + k] = row < h.N - 1 ? (float)(-h.c[row] * h.iw[row]) : 0.f;
+        }
+    }
+    CS3D_CUDA(cudaMalloc(mem, t.size() * 4));
+    CS3D_CUDA(cudaMemcpyAsync(*mem, t.data(), t.size() * 4, cudaMemcpyHostToDevice, s));
+    CS3D_CUDA(cudaStreamSynchronize(s));
+    w.s = *mem;
+    w.f = *mem + 64;
+    w.b = *mem + 128;
+    return CS3D_OK;
 }
 
 // One operator of contiguous FP64 lines in register segments: the launch
@@ -518,6 +548,8 @@ struct cs3d_handle {
     DevOp<float> op32fc[3];  // FP32 filter correction F - I (mixed form)
     SegPlan seg[3] = {};     // mixed form: the periodic directions' segmented solves
     SegOp<float> segop[3][2] = {};  // 1st and 2nd derivative
+    WallOp wallop[3][2] = {};
+    float *wallmem[3][2] = {};
     SegPlan segf[3] = {};    // the filter's, and its correction operator
     SegOp<float> segfop[3] = {};
     // FP64 lines in register segments (post-processor, FP64 adjoint)
@@ -854,6 +886,8 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
                 h->seg[d] = d > 0 ? cluster_plan(Nd[d], ho.periodic) : SegPlan{};
                 if (ho.periodic && !h->seg[d].C) h->seg[d] = seg_plan(Nd[d], d > 0);
                 h->segop[d][k - 1] = seg_op<float>(ho, h->seg[d], 30);
+                if (h->seg[d].wall && (r = wall_op(ho, h->seg[d], h->wallop[d][k - 1], &h->wallmem[d][k - 1], h->stream)))
+                    return fail_free(r);
             } else if (h->mixed && ho.periodic && factors(ho)) {
                 h->segf[d] = seg_plan(Nd[d], false);
                 h->segfop[d] = seg_op<float>(make_filter_correction(ho), h->segf[d], 30);
@@ -945,6 +979,7 @@ extern "C" int cs3d_destroy(cs3d_handle *h) {
             if (h->op64[d][k].mem) cudaFree(h->op64[d][k].mem);
             if (h->op32[d][k].mem) cudaFree(h->op32[d][k].mem);
             if (h->lseg[d][k].mem) cudaFree(h->lseg[d][k].mem);
+            if (k < 2 && h->wallmem[d][k]) cudaFree(h->wallmem[d][k]);
         }
     for (int d = 0; d < 3; d++)
         if (h->op32fc[d].mem) cudaFree(h->op32fc[d].mem);
@@ -1115,10 +1150,12 @@ static int run_stage(cs3d_handle *h, int st, int last) {
             for (int f = 0; f < 6; f++) {
                 if (h->cfg.bc_kind[f] != kind) continue;
                 b.face = f;
-                wall_velocity(&h->cfg, f, b.uw);
+                b.nfaces = f % 2 == 0 && h->cfg.bc_kind[f + 1] == kind ? 2 : 1;
+                for (int k = 0; k < b.nfaces; k++) wall_velocity(&h->cfg, f + k, b.uw[k]);
                 tstart(h, CS3D_K_BOUNDARY);
                 CS3D_CUDA(launch_wall_pre(b, h->stream));
                 tend(h);
+                f += b.nfaces - 1;
             }
         }
     }
@@ -1178,6 +1215,8 @@ static int run_stage(cs3d_handle *h, int st, int last) {
         a.seg = h->seg[d];
         a.g1 = h->segop[d][0];
         a.g2 = h->segop[d][1];
+        a.w1 = h->wallop[d][0];
+        a.w2 = h->wallop[d][1];
         a.h1 = h->seqop[d][0];
         a.h2 = h->seqop[d][1];
         if (sizeof(T) == 8) {
@@ -1264,8 +1303,8 @@ extern "C" int cs3d_post_step(cs3d_handle *h) {
     a.dt = h->scal;
     a.avgT = 15.0;         // SpongeBC.hpp:56-58
     a.epsP = 0.005;
-    a.spongeP = 1.0 / h->gas.gamma;
-    a.gm1 = h->gas.gamma - 1.0;
+    a.eP = 1.0 - a.epsP;
+    a.sP = 1.0 / h->gas.gamma / (h->gas.gamma - 1.0);
     a.q1 = h->q1;
     a.savg = h->savg;
     a.backup = h->backup;

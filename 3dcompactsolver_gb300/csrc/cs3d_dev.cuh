@@ -60,6 +60,7 @@ struct SegPlan {
     int pad;   // full only: shared-memory elements between a line's segments
     int kS;    // SEG - S
     int pair;  // array elements are float2 (y and z sweeps), else float
+    int wall;  // cluster: a line between walls (WallOp)
     int C, B;  // C > 0: a cluster of C blocks holds the line, B segments each
                // (G = B C, not restricted to a power of two)
 };

@@ -49,6 +49,7 @@ struct SweepArgs {
     LineOp<T> d1, d2;
     SegPlan seg;    // mixed form, periodic lines (seg.SEG > 0): the segmented
     SegOp<float> g1, g2;  // solves' plan and operators; plain form: the
+    WallOp w1, w2;  // (lines between walls)
     SeqOp h1, h2;   // sequential solves' (seg: G = C blocks' rows of a line)
     GasParams gas;
     const T *qs[5]; // stage input q* in the work precision (FP64 q* itself, or
@@ -145,8 +146,8 @@ struct ColumnArgs {
 
 struct BCArgs {
     Geom g;
-    int face;
-    double uw[3];
+    int face, nfaces;    // first face, and 2 where the opposite one goes along
+    double uw[2][3];
     GasParams gas;
     Q5 q;                 // stage input (FP64)
     const float *qs[5];   // ... or its FP32 shadow, when q holds null pointers
@@ -178,7 +179,7 @@ struct DtArgs {
 struct SpongeArgs {
     Geom g;
     const double *dt;
-    double avgT, epsP, spongeP, gm1;
+    double avgT, epsP, eP, sP;  // 1 - epsP; spongeP / (gamma - 1)
     Q5 q1, savg, backup;
     float *q1s[5];  // FP32 shadow of q1 to keep in step (mixed)
     int sponge_kind_faces;

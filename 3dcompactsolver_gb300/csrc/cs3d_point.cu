@@ -11,7 +11,9 @@ namespace cs3d {
 // ---------------------------------------------------------------------
 // wall boundary conditions before the derivatives (CSolver_AWS.cpp:553-826)
 // ---------------------------------------------------------------------
-// One launch per face, in the reference's order.  Temperatures of interior
+// One launch per face, in the reference's order; the two faces of a direction
+// share one where both are walls of the kind (neither reads a row that the other writes: 8 points
+// at least lie between them).  Temperatures of interior
 // points come from the current state; on stage 1, points of SPONGE faces that
 // are not on a wall use the state saved before the previous step's sponge
 // overwrite.  The state is FP64 (q), or only its FP32 shadow (qs) for the
@@ -43,7 +45,8 @@ __device__ __forceinline__ float temp_at32(const BCArgs &a, long long gi, int fc
 
 __global__ void k_wall_pre(BCArgs a) {
     const Geom g = a.g;
-    const int dir = a.face / 2, hi = a.face % 2;
+    const int face = a.face + blockIdx.y, dir = face / 2, hi = face % 2;
+    const double *uw = a.uw[blockIdx.y];
     const int n1 = dir == 0 ? g.Ny : g.Nx, n2 = dir == 2 ? g.Ny : g.Nz;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long long)n1 * n2) return;
@@ -84,11 +87,11 @@ __global__ void k_wall_pre(BCArgs a) {
     const double r = a.q.f[0] ? a.q.f[0][gi] : widen(a.qs[0][gi]);
     double nq[5];
     nq[0] = r;
-    nq[1] = dir == 0 ? 0.0 : r * a.uw[0];
-    nq[2] = dir == 1 ? 0.0 : r * a.uw[1];
-    nq[3] = dir == 2 ? 0.0 : r * a.uw[2];
+    nq[1] = dir == 0 ? 0.0 : r * uw[0];
+    nq[2] = dir == 1 ? 0.0 : r * uw[1];
+    nq[3] = dir == 2 ? 0.0 : r * uw[2];
     const double p = r * a.gas.R * Tw;
-    nq[4] = p / a.gas.gm1 + 0.5 * r * (a.uw[0] * a.uw[0] + a.uw[1] * a.uw[1] + a.uw[2] * a.uw[2]);
+    nq[4] = p / a.gas.gm1 + 0.5 * r * (uw[0] * uw[0] + uw[1] * uw[1] + uw[2] * uw[2]);
     if (a.q.f[0])
         for (int f = 1; f < 5; ++f) a.q.f[f][gi] = nq[f];
     if (a.qs_out[0])
@@ -230,8 +233,8 @@ __global__ void k_sponge_update(SpongeArgs a) {
             s += eps * (a.q1.f[f][gi] - s);
             av[f] = s;
         }
-        av[4] = a.epsP * av[4] +
-                (1.0 - a.epsP) * (a.spongeP / a.gm1 + 0.5 * (av[1] * av[1] + av[2] * av[2] + av[3] * av[3]) / av[0]);
+        // (FP64 operations bound this pass: no division per point)
+        av[4] = a.epsP * av[4] + a.eP * (a.sP + 0.5 * (av[1] * av[1] + av[2] * av[2] + av[3] * av[3]) * rcp_f64(av[0]));
 #pragma unroll
         for (int f = 0; f < 5; ++f) a.savg.f[f][gi] = av[f];
         if (a.sponge_kind_faces) {
@@ -426,7 +429,7 @@ static long long face_points(const Geom &g, int face) {
 }
 
 cudaError_t launch_wall_pre(const BCArgs &a, cudaStream_t s) {
-    k_wall_pre<<<(unsigned)((face_points(a.g, a.face) + 255) / 256), 256, 0, s>>>(a);
+    k_wall_pre<<<dim3((unsigned)((face_points(a.g, a.face) + 63) / 64), a.nfaces), 64, 0, s>>>(a);
     return cudaGetLastError();
 }
 cudaError_t launch_cfl(const CflArgs &a, cudaStream_t s) {

@@ -324,13 +324,82 @@ __device__ __forceinline__ E *cluster_map(E *p, int rank) {
     return r;
 }
 
+// Lines between walls: the first and last two rows' stencils are one-sided and
+// the factors converge to the periodic ones within 20 rows of the ends (they
+// approach like l^2n), so the first and last segment of a line take their
+// factors from tables (32 register rows each, the same for all lanes) and the
+// others run as on a periodic line, as does every exchange.
+struct WallOp {
+    float bt[4][6];         // the explicit rows (scaled as the taps): 0, 1 from row 0 on, N-2, N-1 from row N-6 on
+    const float *s, *f, *b; // [2][32]: y_n = s_n r_n + f_n y_{n-1}, x_n = y_n + b_n x_{n+1}
+};
+
+// The explicit rows of the first (end = 0) or last segment into y, from the
+// tile (lane LN of the pair, or both fields' own).
+template <int SEG, bool FULL>
+__device__ __forceinline__ void wall_rows(float (&y)[SEG], const float *x, int P2, const WallOp &w, int end, int k0) {
+    const float *p = x + (end ? SEG - 6 : FULL ? 0 : k0) * P2;
+    float r0 = 0.f, r1 = 0.f;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+        const float v = p[j * P2];
+        r0 = fmaf(w.bt[2 * end][j], v, r0);
+        r1 = fmaf(w.bt[2 * end + 1][j], v, r1);
+    }
+    if (end) {
+        y[SEG - 2] = r0;
+        y[SEG - 1] = r1;
+    } else if (FULL) {
+        y[0] = r0;
+        y[1] = r1;
+    } else {
+#pragma unroll
+        for (int k = 0; k < kSegSlack + 2; ++k) {
+            if (k == k0) y[k] = r0;
+            if (k == k0 + 1) y[k] = r1;
+        }
+    }
+}
+template <int SEG>
+__device__ __forceinline__ float wall_fwd(float (&y)[SEG], const WallOp &w, int end) {
+    const float *s = w.s + 32 * end, *f = w.f + 32 * end;
+    float c = 0.f;
+#pragma unroll
+    for (int k = 0; k < SEG; k += 4) {
+        float s4[4], f4[4];
+        load4(s + k, s4);
+        load4(f + k, f4);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) y[k + j] = c = fmaf(f4[j], c, s4[j] * y[k + j]);
+    }
+    return c;
+}
+template <int SEG, bool FULL>
+__device__ __forceinline__ float wall_bwd(float (&y)[SEG], const WallOp &w, int end, int k0) {
+    const float *b = w.b + 32 * end;
+    float c = 0.f, first = 0.f;
+#pragma unroll
+    for (int k = SEG - 4; k >= 0; k -= 4) {
+        float b4[4];
+        load4(b + k, b4);
+#pragma unroll
+        for (int j = 3; j >= 0; --j) {
+            y[k + j] = c = fmaf(b4[j], c, y[k + j]);
+            if (!FULL && k + j <= kSegSlack) first = k + j == k0 ? c : first;
+        }
+    }
+    return FULL ? c : first;
+}
+
 // The solves of a sweep tile (tasks as run_seg_tasks), one unit a warp: pl.B
 // segments of 32 / pl.B lines of one task.  MIX: tasks 0..3 take the second
 // derivative of the lane y field.  mail: 2 * 8 * kClLines float2s.  Every
 // thread of every block of the cluster calls it.
-template <bool FULL, int NT, bool SINGLE, bool MIX = false>
+// WALL: w1, w2 (one segment a block).
+template <bool FULL, int NT, bool SINGLE, bool MIX = false, bool WALL = false>
 __device__ __forceinline__ void run_cluster_tasks(float2 *tile, int pstride2, float2 *mail, const SegPlan &pl,
-                                                  const SegOp<float> &o1, const SegOp<float> &o2, int rank, int tid) {
+                                                  const SegOp<float> &o1, const SegOp<float> &o2, int rank, int tid,
+                                                  const WallOp *w1 = nullptr, const WallOp *w2 = nullptr) {
     constexpr int SEG = 32, P = kClLines;
     const int B = pl.B, warp = tid >> 5, t = B == 2 ? warp >> 1 : warp, half = B == 2 ? (tid >> 4) & 1 : 0;
     const int l = B == 2 ? ((warp & 1) << 4) | (tid & 15) : tid & 31;
@@ -354,13 +423,27 @@ __device__ __forceinline__ void run_cluster_tasks(float2 *tile, int pstride2, fl
     else if (single) seg_pair_rhs<SEG, FULL, 2>(y1, y2, s, P, o1, o2);
     else seg_pair_rhs<SEG, FULL, 1>(y1, y2, s, P, o1, o2);
     float2 e, b;  // the segment's last forward value, its first solution value
-    e.x = seg_fwd<SEG>(y1, o1);
-    b.x = seg_bwd0<SEG, FULL>(y1, o1, s.k0);
-    if (!single) {
-        e.y = seg_fwd<SEG>(y2, ob);
-        b.y = seg_bwd0<SEG, FULL>(y2, ob, s.k0);
-    } else {
+    if (WALL && (rank == 0 || rank == C - 1)) {
+        const int end = rank > 0;
+        const WallOp &wb = dd ? *w2 : *w1;
+        const float *x = reinterpret_cast<const float *>(s.row);
+        wall_rows<SEG, FULL>(y1, x, 2 * P, *w1, end, s.k0);
+        e.x = wall_fwd<SEG>(y1, *w1, end);
+        b.x = wall_bwd<SEG, FULL>(y1, *w1, end, s.k0);
         e.y = b.y = 0.f;
+        if (!single) {
+            wall_rows<SEG, FULL>(y2, dd && !MIX ? x : x + 1, 2 * P, wb, end, s.k0);
+            e.y = wall_fwd<SEG>(y2, wb, end);
+            b.y = wall_bwd<SEG, FULL>(y2, wb, end, s.k0);
+        }
+    } else {
+        e.x = seg_fwd<SEG>(y1, o1);
+        b.x = seg_bwd0<SEG, FULL>(y1, o1, s.k0);
+        e.y = b.y = 0.f;
+        if (!single) {
+            e.y = seg_fwd<SEG>(y2, ob);
+            b.y = seg_bwd0<SEG, FULL>(y2, ob, s.k0);
+        }
     }
     float2 *box = mail + t * kClLines + l, *box2 = box + 8 * kClLines;
     if (last) *cluster_map(box, next) = e;
@@ -376,9 +459,13 @@ __device__ __forceinline__ void run_cluster_tasks(float2 *tile, int pstride2, fl
     if (first) in = *box;
     if (last) nb = *box2;
     // the next segment's first value answers this one's forward value too
-    seg_close<SEG, FULL, kSegRows1>(y1, o1, pl, s.k0, in.x, fmaf(e.x, o1.nl * o1.geo, nb.x));
-    if (dd) seg_close<SEG, FULL, kSegRows2>(y2, o2, pl, s.k0, in.y, fmaf(e.y, o2.nl * o2.geo, nb.y));
-    else if (!single) seg_close<SEG, FULL, kSegRows1>(y2, o1, pl, s.k0, in.y, fmaf(e.y, o1.nl * o1.geo, nb.y));
+    nb.x = fmaf(e.x, o1.nl * o1.geo, nb.x);
+    nb.y = fmaf(e.y, ob.nl * ob.geo, nb.y);
+    if (WALL && rank == 0) in = make_float2(0.f, 0.f);
+    if (WALL && rank == C - 1) nb = make_float2(0.f, 0.f);
+    seg_close<SEG, FULL, kSegRows1>(y1, o1, pl, s.k0, in.x, nb.x);
+    if (dd) seg_close<SEG, FULL, kSegRows2>(y2, o2, pl, s.k0, in.y, nb.y);
+    else if (!single) seg_close<SEG, FULL, kSegRows1>(y2, o1, pl, s.k0, in.y, nb.y);
     seg_store<SEG, FULL>(s, P, [&](float2 *p, int k) { *p = make_float2(y1[k], y2[k]); });
 }
 

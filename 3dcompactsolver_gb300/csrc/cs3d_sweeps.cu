@@ -292,7 +292,7 @@ __constant__ Task kTasksY2[8] = {{YU, YU, 0, YU, YU2, 1}, {YV, YV, 0, YV, YV2, 1
 
 // FP64: 3 blocks per SM (168 registers, no spills): 2.93 -> 2.67 ms per step at
 // TGV 128^3, 37.5 -> 27.1 at HIT 256^3, the same bits
-template <typename T, int PC, int SEG = 0, bool FULL = false, bool CL = false>
+template <typename T, int PC, int SEG = 0, bool FULL = false, bool CL = false, bool WALL = false>
 __global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBlocksY : 3) k_sweep_y(SweepArgs<T> a) {
     using TS = TileOf<T, SEG>;
     constexpr bool SQ = SEG == kSeq;
@@ -335,8 +335,8 @@ __global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBloc
     if constexpr (SQ)
         run_seq_tasks(sm.buf, sm.stride, TS::mail(sm), kSeqN1Y, L, lgL, N, a.seg, a.h1, a.h2, rank, threadIdx.x);
     else if constexpr (CL)
-        run_cluster_tasks<FULL, 8, true>(sm.pair(0), sm.pstride / 2, cluster_mail(sm), a.seg, a.g1, a.g2, rank,
-                                         threadIdx.x);
+        run_cluster_tasks<FULL, 8, true, false, WALL>(sm.pair(0), sm.pstride / 2, cluster_mail(sm), a.seg, a.g1, a.g2,
+                                                      rank, threadIdx.x, &a.w1, &a.w2);
     else if constexpr (SEG > 0)
         run_seg_tasks<SEG, FULL, 8, true>(sm, P, L, N, a.seg, a.g1, a.g2, threadIdx.x, blockDim.x);
     else
@@ -402,7 +402,7 @@ __constant__ Task kTasksZ[8] = {{ZU, ZU, 0, ZU, ZU2, 1}, {ZV, ZV, 0, ZV, ZV2, 1}
 
 // The z sweep's three phases as functions of (tile, shared-memory layout,
 // thread range).
-template <typename T, int PC, int SEG, bool FULL, bool CL>
+template <typename T, int PC, int SEG, bool FULL, bool CL, bool WALL>
 struct ZSweep {
     static constexpr bool SQ = SEG == kSeq;
     using TS = TileOf<T, SEG>;
@@ -450,8 +450,8 @@ struct ZSweep {
         if constexpr (SQ)
             run_seq_tasks(sm.buf, sm.stride, TS::mail(sm), kSeqN1Z, a.L, a.lgL, t.N, a.seg, a.h1, a.h2, rank, tid);
         else if constexpr (CL)
-            run_cluster_tasks<FULL, 8, false>(sm.pair(0), sm.pstride / 2, cluster_mail(sm), a.seg, a.g1, a.g2,
-                                              rank, tid);
+            run_cluster_tasks<FULL, 8, false, false, WALL>(sm.pair(0), sm.pstride / 2, cluster_mail(sm), a.seg, a.g1,
+                                                           a.g2, rank, tid, &a.w1, &a.w2);
         else if constexpr (SEG > 0)
             run_seg_tasks<SEG, FULL, 8, false>(sm, PC > 0 ? PC : a.P, a.L, t.N, a.seg, a.g1, a.g2, tid, nthr);
         else
@@ -640,9 +640,9 @@ struct ZSweep {
 
 // FP64: 3 blocks per SM (168 registers; 88 bytes of spill stores): 4.70 ->
 // 4.52 ms per step at TGV 128^3, 52.5 -> 44.9 at HIT 256^3, the same bits
-template <typename T, int PC, int SEG = 0, bool FULL = false, bool CL = false>
+template <typename T, int PC, int SEG = 0, bool FULL = false, bool CL = false, bool WALL = false>
 __global__ void __launch_bounds__(sweep_threads<T>(2), sizeof(T) == 4 ? kMinBlocksZ : 3) k_sweep_z(SweepArgs<T> a) {
-    using Z = ZSweep<T, PC, SEG, FULL, CL>;
+    using Z = ZSweep<T, PC, SEG, FULL, CL, WALL>;
     const int rank = CL ? (int)blockIdx.x % a.seg.C : 0;
     const Tile t = Z::SQ ? make_seq_tile<2>(a.g, a.seg, a.L, rank)
                          : CL ? make_cluster_tile<2>(a.g, a.seg, rank) : make_tile<2>(a.g, a.L);
@@ -923,6 +923,10 @@ static dim3 tile_grid(int dir, const Geom &g, int L) {
 static cudaError_t launch_seg_sweep(int dir, const SweepArgs<float> &a, dim3 grid, size_t sm, cudaStream_t s) {
     if (a.seg.C) {
         const bool f = a.seg.full;
+        if (a.seg.wall) {
+            if (dir == 1) return launch_cluster(f ? k_sweep_y<float, 32, 32, true, true, true> : k_sweep_y<float, 32, 32, false, true, true>, a, grid, sm, s);
+            return launch_cluster(f ? k_sweep_z<float, 32, 32, true, true, true> : k_sweep_z<float, 32, 32, false, true, true>, a, grid, sm, s);
+        }
         if (dir == 1) return launch_cluster(f ? k_sweep_y<float, 32, 32, true, true> : k_sweep_y<float, 32, 32, false, true>, a, grid, sm, s);
         return launch_cluster(f ? k_sweep_z<float, 32, 32, true, true> : k_sweep_z<float, 32, 32, false, true>, a, grid, sm, s);
     }

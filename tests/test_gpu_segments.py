@@ -81,3 +81,38 @@ def test_repeated_steps_equal_single_handles(gpu_pkg, kind):
     assert np.array_equal(a.conserved(), c.conserved())
     for s in (a, b, c):
         s.close()
+
+
+@pytest.mark.parametrize("N", [43, 44, 45, 63, 64, 65, 66, 101, 127, 128, 176, 255, 256, 257])
+@pytest.mark.parametrize("d", [1, 2])
+def test_mixed_step_tracks_fp64_between_walls(gpu_pkg, N, d):
+    """Wall lines over a cluster (44..256 points but for 65; the others by the
+    Thomas solves).  The one-sided rows' taps sum to about ten times the
+    interior's, and the walls' no-slip rows drive the largest increments."""
+    abi = gpu_pkg._abi
+    n = [19, 12, 12]
+    n[d] = N
+    n[3 - d] = 13
+    rho, p, U, V, W = _noise((n[2], n[1], n[0]), 500 * d + N)
+    shape = [1, 1, 1]
+    shape[2 - d] = N
+    ramp = np.sin(np.pi * np.arange(N) / (N - 1.0)).reshape(shape)
+    ic = (rho, p, U * ramp, V * ramp, W * ramp)
+    bt = [abi.PERIODIC_SOLVE] * 3
+    bt[d] = abi.DIRICHLET_SOLVE
+    kind = [abi.PERIODIC] * 6
+    kind[2 * d] = abi.ADIABATIC_WALL
+    kind[2 * d + 1] = abi.MOVING_ADIABATIC_WALL if N % 2 else abi.ADIABATIC_WALL
+    out = []
+    for prec in (abi.FP64, abi.FP32_MIXED):
+        L = [6.283185307179586 * (1.0 - 1.0 / k) for k in n]
+        s = gpu_pkg.Solver(gpu_pkg.make_config(
+            tuple(n), tuple(L), bc_type=tuple(bt), bc_kind=tuple(kind), mu_ref=1e-3, CFL=0.3, precision=prec,
+            wall_vel=(0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.05, -0.02, 0.0, 0.0, 0.03, 0.01)))
+        s.set_initial_conditions(*ic)
+        s.step()
+        s.sync()
+        out.append(s.conserved())
+        s.close()
+    scale = np.maximum(np.abs(out[0]).reshape(5, -1).max(1), 1.0).reshape(5, 1, 1, 1)
+    assert float((np.abs(out[1] - out[0]) / scale).max()) <= 10 * TOL
