@@ -338,11 +338,14 @@ struct WallOp {
 // tile (lane LN of the pair, or both fields' own).
 template <int SEG, bool FULL>
 __device__ __forceinline__ void wall_rows(float (&y)[SEG], const float *x, int P2, const WallOp &w, int end, int k0) {
+    // (the rows' coefficients sum to zero: differences from the wall value, so
+    // that rounded coefficients make no derivative of a constant)
     const float *p = x + (end ? SEG - 6 : FULL ? 0 : k0) * P2;
+    const float v0 = p[end ? 5 * P2 : 0];
     float r0 = 0.f, r1 = 0.f;
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
-        const float v = p[j * P2];
+        const float v = p[j * P2] - v0;
         r0 = fmaf(w.bt[2 * end][j], v, r0);
         r1 = fmaf(w.bt[2 * end + 1][j], v, r1);
     }

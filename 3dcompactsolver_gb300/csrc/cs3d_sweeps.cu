@@ -614,7 +614,7 @@ struct ZSweep {
                             const double dd = to_f64(d);
                             double nv;
                             if (st == 1) { nv = in.qa[f] + dd; a.qk.f[f][gi] = nv; }
-                            else if (st == 2) { nv = 0.75 * in.qa[f] + 0.25 * in.qb[f] + 0.25 * dd; a.qk.f[f][gi] = nv; }
+                            else if (st == 2) { nv = 0.75 * in.qa[f] + (0.25 * in.qb[f] + to_f64(T(0.25) * d)); a.qk.f[f][gi] = nv; }
                             else { nv = (1.0 / 3.0) * in.qa[f] + (2.0 / 3.0) * in.qb[f] + (2.0 / 3.0) * dd; a.q2.f[f][gi] = nv; }
                             if (a.shadow_target != SHADOW_NONE) a.shadow_out[f][gi] = narrow(nv);
                         } else {
