@@ -883,7 +883,10 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
                 h->segf[d] = seg_plan(Nd[d], true);
                 h->segfop64[d] = seg_op<double>(ho, h->segf[d], 60);
             } else if (h->mixed && k < 3) {
-                h->seg[d] = d > 0 ? cluster_plan(Nd[d], ho.periodic) : SegPlan{};
+                // (tiles of 32 lines across x: not for grids narrower than 18,
+                // 12x200x200 0.67 ms a step by clusters, 0.54 by one block a line; 18x200x200
+                // 0.96 (one block, 20x200x200) and 0.75)
+                h->seg[d] = d > 0 && cfg->Nx >= 18 ? cluster_plan(Nd[d], ho.periodic) : SegPlan{};
                 if (ho.periodic && !h->seg[d].C) h->seg[d] = seg_plan(Nd[d], d > 0);
                 h->segop[d][k - 1] = seg_op<float>(ho, h->seg[d], 30);
                 if (h->seg[d].wall && (r = wall_op(ho, h->seg[d], h->wallop[d][k - 1], &h->wallmem[d][k - 1], h->stream)))
@@ -924,6 +927,7 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
         // fewer lines a tile where the grid would leave SMs without a block
         // (16^3: 2 lines, 128 blocks a launch)
         auto spread = [&](int &L) {
+            while (L > 2 && L / 2 >= other) L /= 2;
             while (L > 2 && (long long)std::max(1, h->seg[d].C) * ((other + L - 1) / L) * planes < 152) L /= 2;
         };
         if (!h->mixed && h->seg[d].SEG) {
@@ -948,6 +952,7 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
             // 128-byte rows where a block of them fits; half of that along x,
             // whose lines are contiguous
             int L = h->mixed ? (d == 0 ? 16 : 32) : (d == 0 ? 8 : 16);
+            while (L > 4 && L / 2 >= other) L /= 2;
             while (L > 1 && filter_seg_smem((int)h->tb, L, L + (d == 0), Nd[d], h->segf[d]) > 200 * 1024) L /= 2;
             h->Lf[d] = L;
         }
