@@ -884,8 +884,8 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
                 h->segfop64[d] = seg_op<double>(ho, h->segf[d], 60);
             } else if (h->mixed && k < 3) {
                 // (tiles of 32 lines across x: not for grids narrower than 18,
-                // 12x200x200 0.67 ms a step by clusters, 0.54 by one block a line; 18x200x200
-                // 0.96 (one block, 20x200x200) and 0.75)
+                // 12x200x200 0.67 ms a step by clusters, 0.54 by one block a line;
+                // 20x200x200 0.76 and 0.96)
                 h->seg[d] = d > 0 && cfg->Nx >= 18 ? cluster_plan(Nd[d], ho.periodic) : SegPlan{};
                 if (ho.periodic && !h->seg[d].C) h->seg[d] = seg_plan(Nd[d], d > 0);
                 h->segop[d][k - 1] = seg_op<float>(ho, h->seg[d], 30);

@@ -215,6 +215,20 @@ __device__ __forceinline__ double sqrt_f64(double x) {
     return fma(g * e, fma(0.375, e, 0.5), g);
 }
 
+// a / b in FP32 from ib, b's hardware reciprocal (rcp_est, one ulp): the
+// product's residual, exact by FMA, corrects it (Markstein, IBM J. Res. Dev. 34,
+// 1990), to within a few thousandths of an ulp of the rounded quotient.  Several
+// quotients of one b share the reciprocal; b must be normal.
+__device__ __forceinline__ float rcp_est(float b) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+    return r;
+}
+__device__ __forceinline__ float quot(float a, float b, float ib) {
+    const float q = a * ib;
+    return fmaf(fmaf(-q, b, a), ib, q);
+}
+
 // T^-0.24, from which both the viscosity law mu = mu_ref T^0.76 (IdealGas.hpp)
 // and its slope 0.76 mu / T follow by multiplications.
 // FP32: exp2(-0.24 log2 T) with the hardware log2 (absolute error about 2^-22,

@@ -506,13 +506,14 @@ struct ZSweep {
 #pragma unroll
                 for (int f = 0; f < 5; ++f) {
                     in.v[13 + f] = a.R[f][gi];
-                    in.qa[f] = use_q1a ? a.q1.f[f][gi] : a.q2.f[f][gi];
                     if constexpr (sizeof(T) == 4) {
+                        in.qa[f] = use_q1a ? a.q1.f[f][gi] : a.q2.f[f][gi];
                         if (need_qs || need_q1s)
                             in.qb[f] = __hiloint2double(0, __float_as_int(need_qs ? a.qs[f][gi] : a.q1s[f][gi]));
                         else in.qb[f] = need_qb ? a.qk.f[f][gi] : 0.0;
                     } else {
                         in.qb[f] = need_qb ? (tvd ? a.qk.f[f][gi] : a.q1.f[f][gi]) : 0.0;
+                        in.qa[f] = use_q1a ? a.q1.f[f][gi] : a.q2.f[f][gi];
                     }
                 }
             },

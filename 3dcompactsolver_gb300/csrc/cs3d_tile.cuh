@@ -863,11 +863,12 @@ __device__ __forceinline__ PrimW<T> prim_w(const GasParams &gp, T r0, T r1, T r2
         // FP32 keeps the quotients: the reciprocal's rounding, shared by the
         // points of a region of near-uniform density, doubled the mixed
         // form's error in the shear layer's fluctuation statistics
-        s.U = r1 / r0;
-        s.V = r2 / r0;
-        s.W = r3 / r0;
+        const float ir = rcp_est(r0), rR = r0 * (T)gp.R;
+        s.U = quot(r1, r0, ir);
+        s.V = quot(r2, r0, ir);
+        s.W = quot(r3, r0, ir);
         s.p = (T)gp.gm1 * (r4 - T(0.5) * r0 * (s.U * s.U + s.V * s.V + s.W * s.W));
-        s.Tt = s.p / (r0 * (T)gp.R);
+        s.Tt = quot(s.p, rR, ir * (T)(1.0 / gp.R));
     }
     return s;
 }
