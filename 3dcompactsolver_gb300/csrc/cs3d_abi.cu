@@ -949,11 +949,13 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
         // N = 128 the 8-line tile stays (16 lines measured slower)
         if (h->mixed && h->Lf[d] < 8) h->Lf[d] = pick_L(h->tb, 10, Nd[d], d == 0 ? 1 : 0, 110);
         if (h->segf[d].SEG) {
-            // 128-byte rows where a block of them fits; half of that along x,
-            // whose lines are contiguous
-            int L = h->mixed ? (d == 0 ? 16 : 32) : (d == 0 ? 8 : 16);
+            // 128-byte rows where two blocks of them fit an SM; half of that along
+            // x, whose lines are contiguous (256^3 mixed: 32 lines, one block,
+            // 1.08 ms a step; 16 lines, two blocks, 0.86); FP64 8 lines, 3 blocks
+            // (16 lines: 128^3 0.85 instead of 0.83 ms, 256^3 7.37 instead of 6.47)
+            int L = h->mixed ? (d == 0 ? 16 : 32) : 8;
             while (L > 4 && L / 2 >= other) L /= 2;
-            while (L > 1 && filter_seg_smem((int)h->tb, L, L + (d == 0), Nd[d], h->segf[d]) > 200 * 1024) L /= 2;
+            while (L > 1 && filter_seg_smem((int)h->tb, L, L + (d == 0), Nd[d], h->segf[d]) > 100 * 1024) L /= 2;
             h->Lf[d] = L;
         }
         while (h->Lf[d] > 2 && (long long)((other + h->Lf[d] - 1) / h->Lf[d]) * planes < 152) h->Lf[d] /= 2;
@@ -2153,12 +2155,11 @@ static int adj_tape(cs3d_handle *h, const T *const qin[5]) {
 // (primitives and derivative values at q) is G
 // Optional fusions of the RK combination of the adjoint stage: the
 // cotangent lam = ca qb2 + cb yt formed inside the pointwise VJP (qb2 set;
-// yt optional), and acc = out (acc_set) or acc + out inside the chain rule.
+// yt optional), and acc = base + out inside the chain rule.
 struct VjpFuse {
     double *const *qb2 = nullptr, *const *yt = nullptr;
     double ca = 0.0, cb = 0.0;
-    double *const *acc = nullptr;
-    int acc_set = 0;
+    double *const *acc = nullptr, *const *base = nullptr;
 };
 
 template <typename T>
@@ -2242,8 +2243,8 @@ static int adj_vjp_tape(cs3d_handle *h, const T *const qin[5], void *const Gv[48
         ca.qin[f] = qin[f];
         ca.out[f] = out[f];
         ca.acc[f] = fz.acc ? fz.acc[f] : nullptr;
+        ca.base[f] = fz.acc ? fz.base[f] : nullptr;
     }
-    ca.acc_set = fz.acc_set;
     for (int i = 0; i < 48; i++) ca.gbar[i] = B[i];
     tstart(h, CS3D_K_OTHER);
     CS3D_CUDA(launch_chain<T>(ca, h->stream));
@@ -2278,11 +2279,22 @@ static int adj_lin(cs3d_handle *h, double *const out[5], double a, double *const
     return CS3D_OK;
 }
 
-static int copy5(cs3d_handle *h, double *const dst[5], double *const src[5]) {
-    const size_t bytes = (size_t)h->g.npts * 8;
-    for (int f = 0; f < 5; f++)
-        CS3D_CUDA(cudaMemcpyAsync(dst[f], src[f], bytes, cudaMemcpyDeviceToDevice, h->stream));
+// five fields of `bytes` each in one launch (five copies of 2 MB take 2.5 us each)
+static int copy_fields(cs3d_handle *h, void *const dst[5], const void *const src[5], size_t bytes) {
+    Copy5Args a{};
+    a.bytes = bytes;
+    for (int f = 0; f < 5; f++) {
+        a.dst[f] = dst[f];
+        a.src[f] = src[f];
+    }
+    tstart(h, CS3D_K_OTHER);
+    CS3D_CUDA(launch_copy5(a, h->stream));
+    tend(h);
     return CS3D_OK;
+}
+
+static int copy5(cs3d_handle *h, double *const dst[5], double *const src[5]) {
+    return copy_fields(h, (void *const *)dst, (const void *const *)src, (size_t)h->g.npts * 8);
 }
 
 static void slab5(cs3d_handle *h, double *base, double *out[5]) {
@@ -2367,7 +2379,7 @@ static int adj_back(cs3d_handle *h, int fts, bool filtered, const T *const yin[4
         VjpFuse f1;
         f1.qb2 = LAM;
         f1.ca = dt;
-        f1.acc = QB;
+        f1.acc = f1.base = QB;
         return adj_vjp_tape<T>(h, yin[0], tapes[0], nullptr, YT, f1);
     }
     // RK4 (RK4.hpp:35-118) in reverse: q+ = q + dt/6 (k1 + 2 k2 + 2 k3 + k4),
@@ -2376,18 +2388,18 @@ static int adj_back(cs3d_handle *h, int fts, bool filtered, const T *const yin[4
     const double cb[4] = {dt / 2.0, dt / 2.0, dt, 0.0};             // weight of k_s in y_{s+1}
     for (int s = 3; s >= 0; s--) {
         // lam_s = ca_s qbar+ + cb_s ybar_{s+1} (formed in the VJP kernel);
-        // ybar_s = J(y_s)^T lam_s into YT, and YS = sum of the ybar_s (in the
-        // chain-rule kernel)
+        // ybar_s = J(y_s)^T lam_s into YT, and QB = QB2 + the sum of the ybar_s
+        // (in the chain-rule kernel)
         VjpFuse fz;
         fz.qb2 = QB2;
         fz.yt = s == 3 ? nullptr : YT;
         fz.ca = ca[s];
         fz.cb = cb[s];
-        fz.acc = YS;
-        fz.acc_set = s == 3;
+        fz.acc = QB;
+        fz.base = s == 3 ? QB2 : QB;
         if ((rc = adj_vjp_tape<T>(h, yin[s], tapes[s], nullptr, YT, fz))) return rc;
     }
-    return adj_lin(h, QB, 1.0, QB2, 1.0, YS);
+    return CS3D_OK;
 }
 
 // Adjoint of one time step taken from the state q0 with counters (ts, fts):
@@ -2416,11 +2428,12 @@ static int adj_step(cs3d_handle *h, int ts, int fts, double *const q0[5]) {
         for (int i = 0; i < 48; i++) h->tape_out[i] = nullptr;
         if (rc) return rc;
         if (st == h->nstages) break;
+        const void *src[5];
         for (int f = 0; f < 5; f++) {
-            const void *src = sizeof(T) == 8 ? (const void *)h->qk.f[f] : (const void *)h->qks[f];
-            CS3D_CUDA(cudaMemcpyAsync(Y[st - 1][f], src, n * sizeof(T), cudaMemcpyDeviceToDevice, h->stream));
+            src[f] = sizeof(T) == 8 ? (const void *)h->qk.f[f] : (const void *)h->qks[f];
             yin[st][f] = (const T *)Y[st - 1][f];
         }
+        if ((rc = copy_fields(h, (void *const *)Y[st - 1], src, n * sizeof(T)))) return rc;
     }
     const bool filtered = h->timeStep % h->cfg.filter_step == 0;
     return adj_back<T>(h, fts, filtered, yin, h->adj_tapes);
@@ -2436,11 +2449,14 @@ static int adj_taped_step(cs3d_handle *h, int j) {
     if ((rc = cs3d_pre_step(h))) return rc;
     for (int st = 1; st <= h->nstages; st++) {
         char *yb = h->adj_segyin + (size_t)((j * 4 + st - 1) * 5) * fb;
+        const void *src[5];
+        void *dst[5];
         for (int f = 0; f < 5; f++) {
-            const void *src = st == 1 ? (sizeof(T) == 8 ? (const void *)h->q1.f[f] : (const void *)h->q1s[f])
-                                      : (sizeof(T) == 8 ? (const void *)h->qk.f[f] : (const void *)h->qks[f]);
-            CS3D_CUDA(cudaMemcpyAsync(yb + f * fb, src, fb, cudaMemcpyDeviceToDevice, h->stream));
+            src[f] = st == 1 ? (sizeof(T) == 8 ? (const void *)h->q1.f[f] : (const void *)h->q1s[f])
+                             : (sizeof(T) == 8 ? (const void *)h->qk.f[f] : (const void *)h->qks[f]);
+            dst[f] = yb + f * fb;
         }
+        if ((rc = copy_fields(h, dst, src, fb))) return rc;
         char *tb = h->adj_segtape + (size_t)((j * 4 + st - 1) * 48) * fb;
         for (int i = 0; i < 48; i++) h->tape_out[i] = tb + i * fb;
         rc = run_stage<T>(h, st, st == h->nstages);

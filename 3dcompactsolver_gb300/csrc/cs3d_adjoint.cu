@@ -17,6 +17,7 @@
 //   D1^T = -D1,  D2^T = D2,  F^T = F,
 // which k_apply evaluates with the forward solve and a sign.
 #include <cstdio>
+#include <algorithm>
 #include <cmath>
 #include "cs3d_tile.cuh"
 #include "cs3d_rhs_adjoint.cuh"
@@ -538,7 +539,7 @@ __global__ void k_chain(ChainArgs<T> a) {
 #pragma unroll
         for (int f = 0; f < 5; ++f) {
             a.out[f][gi] = o[f];
-            if (a.acc[0]) a.acc[f][gi] = a.acc_set ? o[f] : a.acc[f][gi] + o[f];
+            if (a.acc[0]) a.acc[f][gi] = a.base[f][gi] + o[f];
         }
     }
 }
@@ -552,6 +553,24 @@ __global__ void k_lin5(Lin5Args a) {
             if (a.z[f]) v += a.c * a.z[f][i];
             a.out[f][i] = v;
         }
+    }
+}
+
+// blockIdx.y: the field; 16-byte words, or 4-byte ones where a field is not
+// aligned (four words a thread in flight)
+template <typename W>
+__global__ void k_copy5(Copy5Args a) {
+    const W *src = static_cast<const W *>(a.src[blockIdx.y]);
+    W *dst = static_cast<W *>(a.dst[blockIdx.y]);
+    const long long n = (long long)(a.bytes / sizeof(W));
+    for (long long i = gfirst(); i < n; i += 4 * gstride()) {
+        W v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (i + u * gstride() < n) v[u] = src[i + u * gstride()];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (i + u * gstride() < n) dst[i + u * gstride()] = v[u];
     }
 }
 
@@ -710,6 +729,15 @@ cudaError_t launch_rhs_eval(const RhsEvalArgs<T> &a, cudaStream_t s) {
 }
 cudaError_t launch_lin5(const Lin5Args &a, cudaStream_t s) {
     k_lin5<<<pw_grid(a.n, 256), 256, 0, s>>>(a);
+    return cudaGetLastError();
+}
+cudaError_t launch_copy5(const Copy5Args &a, cudaStream_t s) {
+    bool wide = a.bytes % 16 == 0;
+    for (int f = 0; f < 5; f++) wide = wide && ((uintptr_t)a.src[f] | (uintptr_t)a.dst[f]) % 16 == 0;
+    const long long n = (long long)(a.bytes / (wide ? 16 : 4));
+    const dim3 grid((unsigned)std::min<long long>((n + 4 * 256 - 1) / (4 * 256), 152 * 8), 5);
+    if (wide) k_copy5<uint4><<<grid, 256, 0, s>>>(a);
+    else k_copy5<unsigned><<<grid, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 cudaError_t launch_ke_seed(const KeSeedArgs &a, cudaStream_t s) {

@@ -369,8 +369,8 @@ struct ChainArgs {
     const T *qin[5];
     const T *gbar[48];
     double *out[5];
-    double *acc[5];  // optional: acc = out (acc_set) or acc + out
-    int acc_set;
+    double *acc[5];  // optional: acc = base + out (base may be acc)
+    const double *base[5];
 };
 template <typename T>
 struct RhsEvalArgs {
@@ -386,6 +386,13 @@ struct Lin5Args {
     const double *x[5], *y[5], *z[5];
     double a, b, c;
 };
+// five fields copied in one launch
+struct Copy5Args {
+    size_t bytes;
+    void *dst[5];
+    const void *src[5];
+};
+cudaError_t launch_copy5(const Copy5Args &a, cudaStream_t s);
 // seed of J = mean over points of rho |u|^2 / 2, and per-block partial sums of J
 struct KeSeedArgs {
     Geom g;
