@@ -322,15 +322,16 @@ SegPlan seg_plan(int N, bool pair, int maxG = 16, int step = 8) {
 }
 
 // The line split over a cluster of C blocks, B segments of at most 32 rows
-// each a block: one to 256 points, else two.  22 rows at least: a segment's
-// carry then reaches no further than the next one (0.382^22 = 6e-10, a
-// hundredth of an FP32 rounding; the second derivative's 0.188 falls faster).  C = 0 where no C <= 8 gives that.
+// each a block: one to 256 points, else two.  20 rows at least, as kSegRows1: a segment's
+// carry then reaches no further than the next one (0.382^20 = 4.4e-9, a fourteenth
+// of an FP32 rounding; the second derivative's 0.188 falls faster).  C = 0 where
+// no C <= 8 gives that.
 // Lines between walls: two blocks at least (their first and last segments differ), one segment each.
 SegPlan cluster_plan(int N, int periodic) {
     SegPlan p{};
     for (int B = 1; B <= (periodic ? 2 : 1); B++) {
         const int C = (N + 32 * B - 1) / (32 * B);
-        if (C > 8 || N < 22 * B * C || (!periodic && C < 2)) continue;
+        if (C > 8 || N < 20 * B * C || (!periodic && C < 2)) continue;
         p.wall = !periodic;
         p.SEG = 32;
         p.B = B;
@@ -1232,6 +1233,11 @@ static int run_stage(cs3d_handle *h, int st, int last) {
         } else {
             a.d1 = *reinterpret_cast<const LineOp<T> *>(&h->op32[d][0].op);
             a.d2 = *reinterpret_cast<const LineOp<T> *>(&h->op32[d][1].op);
+        }
+        if (d == 2 && h->sponge) {
+            tstart(h, CS3D_K_SPONGE);
+            CS3D_CUDA(launch_sponge_source<T>(a, h->stream));
+            tend(h);
         }
         tstart(h, CS3D_K_SWEEP_X + d);
         CS3D_CUDA(launch_sweep<T>(d, a, h->stream));

@@ -276,6 +276,8 @@ cudaError_t launch_wall_pre(const BCArgs &a, cudaStream_t s);
 cudaError_t launch_cfl(const CflArgs &a, cudaStream_t s);
 cudaError_t launch_nan_scan(const CflArgs &a, cudaStream_t s);
 cudaError_t launch_finalize_dt(const DtArgs &a, cudaStream_t s);
+template <typename T>
+cudaError_t launch_sponge_source(const SweepArgs<T> &a, cudaStream_t s);
 cudaError_t launch_sponge_update(const SpongeArgs &a, cudaStream_t s);
 cudaError_t launch_ic(const IcArgs &a, cudaStream_t s);
 cudaError_t launch_ic_wall(const IcArgs &a, cudaStream_t s);

@@ -253,6 +253,32 @@ __global__ void k_sponge_update(SpongeArgs a) {
     }
 }
 
+// The sponge's source sigma (avg - q) onto the right-hand side, between the y
+// and the z sweep (SpongeBC / CSolver_AWS.hpp:228); the continuity equation of
+// a wall point has none.  Memory-bound: where sigma is zero nothing else is
+// read, and a thread has one point (shear layer 256x128x42: 16.7 us; two or
+// four points a thread 18 and 21).  Inside the z sweep its branch held back
+// the update's loads: 119 us a stage there, now 98 + 17.
+template <typename T>
+__global__ void k_sponge_source(SweepArgs<T> a) {
+    const unsigned gi = blockIdx.x * blockDim.x + threadIdx.x;
+    if (gi >= a.g.npts) return;
+    const T sg = to_work<T>(a.sigma[gi]);
+    if (sg == T(0)) return;
+    T d[5];
+#pragma unroll
+    for (int f = 0; f < 5; ++f)
+        d[f] = a.R[f][gi] + (f == 4 ? T(2.0) * sg : sg) * (to_work<T>(a.savg.f[f][gi]) - a.qs[f][gi]);
+    bool wall = false;
+    if (a.wall_faces) {
+        const unsigned nxy = (unsigned)a.g.Nx * a.g.Ny, k = gi / nxy, rem = gi - k * nxy, j = rem / a.g.Nx;
+        wall = faces_of(a.g, (int)(rem - j * a.g.Nx), (int)j, (int)k) & a.wall_faces;
+    }
+    if (!wall) a.R[0][gi] = d[0];
+#pragma unroll
+    for (int f = 1; f < 5; ++f) a.R[f][gi] = d[f];
+}
+
 // ---------------------------------------------------------------------
 // initial conditions (CSolver_AWS.cpp:199-504)
 // ---------------------------------------------------------------------
@@ -447,6 +473,14 @@ cudaError_t launch_finalize_dt(const DtArgs &a, cudaStream_t s) {
     k_finalize_dt<<<1, 1, 0, s>>>(a);
     return cudaGetLastError();
 }
+template <typename T>
+cudaError_t launch_sponge_source(const SweepArgs<T> &a, cudaStream_t s) {
+    k_sponge_source<T><<<(unsigned)((a.g.npts + 255) / 256), 256, 0, s>>>(a);
+    return cudaGetLastError();
+}
+template cudaError_t launch_sponge_source<float>(const SweepArgs<float> &, cudaStream_t);
+template cudaError_t launch_sponge_source<double>(const SweepArgs<double> &, cudaStream_t);
+
 cudaError_t launch_sponge_update(const SpongeArgs &a, cudaStream_t s) {
     k_sponge_update<<<grid_for(a.g.npts, 256), 256, 0, s>>>(a);
     return cudaGetLastError();

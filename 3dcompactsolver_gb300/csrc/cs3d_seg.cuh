@@ -38,8 +38,8 @@ namespace cs3d {
 // 0.188; the filter's l depends on its coefficient (all rows).
 constexpr int kSegRows1 = 20, kSegRows2 = 12, kSegRowsAll = 64;
 // Segments are at most kSegSlack rows shorter than the compiled length (seg_plan keeps
-// 8, cluster_plan 10).
-constexpr int kSegSlack = 10;
+// 8, cluster_plan 12).
+constexpr int kSegSlack = 12;
 
 // One lane's place in its line's segments, in elements of the array walked:
 // register row k is at row[k * P] (k >= k0), rows before the segment at

@@ -172,7 +172,7 @@ __constant__ Task kTasksX2[7] = {{XU, XU, 0, XU, XU2, 1}, {XV, XV, 0, XV, XV2, 1
 // FP64 segmented: 256 threads (128 registers), the 13 solves' segments of a tile
 // fill 7 of 8 warps.  As 4-line tiles of 128 threads, 3 blocks an SM (3 of 4
 // warps, a quarter of the lanes idle): 128^3 2.62 -> 2.52 ms a step.
-template <typename T, int PC, int SEG = 0, bool FULL = false>
+template <typename T, int PC, int SEG = 0, bool FULL = false, int PLAIN = 0>
 __global__ void __launch_bounds__(SEG == kSeq ? kSeqTpbX : sweep_threads<T>(0),
                                   sizeof(T) == 4 && (SEG == 0 || FULL) ? kMinBlocksX : 2) k_sweep_x(SweepArgs<T> a) {
     using TS = std::conditional_t<(SEG > 0 && sizeof(T) == 4), TileSegX<SEG>, TileOf<T, SEG>>;
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(SEG == kSeq ? kSeqTpbX : sweep_threads<T>(0),
             // on a wall) use the state before the previous step's sponge
             // overwrite, which the reference's U,V,W,p,T arrays still hold.
             PrimW<T> ss = s;
-            if (a.use_backup) {
+            if (!PLAIN && a.use_backup) {
                 int i, j, k;
                 coords<0>(t, in.pt.l, in.pt.n, i, j, k);
                 const int f = faces_of(a.g, i, j, k);
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(SEG == kSeq ? kSeqTpbX : sweep_threads<T>(0),
             TS::two(sm, 5, p, L, zz.z1, zz.z1, f2, f3);
             const T f4 = TS::one(sm, XF4, p, L, zz.z1);
             a.dx[0][gi] = Ux; a.dx[1][gi] = Vx; a.dx[2][gi] = Wx; a.dx[3][gi] = Tx;
-            if (a.tape[0]) {  // the tape's x entries (kIn* 0..16)
+            if (!PLAIN && a.tape[0]) {  // the tape's x entries (kIn* 0..16)
                 T *const *g = a.tape;
                 g[0][gi] = U; g[1][gi] = V; g[2][gi] = W; g[3][gi] = Tt;
                 g[4][gi] = Ux; g[5][gi] = Vx; g[6][gi] = Wx; g[7][gi] = Tx;
@@ -292,7 +292,7 @@ __constant__ Task kTasksY2[8] = {{YU, YU, 0, YU, YU2, 1}, {YV, YV, 0, YV, YV2, 1
 
 // FP64: 3 blocks per SM (168 registers, no spills): 2.93 -> 2.67 ms per step at
 // TGV 128^3, 37.5 -> 27.1 at HIT 256^3, the same bits
-template <typename T, int PC, int SEG = 0, bool FULL = false, bool CL = false, bool WALL = false>
+template <typename T, int PC, int SEG = 0, bool FULL = false, bool CL = false, bool WALL = false, int PLAIN = 0>
 __global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBlocksY : 3) k_sweep_y(SweepArgs<T> a) {
     using TS = TileOf<T, SEG>;
     constexpr bool SQ = SEG == kSeq;
@@ -371,18 +371,22 @@ __global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBloc
             TS::two(sm, 6, p, L, zz.z1, zz.z1, f2, f3);
             const T f4 = TS::one(sm, YF4, p, L, zz.z1);
             a.dy[0][gi] = Uy; a.dy[1][gi] = Vy; a.dy[2][gi] = Wy; a.dy[3][gi] = Ty;
-            if (a.tape[0]) {  // the tape's y entries (kIn* 17..31)
+            if (!PLAIN && a.tape[0]) {  // the tape's y entries (kIn* 17..31)
                 T *const *g = a.tape;
                 g[17][gi] = Uy; g[18][gi] = Vy; g[19][gi] = Wy; g[20][gi] = Ty;
                 g[21][gi] = Uyy; g[22][gi] = Vyy; g[23][gi] = Wyy; g[24][gi] = Tyy;
                 g[25][gi] = Uxy; g[26][gi] = Vxy; g[27][gi] = cey;
                 g[28][gi] = f1; g[29][gi] = f2; g[30][gi] = f3; g[31][gi] = f4;
             }
-            int i, j, k;
-            coords<1>(t, p.l, p.n, i, j, k);
-            const int wd = a.wall_faces ? wall_dir(faces_of(a.g, i, j, k) & a.wall_faces) : -1;
-            if (wd == 1) a.R[0][gi] = -cey;
-            else if (wd < 0) a.R[0][gi] = in.v[4] - cey;
+            if constexpr (PLAIN != 0) {
+                a.R[0][gi] = in.v[4] - cey;
+            } else {
+                int i, j, k;
+                coords<1>(t, p.l, p.n, i, j, k);
+                const int wd = a.wall_faces ? wall_dir(faces_of(a.g, i, j, k) & a.wall_faces) : -1;
+                if (wd == 1) a.R[0][gi] = -cey;
+                else if (wd < 0) a.R[0][gi] = in.v[4] - cey;
+            }
             const T v1 = mu * (Uyy + c13 * Vxy), v2 = mu * (c43 * Vyy + c13 * Uxy), v3 = mu * Wyy;
             a.R[1][gi] = in.v[5] + (v1 - f1);
             a.R[2][gi] = in.v[6] + (v2 - f2);
@@ -402,7 +406,7 @@ __constant__ Task kTasksZ[8] = {{ZU, ZU, 0, ZU, ZU2, 1}, {ZV, ZV, 0, ZV, ZV2, 1}
 
 // The z sweep's three phases as functions of (tile, shared-memory layout,
 // thread range).
-template <typename T, int PC, int SEG, bool FULL, bool CL, bool WALL>
+template <typename T, int PC, int SEG, bool FULL, bool CL, bool WALL, int PLAIN>
 struct ZSweep {
     static constexpr bool SQ = SEG == kSeq;
     using TS = TileOf<T, SEG>;
@@ -467,7 +471,7 @@ struct ZSweep {
         const double dt = *a.dt;
         const T dtw = (T)dt;
         const int st = a.rk_step;
-        const bool tvd = a.rk == 1;
+        const bool tvd = PLAIN ? PLAIN == 2 : a.rk == 1;
         // which state arrays the update reads (uniform over the launch):
         //   qa = q1 (RK4 stage 1, all TVD-RK3 stages) or q2 (RK4 stages 2-4)
         //   qb = q1 for the FP64 RK4 qk update on stages 2-3, or the FP64 qk of
@@ -554,27 +558,24 @@ struct ZSweep {
                 R[3] = in.v[16] + (w3 - f3);
                 R[4] = in.v[17] + (cpPr * (MuX * Tx + MuY * Ty + MuZ * Tz + mu * Tzz) +
                                    (U * w1 + V * w2 + W * w3 + mu * diss) - f4);
-                T src0 = T(0);
-                if (a.sponge) {  // sigma (avg - q), SpongeBC / CSolver_AWS.hpp:228
-                    const T sg = to_work<T>(a.sigma[gi]);
-                    src0 = sg * (to_work<T>(a.savg.f[0][gi]) - a.qs[0][gi]);
-#pragma unroll
-                    for (int f = 1; f < 5; ++f)
-                        R[f] += (f == 4 ? T(2.0) * sg : sg) * (to_work<T>(a.savg.f[f][gi]) - a.qs[f][gi]);
-                }
                 // continuity and the post-step boundary fix-up (CSolver_AWS.cpp:1506-1679)
-                int i, j, k;
-                coords<2>(t, p.l, p.n, i, j, k);
-                const int fc = faces_of(a.g, i, j, k);
-                const int wd = a.wall_faces ? wall_dir(fc & a.wall_faces) : -1;
-                if (wd == 2) R[0] = -cez;
-                else if (wd < 0) R[0] = a.sponge ? R[0] - cez + src0 : R[0] - cez;
-                const bool zero_all = (fc & a.sponge_kind_faces) != 0;
-                const bool zero_mom = wd >= 0;
-                if (a.diag[0]) {  // derivative fields of the last stage, for diagnostics
+                bool zero_all = false, zero_mom = false;
+                if constexpr (PLAIN) {
+                    R[0] -= cez;
+                } else {
+                    int i, j, k;
+                    coords<2>(t, p.l, p.n, i, j, k);
+                    const int fc = faces_of(a.g, i, j, k);
+                    const int wd = a.wall_faces ? wall_dir(fc & a.wall_faces) : -1;
+                    if (wd == 2) R[0] = -cez;
+                    else if (wd < 0) R[0] -= cez;
+                    zero_all = (fc & a.sponge_kind_faces) != 0;
+                    zero_mom = wd >= 0;
+                }
+                if (!PLAIN && a.diag[0]) {  // derivative fields of the last stage, for diagnostics
                     a.diag[0][gi] = Uz; a.diag[1][gi] = Vz; a.diag[2][gi] = Wz;
                 }
-                if (a.tape[0]) {  // the tape's z entries (kIn* 32..47)
+                if (!PLAIN && a.tape[0]) {  // the tape's z entries (kIn* 32..47)
                     T *const *g = a.tape;
                     g[32][gi] = Uz; g[33][gi] = Vz; g[34][gi] = Wz; g[35][gi] = Tz;
                     g[36][gi] = Uzz; g[37][gi] = Vzz; g[38][gi] = Wzz; g[39][gi] = Tzz;
@@ -586,7 +587,7 @@ struct ZSweep {
                     // plain form: dq = dt * RHS in FP64; mixed form: in FP32
                     T d = sizeof(T) == 8 ? (T)(dt * (double)R[f]) : dtw * R[f];
                     if (zero_all || (f > 0 && zero_mom)) d = T(0);
-                    if (a.dq_out[0]) a.dq_out[f][gi] = to_f64(d);
+                    if (!PLAIN && a.dq_out[0]) a.dq_out[f][gi] = to_f64(d);
                     R[f] = d;
                 }
                 if (sizeof(T) == 8) {
@@ -641,9 +642,10 @@ struct ZSweep {
 
 // FP64: 3 blocks per SM (168 registers; 88 bytes of spill stores): 4.70 ->
 // 4.52 ms per step at TGV 128^3, 52.5 -> 44.9 at HIT 256^3, the same bits
-template <typename T, int PC, int SEG = 0, bool FULL = false, bool CL = false, bool WALL = false>
+// PLAIN: as plain_kind below (x and y: 1 for either integrator)
+template <typename T, int PC, int SEG = 0, bool FULL = false, bool CL = false, bool WALL = false, int PLAIN = 0>
 __global__ void __launch_bounds__(sweep_threads<T>(2), sizeof(T) == 4 ? kMinBlocksZ : 3) k_sweep_z(SweepArgs<T> a) {
-    using Z = ZSweep<T, PC, SEG, FULL, CL, WALL>;
+    using Z = ZSweep<T, PC, SEG, FULL, CL, WALL, PLAIN>;
     const int rank = CL ? (int)blockIdx.x % a.seg.C : 0;
     const Tile t = Z::SQ ? make_seq_tile<2>(a.g, a.seg, a.L, rank)
                          : CL ? make_cluster_tile<2>(a.g, a.seg, rank) : make_tile<2>(a.g, a.L);
@@ -919,6 +921,17 @@ static dim3 tile_grid(int dir, const Geom &g, int L) {
     return dim3((g.Nx + L - 1) / L, g.Ny);
 }
 
+// 1 (RK4) or 2 (TVD-RK3) where a launch has no walls, sponge faces, tape,
+// diagnostics or increments to store, else 0.  An instance without their code
+// has shorter load and update phases: 128^3 z 443 -> 425, y 238 -> 230, x 168 ->
+// 164 us a step, 256^3 z 3.32 -> 3.20 ms, y 1.84 -> 1.78.  One instance per RK
+// stage gave 454 and was dropped; between walls the same split gave nothing.
+template <typename T>
+static int plain_kind(const SweepArgs<T> &a) {
+    if (a.wall_faces || a.sponge_kind_faces || a.diag[0] || a.tape[0] || a.dq_out[0]) return 0;
+    return a.rk == 1 ? 2 : sizeof(T) == 8 || a.mixed_rk4 ? 1 : 0;
+}
+
 // the segmented instances: compile-time pitches for the full segments, the
 // three segment lengths at run-time pitch for the others
 static cudaError_t launch_seg_sweep(int dir, const SweepArgs<float> &a, dim3 grid, size_t sm, cudaStream_t s) {
@@ -928,36 +941,48 @@ static cudaError_t launch_seg_sweep(int dir, const SweepArgs<float> &a, dim3 gri
             if (dir == 1) return launch_cluster(f ? k_sweep_y<float, 32, 32, true, true, true> : k_sweep_y<float, 32, 32, false, true, true>, a, grid, sm, s);
             return launch_cluster(f ? k_sweep_z<float, 32, 32, true, true, true> : k_sweep_z<float, 32, 32, false, true, true>, a, grid, sm, s);
         }
-        if (dir == 1) return launch_cluster(f ? k_sweep_y<float, 32, 32, true, true> : k_sweep_y<float, 32, 32, false, true>, a, grid, sm, s);
-        return launch_cluster(f ? k_sweep_z<float, 32, 32, true, true> : k_sweep_z<float, 32, 32, false, true>, a, grid, sm, s);
+        const int plain = plain_kind(a);
+#define CL_CASE(K, PL) return launch_cluster(f ? K<float, 32, 32, true, true, false, PL> : K<float, 32, 32, false, true, false, PL>, a, grid, sm, s)
+        if (dir == 1) {
+            if (plain) CL_CASE(k_sweep_y, 1);
+            CL_CASE(k_sweep_y, 0);
+        }
+        if (plain == 1) CL_CASE(k_sweep_z, 1);
+        if (plain == 2) CL_CASE(k_sweep_z, 2);
+        CL_CASE(k_sweep_z, 0);
+#undef CL_CASE
     }
 #define SEG_CASE(K, PC, SEG, FULL) return launch_tile_kernel(K<float, PC, SEG, FULL>, a, grid, sm, s)
+#define X_CASE(PC, SEG, FULL) \
+    return plain_kind(a) ? launch_tile_kernel(k_sweep_x<float, PC, SEG, FULL, 1>, a, grid, sm, s) \
+                         : launch_tile_kernel(k_sweep_x<float, PC, SEG, FULL>, a, grid, sm, s)
     if (a.seg.full) {
-        if (dir == 0 && a.P == 17) SEG_CASE(k_sweep_x, 17, 32, true);
-        if (dir == 0 && a.P == 9) SEG_CASE(k_sweep_x, 9, 32, true);
-        if (dir == 0 && a.P == 5) SEG_CASE(k_sweep_x, 5, 32, true);
+        if (dir == 0 && a.P == 17) X_CASE(17, 32, true);
+        if (dir == 0 && a.P == 9) X_CASE(9, 32, true);
+        if (dir == 0 && a.P == 5) X_CASE(5, 32, true);
         if (dir == 1 && a.P == 16) SEG_CASE(k_sweep_y, 16, 32, true);
         if (dir == 1 && a.P == 8) SEG_CASE(k_sweep_y, 8, 32, true);
         if (dir == 2 && a.P == 16) SEG_CASE(k_sweep_z, 16, 32, true);
         if (dir == 2 && a.P == 8) SEG_CASE(k_sweep_z, 8, 32, true);
-        if (dir == 0) SEG_CASE(k_sweep_x, 0, 32, true);
+        if (dir == 0) X_CASE(0, 32, true);
         if (dir == 1) SEG_CASE(k_sweep_y, 0, 32, true);
         SEG_CASE(k_sweep_z, 0, 32, true);
     }
     if (a.seg.SEG == 32) {
-        if (dir == 0) SEG_CASE(k_sweep_x, 0, 32, false);
+        if (dir == 0) X_CASE(0, 32, false);
         if (dir == 1) SEG_CASE(k_sweep_y, 0, 32, false);
         SEG_CASE(k_sweep_z, 0, 32, false);
     }
     if (a.seg.SEG == 24) {
-        if (dir == 0) SEG_CASE(k_sweep_x, 0, 24, false);
+        if (dir == 0) X_CASE(0, 24, false);
         if (dir == 1) SEG_CASE(k_sweep_y, 0, 24, false);
         SEG_CASE(k_sweep_z, 0, 24, false);
     }
-    if (dir == 0) SEG_CASE(k_sweep_x, 0, 16, false);
+    if (dir == 0) X_CASE(0, 16, false);
     if (dir == 1) SEG_CASE(k_sweep_y, 0, 16, false);
     SEG_CASE(k_sweep_z, 0, 16, false);
 #undef SEG_CASE
+#undef X_CASE
 }
 
 template <typename T>
@@ -969,8 +994,14 @@ cudaError_t launch_sweep(int dir, const SweepArgs<T> &a, cudaStream_t s) {
         if (a.seg.SEG) return launch_seg_sweep(dir, a, grid, sm, s);
     } else if (a.seg.SEG == kSeq) {
         if (dir == 0) return launch_tile_kernel(k_sweep_x<T, 0, kSeq>, a, grid, sm, s);
-        return launch_cluster(dir == 1 ? k_sweep_y<T, 0, kSeq, false, true> : k_sweep_z<T, 0, kSeq, false, true>, a, grid,
-                                 sm, s);
+        // the y sweep of this form gains nothing from it (2.31 against 2.32 ms)
+        const int plain = plain_kind(a);
+#define SEQ_CASE(K, PL) return launch_cluster(K<T, 0, kSeq, false, true, false, PL>, a, grid, sm, s)
+        if (dir == 1) SEQ_CASE(k_sweep_y, 0);
+        if (plain == 1) SEQ_CASE(k_sweep_z, 1);
+        if (plain == 2) SEQ_CASE(k_sweep_z, 2);
+        SEQ_CASE(k_sweep_z, 0);
+#undef SEQ_CASE
     }
     if constexpr (sizeof(T) == 4) {
         if (dir == 0 && a.P == 9) return launch_tile_kernel(k_sweep_x<T, 9>, a, grid, sm, s);

@@ -1,15 +1,15 @@
 """The mixed form's segmented line solves (csrc/cs3d_seg.cuh) at the line
 lengths where their plan changes: the shortest and longest of each segment
 count, full and ragged segments, lines split over a cluster of blocks and
-lines in one block, and the lengths left to the Thomas solves (16, 87, 513)."""
+lines in one block, and the lengths left to the Thomas solves."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
-# clusters of one-segment blocks: 22..32, 44..64, 66..256; of two-segment
-# blocks: 264..512; one block: the others
-LENGTHS = [9, 15, 16, 17, 18, 21, 22, 31, 32, 33, 42, 43, 44, 63, 64, 65, 66, 77, 96, 97, 101, 127, 128, 129, 131, 176, 192, 193,
+# clusters of one-segment blocks: 20..32, 40..256; of two-segment blocks:
+# 257..512; one block: the others
+LENGTHS = [9, 15, 16, 17, 18, 19, 20, 21, 22, 31, 32, 33, 39, 40, 41, 42, 43, 44, 60, 61, 63, 64, 65, 66, 77, 96, 97, 101, 127, 128, 129, 131, 176, 192, 193,
            256, 257, 263, 264, 320, 511, 512, 513]
 
 # One RK4 step plus filter of a state of order one at CFL 0.5: each of the four
@@ -48,6 +48,31 @@ def test_mixed_step_tracks_fp64_at_plan_edges(gpu_pkg, N, d):
     assert float((np.abs(out[1] - out[0]) / scale).max()) <= TOL
 
 
+@pytest.mark.parametrize("rk", ["RK4", "TVDRK3"])
+@pytest.mark.parametrize("prec", ["FP64", "FP32_MIXED"])
+@pytest.mark.parametrize("n", [(32, 64, 32), (33, 45, 101), (12, 12, 12)])
+def test_steps_do_not_depend_on_what_is_stored(gpu_pkg, n, prec, rk):
+    """The sweeps' instances without the code of diagnostics and increments
+    compute what the general instances do: the same operations in the same
+    order but for contractions, a rounding of the working type a stage."""
+    abi = gpu_pkg._abi
+    ic = _noise((n[2], n[1], n[0]), 7)
+    out = []
+    for store in (0, 1):
+        s = gpu_pkg.Solver(gpu_pkg.make_config(n, tuple(6.283185307179586 * (1.0 - 1.0 / k) for k in n), mu_ref=1e-3, CFL=0.5,
+                                               rk=getattr(abi, rk), precision=getattr(abi, prec)))
+        s.set_option(gpu_pkg.OPT_STORE_DIAGNOSTICS, store)
+        s.set_option(gpu_pkg.OPT_STORE_INCREMENTS, store)
+        s.set_initial_conditions(*ic)
+        s.step()
+        s.sync()
+        out.append(s.conserved())
+        s.close()
+    eps = 2.0 ** -24 if prec == "FP32_MIXED" else 2.0 ** -53
+    scale = np.maximum(np.abs(out[0]).reshape(5, -1).max(1), 1.0).reshape(5, 1, 1, 1)
+    assert float((np.abs(out[1] - out[0]) / scale).max()) <= 5 * 4 * 4 * eps
+
+
 @pytest.mark.parametrize("kind", ["mixed", "fp64", "sponge"])
 def test_repeated_steps_equal_single_handles(gpu_pkg, kind):
     """Steps launched as a recorded graph (small grids, after eight of a form)
@@ -83,11 +108,11 @@ def test_repeated_steps_equal_single_handles(gpu_pkg, kind):
         s.close()
 
 
-@pytest.mark.parametrize("N", [43, 44, 45, 63, 64, 65, 66, 101, 127, 128, 176, 255, 256, 257])
+@pytest.mark.parametrize("N", [39, 40, 41, 43, 44, 45, 60, 61, 63, 64, 65, 66, 101, 127, 128, 176, 255, 256, 257])
 @pytest.mark.parametrize("d", [1, 2])
 def test_mixed_step_tracks_fp64_between_walls(gpu_pkg, N, d):
-    """Wall lines over a cluster (44..256 points but for 65; the others by the
-    Thomas solves).  The one-sided rows' taps sum to about ten times the
+    """Wall lines over a cluster (40..256 points; the others by the Thomas
+    solves).  The one-sided rows' taps sum to about ten times the
     interior's, and the walls' no-slip rows drive the largest increments."""
     abi = gpu_pkg._abi
     n = [19, 12, 12]
