@@ -412,8 +412,8 @@ SeqOp seq_op(const HostOp &h, const SegPlan &p) {
 }
 
 // The walls' rows of such a line: explicit rows, and the tables of the first
-// and last segment (device memory).
-int wall_op(const HostOp &h, const SegPlan &p, WallOp &w, float **mem, cudaStream_t s) {
+// and last segment.
+void wall_op(const HostOp &h, const SegPlan &p, WallOp &w) {
     const double a = h.alo[h.N / 2], l = (1.0 - std::sqrt(1.0 - 4.0 * a * a)) / (2.0 * a), q = 1.0 + l * l;
     for (int b = 0; b < 4; b++)
         for (int j = 0; j < 6; j++) {
@@ -421,23 +421,15 @@ int wall_op(const HostOp &h, const SegPlan &p, WallOp &w, float **mem, cudaStrea
             const int k = b < 2 ? j : h.N - 6 + j - h.boff[b];
             w.bt[b][j] = k >= 0 ? (float)(h.btaps[b][k] * h.scale * q) : 0.f;
         }
-    std::vector<float> t(3 * 64, 0.f);
     for (int e = 0; e < 2; e++) {
         const int len = e ? p.S - (p.G - 1 >= p.nS) : p.S, row0 = e ? h.N - len : 0;
         for (int k = 32 - len; k < 32; k++) {
             const int row = row0 + k - (32 - len);
-            t[32 * e + k] = (float)(h.iw[row] / q);
-            t[64 + 32 * e + k] = row > 0 ? (float)(-h.alo[row] * h.iw[row]) : 0.f;
-            t[128 + 32 * e + k] = row < h.N - 1 ? (float)(-h.c[row] * h.iw[row]) : 0.f;
+            w.s[e][k] = (float)(h.iw[row] / q);
+            w.f[e][k] = row > 0 ? (float)(-h.alo[row] * h.iw[row]) : 0.f;
+            w.b[e][k] = row < h.N - 1 ? (float)(-h.c[row] * h.iw[row]) : 0.f;
         }
     }
-    CS3D_CUDA(cudaMalloc(mem, t.size() * 4));
-    CS3D_CUDA(cudaMemcpyAsync(*mem, t.data(), t.size() * 4, cudaMemcpyHostToDevice, s));
-    CS3D_CUDA(cudaStreamSynchronize(s));
-    w.s = *mem;
-    w.f = *mem + 64;
-    w.b = *mem + 128;
-    return CS3D_OK;
 }
 
 // One operator of contiguous FP64 lines in register segments: the launch
@@ -550,7 +542,6 @@ struct cs3d_handle {
     SegPlan seg[3] = {};     // mixed form: the periodic directions' segmented solves
     SegOp<float> segop[3][2] = {};  // 1st and 2nd derivative
     WallOp wallop[3][2] = {};
-    float *wallmem[3][2] = {};
     SegPlan segf[3] = {};    // the filter's, and its correction operator
     SegOp<float> segfop[3] = {};
     // FP64 lines in register segments (post-processor, FP64 adjoint)
@@ -890,8 +881,7 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
                 h->seg[d] = d > 0 && cfg->Nx >= 18 ? cluster_plan(Nd[d], ho.periodic) : SegPlan{};
                 if (ho.periodic && !h->seg[d].C) h->seg[d] = seg_plan(Nd[d], d > 0);
                 h->segop[d][k - 1] = seg_op<float>(ho, h->seg[d], 30);
-                if (h->seg[d].wall && (r = wall_op(ho, h->seg[d], h->wallop[d][k - 1], &h->wallmem[d][k - 1], h->stream)))
-                    return fail_free(r);
+                if (h->seg[d].wall) wall_op(ho, h->seg[d], h->wallop[d][k - 1]);
             } else if (h->mixed && ho.periodic && factors(ho)) {
                 h->segf[d] = seg_plan(Nd[d], false);
                 h->segfop[d] = seg_op<float>(make_filter_correction(ho), h->segf[d], 30);
@@ -987,7 +977,6 @@ extern "C" int cs3d_destroy(cs3d_handle *h) {
             if (h->op64[d][k].mem) cudaFree(h->op64[d][k].mem);
             if (h->op32[d][k].mem) cudaFree(h->op32[d][k].mem);
             if (h->lseg[d][k].mem) cudaFree(h->lseg[d][k].mem);
-            if (k < 2 && h->wallmem[d][k]) cudaFree(h->wallmem[d][k]);
         }
     for (int d = 0; d < 3; d++)
         if (h->op32fc[d].mem) cudaFree(h->op32fc[d].mem);

@@ -559,7 +559,7 @@ __global__ void k_lin5(Lin5Args a) {
 // blockIdx.y: the field; 16-byte words, or 4-byte ones where a field is not
 // aligned (four words a thread in flight)
 template <typename W>
-__global__ void k_copy5(Copy5Args a) {
+__global__ void k_copy5(const __grid_constant__ Copy5Args a) {
     const W *src = static_cast<const W *>(a.src[blockIdx.y]);
     W *dst = static_cast<W *>(a.dst[blockIdx.y]);
     const long long n = (long long)(a.bytes / sizeof(W));

@@ -134,13 +134,12 @@ __global__ void __launch_bounds__(kLineSegTpb, WALL && SEG > 24 ? 3 : 4) k_line_
 #pragma unroll
             for (int b = 0; b < H; ++b) {
                 const double v = explicit_row(seg == 0 ? b : H + b, seg == 0 ? 0 : max(G - 2, 0));
-                if (seg == 0) {
+                // (selects: as an assignment to row k0 + b the array leaves the
+                // registers)
+                const bool lo = seg == 0;
 #pragma unroll
-                    for (int k = 0; k < kSegSlack + H; ++k)
-                        if (k == k0 + b) y[k] = v;
-                } else {
-                    y[SEG - H + b] = v;
-                }
+                for (int k = 0; k < kSegSlack + H; ++k) y[k] = lo && k == k0 + b ? v : y[k];
+                y[SEG - H + b] = lo ? y[SEG - H + b] : v;
                 if (G == 1) y[SEG - H + b] = explicit_row(H + b, 0);
             }
         }

@@ -331,67 +331,62 @@ __device__ __forceinline__ E *cluster_map(E *p, int rank) {
 // others run as on a periodic line, as does every exchange.
 struct WallOp {
     float bt[4][6];         // the explicit rows (scaled as the taps): 0, 1 from row 0 on, N-2, N-1 from row N-6 on
-    const float *s, *f, *b; // [2][32]: y_n = s_n r_n + f_n y_{n-1}, x_n = y_n + b_n x_{n+1}
+    float s[2][32], f[2][32], b[2][32];  // y_n = s_n r_n + f_n y_{n-1}, x_n = y_n + b_n x_{n+1}
 };
 
-// The explicit rows of the first (end = 0) or last segment into y, from the
-// tile (lane LN of the pair, or both fields' own).
-template <int SEG, bool FULL>
-__device__ __forceinline__ void wall_rows(float (&y)[SEG], const float *x, int P2, const WallOp &w, int end, int k0) {
-    // (the rows' coefficients sum to zero: differences from the wall value, so
-    // that rounded coefficients make no derivative of a constant)
-    const float *p = x + (end ? SEG - 6 : FULL ? 0 : k0) * P2;
-    const float v0 = p[end ? 5 * P2 : 0];
+// One solve of the first (END = 0) or last segment from zero: its last forward
+// value into e, its first solution value into b.  x: the segment's first row,
+// in the tile (of one lane of the pair).  END and the rows are
+// known to the compiler, so that a table's entry is an operand of its operation
+// and not a load (y of 256x128x42, 64 of 128 rows in such segments: 49.3 us a
+// stage with tables in memory, 44.8 so).
+template <int SEG, bool FULL, int END>
+__device__ __forceinline__ void wall_solve(float (&y)[SEG], const float *x, int P2, const WallOp &w, int k0, float &e,
+                                           float &b) {
+    // the explicit rows.  (Their coefficients sum to zero: differences from the
+    // wall value, so that rounded coefficients make no derivative of a constant.)
+    const float *p = x + (END ? SEG - 6 : FULL ? 0 : k0) * P2;
+    const float v0 = p[END ? 5 * P2 : 0];
     float r0 = 0.f, r1 = 0.f;
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
         const float v = p[j * P2] - v0;
-        r0 = fmaf(w.bt[2 * end][j], v, r0);
-        r1 = fmaf(w.bt[2 * end + 1][j], v, r1);
+        r0 = fmaf(w.bt[2 * END][j], v, r0);
+        r1 = fmaf(w.bt[2 * END + 1][j], v, r1);
     }
-    if (end) {
+    if (END) {
         y[SEG - 2] = r0;
         y[SEG - 1] = r1;
     } else if (FULL) {
         y[0] = r0;
         y[1] = r1;
     } else {
+        // (selects: as an assignment to row k0 the array leaves the registers:
+        // y of 128x127x128 101 us a stage, 73 so)
 #pragma unroll
-        for (int k = 0; k < kSegSlack + 2; ++k) {
-            if (k == k0) y[k] = r0;
-            if (k == k0 + 1) y[k] = r1;
-        }
+        for (int k = 0; k < kSegSlack + 2; ++k) y[k] = k == k0 ? r0 : k == k0 + 1 ? r1 : y[k];
     }
-}
-template <int SEG>
-__device__ __forceinline__ float wall_fwd(float (&y)[SEG], const WallOp &w, int end) {
-    const float *s = w.s + 32 * end, *f = w.f + 32 * end;
     float c = 0.f;
 #pragma unroll
-    for (int k = 0; k < SEG; k += 4) {
-        float s4[4], f4[4];
-        load4(s + k, s4);
-        load4(f + k, f4);
+    for (int k = 0; k < SEG; ++k) y[k] = c = fmaf(w.f[END][k], c, w.s[END][k] * y[k]);
+    e = c;
+    c = b = 0.f;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) y[k + j] = c = fmaf(f4[j], c, s4[j] * y[k + j]);
+    for (int k = SEG - 1; k >= 0; --k) {
+        y[k] = c = fmaf(w.b[END][k], c, y[k]);
+        if (!FULL && k <= kSegSlack) b = k == k0 ? c : b;
     }
-    return c;
+    if (FULL) b = c;
 }
-template <int SEG, bool FULL>
-__device__ __forceinline__ float wall_bwd(float (&y)[SEG], const WallOp &w, int end, int k0) {
-    const float *b = w.b + 32 * end;
-    float c = 0.f, first = 0.f;
-#pragma unroll
-    for (int k = SEG - 4; k >= 0; k -= 4) {
-        float b4[4];
-        load4(b + k, b4);
-#pragma unroll
-        for (int j = 3; j >= 0; --j) {
-            y[k + j] = c = fmaf(b4[j], c, y[k + j]);
-            if (!FULL && k + j <= kSegSlack) first = k + j == k0 ? c : first;
-        }
-    }
-    return FULL ? c : first;
+// A task's two solves there: y1 by w1, y2 by w2 (dd: a second derivative, of the
+// lane x field unless MIX) or w1.
+template <int SEG, bool FULL, bool MIX, int END>
+__device__ __forceinline__ void wall_task(float (&y1)[SEG], float (&y2)[SEG], const float *x, int P2, const WallOp &w1,
+                                          const WallOp &w2, int k0, bool dd, bool single, float2 &e, float2 &b) {
+    wall_solve<SEG, FULL, END>(y1, x, P2, w1, k0, e.x, b.x);
+    if (dd) wall_solve<SEG, FULL, END>(y2, MIX ? x + 1 : x, P2, w2, k0, e.y, b.y);
+    else if (!single) wall_solve<SEG, FULL, END>(y2, x + 1, P2, w1, k0, e.y, b.y);
+    else e.y = b.y = 0.f;
 }
 
 // The solves of a sweep tile (tasks as run_seg_tasks), one unit a warp: pl.B
@@ -427,18 +422,9 @@ __device__ __forceinline__ void run_cluster_tasks(float2 *tile, int pstride2, fl
     else seg_pair_rhs<SEG, FULL, 1>(y1, y2, s, P, o1, o2);
     float2 e, b;  // the segment's last forward value, its first solution value
     if (WALL && (rank == 0 || rank == C - 1)) {
-        const int end = rank > 0;
-        const WallOp &wb = dd ? *w2 : *w1;
         const float *x = reinterpret_cast<const float *>(s.row);
-        wall_rows<SEG, FULL>(y1, x, 2 * P, *w1, end, s.k0);
-        e.x = wall_fwd<SEG>(y1, *w1, end);
-        b.x = wall_bwd<SEG, FULL>(y1, *w1, end, s.k0);
-        e.y = b.y = 0.f;
-        if (!single) {
-            wall_rows<SEG, FULL>(y2, dd && !MIX ? x : x + 1, 2 * P, wb, end, s.k0);
-            e.y = wall_fwd<SEG>(y2, wb, end);
-            b.y = wall_bwd<SEG, FULL>(y2, wb, end, s.k0);
-        }
+        if (rank == 0) wall_task<SEG, FULL, MIX, 0>(y1, y2, x, 2 * P, *w1, *w2, s.k0, dd, single, e, b);
+        else wall_task<SEG, FULL, MIX, 1>(y1, y2, x, 2 * P, *w1, *w2, s.k0, dd, single, e, b);
     } else {
         e.x = seg_fwd<SEG>(y1, o1);
         b.x = seg_bwd0<SEG, FULL>(y1, o1, s.k0);

@@ -141,3 +141,28 @@ def test_mixed_step_tracks_fp64_between_walls(gpu_pkg, N, d):
         s.close()
     scale = np.maximum(np.abs(out[0]).reshape(5, -1).max(1), 1.0).reshape(5, 1, 1, 1)
     assert float((np.abs(out[1] - out[0]) / scale).max()) <= 10 * TOL
+
+
+@pytest.mark.parametrize("N", [19, 20, 21, 22, 31, 32, 33, 39, 40, 41, 42, 44, 65, 101, 256, 257, 511])
+@pytest.mark.parametrize("d", [0, 1, 2])
+def test_mixed_transposed_sweep_tracks_fp64_at_plan_edges(gpu_pkg, N, d):
+    """The transposed sweeps use the same plans.  FP32 rounds each of about
+    forty products of a seed of order one and a coefficient at 2^-24, against the
+    largest entry of a field; 2e-3 leaves the cancellation of the second
+    derivatives' taps (four orders), a wrong neighbour is of order one."""
+    abi = gpu_pkg._abi
+    n = [20, 20, 20]
+    n[d] = N
+    n[(d + 1) % 3] = 19
+    rho, p, U, V, W = _noise((n[2], n[1], n[0]), 900 * d + N)
+    q = np.stack([rho, rho * U, rho * V, rho * W, p / 0.4 + 0.5 * rho * (U * U + V * V + W * W)])
+    w = np.random.default_rng(N).standard_normal(q.shape)
+    out = []
+    for prec in (abi.FP64, abi.FP32_MIXED):
+        s = gpu_pkg.Solver(gpu_pkg.make_config(tuple(n), tuple(6.283185307179586 * (1.0 - 1.0 / k) for k in n), mu_ref=1e-3, CFL=0.5,
+                                               precision=prec))
+        s.set_initial_conditions(rho, p, U, V, W)
+        out.append(s.rhs_vjp(q, w))
+        s.close()
+    for f in range(5):
+        assert np.abs(out[1][f] - out[0][f]).max() <= 2e-3 * np.abs(out[0][f]).max(), f
