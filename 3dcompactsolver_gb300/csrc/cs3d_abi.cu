@@ -1210,12 +1210,14 @@ static int run_stage(cs3d_handle *h, int st, int last) {
         a.divN = make_fastdiv((unsigned)(d == 0 ? h->g.Nx : d == 1 ? h->g.Ny : h->g.Nz));
         a.P = a.L + x_pitch_plus(h, d);
         a.seg = h->seg[d];
-        a.g1 = h->segop[d][0];
-        a.g2 = h->segop[d][1];
-        a.w1 = h->wallop[d][0];
-        a.w2 = h->wallop[d][1];
-        a.h1 = h->seqop[d][0];
-        a.h2 = h->seqop[d][1];
+        if constexpr (sizeof(T) == 4) {
+            a.g1 = h->segop[d][0];
+            a.g2 = h->segop[d][1];
+            a.wall = h->wallop[d];
+        } else {
+            a.h1 = h->seqop[d][0];
+            a.h2 = h->seqop[d][1];
+        }
         if (sizeof(T) == 8) {
             a.d1 = *reinterpret_cast<const LineOp<T> *>(&h->op64[d][0].op);
             a.d2 = *reinterpret_cast<const LineOp<T> *>(&h->op64[d][1].op);

@@ -38,8 +38,24 @@ struct GasParams {
 // What the z sweep writes as the FP32 shadow of the next stage's input.
 enum ShadowTarget { SHADOW_NONE = 0, SHADOW_QK = 1, SHADOW_Q2 = 2 };
 
+// The solves' operators by form (what a launch does not read it does not carry:
+// the host pays for every byte: with all of them, 4.7 KB, small grids took
+// 1-3 us more a step).  seg.SEG > 0: the mixed form's segmented solves, or the plain
+// form's sequential ones (seg: G = C blocks' rows of a line).
 template <typename T>
-struct SweepArgs {
+struct SolveArgs {
+    SegPlan seg;
+    SegOp<float> g1, g2;
+    const WallOp *wall;  // (host) two, for lines between walls
+};
+template <>
+struct SolveArgs<double> {
+    SegPlan seg;
+    SeqOp h1, h2;
+};
+
+template <typename T>
+struct SweepArgs : SolveArgs<T> {
     Geom g;
     int L;          // lines per tile (a power of two)
     int lgL;        // log2(L)
@@ -47,10 +63,6 @@ struct SweepArgs {
     int P;          // shared-memory pitch between positions of a line
     int threads;    // threads per block
     LineOp<T> d1, d2;
-    SegPlan seg;    // mixed form, periodic lines (seg.SEG > 0): the segmented
-    SegOp<float> g1, g2;  // solves' plan and operators; plain form: the
-    WallOp w1, w2;  // (lines between walls)
-    SeqOp h1, h2;   // sequential solves' (seg: G = C blocks' rows of a line)
     GasParams gas;
     const T *qs[5]; // stage input q* in the work precision (FP64 q* itself, or
                     // its FP32 shadow in the mixed form)
@@ -84,6 +96,10 @@ struct SweepArgs {
     // U, V, W, T and the 44 derivative values of the right-hand side, in the
     // order of cs3d_rhs_adjoint.cuh's kIn* indices; null = not written
     T *tape[48];
+};
+template <typename T>
+struct WallSweepArgs : SweepArgs<T> {
+    WallOp w1, w2;
 };
 
 template <typename T>

@@ -1,27 +1,30 @@
 // cs3d_sweeps.cu -- the directional sweep kernels of one RK stage, the
 // compact filter and the single-operator kernel (sm_103a).
 //
-// One stage is three fused directional sweeps.  Each sweep kernel takes a
-// pencil tile -- L complete grid lines along the sweep direction -- and runs
-// three phases:
+// One stage is three fused directional sweeps.  A block takes a tile of lines
+// along the sweep direction -- whole lines, or 32 lines' rows of one block of a
+// cluster -- and runs three phases:
 //
 //   A  load the tile's inputs (batched, several points per thread in
 //      flight), form primitives and fluxes, stage every line-solve input in
 //      shared memory ([position][line] layout);
-//   B  solve: one thread per (line, task); a task is two line solves run
-//      interleaved -- the 1st and 2nd derivative of one field, or the 1st
-//      derivative of two fields -- each a Thomas sweep with precomputed
-//      factors, unrolled in chunks of 4 rows with the next chunk's loads
-//      issued ahead;
+//   B  solve.  A task is two line solves run together -- the 1st and 2nd
+//      derivative of one field, or the 1st derivative of two.  Mixed form:
+//      segments of 16 to 32 rows in registers (run_seg_x, run_cluster_tasks);
+//      plain form: one thread walks its block's rows (run_seq_tasks); Thomas
+//      sweeps with precomputed factors for the lines that neither cuts (FP64
+//      wall lines, lines of 8 or above 512 points);
 //   C  consume the derivatives point by point.
 //
 //   sweep x : primitives, Euler x-fluxes, 13 x-solves; writes Ux,Vx,Wx,Tx,
-//             mu, mu'(T) and the linear x-part of the five right-hand sides
+//             the plain form's p, mu, mu'(T) and the linear x-part of the
+//             five right-hand sides
 //   sweep y : 15 y-solves (incl. the cross derivatives Uxy, Vxy); writes
 //             Uy,Vy,Wy,Ty and adds the linear y-part
 //   sweep z : 16 z-solves (incl. d/dz of Ux+Vy, Wx, Wy), the nonlinear viscous
-//             terms, sponge sources, dt, the wall/sponge increment fix-up and
-//             the RK4 / TVD-RK3 update of the conserved state
+//             terms, dt, the wall/sponge increment fix-up and the RK4 /
+//             TVD-RK3 update of the conserved state (k_sponge_source, where
+//             there is a sponge, runs before it)
 //
 // The reference instead stores ~48 derivative fields and makes ~54 layout
 // transposes per stage (CSolver_AWS.cpp:829-1243).  Lines along y and z are
@@ -38,14 +41,14 @@
 namespace cs3d {
 
 // Points per thread in flight in the point loops of the mixed form (measured
-// at 128^3 and 256^3; deeper batches spill or run no faster).
+// at 128^3 and 256^3; deeper batches spill or run no faster).  The x sweep and
+// every load phase: 4; the z update: 1 (its 33 loads a point are enough).
 constexpr int kFilterBatch = 4;         // the mixed filter's load and store loops
 constexpr int kFilterConsumeBatch = 2;  // the mixed filter's consume loop
 constexpr int kYConsumeBatch = 4;       // the y sweep's consume phase
-// Resident blocks per SM the mixed-form kernels are compiled for: the filter
-// at 4 (64 registers), the x sweep at 3 blocks of 256 threads (80 registers),
-// y and z at one block of 512 (128 registers); the plain form runs 128
-// threads, 2 blocks.
+// Resident blocks per SM the mixed-form kernels are compiled for: the x sweep 3
+// blocks of 256 threads (80 registers; ragged segments 2), y and z 512 threads
+// (128 registers: two cluster blocks of 256), the Thomas filter 4 (64).
 constexpr int kFilterMinBlocks = 4;
 constexpr int kMinBlocksX = 3, kMinBlocksY = 1, kMinBlocksZ = 1;
 
@@ -62,12 +65,11 @@ constexpr bool kRecompute = sizeof(T) == 4;
 // shared-memory access of a solve chunk becomes an immediate off one base
 // register: x 0.358 -> 0.336 ms, y and z 2-4% faster per step at 128^3.
 //
-// SEG > 0 (mixed form, periodic lines): the segmented solves of cs3d_seg.cuh,
-// SEG rows a segment, FULL when the line length is a multiple; the tile then
-// has no line factors and its solutions need no correction on read.  SEG = 0:
-// the Thomas solves with precomputed factors (the plain form, wall lines, and
-// lengths that seg_plan does not cut).
-constexpr int ZS_ = 8;  // the first of the z tile's slots that park dq (ZS)
+// SEG > 0: the segmented solves of cs3d_seg.cuh, SEG rows a segment (kSeq: the
+// plain form's sequential ones), FULL when the line length is a multiple; CL: the
+// line over a cluster; WALL: between walls.  The tile then has no line factors
+// and its solutions need no correction on read.  SEG = 0: the Thomas solves with
+// precomputed factors (FP64 wall lines, and lengths that no plan cuts).
 template <typename T, int SEG>
 struct TileOf {
     using SM = typename SweepSmem<T>::type;
@@ -80,8 +82,6 @@ struct TileOf {
         get2(sm, t, p, L, za, zb, a, b);
     }
     static __device__ __forceinline__ T one(const SM &sm, int k, const Pt &p, int L, T z) { return get1(sm, k, p, L, z); }
-    // the z sweep parks dq in five of the point's spent solve slots
-    static __device__ __forceinline__ T &dq(const SM &sm, int f, int o) { return sm.at(ZS_ + f, o); }
 };
 // FP64, periodic lines: planar buffers of the sequential solves, the n1 first
 // derivatives, then the four second derivatives (each solved in place, so the
@@ -112,7 +112,6 @@ struct TileOf<double, kSeq> {
         b = sm.at(t < 4 ? sm.n1 + t : 2 * t - 3, p.o);
     }
     static __device__ __forceinline__ double one(const SM &sm, int, const Pt &p, int, double) { return sm.at(sm.n1 - 1, p.o); }
-    static __device__ __forceinline__ double &dq(const SM &sm, int f, int o) { return sm.at(4 + f, o); }
     static __device__ __forceinline__ double *mail(const SM &sm) { return sm.buf + (sm.n1 + 4) * sm.stride; }
 };
 __device__ __forceinline__ void put2(const SmemSeq &sm, int t, int o, double v0, double v1) {
@@ -147,7 +146,6 @@ struct TileSeg {
         b = v.y;
     }
     static __device__ __forceinline__ float one(const SM &sm, int k, const Pt &p, int, float) { return sm.at(k, p.o); }
-    static __device__ __forceinline__ float &dq(const SM &sm, int f, int o) { return sm.at(ZS_ + f, o); }
 };
 template <> struct TileOf<float, 16> : TileSeg<16> {};
 template <> struct TileOf<float, 24> : TileSeg<24> {};
@@ -293,7 +291,8 @@ __constant__ Task kTasksY2[8] = {{YU, YU, 0, YU, YU2, 1}, {YV, YV, 0, YV, YV2, 1
 // FP64: 3 blocks per SM (168 registers, no spills): 2.93 -> 2.67 ms per step at
 // TGV 128^3, 37.5 -> 27.1 at HIT 256^3, the same bits
 template <typename T, int PC, int SEG = 0, bool FULL = false, bool CL = false, bool WALL = false, int PLAIN = 0>
-__global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBlocksY : 3) k_sweep_y(SweepArgs<T> a) {
+__global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBlocksY : 3)
+k_sweep_y(std::conditional_t<WALL, WallSweepArgs<T>, SweepArgs<T>> a) {
     using TS = TileOf<T, SEG>;
     constexpr bool SQ = SEG == kSeq;
     const int L = CL && !SQ ? kClLines : a.L, P = PC > 0 ? PC : a.P, lgL = CL && !SQ ? 5 : a.lgL;
@@ -334,9 +333,12 @@ __global__ void __launch_bounds__(sweep_threads<T>(1), sizeof(T) == 4 ? kMinBloc
     else __syncthreads();
     if constexpr (SQ)
         run_seq_tasks(sm.buf, sm.stride, TS::mail(sm), kSeqN1Y, L, lgL, N, a.seg, a.h1, a.h2, rank, threadIdx.x);
-    else if constexpr (CL)
-        run_cluster_tasks<FULL, 8, true, false, WALL>(sm.pair(0), sm.pstride / 2, cluster_mail(sm), a.seg, a.g1, a.g2,
+    else if constexpr (WALL)
+        run_cluster_tasks<FULL, 8, true, false, true>(sm.pair(0), sm.pstride / 2, cluster_mail(sm), a.seg, a.g1, a.g2,
                                                       rank, threadIdx.x, &a.w1, &a.w2);
+    else if constexpr (CL)
+        run_cluster_tasks<FULL, 8, true>(sm.pair(0), sm.pstride / 2, cluster_mail(sm), a.seg, a.g1, a.g2, rank,
+                                         threadIdx.x);
     else if constexpr (SEG > 0)
         run_seg_tasks<SEG, FULL, 8, true>(sm, P, L, N, a.seg, a.g1, a.g2, threadIdx.x, blockDim.x);
     else
@@ -449,13 +451,13 @@ struct ZSweep {
     }
     // B: the 16 solves (8 pairs) of every line of the tile
     static __device__ __forceinline__ void solve(const SweepArgs<T> &a, const Tile &t, const SM &sm, int tid,
-                                                 int nthr) {
+                                                 int nthr, const WallOp *w1 = nullptr, const WallOp *w2 = nullptr) {
         const int rank = CL ? (int)blockIdx.x % a.seg.C : 0;
         if constexpr (SQ)
             run_seq_tasks(sm.buf, sm.stride, TS::mail(sm), kSeqN1Z, a.L, a.lgL, t.N, a.seg, a.h1, a.h2, rank, tid);
         else if constexpr (CL)
             run_cluster_tasks<FULL, 8, false, false, WALL>(sm.pair(0), sm.pstride / 2, cluster_mail(sm), a.seg, a.g1,
-                                                           a.g2, rank, tid, &a.w1, &a.w2);
+                                                           a.g2, rank, tid, w1, w2);
         else if constexpr (SEG > 0)
             run_seg_tasks<SEG, FULL, 8, false>(sm, PC > 0 ? PC : a.P, a.L, t.N, a.seg, a.g1, a.g2, tid, nthr);
         else
@@ -487,7 +489,6 @@ struct ZSweep {
         // of the update (two an SM and clock) run under the other warps' FP32
         // work and loads.  As two passes over the tile, the update alone took 8.5 of a
         // block's 20 us at 128^3.
-        static_assert(ZS == ZS_ && ZF1 == ZS_ + 4, "dq slots");
         struct InC {
             Pt pt;
             T v[18];
@@ -644,7 +645,8 @@ struct ZSweep {
 // 4.52 ms per step at TGV 128^3, 52.5 -> 44.9 at HIT 256^3, the same bits
 // PLAIN: as plain_kind below (x and y: 1 for either integrator)
 template <typename T, int PC, int SEG = 0, bool FULL = false, bool CL = false, bool WALL = false, int PLAIN = 0>
-__global__ void __launch_bounds__(sweep_threads<T>(2), sizeof(T) == 4 ? kMinBlocksZ : 3) k_sweep_z(SweepArgs<T> a) {
+__global__ void __launch_bounds__(sweep_threads<T>(2), sizeof(T) == 4 ? kMinBlocksZ : 3)
+k_sweep_z(std::conditional_t<WALL, WallSweepArgs<T>, SweepArgs<T>> a) {
     using Z = ZSweep<T, PC, SEG, FULL, CL, WALL, PLAIN>;
     const int rank = CL ? (int)blockIdx.x % a.seg.C : 0;
     const Tile t = Z::SQ ? make_seq_tile<2>(a.g, a.seg, a.L, rank)
@@ -653,7 +655,8 @@ __global__ void __launch_bounds__(sweep_threads<T>(2), sizeof(T) == 4 ? kMinBloc
     Z::load(a, t, sm, threadIdx.x, blockDim.x);
     if constexpr (CL) cluster_sync();
     else __syncthreads();
-    Z::solve(a, t, sm, threadIdx.x, blockDim.x);
+    if constexpr (WALL) Z::solve(a, t, sm, threadIdx.x, blockDim.x, &a.w1, &a.w2);
+    else Z::solve(a, t, sm, threadIdx.x, blockDim.x);
     __syncthreads();
     Z::consume(a, t, sm, threadIdx.x, blockDim.x);
 }
@@ -938,8 +941,12 @@ static cudaError_t launch_seg_sweep(int dir, const SweepArgs<float> &a, dim3 gri
     if (a.seg.C) {
         const bool f = a.seg.full;
         if (a.seg.wall) {
-            if (dir == 1) return launch_cluster(f ? k_sweep_y<float, 32, 32, true, true, true> : k_sweep_y<float, 32, 32, false, true, true>, a, grid, sm, s);
-            return launch_cluster(f ? k_sweep_z<float, 32, 32, true, true, true> : k_sweep_z<float, 32, 32, false, true, true>, a, grid, sm, s);
+            WallSweepArgs<float> w;
+            static_cast<SweepArgs<float> &>(w) = a;
+            w.w1 = a.wall[0];
+            w.w2 = a.wall[1];
+            if (dir == 1) return launch_cluster(f ? k_sweep_y<float, 32, 32, true, true, true> : k_sweep_y<float, 32, 32, false, true, true>, w, grid, sm, s);
+            return launch_cluster(f ? k_sweep_z<float, 32, 32, true, true, true> : k_sweep_z<float, 32, 32, false, true, true>, w, grid, sm, s);
         }
         const int plain = plain_kind(a);
 #define CL_CASE(K, PL) return launch_cluster(f ? K<float, 32, 32, true, true, false, PL> : K<float, 32, 32, false, true, false, PL>, a, grid, sm, s)

@@ -623,30 +623,6 @@ __device__ __forceinline__ void rhs_pass(const Smem<T> &sm, int src0, int dst0, 
     }
 }
 
-// Per-thread loop over the points of a tile with a software pipeline: the
-// global loads of the thread's next point are issued before the current
-// point is computed, so memory latency overlaps the arithmetic.
-// ld(S&, p) loads point p; cp(S&) computes and stores it.
-// tid / nthr: this thread's index among the nthr threads sharing the loop.
-template <typename S, typename LD, typename CP>
-__device__ __forceinline__ void pipelined(int NL, int tid, int nthr, LD &&ld, CP &&cp) {
-    int p = tid;
-    if (p >= NL) return;
-    S s0, s1;
-    ld(s0, p);
-    for (;;) {
-        const int p1 = p + nthr;
-        if (p1 < NL) ld(s1, p1);
-        cp(s0);
-        if (p1 >= NL) break;
-        const int p2 = p1 + nthr;
-        if (p2 < NL) ld(s0, p2);
-        cp(s1);
-        if (p2 >= NL) break;
-        p = p2;
-    }
-}
-
 // Per-thread loop over the points of a tile in batches of B: the loads of B
 // points are issued together, then the B points are computed and stored.
 template <typename S, int B, typename LD, typename CP>
