@@ -916,10 +916,14 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
         shape(&h->seg[d], h->L[d], h->threads[d]);
         const int other = d == 0 ? cfg->Ny : cfg->Nx, planes = d == 2 ? cfg->Ny : cfg->Nz;
         // fewer lines a tile where the grid would leave SMs without a block
-        // (16^3: 2 lines, 128 blocks a launch)
+        // (16^3: 2 lines, 128 blocks a launch); the mixed y and z tiles only
+        // below half of the SMs, as narrower ones leave solving lanes idle
+        // (44x39x38, three handles, two steps: 178 us, so 147; one handle's
+        // kernels take the same time or less)
+        const int fill = h->mixed && d > 0 ? 76 : 152;
         auto spread = [&](int &L) {
             while (L > 2 && L / 2 >= other) L /= 2;
-            while (L > 2 && (long long)std::max(1, h->seg[d].C) * ((other + L - 1) / L) * planes < 152) L /= 2;
+            while (L > 2 && (long long)std::max(1, h->seg[d].C) * ((other + L - 1) / L) * planes < fill) L /= 2;
         };
         if (!h->mixed && h->seg[d].SEG) {
             // y and z: 8 lines (64-byte rows, a warp's solves of one kind), 3
