@@ -479,14 +479,18 @@ struct SeqOp {
                           // as much as its arithmetic)
 };
 
-// KIND 1, 2.  lo: the two rows before the first, hi: after the last (read
-// before any row is written; sync() between).  Returns the end value.
-template <int KIND, typename SYNC>
-__device__ __forceinline__ double seq_fwd(double *d, int P, int R, const SeqOp &o, const double *lo, const double *hi,
-                                          SYNC &&sync) {
-    double w0 = lo[-2 * P], w1 = lo[-P], w2 = d[0], w3 = d[P];
-    const double h0 = hi[0], h1 = hi[P];
-    sync();
+// The two rows before a segment's first and the two after its last, read
+// before any row is written.
+struct SeqHalo {
+    double lo[2], hi[2];
+};
+__device__ __forceinline__ SeqHalo seq_halo(const double *lo, const double *hi, int P) {
+    return {{lo[-2 * P], lo[-P]}, {hi[0], hi[P]}};
+}
+// KIND 1, 2.  Returns the end value.
+template <int KIND>
+__device__ __forceinline__ double seq_fwd(double *d, int P, int R, const SeqOp &o, const SeqHalo &h) {
+    double w0 = h.lo[0], w1 = h.lo[1], w2 = d[0], w3 = d[P];
     const double nl = o.nl, s0 = o.s0, s1 = o.s1, s2 = o.s2;
     double y = 0.0;
     auto row = [&](double w4) {
@@ -507,7 +511,7 @@ __device__ __forceinline__ double seq_fwd(double *d, int P, int R, const SeqOp &
         }
     }
     for (; n < R; ++n, q += P) {
-        row(n + 2 < R ? q[2 * P] : n + 2 == R ? h0 : h1);
+        row(n + 2 < R ? q[2 * P] : n + 2 == R ? h.hi[0] : h.hi[1]);
         q[0] = y;
     }
     return y;
@@ -572,9 +576,10 @@ __device__ __forceinline__ void run_seq_tasks(double *tile, int stride, double *
     if (C > 1) {
         const int prev = rank > 0 ? rank - 1 : C - 1, next = rank < C - 1 ? rank + 1 : 0;
         const double *lo = cluster_map(d + seg_rows(pl, rank - 1) * L, prev), *hi = cluster_map(d, next);
-        auto sync = [] { cluster_sync(); };
-        if (second) v = seq_fwd<2>(d, L, on ? R : 0, o, lo, hi, sync);
-        else v = seq_fwd<1>(d, L, on ? R : 0, o, lo, hi, sync);
+        const SeqHalo halo = seq_halo(lo, hi, L);
+        cluster_sync();
+        if (second) v = seq_fwd<2>(d, L, on ? R : 0, o, halo);
+        else v = seq_fwd<1>(d, L, on ? R : 0, o, halo);
         if (on) *cluster_map(box, next) = v;
         cluster_sync();
         if (on) {
@@ -586,9 +591,10 @@ __device__ __forceinline__ void run_seq_tasks(double *tile, int stride, double *
     } else if (B > 1) {
         const int hp = (h - 1) & (B - 1), hn = (h + 1) & (B - 1);
         const double *lo = h ? d : line + R * L, *hi = hn ? d + rows * L : line;
-        auto sync = [] { __syncthreads(); };
-        if (second) v = seq_fwd<2>(d, L, on ? rows : 0, o, lo, hi, sync);
-        else v = seq_fwd<1>(d, L, on ? rows : 0, o, lo, hi, sync);
+        const SeqHalo halo = seq_halo(lo, hi, L);
+        __syncthreads();
+        if (second) v = seq_fwd<2>(d, L, on ? rows : 0, o, halo);
+        else v = seq_fwd<1>(d, L, on ? rows : 0, o, halo);
         if (on) mbox[hn * L] = v;
         __syncthreads();
         if (on) {
@@ -598,9 +604,9 @@ __device__ __forceinline__ void run_seq_tasks(double *tile, int stride, double *
         __syncthreads();
         if (on) seq_end(d, L, rows, o, *box2);
     } else if (on) {
-        auto sync = [] {};
-        if (second) v = seq_fwd<2>(d, L, R, o, d + R * L, d, sync);
-        else v = seq_fwd<1>(d, L, R, o, d + R * L, d, sync);
+        const SeqHalo halo = seq_halo(d + R * L, d, L);
+        if (second) v = seq_fwd<2>(d, L, R, o, halo);
+        else v = seq_fwd<1>(d, L, R, o, halo);
         v = seq_bwd(d, L, R, o, v * o.wrap);
         seq_end(d, L, R, o, v * o.wrap);
     }
