@@ -347,26 +347,50 @@ SegPlan cluster_plan(int N, int periodic) {
     return p;
 }
 
-// The periodic operator in that form: left-hand side (a, 1, a) with
-// a = l / (1 + l^2).
-// bits: below 2^-bits a carry is left out.
+// l of the left-hand side (a, 1, a), a = l / (1 + l^2).
+double root_of(const HostOp &h) {
+    const double a = h.alo[h.N / 2];
+    return a == 0.0 ? 0.0 : (1.0 - std::sqrt(1.0 - 4.0 * a * a)) / (2.0 * a);
+}
+
+// below 2^-bits a carry is left out
 template <typename R>
-SegOp<R> seg_op(const HostOp &h, const SegPlan &p, int bits) {
+constexpr int kCarryBits = sizeof(R) == 4 ? 30 : 60;
+
+// Whether the segments' carries of a periodic operator can be formed in R: they are scaled
+// by negative powers of l up to the unused rows of a segment (SegOp::iS,
+// iS1), which an l near zero takes out of R's range.  An l of less than a carry's
+// last bit has no carries.  The derivatives' (0.38^-9, 0.19^-13) and the
+// usual filters' are far inside; in between (|alphaF| below 0.01 at worst in
+// FP32, 1e-10 in FP64) the Thomas solves stay.  A table of powers counted
+// from a segment's own first row instead of iS, iS1 takes any l, but the second table
+// read cost 16^3 FP64 91.1 -> 95.2 us a step, 101x90x77 mixed 724 -> 738.
+template <typename R>
+bool carries(const HostOp &h, const SegPlan &p) {
+    const double l = std::fabs(root_of(h));
+    const int rows = p.full ? 0 : p.kS + (p.nS < p.G);
+    return l < std::ldexp(1.0, -kCarryBits<R>) || std::pow(l, rows) >= std::ldexp(1.0, sizeof(R) == 4 ? -60 : -300);
+}
+
+// The periodic operator in that form.
+template <typename R>
+SegOp<R> seg_op(const HostOp &h, const SegPlan &p) {
     SegOp<R> o{};
     if (!p.SEG) return o;
-    const double a = h.alo[h.N / 2];
-    const double l = a == 0.0 ? 0.0 : (1.0 - std::sqrt(1.0 - 4.0 * a * a)) / (2.0 * a);
+    const double l = root_of(h);
     o.nl = (R)-l;
     o.geo = (R)(1.0 / (1.0 - l * l));
     for (int k = 0; k <= kMaxH; k++) o.s[k] = (R)(h.taps[kMaxH + k] * h.scale * (1.0 + l * l));
     for (int k = 0; k < 32; k++) o.pw[k] = (R)std::pow(-l, k + 1);
     o.qS = (R)std::pow(-l, p.S);
     o.qS1 = (R)std::pow(-l, p.S - 1);
-    o.iS = (R)std::pow(-l, -p.kS);
-    o.iS1 = (R)std::pow(-l, -(p.kS + 1));
+    if (std::fabs(l) >= std::ldexp(1.0, -kCarryBits<R>)) {  // else no carry (the explicit filter, l = 0, has none)
+        o.iS = (R)std::pow(-l, -p.kS);
+        o.iS1 = (R)std::pow(-l, -(p.kS + 1));
+    }
     const int smin = p.nS < p.G ? p.S - 1 : p.S;
     o.T = 1;
-    while (o.T < p.G && std::pow(std::fabs(l), (double)smin * o.T) > std::ldexp(1.0, -bits)) o.T++;
+    while (o.T < p.G && std::pow(std::fabs(l), (double)smin * o.T) > std::ldexp(1.0, -kCarryBits<R>)) o.T++;
     o.wrap = o.T == p.G ? (R)(1.0 / (1.0 - std::pow(-l, h.N))) : R(1);
     return o;
 }
@@ -400,7 +424,7 @@ int seq_slots(int n1, int B, int L) {
 
 SeqOp seq_op(const HostOp &h, const SegPlan &p) {
     SeqOp o{};
-    const SegOp<double> g = seg_op<double>(h, p, 56);
+    const SegOp<double> g = seg_op<double>(h, p);
     o.nl = g.nl;
     o.s0 = g.s[0];
     o.s1 = g.s[1];
@@ -445,6 +469,10 @@ int make_line_seg(const HostOp &h, LineSeg &ls, cudaStream_t s) {
     if (!factors(h)) return CS3D_OK;
     a.seg = seg_plan(N, false, 32, 4);
     if (!a.seg.SEG) return CS3D_OK;
+    if (h.periodic && !carries<double>(h, a.seg)) {
+        a.seg = SegPlan{};
+        return CS3D_OK;
+    }
     const SegPlan &p = a.seg;
     a.N = N;
     while ((1 << a.lgG) < p.G) a.lgG++;
@@ -452,7 +480,7 @@ int make_line_seg(const HostOp &h, LineSeg &ls, cudaStream_t s) {
     a.divN = make_fastdiv((unsigned)N);
     a.divS = make_fastdiv((unsigned)p.S);
     a.divS1 = make_fastdiv((unsigned)(p.S - 1));
-    a.op = seg_op<double>(h, p, 60);
+    a.op = seg_op<double>(h, p);
     if (!a.wall) return CS3D_OK;
     for (int k = 0; k <= kMaxH; k++) a.op.s[k] = h.taps[kMaxH + k] * h.scale;  // (the table scales the rows)
     for (int b = 0; b < 2 * kMaxH; b++) {
@@ -866,25 +894,31 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
             if (r) return fail_free(r);
             if (ho.periodic && factors(ho)) {
                 h->segr[d] = seg_plan(Nd[d], true);
-                h->segrop[d][k - 1] = seg_op<double>(ho, h->segr[d], 60);
+                if (carries<double>(ho, h->segr[d])) h->segrop[d][k - 1] = seg_op<double>(ho, h->segr[d]);
             }
             if (!h->mixed && ho.periodic && k < 3) {
                 h->seg[d] = seq_plan(Nd[d], d);
                 h->seqop[d][k - 1] = seq_op(ho, h->seg[d]);
             } else if (!h->mixed && ho.periodic && factors(ho)) {
-                h->segf[d] = seg_plan(Nd[d], true);
-                h->segfop64[d] = seg_op<double>(ho, h->segf[d], 60);
+                const SegPlan p = seg_plan(Nd[d], true);
+                if (carries<double>(ho, p)) {
+                    h->segf[d] = p;
+                    h->segfop64[d] = seg_op<double>(ho, p);
+                }
             } else if (h->mixed && k < 3) {
                 // (tiles of 32 lines across x: not for grids narrower than 18,
                 // 12x200x200 0.67 ms a step by clusters, 0.54 by one block a line;
                 // 20x200x200 0.76 and 0.96)
                 h->seg[d] = d > 0 && cfg->Nx >= 18 ? cluster_plan(Nd[d], ho.periodic) : SegPlan{};
                 if (ho.periodic && !h->seg[d].C) h->seg[d] = seg_plan(Nd[d], d > 0);
-                h->segop[d][k - 1] = seg_op<float>(ho, h->seg[d], 30);
+                h->segop[d][k - 1] = seg_op<float>(ho, h->seg[d]);
                 if (h->seg[d].wall) wall_op(ho, h->seg[d], h->wallop[d][k - 1]);
             } else if (h->mixed && ho.periodic && factors(ho)) {
-                h->segf[d] = seg_plan(Nd[d], false);
-                h->segfop[d] = seg_op<float>(make_filter_correction(ho), h->segf[d], 30);
+                const SegPlan p = seg_plan(Nd[d], false);
+                if (carries<float>(ho, p)) {
+                    h->segf[d] = p;
+                    h->segfop[d] = seg_op<float>(make_filter_correction(ho), p);
+                }
             }
         }
     for (int d = 0; d < 3; d++) {
