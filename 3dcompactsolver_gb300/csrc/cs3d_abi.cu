@@ -347,10 +347,12 @@ SegPlan cluster_plan(int N, int periodic) {
     return p;
 }
 
-// l of the left-hand side (a, 1, a), a = l / (1 + l^2).
+// l of the left-hand side (a, 1, a), a = l / (1 + l^2): the smaller root, in
+// the form without a difference (the other, (1 - sqrt) / 2a, lost half its digits at
+// a = 1e-6 and all at 1e-9).
 double root_of(const HostOp &h) {
     const double a = h.alo[h.N / 2];
-    return a == 0.0 ? 0.0 : (1.0 - std::sqrt(1.0 - 4.0 * a * a)) / (2.0 * a);
+    return 2.0 * a / (1.0 + std::sqrt((1.0 - 2.0 * a) * (1.0 + 2.0 * a)));
 }
 
 // below 2^-bits a carry is left out
@@ -438,7 +440,7 @@ SeqOp seq_op(const HostOp &h, const SegPlan &p) {
 // The walls' rows of such a line: explicit rows, and the tables of the first
 // and last segment.
 void wall_op(const HostOp &h, const SegPlan &p, WallOp &w) {
-    const double a = h.alo[h.N / 2], l = (1.0 - std::sqrt(1.0 - 4.0 * a * a)) / (2.0 * a), q = 1.0 + l * l;
+    const double l = root_of(h), q = 1.0 + l * l;
     for (int b = 0; b < 4; b++)
         for (int j = 0; j < 6; j++) {
             // (rows N-2 and N-1 from column N - 6 on)

@@ -27,6 +27,13 @@ def test_operator_matches_oracle(gpu_pkg, oracle, N, bc, alphaF):
     assert rel_err(out, oracle.line_op_port(3, bc, N, 1.0 / (N - 1.0), alphaF, lines)) <= 1e-13
 
 
+@pytest.mark.parametrize("alphaF", [1e-12, 1e-9, -1e-7, 1e-6, 1e-5, 1e-4, -1e-3, 1e-2])
+@pytest.mark.parametrize("N", [33, 64, 77, 100])
+def test_operator_at_small_coefficients(gpu_pkg, oracle, N, alphaF):
+    """The root l of a = l / (1 + l^2) keeps its relative accuracy down to l = a."""
+    test_operator_matches_oracle(gpu_pkg, oracle, N, 0, alphaF)
+
+
 def _steps(gpu_pkg, cfg, ic, n):
     s = gpu_pkg.Solver(cfg)
     s.set_initial_conditions(*ic)
