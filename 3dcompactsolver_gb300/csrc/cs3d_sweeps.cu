@@ -674,6 +674,15 @@ k_sweep_z(std::conditional_t<WALL, WallSweepArgs<T>, SweepArgs<T>> a) {
 // q1 = q2 + (filtered - unfiltered) in FP64 plus q1's FP32 shadow.
 __constant__ Task kTasksF[3] = {{0, 0, 2, 1, 1, 2}, {2, 2, 2, 3, 3, 2}, {4, 4, 2, 4, 4, 2}};
 
+// What a filter pass starts from: q2 itself (plain form), or its fluctuation.  One
+// function for both kernels: the first and the last pass of a step may run different
+// ones (a direction between walls), and q1 takes the difference of what they form.
+template <typename T>
+__device__ __forceinline__ T unfiltered(const FilterArgs<T> &a, int f, double q) {
+    if constexpr (sizeof(T) == 8) return q;
+    else return fluct_of(q, a.ref_hi[f], a.ref_lo[f]);
+}
+
 template <typename T, int DIR, int PC>
 __global__ void __launch_bounds__(filter_threads<T>(), sizeof(T) == 4 ? kFilterMinBlocks : 4) k_filter(FilterArgs<T> a) {
     constexpr int B = sizeof(T) == 4 ? kFilterBatch : 2;
@@ -691,7 +700,7 @@ __global__ void __launch_bounds__(filter_threads<T>(), sizeof(T) == 4 ? kFilterM
             const unsigned gi = pt[b].gi;
 #pragma unroll
             for (int f = 0; f < 5; ++f)
-                v[b][f] = a.src64.f[f] ? to_work<T>(a.src64.f[f][gi] - a.ref[f]) : a.src32[f][gi];
+                v[b][f] = a.src64.f[f] ? unfiltered(a, f, a.src64.f[f][gi]) : a.src32[f][gi];
         }
 #pragma unroll
         for (int b = 0; b < B; ++b) {
@@ -742,7 +751,7 @@ __global__ void __launch_bounds__(filter_threads<T>(), sizeof(T) == 4 ? kFilterM
                     if (a.delta_from.f[f]) {
                         // the unfiltered value: the first pass's FP32 input, or
                         // formed again from q2 (the same number either way)
-                        const T v0 = kCorr && a.unf[f] ? u[b][f] : to_work<T>(q[b][f] - a.ref[f]);
+                        const T v0 = kCorr && a.unf[f] ? u[b][f] : unfiltered(a, f, q[b][f]);
                         nv = q[b][f] + to_f64(v - v0);
                     } else {
                         nv = to_f64(v) + a.ref[f];
@@ -776,8 +785,7 @@ k_filter_seg(FilterArgs<T> a) {
             const unsigned gi = in.pt.gi;
 #pragma unroll
             for (int f = 0; f < 5; ++f) {
-                if constexpr (sizeof(T) == 8) in.v[f] = a.src64.f[0] ? a.src64.f[f][gi] : a.src32[f][gi];
-                else in.v[f] = a.src64.f[0] ? fluct_of(a.src64.f[f][gi], a.ref_hi[f], a.ref_lo[f]) : a.src32[f][gi];
+                in.v[f] = a.src64.f[0] ? unfiltered(a, f, a.src64.f[f][gi]) : a.src32[f][gi];
             }
         },
         [&](In &in) {
@@ -826,7 +834,7 @@ k_filter_seg(FilterArgs<T> a) {
                     // q1 = q2 + (filtered - unfiltered); the unfiltered value is
                     // the first pass's FP32 input, or formed again from q2 (the
                     // same number either way)
-                    const float v0 = a.unf[0] ? o.u[f] : fluct_of(o.q[f], a.ref_hi[f], a.ref_lo[f]);
+                    const float v0 = a.unf[0] ? o.u[f] : unfiltered(a, f, o.q[f]);
                     const double nv = o.q[f] + widen(v - v0);
                     a.dst64.f[f][gi] = nv;
                     a.shadow_out[f][gi] = narrow(nv);
