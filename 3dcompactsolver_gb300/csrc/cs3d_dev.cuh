@@ -200,8 +200,8 @@ __device__ __forceinline__ int faces_of(const Geom &g, int i, int j, int k) {
 // Reciprocal and square root in FP64 from FP32 estimates by one step of a
 // cubically convergent Newton series (1/x = r (1 + e + e^2 + ...), e = 1 - x r;
 // sqrt x = g (1 - e)^(-1/2), g = x r, e = 1 - g r with r near 1/sqrt x): three and
-// five operations on the FP64 pipe, within an ulp.  Outside the FP32 range,
-// and for NaN, the library's.
+// five operations on the FP64 pipe, within an ulp (the square root: one and a
+// half).  Outside the FP32 range, and for NaN, the library's.
 __device__ __forceinline__ double rcp_f64(double x) {
     if (!(fabs(x) > 1e-30 && fabs(x) < 1e30)) return 1.0 / x;
     const double r = widen(__frcp_rn(narrow(x)));
@@ -229,28 +229,42 @@ __device__ __forceinline__ float quot(float a, float b, float ib) {
     return fmaf(fmaf(-q, b, a), ib, q);
 }
 
-// T^-0.24, from which both the viscosity law mu = mu_ref T^0.76 (IdealGas.hpp)
-// and its slope 0.76 mu / T follow by multiplications.
+// T^-0.24 and T^0.76, for the viscosity law mu = mu_ref T^0.76 (IdealGas.hpp)
+// and its slope 0.76 mu / T = 0.76 mu_ref T^-0.24.
 // FP32: exp2(-0.24 log2 T) with the hardware log2 (absolute error about 2^-22,
-// so about 4e-8 relative in the result).  FP64, whose pipe issues two
-// operations per SM and clock: y = T^-0.24 solves T^6 y^25 = 1; from an FP32
-// estimate (relative error below 6e-7) the residual e = 1 - T^6 y^25 gives
-// y (1 - e)^(-1/25) = y (1 + e/25 + 13 e^2/625 + ...), the next term below
-// 5e-17: 14 FP64 operations and no division, within 1 ulp of the library pow
-// on [1e-6, 1e6].  Outside that range, and for NaN, the library pow.
+// so about 4e-8 relative in the result), and T times that.
 __device__ __forceinline__ float visc_rpow(float T) { return exp2f(-0.24f * __log2f(T)); }
-__device__ __forceinline__ double visc_rpow(double T) {
-    if (!(T > 1e-6 && T < 1e6)) return pow(T, -0.24);
-    const double y = widen(exp2f(-0.24f * log2f(narrow(T))));
-    const double t2 = T * T, t6 = t2 * t2 * t2;
-    const double y2 = y * y, y4 = y2 * y2, y8 = y4 * y4, y16 = y8 * y8;
-    const double e = fma(-t6, y16 * y8 * y, 1.0);
-    return fma(y, e * fma(e, 13.0 / 625.0, 1.0 / 25.0), y);
+__device__ __forceinline__ float visc_pow(float T) { return T * visc_rpow(T); }
+// FP64, whose pipe issues two operations per SM and clock: y = T^-0.24 solves
+// T^6 y^25 = 1; from an FP32 estimate (relative error below 6e-7) the residual
+// e = 1 - T^6 y^25 gives the factor (1 - e)^(-1/25) = 1 + e/25 + 13 e^2/625 + ...,
+// the next term below 5e-17, of both powers.  T^0.76 is T y with the rounding
+// of that product and the factor's excess added: as T times T^-0.24 it had two
+// roundings more (1.8 ulp at most, 0.9 so; three FP64 operations more, as many as
+// (T y^4)^6 y takes less than T^6 times y^25).  No division; both within 1.3 ulp
+// on [1e-6, 1e6], 1.0 near T = 1.  Outside that range, and for NaN, the library
+// pow.
+__device__ __forceinline__ double visc_powers(double T, double &rpow) {
+    if (!(T > 1e-6 && T < 1e6)) {
+        rpow = pow(T, -0.24);
+        return pow(T, 0.76);
+    }
+    const double y = widen(exp2f(-0.24f * log2f(narrow(T)))), ty = T * y;
+    const double y2 = y * y, u = T * (y2 * y2), u2 = u * u;  // (T y^4)^6 y
+    const double e = fma(-(u2 * u2 * u2), y, 1.0);
+    const double g = e * fma(e, 13.0 / 625.0, 1.0 / 25.0);
+    rpow = fma(y, g, y);
+    return ty + fma(ty, g, fma(T, y, -ty));
 }
-
-// T^0.76
-template <typename T>
-__device__ __forceinline__ T visc_pow(T t) { return t * visc_rpow(t); }
+__device__ __forceinline__ double visc_pow(double T) {
+    double r;
+    return visc_powers(T, r);
+}
+__device__ __forceinline__ double visc_rpow(double T) {
+    double r;
+    visc_powers(T, r);
+    return r;
+}
 
 // Direction whose continuity derivative survives at a wall point: the
 // reference applies the wall faces in the order X0,X1,Y0,Y1,Z0,Z1 and the

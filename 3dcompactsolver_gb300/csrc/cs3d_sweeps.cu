@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(SEG == kSeq ? kSeqTpbX : sweep_threads<T>(0),
                                 blockDim.x, XDUM);
     __syncthreads();
     // phase C
-    const T c43 = T(4.0 / 3.0), cpPr = (T)gp.cpPr, muref = (T)gp.mu_ref;
+    const T c43 = T(4.0 / 3.0), cpPr = (T)gp.cpPr, muref = (T)gp.mu_ref, slope = (T)0.76 * muref;
     struct InC { Pt pt; T v[4]; };
     batched<InC, sizeof(T) == 4 ? 4 : 2>(NL,
         [&](InC &in, int p) {
@@ -242,11 +242,14 @@ __global__ void __launch_bounds__(SEG == kSeq ? kSeqTpbX : sweep_threads<T>(0),
             const unsigned gi = p.gi;
             const Zn<T> zz = TS::z(a.d1, a.d2, p.n);
             const T U = in.v[0], V = in.v[1], W = in.v[2], Tt = in.v[3];
-            const T vz = muref * visc_rpow(Tt);
-            const T mu = vz * Tt;
-            if constexpr (!kRecompute<T>) {
+            T mu;
+            if constexpr (kRecompute<T>) {
+                mu = muref * visc_rpow(Tt) * Tt;
+            } else {
+                T rp;
+                mu = muref * visc_powers(Tt, rp);
                 a.mu[gi] = mu;
-                a.amu[gi] = (T)0.76 * vz;
+                a.amu[gi] = slope * rp;
             }
             T Ux, Uxx, Vx, Vxx, Wx, Wxx, Tx, Txx, cex, f1, f2, f3;
             TS::two(sm, 0, p, L, zz.z1, zz.z2, Ux, Uxx);
