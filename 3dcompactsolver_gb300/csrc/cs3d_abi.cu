@@ -347,6 +347,31 @@ SegPlan cluster_plan(int N, int periodic) {
     return p;
 }
 
+// The mixed form's lines.  x: segments in one block.  y and z: clusters, whose tiles
+// are 32 lines across x, where the grid is wide enough; else segments in one
+// block, whose tiles are at most 16 lines wide; else the Thomas solves (SEG =
+// 0).  Times in us a step of Nx x N x N, three ways (cluster / block / Thomas):
+//   Nx = 9    N = 100 265 220 224   160 383 473 438   200 644 652 543   256 832 674 786
+//   Nx = 16   N = 100 264 216 223   160 399 470 441   200 692 692 576   256 904 718 829
+//   Nx = 17   N = 32  111 101 105   40  111 115 123   100 292 322 338   200 775 1002 769
+//   Nx = 18   N = 32  111 101 105   100 291 322 336   200 782 1012 781  256 1019 1032 1186
+// So clusters from 17 columns on (a second block tile for one column more), and
+// narrower grids' lines above 128 points by segments only where those are
+// 32 rows long and four fifths full (24-row segments, 129 to 192 and 257 to 384
+// points: 5 to 15% behind Thomas at every length measured; 200, 300 and 400
+// points 17, 6 and 10%).  From 385 points the Thomas tiles are 4 lines wide and lose
+// to the block's 8 from 13 columns on (400: 2592 and 3161).
+SegPlan mixed_plan(int N, int d, int Nx, int periodic) {
+    if (d > 0 && (Nx >= 18 || (Nx == 17 && N >= 40 && periodic))) {
+        const SegPlan c = cluster_plan(N, periodic);
+        if (c.C) return c;
+    }
+    if (!periodic) return SegPlan{};
+    const SegPlan p = seg_plan(N, d > 0);
+    if (d > 0 && N > 128 && !(p.SEG == 32 && (5 * N >= 4 * 32 * p.G || (N > 384 && Nx > 12)))) return SegPlan{};
+    return p;
+}
+
 // l of the left-hand side (a, 1, a), a = l / (1 + l^2): the smaller root, in
 // the form without a difference (the other, (1 - sqrt) / 2a, lost half its digits at
 // a = 1e-6 and all at 1e-9).
@@ -937,11 +962,7 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
                     h->segfop64[d] = seg_op<double>(ho, p);
                 }
             } else if (h->mixed && k < 3) {
-                // (tiles of 32 lines across x: not for grids narrower than 18,
-                // 12x200x200 0.67 ms a step by clusters, 0.54 by one block a line;
-                // 20x200x200 0.76 and 0.96)
-                h->seg[d] = d > 0 && cfg->Nx >= 18 ? cluster_plan(Nd[d], ho.periodic) : SegPlan{};
-                if (ho.periodic && !h->seg[d].C) h->seg[d] = seg_plan(Nd[d], d > 0);
+                h->seg[d] = mixed_plan(Nd[d], d, cfg->Nx, ho.periodic);
                 h->segop[d][k - 1] = seg_op<float>(ho, h->seg[d]);
                 if (h->seg[d].wall) wall_op(ho, h->seg[d], h->wallop[d][k - 1]);
             } else if (h->mixed && ho.periodic && factors(ho)) {
