@@ -1724,11 +1724,29 @@ extern "C" int cs3d_kernel_times(cs3d_handle *h, double *ms, long long *count, i
 // ---------------------------------------------------------------------
 // single operators
 // ---------------------------------------------------------------------
+// Lines of one or two segments that the Thomas kernel serves better: it spreads
+// 32 lines a block where a block of segments takes 64 or 128, and has no idle rows.
+// Thomas against segments in us, operators 1 / 2 / 3:
+//   walls, 9 points      4096 lines 8.4 8.4 10.3, 14.4 14.5 18.6    131072: 53 53 65, 49 53 76
+//   walls, 12            4096: 10.4 10.4 11.4, 14.5 14.5 18.6       131072: 66 66 84, 50 53 77
+//   walls, 18            4096: 12.4 12.4 14.5, 14.5 14.4 18.5       131072: 92 92 123, 88 95 137
+//   walls, 24            4096: 14.5 14.5 16.6, 14.5 14.5 18.6       131072: 115 115 159, 90 96 138
+//   periodic, 9          4096: 8.4 8.4 10.4, 10.4 10.4 13.4         131072: 53 53 66, 39 43 61
+//   periodic, 15         4096: 11.4 11.3 12.5, 10.4 12.4 14.5       131072: 80 80 103, 41 45 62
+// The lines cross at 2^18 points between walls and 2^17 periodic; up to
+// five eighths of the rows in use (9, 10 and 17 to 20 points) walls never cross for all
+// three operators.
+static bool short_lines(const LineSegArgs &a, int kind, long long npts) {
+    const int rows = a.seg.G * a.seg.SEG;
+    if (a.wall) return 8 * a.N <= 5 * rows || (a.N <= 24 && npts < 1 << 18);
+    return a.N <= 16 && npts < 1 << 17 && (kind > 1 || a.N < 11);
+}
+
 // The operator on every line of npts points: in register segments where the
 // line is cut, else one Thomas solve a thread.
 static int line_op_on(const LineOp<double> &op, const LineSegArgs &seg, int kind, long long npts, const double *in,
                       double *out, cudaStream_t s) {
-    if (seg.seg.SEG) {
+    if (seg.seg.SEG && !short_lines(seg, kind, npts)) {
         LineSegArgs a = seg;
         a.nlines = npts / op.N;
         a.in = in;
