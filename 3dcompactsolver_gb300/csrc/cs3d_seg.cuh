@@ -578,8 +578,8 @@ __device__ __forceinline__ void run_seq_tasks(double *tile, int stride, double *
         const double *lo = cluster_map(d + seg_rows(pl, rank - 1) * L, prev), *hi = cluster_map(d, next);
         const SeqHalo halo = seq_halo(lo, hi, L);
         cluster_sync();
-        if (second) v = seq_fwd<2>(d, L, on ? R : 0, o, halo);
-        else v = seq_fwd<1>(d, L, on ? R : 0, o, halo);
+        // (idle lanes have the first line's addresses, whose rows are being written now)
+        if (on) v = second ? seq_fwd<2>(d, L, R, o, halo) : seq_fwd<1>(d, L, R, o, halo);
         if (on) *cluster_map(box, next) = v;
         cluster_sync();
         if (on) {
@@ -593,8 +593,8 @@ __device__ __forceinline__ void run_seq_tasks(double *tile, int stride, double *
         const double *lo = h ? d : line + R * L, *hi = hn ? d + rows * L : line;
         const SeqHalo halo = seq_halo(lo, hi, L);
         __syncthreads();
-        if (second) v = seq_fwd<2>(d, L, on ? rows : 0, o, halo);
-        else v = seq_fwd<1>(d, L, on ? rows : 0, o, halo);
+        // (idle lanes have the first line's addresses, whose rows are being written now)
+        if (on) v = second ? seq_fwd<2>(d, L, rows, o, halo) : seq_fwd<1>(d, L, rows, o, halo);
         if (on) mbox[hn * L] = v;
         __syncthreads();
         if (on) {
