@@ -18,7 +18,10 @@ LIB = os.path.join(HERE, "libcs3d_gb300.so")
 OBJDIR = os.path.join(HERE, "_build")
 SOURCES = ["cs3d_sweeps.cu", "cs3d_point.cu", "cs3d_abi.cu", "cs3d_adjoint.cu", "cs3d_lineop.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wno-enum-compare",
+# --no-compress: the line information of the unrolled solves makes the device code large, and
+# unpacking it took 24 ms of a process's first mixed step and 20 ms of its first adjoint (3 and 5
+# so; a library of 51 instead of 15 MB)
+FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--no-compress", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wno-enum-compare",
          f"-I{INC}"]
 
 
