@@ -361,10 +361,18 @@ SegPlan cluster_plan(int N, int periodic) {
 // points: 5 to 15% behind Thomas at every length measured; 200, 300 and 400
 // points 17, 6 and 10%).  From 385 points the Thomas tiles are 4 lines wide and lose
 // to the block's 8 from 13 columns on (400: 2592 and 3161).
-SegPlan mixed_plan(int N, int d, int Nx, int periodic) {
+// Lines between walls of planes x Nx lines: where an eighth or more of the clusters' columns
+// is idle, they take a second wave (two blocks an SM) and the Thomas tiles of 16 lines do not,
+// the latter.  us a step, cluster / Thomas: 48x100x50 304 and 275, 48x100x40
+// 258 and 234, 33x190x50 375 and 341, 40x250x48 458 and 452, 80x100x30 252 and
+// 226.  (One wave, 48x96x44: 228 and 263.  No idle columns, 64x250x30: 320 and 353.)
+SegPlan mixed_plan(int N, int d, int Nx, int planes, int periodic) {
     if (d > 0 && (Nx >= 18 || (Nx == 17 && N >= 40 && periodic))) {
         const SegPlan c = cluster_plan(N, periodic);
-        if (c.C) return c;
+        const long long tiles = (Nx + 31) / 32;
+        const bool waves = !periodic && 8 * Nx <= 7 * 32 * tiles && tiles * planes * c.C > 2 * 152 &&
+                           (Nx + 15) / 16 * (long long)planes <= 152;
+        if (c.C && !waves) return c;
     }
     if (!periodic) return SegPlan{};
     const SegPlan p = seg_plan(N, d > 0);
@@ -962,7 +970,7 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
                     h->segfop64[d] = seg_op<double>(ho, p);
                 }
             } else if (h->mixed && k < 3) {
-                h->seg[d] = mixed_plan(Nd[d], d, cfg->Nx, ho.periodic);
+                h->seg[d] = mixed_plan(Nd[d], d, cfg->Nx, d == 2 ? cfg->Ny : cfg->Nz, ho.periodic);
                 h->segop[d][k - 1] = seg_op<float>(ho, h->seg[d]);
                 if (h->seg[d].wall) wall_op(ho, h->seg[d], h->wallop[d][k - 1]);
             } else if (h->mixed && ho.periodic && factors(ho)) {
