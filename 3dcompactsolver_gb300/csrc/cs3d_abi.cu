@@ -1012,11 +1012,13 @@ extern "C" int cs3d_create(const cs3d_config *cfg, cs3d_handle **out) {
         shape(&h->seg[d], h->L[d], h->threads[d]);
         const int other = d == 0 ? cfg->Ny : cfg->Nx, planes = d == 2 ? cfg->Ny : cfg->Nz;
         // fewer lines a tile where the grid would leave SMs without a block
-        // (16^3: 2 lines, 128 blocks a launch); the mixed y and z tiles only
-        // below half of the SMs, as narrower ones leave solving lanes idle
-        // (44x39x38, three handles, two steps: 178 us, so 147; one handle's
-        // kernels take the same time or less)
-        const int fill = h->mixed && d > 0 ? 76 : 152;
+        // (16^3: 2 lines, 128 blocks a launch).  Narrower tiles leave solving lanes
+        // idle, which several handles in flight pay for: the mixed y and z tiles
+        // only below half of the SMs (44x39x38, three handles, two steps: 178
+        // us, so 147), the plain form's below 100 blocks (24^3 in 144 blocks of 4 lines
+        // instead of 288 of 2, three handles: 592 -> 494 us a step of each, one handle
+        // 283 -> 281; below 76 blocks 40x9x40 between walls takes 397 instead of 335)
+        const int fill = h->mixed ? (d > 0 ? 76 : 152) : 100;
         auto spread = [&](int &L) {
             while (L > 2 && L / 2 >= other) L /= 2;
             while (L > 2 && (long long)std::max(1, h->seg[d].C) * ((other + L - 1) / L) * planes < fill) L /= 2;
