@@ -2935,11 +2935,15 @@ extern "C" int cs3d_vorticity_q(cs3d_handle *h, double *vort, double *qcrit) {
     a.qcrit = h->post_buf + 13 * n;
     CS3D_CUDA(launch_velocity(a, h->stream));
     h->launches++;
-    // the nine first derivatives with the solver's FP64 operators, one launch per direction
+    // the nine first derivatives with the solver's FP64 operators
     for (int e = 0; e < 3; e++) {
         const LineSegArgs &ls = h->lseg[e][0].a;
         int rc = CS3D_OK;
-        if (e == 0 && ls.seg.SEG) {
+        // (x: short lines of small grids go in one launch below, as three cost more than the
+        // solves: us a call with walls in x 16^3 91, so 73, 33^3 116 and 93, 60x16x16 124 and
+        // 99.  On 33x100x100 three launches take 216, one 225; from 65 points on the one is
+        // slower between walls, 100x20x20 120 and 125)
+        if (e == 0 && ls.seg.SEG && (ls.N > 64 || h->g.npts > 1 << 18)) {
             for (int c = 0; c < 3 && !rc; c++)
                 rc = line_op_on(h->op64[e][0].op, ls, 1, h->g.npts, a.vel[c], d[c][e], h->stream);
             h->launches += 3;
