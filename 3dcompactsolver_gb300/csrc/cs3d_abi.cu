@@ -407,6 +407,8 @@ bool carries(const HostOp &h, const SegPlan &p) {
     return l < std::ldexp(1.0, -kCarryBits<R>) || std::pow(l, rows) >= std::ldexp(1.0, sizeof(R) == 4 ? -60 : -300);
 }
 
+bool second_derivative(const HostOp &h) { return h.H == 2 && h.taps[kMaxH] != 0.0; }
+
 // The periodic operator in that form.
 template <typename R>
 SegOp<R> seg_op(const HostOp &h, const SegPlan &p) {
@@ -416,6 +418,7 @@ SegOp<R> seg_op(const HostOp &h, const SegPlan &p) {
     o.nl = (R)-l;
     o.geo = (R)(1.0 / (1.0 - l * l));
     for (int k = 0; k <= kMaxH; k++) o.s[k] = (R)(h.taps[kMaxH + k] * h.scale * (1.0 + l * l));
+    if (second_derivative(h)) o.s[0] = o.s[1] + R(2) * o.s[2];  // (by second differences, seg_r2)
     for (int k = 0; k < 32; k++) o.pw[k] = (R)std::pow(-l, k + 1);
     o.qS = (R)std::pow(-l, p.S);
     o.qS1 = (R)std::pow(-l, p.S - 1);
@@ -490,9 +493,18 @@ SeqOp seq_op(const HostOp &h, const SegPlan &p) {
     SeqOp o{};
     const SegOp<double> g = seg_op<double>(h, p);
     o.nl = g.nl;
-    o.s0 = g.s[0];
     o.s1 = g.s[1];
     o.s2 = g.s[2];
+    if (second_derivative(h)) {
+        // The taps' sum is zero.  Rounded each by itself, after the factors 1/h^2 and 1 + l^2,
+        // they make a derivative of a constant (rms error at 128 points 4.1e-15 of
+        // the result; 2.7e-15 so, 2.8e-15 by the Thomas solves): multiples of the
+        // centre's last place, their second moment kept.
+        const double c = 2.0 * std::fabs(o.s1 + o.s2), u = std::nextafter(c, INFINITY) - c;
+        o.s2 = std::rint(o.s2 / u) * u;
+        o.s1 = std::rint((o.s1 + 4.0 * (g.s[2] - o.s2)) / u) * u;
+        o.s0 = -2.0 * (o.s1 + o.s2);
+    }
     o.wrap = p.G == 1 ? 1.0 / (1.0 - std::pow(g.nl, h.N)) : 1.0;
     while (o.K < kSeqRows && std::pow(std::fabs(g.nl), o.K) > std::ldexp(1.0, -56)) o.K++;
     for (int k = 0; k < kSeqRows; k++) o.pw[k] = std::pow(g.nl, k + 1);
@@ -547,6 +559,7 @@ int make_line_seg(const HostOp &h, LineSeg &ls, cudaStream_t s) {
     a.op = seg_op<double>(h, p);
     if (!a.wall) return CS3D_OK;
     for (int k = 0; k <= kMaxH; k++) a.op.s[k] = h.taps[kMaxH + k] * h.scale;  // (the table scales the rows)
+    if (second_derivative(h)) a.op.s[0] = a.op.s[1] + 2.0 * a.op.s[2];
     for (int b = 0; b < 2 * kMaxH; b++) {
         for (int k = 0; k < kTaps; k++) a.btaps[b][k] = h.btaps[b][k] * h.scale;
         a.boff[b] = h.boff[b];

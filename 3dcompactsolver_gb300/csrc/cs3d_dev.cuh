@@ -65,7 +65,7 @@ struct SegPlan {
                // (G = B C, not restricted to a power of two)
 };
 
-// A periodic operator in that form: -l, the scaled taps (centre outwards),
+// A periodic operator in that form: -l, the scaled taps (centre outwards; second derivative: seg_r2),
 // the powers (-l)^(k+1), and what weights the carries between segments.
 template <typename R>
 struct SegOp {
