@@ -160,7 +160,7 @@ __global__ void k_cfl(CflArgs a) {
     } else {
         // FP32 bounds of every point first; FP64 arithmetic, two operations an
         // SM and clock, only for points whose upper bound reaches the largest
-        // lower bound of the block (128^3: 137 -> 20 us a step, the same maximum)
+        // lower bound of the block (Taylor-Green 128^3: 137 -> 81 us a step, the same maximum)
         const long long i0 = (long long)blockIdx.x * (B * blockDim.x) + threadIdx.x;
         float up[B], low = 0.f;
 #pragma unroll

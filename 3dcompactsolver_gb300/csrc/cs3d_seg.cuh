@@ -25,9 +25,9 @@
 // a row is read once and written once in about 11 instructions, the chain is a
 // segment, and a warp holds all segments of its lines (no block barrier inside
 // a solve).  The consume phases read solutions without a correction.  Against
-// solve_lanes, per step: 128^3 y 0.359 -> 0.283 ms, z 0.602 -> 0.527; 256^3 y
-// 2.92 -> 2.19 ms; the error against 64 bits falls by a tenth (differences
-// before products).
+// solve_lanes, per step, y and z by the clusters below: 128^3 x 0.250 -> 0.166 ms, y
+// 0.358 -> 0.232, z 0.603 -> 0.426; the error against 64 bits falls by a tenth
+// (differences before products).
 #pragma once
 #include "cs3d_dev.cuh"
 
@@ -313,7 +313,8 @@ __device__ __forceinline__ void seg_filter(const SegLane<R> &s, int P, const Seg
 // tile's row takes of its 128-byte line -- a copy kernel of z tiles on 256^3
 // measured 2.0 / 3.9 / 6.5 TB/s at 8 / 16 / 32 FP32 lines a row (5.2 / 5.6 /
 // 5.3 TB/s at 128^3, which the L2 holds).  The 8-line tiles that whole lines
-// leave room for at N = 256: z 6.66 ms a step; clusters of 4: 4.03.
+// leave room for at N = 256: z 6.66 ms a step; clusters of 4 with two segments a block
+// 4.03, of 8 with one 3.20.
 constexpr int kClLines = 32;  // (kClusterLines)
 
 __device__ __forceinline__ void cluster_sync() {

@@ -13,7 +13,8 @@
 //      segments of 16 to 32 rows in registers (run_seg_x, run_cluster_tasks);
 //      plain form: one thread walks its block's rows (run_seq_tasks); Thomas
 //      sweeps with precomputed factors for the lines that neither cuts (FP64
-//      wall lines, lines of 8 or above 512 points);
+//      wall lines; mixed ones along x, below 40 or above 256 points, or where
+//      mixed_plan says so; mixed periodic ones of 8 or above 512 points);
 //   C  consume the derivatives point by point.
 //
 //   sweep x : primitives, Euler x-fluxes, 13 x-solves; writes Ux,Vx,Wx,Tx,

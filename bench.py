@@ -83,7 +83,8 @@ def kernel_bytes_per_point(kernel, wb, rk_stages):
 # width H: the (2H+1)-tap right-hand side (2H+1 FMAs), the forward recurrence
 # (one FMA), the back substitution (one FMA and one multiply) and the
 # Sherman-Morrison correction on read (one FMA): 17 operations for the
-# derivatives (H = 2), 25 for the filter (H = 4).
+# derivatives (H = 2), 25 for the filter (H = 4).  These are the Thomas form's; the
+# constant-coefficient solves take 13 to 15 for a derivative.
 SOLVE_FLOPS_D = 17
 SOLVE_FLOPS_F = 25
 
@@ -570,7 +571,7 @@ def run_ours(args):
             "warmup": args.warmup, "ms_per_step": round(ms / args.steps, 4), "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f32" if args.precision == "mixed" else "f64",
             "precision": ("FP32-mixed: FP32 derivative/RHS/flux/filter arithmetic; FP64 conserved state, "
-                          "RK accumulation q2 += a_s dq on every stage and Sherman-Morrison factor; "
+                          "RK accumulation q2 += a_s dq on every stage; "
                           "the RK4 stage input qk as an FP32 shadow") if args.precision == "mixed"
                          else "FP64 throughout",
             "data": "synthetic",

@@ -52,11 +52,10 @@ extern "C" {
 /* arithmetic of the stage */
 #define CS3D_FP64        0  /* plain form: every operation in FP64        */
 #define CS3D_FP32_MIXED  1  /* RHS, flux, derivative and filter arithmetic in
-                               FP32; conserved state q1/q2, the RK
-                               accumulation q2 += a_s dq of every stage and
-                               the cyclic Sherman-Morrison factor in FP64;
-                               the RK4 stage input qk = q1 + b_s dq is kept
-                               as an FP32 shadow only                       */
+                               FP32; conserved state q1/q2 and the RK
+                               accumulation q2 += a_s dq of every stage in
+                               FP64; the RK4 stage input qk = q1 + b_s dq is
+                               kept as an FP32 shadow only                  */
 /* sponge construction */
 #define CS3D_SPONGE_REFERENCE 0 /* sigma built only on SPONGE faces with the
                                    reference's band widths 0.25Lx, 0.125Ly,
